@@ -13,13 +13,14 @@
 // 4 * 128 / ds columns of one head of one sequence and walks the sequence's tokens in order, RT_CHUNK at a time:
 // the chunk's rotated q and k and its v columns are staged in shared memory by the whole block.
 //
-// Long prompts, three kernels (retention_parts): the sequence is cut into pieces of `piece` tokens;
+// Long prompts, three kernels (retention_parts): the sequence is cut into pieces of `piece` tokens; in bfloat16 with heads of up
+// to 128 rotated coordinates as products on the tensor cores (further down), otherwise
 //   1. every piece runs the recurrence from a zero state (the same code): its local outputs, and the state
 //      it would leave, A_c
 //   2. the pieces' states are chained: S_c = decay^len_c * S_(c-1) + A_c   (S_(-1) is the sequence's state)
 //   3. every piece adds what the state before it contributes: o_t += decay^(t - t0 + 1) * S_(c-1)^T q_t
 // so that the pieces run side by side; the sums are the same up to their order.
-#include "common.cuh"
+#include "split_mma.cuh"
 
 #define RT_THREADS 128
 #define RT_CHUNK 64          // tokens staged at a time, at most (a piece of a long prompt)
@@ -253,43 +254,231 @@ retention_kernel(float* __restrict__ o, const TA* __restrict__ proj, int ld, int
     }
 }
 
+// ---------------------------------------------------------------------------- the pieces as products on the tensor cores
+// bfloat16 projections, heads of up to 128 rotated coordinates: with w_i = decay^i, a piece of n tokens from state S is
+//   state    S' = w_n S + sum_l w_(n-1-l) k_l v_l^T                                  one product (keys^T values)
+//   outputs  o_j = sum_(l <= j) w_(j-l) (q_j . k_l) v_l + w_(j+1) S^T q_j            scores, weights times values, queries times state
+// All of it stays fp32: rotated queries and keys, weights and states are cut into three bfloat16 pieces (split_mma.cuh).
+// The token-by-token walk of the same pieces issues two packed FMAs and two shared-memory reads for 8 numbers of the state and
+// waits for itself: 287 us with the chain for 2,048 tokens of 16 heads of 128 x 128, 78 us as products (22 states, 11 chain, 45
+// outputs; the tensor pipe 41 % busy in the outputs, bound by a block's phases between barriers at 16 warps an SM), and no
+// further from 64-bit sums (outputs 2.4e-7 of their norm before, 1.7e-7 now; states 2.4e-7 and 2.0e-7).  Pieces of 64 tokens:
+// the states of longer ones are fewer, but scores and weights grow with the square.
+#define RM_THREADS 256
+
+// rotated and scaled coordinates of the piece's tokens into pieces [SM_L][128] (zeros beyond n tokens and D coordinates): a
+// thread turns eight neighbouring pairs (f, f + half) of one token's q and k with the same cosines and sines
+struct RmRot {
+    const float* inv_freq; const float* table;        // table [2][half][T], or null
+    int n_rot, T;
+};
+template <bool Q>
+__device__ __forceinline__ void rm_stage(__nv_bfloat16* qt, __nv_bfloat16* kt, const __nv_bfloat16* q, const __nv_bfloat16* k,
+                                         size_t stride, int row0, int pos0, int n, int D, const RmRot& rot, float k_scale,
+                                         const float* k_weight, int tid) {
+    const int half = rot.n_rot >> 1, pairs = half >> 3, items = (D >> 3) - pairs;       // items: pairs of groups, then single groups
+    for (int x = tid; x < items * SM_L; x += RM_THREADS) {
+        const int l = x % SM_L, it = x / SM_L;
+        const bool turn = it < pairs;
+        const int f0 = turn ? it * 8 : rot.n_rot + (it - pairs) * 8, f1 = f0 + half;
+        float cs[8], sn[8];
+        const bool live = l < n;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) { cs[e] = 1.f; sn[e] = 0.f; }
+        if (turn && live) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                if (rot.table) {
+                    const float* c = rot.table + (size_t)(f0 + e) * rot.T + row0 + l;
+                    const float* s = c + (size_t)half * rot.T;
+                    if (ZLM_CHK(c, 4)) cs[e] = *c;
+                    if (ZLM_CHK(s, 4)) sn[e] = *s;
+                } else {
+                    sincosf((float)(pos0 + l) * rot.inv_freq[f0 + e], &sn[e], &cs[e]);
+                }
+            }
+        }
+        const float kw = k_scale * (k_weight ? k_weight[l] : 1.f);
+#pragma unroll
+        for (int y = Q ? 0 : 1; y < 2; ++y) {
+            const __nv_bfloat16* p = (y ? k : q) + (size_t)l * stride;
+            __nv_bfloat16* dst = y ? kt : qt;
+            uint4 a = make_uint4(0, 0, 0, 0), b = a;
+            if (live && ZLM_CHK(p + f0, 16)) a = *(const uint4*)(p + f0);
+            if (turn && live && ZLM_CHK(p + f1, 16)) b = *(const uint4*)(p + f1);
+            float u[8], v[8], r[8];
+            widen8(a, u);
+            widen8(b, v);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) r[e] = (turn ? u[e] * cs[e] - v[e] * sn[e] : u[e]) * (y ? kw : 1.f);
+            split8(dst, SM_L * 128, tile_off<128>(l, f0 >> 3), r);
+            if (turn) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) r[e] = (v[e] * cs[e] + u[e] * sn[e]) * (y ? kw : 1.f);
+                split8(dst, SM_L * 128, tile_off<128>(l, f1 >> 3), r);
+            }
+        }
+    }
+}
+// decay^0 .. decay^64, each rounded once
+__device__ __forceinline__ void rm_powers(float* pw, float d, int tid) {
+    if (tid <= SM_L) pw[tid] = (float)pow((double)d, (double)tid);
+}
+
+// grid (R * maxp, H, ceil(V / 128))
+__global__ void __launch_bounds__(RM_THREADS, 2)
+retention_piece_state_kernel(float* __restrict__ part, const __nv_bfloat16* __restrict__ proj, int ld, int k_off, int v_off,
+                             RmRot rot, const float* __restrict__ decay, const int* __restrict__ cu_seqlens,
+                             const int* __restrict__ seq_start, int maxp, int H, int D, int V, float k_scale) {
+    extern __shared__ __align__(128) __nv_bfloat16 rm_smem[];
+    __nv_bfloat16* kt = rm_smem;                     // [3][SM_L][128]
+    __nv_bfloat16* vt = kt + 3 * SM_L * 128;         // [SM_L][128]
+    __shared__ float pw[SM_L + 1], kw[SM_L];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y, c0 = blockIdx.z * 128;
+    const int r = blockIdx.x / maxp, first = (blockIdx.x % maxp) * SM_L;
+    if (!ZLM_CHK(cu_seqlens + r, 8) || !ZLM_CHK(seq_start + r, 4) || !ZLM_CHK(decay + h, 4)) return;
+    const int n = min(SM_L, cu_seqlens[r + 1] - cu_seqlens[r] - first);
+    if (n <= 0) return;
+    rm_powers(pw, decay[h], tid);
+    __syncthreads();
+    if (tid < SM_L) kw[tid] = tid < n ? pw[n - 1 - tid] : 0.f;
+    __syncthreads();
+    const int row0 = cu_seqlens[r] + first;
+    pdl_wait();
+    const __nv_bfloat16* rows = proj + (size_t)row0 * ld;
+    sm_stage_values(vt, rows + v_off + (size_t)h * V, ld, n, c0, V, tid);
+    rm_stage<false>(nullptr, kt, nullptr, rows + k_off + (size_t)h * D, ld, row0, seq_start[r] + first, n, D, rot, k_scale, kw, tid);
+    dec_wait<0>();
+    __syncthreads();
+    const int d0 = warp * 16;
+    if (d0 >= D) return;
+#pragma unroll 1
+    for (int n0 = 0; n0 < 128 && c0 + n0 < V; n0 += 64) {
+        SmSum<8> acc;
+        acc.zero();
+        sm_piece_state(acc, kt, vt, d0, n0, lane);
+        float* dst = part + (((size_t)blockIdx.x * H + h) * D + d0 + (lane >> 2)) * V + c0 + n0 + (lane & 3) * 2;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                float* p = dst + (size_t)8 * e * V + i * 8;
+                if (c0 + n0 + i * 8 < V && ZLM_CHK(p, 8)) *(float2*)p = make_float2(acc.get(i, 2 * e), acc.get(i, 2 * e + 1));
+            }
+    }
+}
+
+// grid (R * maxp, H, ceil(V / 128)); a warp owns 16 queries and 64 value columns
+__global__ void __launch_bounds__(RM_THREADS, 2)
+retention_piece_out_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, int ld, int q_off, int k_off, int v_off,
+                           RmRot rot, const float* __restrict__ decay, const float* __restrict__ before,
+                           const int* __restrict__ cu_seqlens, const int* __restrict__ seq_start, int maxp, int H, int D, int V,
+                           float k_scale) {
+    extern __shared__ __align__(128) __nv_bfloat16 rm_smem[];
+    __nv_bfloat16* qt = rm_smem;                     // [3][SM_L][128]
+    __nv_bfloat16* kt = qt + 3 * SM_L * 128;         // [3][SM_L][128], later the weights and the state's rows:
+    __nv_bfloat16* pt = kt;                          // [3][SM_L][SM_L]
+    __nv_bfloat16* st = pt + 3 * SM_L * SM_L;        // [3][32][128]
+    __nv_bfloat16* vt = kt + 3 * SM_L * 128;         // [SM_L][128]
+    __shared__ float pw[SM_L + 1], red[SM_L][2];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y, c0 = blockIdx.z * 128;
+    const int r = blockIdx.x / maxp, first = (blockIdx.x % maxp) * SM_L;
+    if (!ZLM_CHK(cu_seqlens + r, 8) || !ZLM_CHK(seq_start + r, 4) || !ZLM_CHK(decay + h, 4)) return;
+    const int n = min(SM_L, cu_seqlens[r + 1] - cu_seqlens[r] - first);
+    if (n <= 0) return;
+    rm_powers(pw, decay[h], tid);
+    const int row0 = cu_seqlens[r] + first;
+    pdl_wait();
+    const __nv_bfloat16* rows = proj + (size_t)row0 * ld;
+    sm_stage_values(vt, rows + v_off + (size_t)h * V, ld, n, c0, V, tid);
+    rm_stage<true>(qt, kt, rows + q_off + (size_t)h * D, rows + k_off + (size_t)h * D, ld, row0, seq_start[r] + first, n, D, rot,
+                   k_scale, nullptr, tid);
+    const float* S = before + ((size_t)blockIdx.x * H + h) * D * V;
+    SmRows next = sm_fetch_state(S, 0, D, V, c0, tid);
+    dec_wait<0>();
+    __syncthreads();
+    const int r0 = (warp >> 1) * 16, part = warp & 1;
+    SmSum<4> dots;
+    sm_scores(dots, qt, kt, r0, part * 32, D, lane);
+    float s[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int j = r0 + (lane >> 2) + 8 * (e >> 1), l = part * 32 + i * 8 + (lane & 3) * 2 + (e & 1);
+            s[i][e] = l <= j ? dots.get(i, e) * pw[l <= j ? j - l : 0] : 0.f;
+        }
+    __syncthreads();                                 // (the keys are read: weights and the state take their place)
+    sm_put_weights(pt, s, r0, part * 32, lane);
+    SmSum<8> acc;
+    acc.zero();
+    for (int d0 = 0; d0 < D; d0 += 32) {
+        sm_put_state(st, next, tid);
+        if (d0 + 32 < D) next = sm_fetch_state(S, d0 + 32, D, V, c0, tid);
+        __syncthreads();
+        sm_read_state(acc, qt, st, r0, part * 64, d0, D, lane);
+        __syncthreads();
+    }
+    if (out.y) sm_stage_values(qt, out.g + (size_t)row0 * out.g_stride + (size_t)h * V, out.g_stride, n, 0, V, tid);      // (the queries are read)
+    acc.scale(pw[r0 + (lane >> 2) + 1], pw[r0 + (lane >> 2) + 9]);
+    sm_read_values(acc, pt, vt, r0, part * 64, lane);
+    sm_write(acc, 1.f, 1.f, out, qt, red, row0, n, h, H, V, c0, r0, part, lane);
+}
+
+// what the tensor-core form takes: 16-byte reads of 8 neighbouring coordinates (also of the halves of a rotation)
+extern "C" int zlm_retention_products(int dtype, int ld, int q_off, int k_off, int v_off, int n_rot, int D, int V) {
+    return dtype == ZLM_DTYPE_BF16 && D > 0 && D % 16 == 0 && D <= 128 && V > 0 && V % 8 == 0 && (V + 127) / 128 <= 65535 &&
+           n_rot % 16 == 0 && ld % 8 == 0 && q_off % 8 == 0 && k_off % 8 == 0 && v_off % 8 == 0;
+}
+
 // chains the pieces' states of one sequence: before[c] = S_(c-1), S_c = decay^len_c * S_(c-1) + part[c]; the last S
-// becomes the sequence's state.  grid (ceil(D*V / 256), H, R); the pieces of sequence r are r * maxp .. and `part_state`
-// is overwritten in place by `before`.
-__global__ void __launch_bounds__(256)
+// becomes the sequence's state.  A thread owns VEC neighbouring numbers; grid (ceil(D*V / (128 VEC)), H, R); the pieces of
+// sequence r are r * maxp .. and `part_state` is overwritten in place by `before`.
+template <int VEC>
+__global__ void __launch_bounds__(128)
 retention_chain_kernel(float* __restrict__ part_state, float* __restrict__ state, const float* __restrict__ decay,
                        const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slot, int maxp, int piece, int H,
                        int DV) {
+    struct alignas(4 * VEC) Num { float v[VEC]; };
     pdl_launch_dependents();
-    const int e = blockIdx.x * 256 + threadIdx.x, h = blockIdx.y, r = blockIdx.z;
+    const int e = (blockIdx.x * 128 + threadIdx.x) * VEC, h = blockIdx.y, r = blockIdx.z;
     pdl_wait();
     if (e >= DV) return;
     const int n = cu_seqlens[r + 1] - cu_seqlens[r];
-    const int p0 = r * maxp, np = (n + piece - 1) / piece;
-    float* sp = state + ((size_t)seq_slot[r] * H + h) * DV + e;
-    if (!ZLM_CHK(sp, 4)) return;
-    float S = *sp;
+    const int np = (n + piece - 1) / piece;
+    Num* sp = (Num*)(state + ((size_t)seq_slot[r] * H + h) * DV + e);
+    if (!ZLM_CHK(sp, 4 * VEC)) return;
+    Num S = *sp;
     const float d = decay[h];
     const float dl = powf(d, (float)piece);            // every piece but the last is whole
-    for (int c0 = 0; c0 < np; c0 += 8) {
+    const float dn = n == np * piece ? dl : powf(d, (float)(n - (np - 1) * piece));
+    const size_t step = (size_t)H * DV;
+    float* pp = part_state + ((size_t)r * maxp * H + h) * DV + e;
+    for (int c0 = 0; c0 < np; c0 += 8, pp += 8 * step) {
         // eight pieces' states at a time: their loads do not wait for each other
-        float a[8];
+        Num a[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (c0 + u < np && ZLM_CHK(pp + u * step, 4 * VEC)) a[u] = *(const Num*)(pp + u * step);
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            const float* pp = part_state + ((size_t)(p0 + c0 + u) * H + h) * DV + e;
-            a[u] = (c0 + u < np && ZLM_CHK(pp, 4)) ? *pp : 0.f;
-        }
+            if (c0 + u >= np) break;
+            if (ZLM_CHK(pp + u * step, 4 * VEC)) *(Num*)(pp + u * step) = S;
+            const float f = c0 + u == np - 1 ? dn : dl;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int c = c0 + u;
-            if (c >= np) break;
-            float* pp = part_state + ((size_t)(p0 + c) * H + h) * DV + e;
-            if (ZLM_CHK(pp, 4)) *pp = S;
-            const int len = min(piece, n - c * piece);
-            S = fmaf(len == piece ? dl : powf(d, (float)len), S, a[u]);
+            for (int x = 0; x < VEC; ++x) S.v[x] = fmaf(f, S.v[x], a[u].v[x]);
         }
     }
     *sp = S;
+}
+static void launch_chain(float* part_state, float* state, const float* decay, const int* cu_seqlens, const int* seq_slot, int R, int maxp,
+                         int piece, int H, int DV, cudaStream_t st) {
+    if (DV % 4 == 0 && (uintptr_t)state % 16 == 0 && (uintptr_t)part_state % 16 == 0)
+        zlm_launch(retention_chain_kernel<4>, dim3((DV + 511) / 512, H, R), dim3(128), 0, st, part_state, state, decay, cu_seqlens,
+                   seq_slot, maxp, piece, H, DV);
+    else
+        zlm_launch(retention_chain_kernel<1>, dim3((DV + 127) / 128, H, R), dim3(128), 0, st, part_state, state, decay, cu_seqlens,
+                   seq_slot, maxp, piece, H, DV);
 }
 
 static int retention_dpt(int D, int* ds) {
@@ -369,16 +558,44 @@ extern "C" int zlm_retention(float* o, const void* proj, int ld, int q_off, int 
 
 // The same for long prompts, in pieces of `piece` tokens that run side by side: maxp pieces a sequence (those of the
 // step's longest one; a shorter sequence's last pieces are empty); part_state is scratch of R * maxp * H * D * V floats.
+// y (null: none; where zlm_retention_products says yes, heads of up to 128 value columns): [T][y_stride] bfloat16 receives, in
+// the place of o, every head divided by its root mean square times silu (act 1) or sigmoid (0) of g [T][g_stride].
 extern "C" int zlm_retention_parts(float* o, const void* proj, int ld, int q_off, int k_off, int v_off, int dtype,
                                    const float* inv_freq, int n_rot, const float* decay, float* state,
                                    const int* cu_seqlens, const int* seq_slot, const int* seq_start, int R, int maxp, int piece,
                                    float* part_state, int H, int D, int V, float k_scale, const float* table, int T,
-                                   cudaStream_t st) {
+                                   void* y, int y_stride, const void* g, int g_stride, float eps, int act, cudaStream_t st) {
     if (R == 0 || maxp == 0) return ZLM_OK;
     const long long pieces = (long long)R * maxp;
     int rc = retention_check(H, D, V, n_rot, R);
     if (rc) return rc;
     ZLM_REQUIRE(piece > 0 && pieces <= 65535 && part_state, "retention: %lld pieces of %d tokens", pieces, piece);
+    const bool products = zlm_retention_products(dtype, ld, q_off, k_off, v_off, n_rot, D, V) && piece == SM_L &&
+                          (uintptr_t)proj % 16 == 0 && (uintptr_t)part_state % 16 == 0 && (uintptr_t)o % 8 == 0;
+    ZLM_REQUIRE(!y || (products && V <= 128 && y_stride % 8 == 0 && g_stride % 8 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)g % 16 == 0),
+                "retention: heads of %d x %d do not take their gate along", D, V);
+    if (products) {
+        const size_t smem1 = (size_t)4 * SM_L * 128 * sizeof(__nv_bfloat16), smem2 = (size_t)7 * SM_L * 128 * sizeof(__nv_bfloat16);
+        static bool attr_set_dev[64] = {};
+        bool& attr_set = attr_set_dev[zlm_device_index()];
+        if (!attr_set) {
+            cudaError_t e1 = cudaFuncSetAttribute(retention_piece_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
+            cudaError_t e2 = cudaFuncSetAttribute(retention_piece_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
+            if (e1 != cudaSuccess || e2 != cudaSuccess) {
+                zlm_set_error("retention: cannot reserve shared memory");
+                return ZLM_ERR_CUDA;
+            }
+            attr_set = true;
+        }
+        const dim3 grid((unsigned)pieces, H, (V + 127) / 128);
+        const RmRot rot{inv_freq, table, n_rot, T};
+        zlm_launch(retention_piece_state_kernel, grid, dim3(RM_THREADS), smem1, st, part_state, (const __nv_bfloat16*)proj, ld, k_off,
+                   v_off, rot, decay, cu_seqlens, seq_start, maxp, H, D, V, k_scale);
+        launch_chain(part_state, state, decay, cu_seqlens, seq_slot, R, maxp, piece, H, D * V, st);
+        zlm_launch(retention_piece_out_kernel, grid, dim3(RM_THREADS), smem2, st, SmOut{o, (__nv_bfloat16*)y, y_stride, (const __nv_bfloat16*)g, g_stride, VecW{nullptr, 0}, 0, eps, act},
+                   (const __nv_bfloat16*)proj, ld, q_off, k_off, v_off, rot, decay, (const float*)part_state, cu_seqlens, seq_start, maxp, H, D, V, k_scale);
+        return zlm_check_launch("retention_products");
+    }
     int ds;
     const int dpt = retention_dpt(D, &ds);
     const int cols = RT_THREADS / ds * RT_CPT;
@@ -411,8 +628,7 @@ extern "C" int zlm_retention_parts(float* o, const void* proj, int ld, int q_off
         rc = zlm_check_launch("retention_parts");
         if (rc) return rc;
         if (mode == 1) {
-            zlm_launch(retention_chain_kernel, dim3((D * V + 255) / 256, H, R), dim3(256), 0, st, part_state, state, decay,
-                       cu_seqlens, seq_slot, maxp, piece, H, D * V);
+            launch_chain(part_state, state, decay, cu_seqlens, seq_slot, R, maxp, piece, H, D * V, st);
             rc = zlm_check_launch("retention_chain");
             if (rc) return rc;
         }

@@ -1,0 +1,304 @@
+// Products of fp32 numbers on the bfloat16 tensor cores without giving up fp32: an operand is cut into three bfloat16
+// pieces, hi + mid + lo, which together hold all 24 bits of it (each piece rounds what the pieces before it left), and the
+// pieces' products that matter are added up: hi*hi, hi*mid, mid*hi, hi*lo, lo*hi, mid*mid where both operands are cut (what is
+// left out is below 2^-25 of the product), three products where the other one is bfloat16 as it is.
+// The tensor cores cut off what their accumulator cannot hold instead of rounding, which adds up along a chain (one
+// accumulator for all products: 1.1e-6 of the outputs against 2.4e-7 of the FFMA chain that this stands in for).  So the
+// large products of 16 terms start from zero each time and are added by the rounding FADD, and the small ones, of which the
+// cut-off matters 2^-8 as much, have an accumulator of their own that joins at the end (1.7e-7).
+// The helpers work on tiles in shared memory, one tile for each piece, rows swizzled as tile_off says.
+#pragma once
+#include "attn_common.cuh"
+
+#define SM_L 64                      // tokens of a piece of a long prompt
+
+// the three pieces of two neighbouring numbers
+struct Split2 { unsigned p[3]; };
+__device__ __forceinline__ Split2 split2(float a, float b) {
+    Split2 s;
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+        s.p[x] = pack_bf16(a, b);
+        a -= __uint_as_float(s.p[x] << 16);
+        b -= __uint_as_float(s.p[x] & 0xffff0000u);
+    }
+    return s;
+}
+// eight neighbouring numbers into the three tiles at element offset `off`
+__device__ __forceinline__ void split8(__nv_bfloat16* tile, int tile_elems, int off, const float* f) {
+    unsigned u[3][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const Split2 s = split2(f[2 * e], f[2 * e + 1]);
+#pragma unroll
+        for (int x = 0; x < 3; ++x) u[x][e] = s.p[x];
+    }
+#pragma unroll
+    for (int x = 0; x < 3; ++x) *(uint4*)(tile + (size_t)x * tile_elems + off) = make_uint4(u[x][0], u[x][1], u[x][2], u[x][3]);
+}
+__device__ __forceinline__ void widen8(const uint4& u, float* f) {
+    f[0] = __uint_as_float(u.x << 16); f[1] = __uint_as_float(u.x & 0xffff0000u);
+    f[2] = __uint_as_float(u.y << 16); f[3] = __uint_as_float(u.y & 0xffff0000u);
+    f[4] = __uint_as_float(u.z << 16); f[5] = __uint_as_float(u.z & 0xffff0000u);
+    f[6] = __uint_as_float(u.w << 16); f[7] = __uint_as_float(u.w & 0xffff0000u);
+}
+
+// where a lane reads, for the four 8 x 8 matrices of an ldmatrix:
+//   A of a product from rows of A (16 rows from r0, 16 columns from c0)
+template <int HD> __device__ __forceinline__ const __nv_bfloat16* sm_a_rows(const __nv_bfloat16* t, int r0, int c0, int lane) {
+    return t + tile_off<HD>(r0 + (lane & 15), (c0 >> 3) + (lane >> 4));
+}
+//   A from rows of A^T (16 rows of A^T from c0, 16 columns from r0), transposed on the way
+template <int HD> __device__ __forceinline__ const __nv_bfloat16* sm_a_cols(const __nv_bfloat16* t, int r0, int c0, int lane) {
+    return t + tile_off<HD>(c0 + (lane & 7) + ((lane >> 4) << 3), (r0 >> 3) + ((lane >> 3) & 1));
+}
+//   B of two neighbouring tiles of 8 outputs from rows of B^T (an output a row)
+template <int HD> __device__ __forceinline__ const __nv_bfloat16* sm_b_rows(const __nv_bfloat16* t, int n0, int k0, int lane) {
+    return t + tile_off<HD>(n0 + (lane & 7) + ((lane >> 4) << 3), (k0 >> 3) + ((lane >> 3) & 1));
+}
+//   the same from rows of B (an output a column), transposed on the way
+template <int HD> __device__ __forceinline__ const __nv_bfloat16* sm_b_cols(const __nv_bfloat16* t, int n0, int k0, int lane) {
+    return t + tile_off<HD>(k0 + (lane & 15), (n0 >> 3) + (lane >> 4));
+}
+
+// sums of NT tiles of 16 x 8 outputs: the large products' and the small ones'
+template <int NT> struct SmSum {
+    float hi[NT][4], lo[NT][4];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) hi[n][e] = lo[n][e] = 0.f;
+    }
+    // both times a factor by row (of a lane's two rows)
+    __device__ __forceinline__ void scale(float r0, float r8) {
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                hi[n][e] *= e < 2 ? r0 : r8;
+                lo[n][e] *= e < 2 ? r0 : r8;
+            }
+    }
+    __device__ __forceinline__ float get(int n, int e) const { return hi[n][e] + lo[n][e]; }
+};
+// acc += a b, 16 terms from zero on, added by FADD
+__device__ __forceinline__ void sm_mma_add(float* acc, const unsigned* a, unsigned b0, unsigned b1) {
+    float d[4];
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[e] += d[e];
+}
+// tiles n and n + 1 += A B with both operands in pieces
+template <int NT> __device__ __forceinline__ void sm_mma6(SmSum<NT>& s, int n, const unsigned (&a)[3][4], const unsigned (&b)[3][4]) {
+    constexpr int ia[5] = {1, 0, 2, 0, 1}, ib[5] = {1, 2, 0, 1, 0};
+    sm_mma_add(s.hi[n], a[0], b[0][0], b[0][1]);
+    sm_mma_add(s.hi[n + 1], a[0], b[0][2], b[0][3]);
+#pragma unroll
+    for (int x = 0; x < 5; ++x) {
+        dec_mma(s.lo[n], a[ia[x]], b[ib[x]][0], b[ib[x]][1]);
+        dec_mma(s.lo[n + 1], a[ia[x]], b[ib[x]][2], b[ib[x]][3]);
+    }
+}
+// the same with B in bfloat16 as it is
+template <int NT> __device__ __forceinline__ void sm_mma3(SmSum<NT>& s, int n, const unsigned (&a)[3][4], const unsigned (&b)[4]) {
+    sm_mma_add(s.hi[n], a[0], b[0], b[1]);
+    sm_mma_add(s.hi[n + 1], a[0], b[2], b[3]);
+#pragma unroll
+    for (int x = 2; x >= 1; --x) {
+        dec_mma(s.lo[n], a[x], b[0], b[1]);
+        dec_mma(s.lo[n + 1], a[x], b[2], b[3]);
+    }
+}
+
+// ---------------------------------------------------------------------------- a piece of 64 tokens, one head, 128 value columns
+// Blocks of 256 threads.  What a piece adds to a state:
+//   acc += (keys)^T (values): the warp's 16 rows of the state from d0 on, 64 columns from n0 on;
+//   kt: the weighted keys [SM_L][128] in pieces, vt: the values [SM_L][128]
+__device__ __forceinline__ void sm_piece_state(SmSum<8>& acc, const __nv_bfloat16* kt, const __nv_bfloat16* vt, int d0, int n0, int lane) {
+#pragma unroll
+    for (int k0 = 0; k0 < SM_L; k0 += 16) {
+        unsigned a[3][4];
+#pragma unroll
+        for (int x = 0; x < 3; ++x) dec_ldsm4t(a[x][0], a[x][1], a[x][2], a[x][3], sm_a_cols<128>(kt + x * SM_L * 128, d0, k0, lane));
+#pragma unroll
+        for (int n = 0; n < 8; n += 2) {
+            unsigned b[4];
+            dec_ldsm4t(b[0], b[1], b[2], b[3], sm_b_cols<128>(vt, n0 + n * 8, k0, lane));
+            sm_mma3(acc, n, a, b);
+        }
+    }
+}
+// Scores of 16 queries (rows r0 on) against 32 keys (rows n0 on), `dim` coordinates, both in pieces [SM_L][128]; tiles of
+// keys after the last query stay zero
+__device__ __forceinline__ void sm_scores(SmSum<4>& s, const __nv_bfloat16* qt, const __nv_bfloat16* kt, int r0, int n0, int dim, int lane) {
+    s.zero();
+    if (n0 > r0 + 15) return;
+    for (int k0 = 0; k0 < dim; k0 += 16) {
+        unsigned a[3][4];
+#pragma unroll
+        for (int x = 0; x < 3; ++x) dec_ldsm4(a[x][0], a[x][1], a[x][2], a[x][3], sm_a_rows<128>(qt + x * SM_L * 128, r0, k0, lane));
+#pragma unroll
+        for (int n = 0; n < 4; n += 2) {
+            if (n0 + n * 8 > r0 + 15) continue;
+            unsigned b[3][4];
+#pragma unroll
+            for (int x = 0; x < 3; ++x) dec_ldsm4(b[x][0], b[x][1], b[x][2], b[x][3], sm_b_rows<128>(kt + x * SM_L * 128, n0 + n * 8, k0, lane));
+            sm_mma6(s, n, a, b);
+        }
+    }
+}
+// 32 rows of the state, 128 columns: fetched into registers (a thread's four float4), then cut into pieces [32][128]
+struct SmRows { float4 f[4]; };
+__device__ __forceinline__ SmRows sm_fetch_state(const float* S, int d0, int dim, int V, int c0, int tid) {
+    SmRows r;
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+        const int row = d0 + (tid >> 4) + 16 * x, c = c0 + (tid & 15) * 8;
+        const float* p = S + (size_t)row * V + c;
+        const bool ok = row < dim && c < V && ZLM_CHK(p, 32);
+        r.f[2 * x] = ok ? *(const float4*)p : make_float4(0.f, 0.f, 0.f, 0.f);
+        r.f[2 * x + 1] = ok ? *(const float4*)(p + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    return r;
+}
+__device__ __forceinline__ void sm_put_state(__nv_bfloat16* st, const SmRows& r, int tid) {
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+        const float f[8] = {r.f[2 * x].x, r.f[2 * x].y, r.f[2 * x].z, r.f[2 * x].w, r.f[2 * x + 1].x, r.f[2 * x + 1].y, r.f[2 * x + 1].z, r.f[2 * x + 1].w};
+        split8(st, 32 * 128, tile_off<128>((tid >> 4) + 16 * x, tid & 15), f);
+    }
+}
+// acc (16 queries from r0, 64 columns from n0) += queries, coordinates d0 .. d0 + 31, times the state's pieces [32][128]
+__device__ __forceinline__ void sm_read_state(SmSum<8>& acc, const __nv_bfloat16* qt, const __nv_bfloat16* st, int r0, int n0, int d0, int dim, int lane) {
+#pragma unroll
+    for (int k0 = 0; k0 < 32; k0 += 16) {
+        if (d0 + k0 >= dim) return;
+        unsigned a[3][4];
+#pragma unroll
+        for (int x = 0; x < 3; ++x) dec_ldsm4(a[x][0], a[x][1], a[x][2], a[x][3], sm_a_rows<128>(qt + x * SM_L * 128, r0, d0 + k0, lane));
+#pragma unroll
+        for (int n = 0; n < 8; n += 2) {
+            unsigned b[3][4];
+#pragma unroll
+            for (int x = 0; x < 3; ++x) dec_ldsm4t(b[x][0], b[x][1], b[x][2], b[x][3], sm_b_cols<128>(st + x * 32 * 128, n0 + n * 8, k0, lane));
+            sm_mma6(acc, n, a, b);
+        }
+    }
+}
+// the weights of 16 queries (from r0) on 32 keys (from n0) into pieces [SM_L][SM_L]
+__device__ __forceinline__ void sm_put_weights(__nv_bfloat16* pt, const float (&s)[4][4], int r0, int n0, int lane) {
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const Split2 w = split2(s[n][2 * i], s[n][2 * i + 1]);
+            const int row = r0 + (lane >> 2) + 8 * i;
+#pragma unroll
+            for (int x = 0; x < 3; ++x)
+                *(unsigned*)(pt + x * SM_L * SM_L + tile_off<SM_L>(row, (n0 >> 3) + n) + (lane & 3) * 2) = w.p[x];
+        }
+}
+// acc (16 queries from r0, 64 columns from n0) += weights times values [SM_L][128]; keys after the queries are skipped
+__device__ __forceinline__ void sm_read_values(SmSum<8>& acc, const __nv_bfloat16* pt, const __nv_bfloat16* vt, int r0, int n0, int lane) {
+#pragma unroll
+    for (int k0 = 0; k0 < SM_L; k0 += 16) {
+        if (k0 > r0) return;
+        unsigned a[3][4];
+#pragma unroll
+        for (int x = 0; x < 3; ++x) dec_ldsm4(a[x][0], a[x][1], a[x][2], a[x][3], sm_a_rows<SM_L>(pt + x * SM_L * SM_L, r0, k0, lane));
+#pragma unroll
+        for (int n = 0; n < 8; n += 2) {
+            unsigned b[4];
+            dec_ldsm4t(b[0], b[1], b[2], b[3], sm_b_cols<128>(vt, n0 + n * 8, k0, lane));
+            sm_mma3(acc, n, a, b);
+        }
+    }
+}
+// the values of a piece, 128 columns from c0 (zeros beyond the piece's tokens and the head's columns), by asynchronous copies
+__device__ __forceinline__ void sm_stage_values(__nv_bfloat16* vt, const __nv_bfloat16* v, size_t stride, int n, int c0, int V, int tid) {
+#pragma unroll
+    for (int y = 0; y < SM_L * 16 / 256; ++y) {
+        const int x = tid + y * 256, l = x >> 4, c = x & 15;
+        __nv_bfloat16* dst = vt + tile_off<128>(l, c);
+        if (l < n && c0 + c * 8 < V) dec_cp_async16(dst, v + (size_t)l * stride + c0 + c * 8);
+        else *(uint4*)dst = make_uint4(0, 0, 0, 0);
+    }
+    dec_commit();
+}
+
+// ---------------------------------------------------------------------------- what leaves the kernels of a piece
+// The outputs as they are (o [T][H * V] fp32), or what follows them in the mixers (y): every head divided by its root mean
+// square, times a weight where there is one, times silu (act 1) or sigmoid (0) of a gate's columns, in bfloat16.
+struct SmOut {
+    float* o;
+    __nv_bfloat16* y;                // null: o
+    int y_stride;
+    const __nv_bfloat16* g;
+    int g_stride;
+    VecW w;                          // null, or [w_rows ? H : 1][V]
+    int w_rows;
+    float eps;
+    int act;
+};
+// a warp's 16 rows (of the piece's n) by 64 columns, times a factor for each of a lane's two rows; red [SM_L][2] in shared
+// memory.  The gated form wants all of a head's columns in the block (V <= 128) and every thread of it here; gt is its tile
+// of the gate's columns [SM_L][128], on the way by sm_stage_values, which the results pass through on their way out
+__device__ __forceinline__ void sm_write(const SmSum<8>& acc, float f0, float f8, const SmOut& out, __nv_bfloat16* gt, float (*red)[2],
+                                         int row0, int n, int h, int H, int V, int c0, int r0, int half, int lane) {
+    const int c = c0 + half * 64 + (lane & 3) * 2;
+    if (!out.y) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int j = r0 + (lane >> 2) + 8 * e;
+                float* p = out.o + ((size_t)(row0 + j) * H + h) * V + c + i * 8;
+                const float f = e ? f8 : f0;
+                if (j < n && c + i * 8 < V && ZLM_CHK(p, 8)) *(float2*)p = make_float2(acc.get(i, 2 * e) * f, acc.get(i, 2 * e + 1) * f);
+            }
+        return;
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        float ss = 0.f;                                  // (columns beyond V are zero)
+        const float f = e ? f8 : f0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float a = acc.get(i, 2 * e) * f, b = acc.get(i, 2 * e + 1) * f;
+            ss = fmaf(a, a, fmaf(b, b, ss));
+        }
+        ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+        if ((lane & 3) == 0) red[r0 + (lane >> 2) + 8 * e][half] = ss;
+    }
+    dec_wait<0>();
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int j = r0 + (lane >> 2) + 8 * e;
+        const float f = (e ? f8 : f0) / sqrtf((red[j][0] + red[j][1]) / (float)V + out.eps);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (c + i * 8 >= V) continue;
+            unsigned* at = (unsigned*)(gt + tile_off<128>(j, half * 8 + i) + (lane & 3) * 2);
+            const unsigned z = *at;
+            float v[2];
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const float zz = __uint_as_float(x ? z & 0xffff0000u : z << 16), sg = 1.0f / (1.0f + expf(-zz));
+                const float w = out.w.p ? out.w[(out.w_rows ? h * V : 0) + c + i * 8 + x] : 1.0f;
+                v[x] = acc.get(i, 2 * e + x) * f * w * (out.act == 1 ? zz * sg : sg);
+            }
+            *at = pack_bf16(v[0], v[1]);
+        }
+    }
+    __syncthreads();
+    for (int x = threadIdx.x; x < n * 16; x += 256) {
+        __nv_bfloat16* yp = out.y + (size_t)(row0 + (x >> 4)) * out.y_stride + (size_t)h * V + (x & 15) * 8;
+        if ((x & 15) * 8 < V && ZLM_CHK(yp, 16)) *(uint4*)yp = *(const uint4*)(gt + tile_off<128>(x >> 4, x & 15));
+    }
+}

@@ -869,7 +869,7 @@ class CudaKernels:
     def retention(self, o: torch.Tensor, proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
                   inv_freq: Optional[torch.Tensor], n_rot: int, decay: torch.Tensor, state: torch.Tensor, plan,
                   heads: int, dim: int, v_dim: int, k_scale: float, pieces: Optional[bool] = None,
-                  cos_sin: Optional[torch.Tensor] = None) -> None:
+                  cos_sin: Optional[torch.Tensor] = None, _gate: Optional[tuple] = None) -> None:
         """o [T, heads*v_dim] fp32 = S_t^T q_t with S_t = decay_h S_(t-1) + k_t v_t^T per head, q and k rotated (first
         ``n_rot`` coordinates of a head, halves against each other, by pos * inv_freq) and k scaled by ``k_scale``; q, k,
         v are columns of ``proj`` from q_off, k_off, v_off on; ``state`` [slots, heads, dim, v_dim] fp32 holds S between
@@ -898,9 +898,31 @@ class CudaKernels:
             L = self.RETENTION_PIECE
             maxp = (int(plan.max_new) + L - 1) // L
             part = plan.scratch("retention.part_state", (plan.R * maxp * heads * dim * v_dim,), torch.float32)
-            self._call("zlm_retention_parts", *head, c_int(maxp), c_int(L), self._p(part), *tail)
+            # (the gate rides in the last kernel where the pieces run as products)
+            y, g, eps, act = (_gate[0], _gate[1], _gate[2], _gate[3]) if _gate is not None else (None, None, 0.0, "silu")
+            self._call("zlm_retention_parts", *head, c_int(maxp), c_int(L), self._p(part), *tail[:-1], self._p(y),
+                       c_int(y.stride(0) if y is not None else 0), self._p(g), c_int(g.stride(0) if g is not None else 0),
+                       c_float(eps), c_int({"sigmoid": 0, "silu": 1}[act]), tail[-1])
             return
         self._call("zlm_retention", *head, *tail[:-1], c_int(int(getattr(plan, "max_new", 0) or 0)), tail[-1])
+
+    def retention_gated(self, y: torch.Tensor, g: torch.Tensor, eps: float, act: str, o: torch.Tensor, proj: torch.Tensor,
+                        q_off: int, k_off: int, v_off: int, inv_freq: Optional[torch.Tensor], n_rot: int, decay: torch.Tensor,
+                        state: torch.Tensor, plan, heads: int, dim: int, v_dim: int, k_scale: float,
+                        cos_sin: Optional[torch.Tensor] = None) -> None:
+        """``retention``, then ``head_gate`` with the heads' unit norm: y [T, heads*v_dim] = o / rms(o, per head) * act(g).
+        ``o`` is scratch that a long bfloat16 prompt does not touch (its last kernel writes y)."""
+        args = (proj, q_off, k_off, v_off, inv_freq, n_rot, decay, state, plan, heads, dim, v_dim, k_scale)
+        if (y.dtype == g.dtype == torch.bfloat16 and plan.max_new >= self.RETENTION_PIECES_FROM and v_dim <= 128
+                and y.stride(1) == g.stride(1) == 1 and (y.stride(0) | g.stride(0)) % 8 == 0
+                and (proj.data_ptr() | y.data_ptr() | g.data_ptr()) % 16 == 0
+                and self.lib.zlm_retention_products(c_int(_dt(proj)), c_int(proj.stride(0)), c_int(q_off), c_int(k_off), c_int(v_off),
+                                                    c_int(n_rot if inv_freq is not None else 0), c_int(dim), c_int(v_dim))):
+            assert y.shape == g.shape == (proj.shape[0], heads * v_dim)
+            self.retention(o, *args, cos_sin=cos_sin, _gate=(y, g, eps, act))
+            return
+        self.retention(o, *args, cos_sin=cos_sin)
+        self.head_gate(y, o.view(-1, heads, v_dim), g, heads, v_dim, True, eps, act)
 
     def attn_prep(self, q_out: torch.Tensor, proj: torch.Tensor, conv_w: Optional[torch.Tensor], state: Optional[torch.Tensor],
                   plan, block_table: torch.Tensor, pool: torch.Tensor, nq: int, nkv: int, dim: int, vdim: int, taps: int,

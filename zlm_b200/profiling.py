@@ -259,6 +259,14 @@ class ProfilingKernels:
         return self._timed(kind, n, 4.0 * T * heads * dim * v_dim, self.k.retention, o, proj, q_off, k_off, v_off, inv_freq,
                            n_rot, decay, state, plan, heads, dim, v_dim, k_scale, pieces, cos_sin)
 
+    def retention_gated(self, y, g, eps, act, o, proj, q_off, k_off, v_off, inv_freq, n_rot, decay, state, plan, heads, dim, v_dim,
+                        *args, **kw):
+        T, el = proj.shape[0], proj.element_size()
+        n = T * heads * (2 * dim + v_dim) * el + 2 * _nbytes(y) + 2 * plan.R * heads * dim * v_dim * 4
+        kind = "retention decode, heads norm*gate" if plan.is_decode else "retention prefill, heads norm*gate"
+        return self._timed(kind, n, 4.0 * T * heads * dim * v_dim, self.k.retention_gated, y, g, eps, act, o, proj, q_off, k_off,
+                           v_off, inv_freq, n_rot, decay, state, plan, heads, dim, v_dim, *args, **kw)
+
     # mixers side by side, recurrent mixers, the general q/k/v preparation
     def attn_prep(self, q_out, proj, conv_w, state, plan, block_table, pool, nq, nkv, dim, vdim, *args, **kw):
         T, el = proj.shape[0], proj.element_size()
