@@ -277,52 +277,71 @@ __device__ __forceinline__ void rm_stage(__nv_bfloat16* qt, __nv_bfloat16* kt, c
                                          size_t stride, int row0, int pos0, int n, int D, const RmRot& rot, float k_scale,
                                          const float* k_weight, int tid) {
     const int half = rot.n_rot >> 1, pairs = half >> 3, items = (D >> 3) - pairs;       // items: pairs of groups, then single groups
-    for (int x = tid; x < items * SM_L; x += RM_THREADS) {
+    struct Item { uint4 a[2], b[2]; float cs[8], sn[8]; };
+    auto fetch = [&](int x, Item& t) {
         const int l = x % SM_L, it = x / SM_L;
-        const bool turn = it < pairs;
+        const bool turn = it < pairs, live = l < n;
         const int f0 = turn ? it * 8 : rot.n_rot + (it - pairs) * 8, f1 = f0 + half;
-        float cs[8], sn[8];
-        const bool live = l < n;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) { cs[e] = 1.f; sn[e] = 0.f; }
-        if (turn && live) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                if (rot.table) {
-                    const float* c = rot.table + (size_t)(f0 + e) * rot.T + row0 + l;
-                    const float* s = c + (size_t)half * rot.T;
-                    if (ZLM_CHK(c, 4)) cs[e] = *c;
-                    if (ZLM_CHK(s, 4)) sn[e] = *s;
-                } else {
-                    sincosf((float)(pos0 + l) * rot.inv_freq[f0 + e], &sn[e], &cs[e]);
-                }
-            }
-        }
-        const float kw = k_scale * (k_weight ? k_weight[l] : 1.f);
 #pragma unroll
         for (int y = Q ? 0 : 1; y < 2; ++y) {
             const __nv_bfloat16* p = (y ? k : q) + (size_t)l * stride;
-            __nv_bfloat16* dst = y ? kt : qt;
-            uint4 a = make_uint4(0, 0, 0, 0), b = a;
-            if (live && ZLM_CHK(p + f0, 16)) a = *(const uint4*)(p + f0);
-            if (turn && live && ZLM_CHK(p + f1, 16)) b = *(const uint4*)(p + f1);
-            float u[8], v[8], r[8];
-            widen8(a, u);
-            widen8(b, v);
+            t.a[y] = t.b[y] = make_uint4(0, 0, 0, 0);
+            if (live && ZLM_CHK(p + f0, 16)) t.a[y] = *(const uint4*)(p + f0);
+            if (turn && live && ZLM_CHK(p + f1, 16)) t.b[y] = *(const uint4*)(p + f1);
+        }
 #pragma unroll
-            for (int e = 0; e < 8; ++e) r[e] = (turn ? u[e] * cs[e] - v[e] * sn[e] : u[e]) * (y ? kw : 1.f);
+        for (int e = 0; e < 8; ++e) {
+            t.cs[e] = 1.f;
+            t.sn[e] = 0.f;
+            if (!turn || !live) continue;
+            if (rot.table) {
+                const float* c = rot.table + (size_t)(f0 + e) * rot.T + row0 + l;
+                const float* s = c + (size_t)half * rot.T;
+                if (ZLM_CHK(c, 4)) t.cs[e] = *c;
+                if (ZLM_CHK(s, 4)) t.sn[e] = *s;
+            } else {
+                sincosf((float)(pos0 + l) * rot.inv_freq[f0 + e], &t.sn[e], &t.cs[e]);
+            }
+        }
+    };
+    auto put = [&](int x, const Item& t) {
+        const int l = x % SM_L, it = x / SM_L;
+        const bool turn = it < pairs;
+        const int f0 = turn ? it * 8 : rot.n_rot + (it - pairs) * 8, f1 = f0 + half;
+        const float kw = k_scale * (k_weight ? k_weight[l] : 1.f);
+#pragma unroll
+        for (int y = Q ? 0 : 1; y < 2; ++y) {
+            __nv_bfloat16* dst = y ? kt : qt;
+            float u[8], v[8], r[8];
+            widen8(t.a[y], u);
+            widen8(t.b[y], v);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) r[e] = (turn ? u[e] * t.cs[e] - v[e] * t.sn[e] : u[e]) * (y ? kw : 1.f);
             split8(dst, SM_L * 128, tile_off<128>(l, f0 >> 3), r);
             if (turn) {
 #pragma unroll
-                for (int e = 0; e < 8; ++e) r[e] = (v[e] * cs[e] + u[e] * sn[e]) * (y ? kw : 1.f);
+                for (int e = 0; e < 8; ++e) r[e] = (v[e] * t.cs[e] + u[e] * t.sn[e]) * (y ? kw : 1.f);
                 split8(dst, SM_L * 128, tile_off<128>(l, f1 >> 3), r);
             }
         }
+    };
+    // (two items' loads on their way at a time: the stores into shared memory let no later load past them)
+    for (int x = tid; x < items * SM_L; x += 2 * RM_THREADS) {
+        Item t0, t1;
+        const bool two = x + RM_THREADS < items * SM_L;
+        fetch(x, t0);
+        if (two) fetch(x + RM_THREADS, t1);
+        put(x, t0);
+        if (two) put(x + RM_THREADS, t1);
     }
 }
 // decay^0 .. decay^64, each rounded once
 __device__ __forceinline__ void rm_powers(float* pw, float d, int tid) {
-    if (tid <= SM_L) pw[tid] = (float)pow((double)d, (double)tid);
+    if (tid > SM_L) return;
+    double p = 1.0, q = d;
+    for (int i = tid; i; i >>= 1, q *= q)
+        if (i & 1) p *= q;
+    pw[tid] = (float)p;
 }
 
 // grid (R * maxp, H, ceil(V / 128))
@@ -357,14 +376,7 @@ retention_piece_state_kernel(float* __restrict__ part, const __nv_bfloat16* __re
         SmSum<8> acc;
         acc.zero();
         sm_piece_state(acc, kt, vt, d0, n0, lane);
-        float* dst = part + (((size_t)blockIdx.x * H + h) * D + d0 + (lane >> 2)) * V + c0 + n0 + (lane & 3) * 2;
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                float* p = dst + (size_t)8 * e * V + i * 8;
-                if (c0 + n0 + i * 8 < V && ZLM_CHK(p, 8)) *(float2*)p = make_float2(acc.get(i, 2 * e), acc.get(i, 2 * e + 1));
-            }
+        sm_write_state(part + ((size_t)blockIdx.x * H + h) * D * V, acc, d0, c0 + n0, V, lane);
     }
 }
 

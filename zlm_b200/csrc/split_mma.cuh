@@ -3,9 +3,8 @@
 // pieces' products that matter are added up: hi*hi, hi*mid, mid*hi, hi*lo, lo*hi, mid*mid where both operands are cut (what is
 // left out is below 2^-25 of the product), three products where the other one is bfloat16 as it is.
 // The tensor cores cut off what their accumulator cannot hold instead of rounding, which adds up along a chain (one
-// accumulator for all products: 1.1e-6 of the outputs against 2.4e-7 of the FFMA chain that this stands in for).  So the
-// large products of 16 terms start from zero each time and are added by the rounding FADD, and the small ones, of which the
-// cut-off matters 2^-8 as much, have an accumulator of their own that joins at the end (1.7e-7).
+// accumulator for all products: 1.1e-6 of a retention's outputs against 2.4e-7 of the FFMA chain that this stands in for).  So
+// the products of 16 terms start from zero each time, the small ones first, and are added by the rounding FADD: 1.8e-7.
 // The helpers work on tiles in shared memory, one tile for each piece, rows swizzled as tile_off says.
 #pragma once
 #include "attn_common.cuh"
@@ -61,58 +60,65 @@ template <int HD> __device__ __forceinline__ const __nv_bfloat16* sm_b_cols(cons
     return t + tile_off<HD>(k0 + (lane & 15), (n0 >> 3) + (lane >> 4));
 }
 
-// sums of NT tiles of 16 x 8 outputs: the large products' and the small ones'
-template <int NT> struct SmSum {
-    float hi[NT][4], lo[NT][4];
-    __device__ __forceinline__ void zero() {
-#pragma unroll
-        for (int n = 0; n < NT; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) hi[n][e] = lo[n][e] = 0.f;
-    }
-    // both times a factor by row (of a lane's two rows)
-    __device__ __forceinline__ void scale(float r0, float r8) {
-#pragma unroll
-        for (int n = 0; n < NT; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                hi[n][e] *= e < 2 ? r0 : r8;
-                lo[n][e] *= e < 2 ? r0 : r8;
-            }
-    }
-    __device__ __forceinline__ float get(int n, int e) const { return hi[n][e] + lo[n][e]; }
-};
-// acc += a b, 16 terms from zero on, added by FADD
-__device__ __forceinline__ void sm_mma_add(float* acc, const unsigned* a, unsigned b0, unsigned b1) {
-    float d[4];
+// d = a b
+__device__ __forceinline__ void sm_mma_zero(float* d, const unsigned* a, unsigned b0, unsigned b1) {
     asm volatile(
         "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
-#pragma unroll
-    for (int e = 0; e < 4; ++e) acc[e] += d[e];
 }
-// tiles n and n + 1 += A B with both operands in pieces
-template <int NT> __device__ __forceinline__ void sm_mma6(SmSum<NT>& s, int n, const unsigned (&a)[3][4], const unsigned (&b)[3][4]) {
-    constexpr int ia[5] = {1, 0, 2, 0, 1}, ib[5] = {1, 2, 0, 1, 0};
-    sm_mma_add(s.hi[n], a[0], b[0][0], b[0][1]);
-    sm_mma_add(s.hi[n + 1], a[0], b[0][2], b[0][3]);
+// NP pairs of neighbouring tiles of 16 x 8 sums += A B, 16 terms, both operands in pieces.  (The products of one tile wait for
+// each other; those of the 2 NP tiles take turns.)
+template <int NP> __device__ __forceinline__ void sm_mma6(float (*acc)[4], const unsigned (&a)[3][4], const unsigned (&b)[NP][3][4]) {
+    constexpr int ia[6] = {1, 0, 2, 0, 1, 0}, ib[6] = {1, 2, 0, 1, 0, 0};
+    float d[2 * NP][4];
 #pragma unroll
-    for (int x = 0; x < 5; ++x) {
-        dec_mma(s.lo[n], a[ia[x]], b[ib[x]][0], b[ib[x]][1]);
-        dec_mma(s.lo[n + 1], a[ia[x]], b[ib[x]][2], b[ib[x]][3]);
-    }
+    for (int x = 0; x < 6; ++x)
+#pragma unroll
+        for (int t = 0; t < 2 * NP; ++t) {
+            const unsigned* p = b[t / 2][ib[x]] + (t & 1) * 2;
+            if (x == 0) sm_mma_zero(d[t], a[ia[x]], p[0], p[1]);
+            else dec_mma(d[t], a[ia[x]], p[0], p[1]);
+        }
+#pragma unroll
+    for (int t = 0; t < 2 * NP; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[t][e] += d[t][e];
 }
 // the same with B in bfloat16 as it is
-template <int NT> __device__ __forceinline__ void sm_mma3(SmSum<NT>& s, int n, const unsigned (&a)[3][4], const unsigned (&b)[4]) {
-    sm_mma_add(s.hi[n], a[0], b[0], b[1]);
-    sm_mma_add(s.hi[n + 1], a[0], b[2], b[3]);
+template <int NP> __device__ __forceinline__ void sm_mma3(float (*acc)[4], const unsigned (&a)[3][4], const unsigned (&b)[NP][4]) {
+    float d[2 * NP][4];
 #pragma unroll
-    for (int x = 2; x >= 1; --x) {
-        dec_mma(s.lo[n], a[x], b[0], b[1]);
-        dec_mma(s.lo[n + 1], a[x], b[2], b[3]);
-    }
+    for (int x = 2; x >= 0; --x)
+#pragma unroll
+        for (int t = 0; t < 2 * NP; ++t) {
+            const unsigned* p = b[t / 2] + (t & 1) * 2;
+            if (x == 2) sm_mma_zero(d[t], a[x], p[0], p[1]);
+            else dec_mma(d[t], a[x], p[0], p[1]);
+        }
+#pragma unroll
+    for (int t = 0; t < 2 * NP; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[t][e] += d[t][e];
 }
+// sums of NT tiles of 16 x 8
+template <int NT> struct SmSum {
+    float v[NT][4];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[n][e] = 0.f;
+    }
+    // times a factor by row (of a lane's two rows)
+    __device__ __forceinline__ void scale(float r0, float r8) {
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[n][e] *= e < 2 ? r0 : r8;
+    }
+    __device__ __forceinline__ float get(int n, int e) const { return v[n][e]; }
+};
 
 // ---------------------------------------------------------------------------- a piece of 64 tokens, one head, 128 value columns
 // Blocks of 256 threads.  What a piece adds to a state:
@@ -125,15 +131,27 @@ __device__ __forceinline__ void sm_piece_state(SmSum<8>& acc, const __nv_bfloat1
 #pragma unroll
         for (int x = 0; x < 3; ++x) dec_ldsm4t(a[x][0], a[x][1], a[x][2], a[x][3], sm_a_cols<128>(kt + x * SM_L * 128, d0, k0, lane));
 #pragma unroll
-        for (int n = 0; n < 8; n += 2) {
-            unsigned b[4];
-            dec_ldsm4t(b[0], b[1], b[2], b[3], sm_b_cols<128>(vt, n0 + n * 8, k0, lane));
-            sm_mma3(acc, n, a, b);
+        for (int n = 0; n < 8; n += 4) {
+            unsigned b[2][4];
+#pragma unroll
+            for (int y = 0; y < 2; ++y) dec_ldsm4t(b[y][0], b[y][1], b[y][2], b[y][3], sm_b_cols<128>(vt, n0 + n * 8 + y * 16, k0, lane));
+            sm_mma3<2>(acc.v + n, a, b);
         }
     }
 }
-// Scores of 16 queries (rows r0 on) against 32 keys (rows n0 on), `dim` coordinates, both in pieces [SM_L][128]; tiles of
-// keys after the last query stay zero
+// 16 rows from d0, 64 columns from c of a state [..][V]
+__device__ __forceinline__ void sm_write_state(float* S, const SmSum<8>& acc, int d0, int c, int V, int lane) {
+    float* dst = S + (size_t)(d0 + (lane >> 2)) * V + c + (lane & 3) * 2;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            float* p = dst + (size_t)8 * e * V + i * 8;
+            if (c + i * 8 < V && ZLM_CHK(p, 8)) *(float2*)p = make_float2(acc.get(i, 2 * e), acc.get(i, 2 * e + 1));
+        }
+}
+// Scores of 16 queries (rows r0 on) against 32 keys (rows n0 on), `dim` coordinates, both in pieces [SM_L][128]; where
+// all 32 keys come after the last query the scores stay zero
 __device__ __forceinline__ void sm_scores(SmSum<4>& s, const __nv_bfloat16* qt, const __nv_bfloat16* kt, int r0, int n0, int dim, int lane) {
     s.zero();
     if (n0 > r0 + 15) return;
@@ -141,14 +159,13 @@ __device__ __forceinline__ void sm_scores(SmSum<4>& s, const __nv_bfloat16* qt, 
         unsigned a[3][4];
 #pragma unroll
         for (int x = 0; x < 3; ++x) dec_ldsm4(a[x][0], a[x][1], a[x][2], a[x][3], sm_a_rows<128>(qt + x * SM_L * 128, r0, k0, lane));
+        unsigned b[2][3][4];
 #pragma unroll
-        for (int n = 0; n < 4; n += 2) {
-            if (n0 + n * 8 > r0 + 15) continue;
-            unsigned b[3][4];
+        for (int y = 0; y < 2; ++y)
 #pragma unroll
-            for (int x = 0; x < 3; ++x) dec_ldsm4(b[x][0], b[x][1], b[x][2], b[x][3], sm_b_rows<128>(kt + x * SM_L * 128, n0 + n * 8, k0, lane));
-            sm_mma6(s, n, a, b);
-        }
+            for (int x = 0; x < 3; ++x)
+                dec_ldsm4(b[y][x][0], b[y][x][1], b[y][x][2], b[y][x][3], sm_b_rows<128>(kt + x * SM_L * 128, n0 + y * 16, k0, lane));
+        sm_mma6<2>(s.v, a, b);
     }
 }
 // 32 rows of the state, 128 columns: fetched into registers (a thread's four float4), then cut into pieces [32][128]
@@ -181,11 +198,14 @@ __device__ __forceinline__ void sm_read_state(SmSum<8>& acc, const __nv_bfloat16
 #pragma unroll
         for (int x = 0; x < 3; ++x) dec_ldsm4(a[x][0], a[x][1], a[x][2], a[x][3], sm_a_rows<128>(qt + x * SM_L * 128, r0, d0 + k0, lane));
 #pragma unroll
-        for (int n = 0; n < 8; n += 2) {
-            unsigned b[3][4];
+        for (int n = 0; n < 8; n += 4) {
+            unsigned b[2][3][4];
 #pragma unroll
-            for (int x = 0; x < 3; ++x) dec_ldsm4t(b[x][0], b[x][1], b[x][2], b[x][3], sm_b_cols<128>(st + x * 32 * 128, n0 + n * 8, k0, lane));
-            sm_mma6(acc, n, a, b);
+            for (int y = 0; y < 2; ++y)
+#pragma unroll
+                for (int x = 0; x < 3; ++x)
+                    dec_ldsm4t(b[y][x][0], b[y][x][1], b[y][x][2], b[y][x][3], sm_b_cols<128>(st + x * 32 * 128, n0 + n * 8 + y * 16, k0, lane));
+            sm_mma6<2>(acc.v + n, a, b);
         }
     }
 }
@@ -211,10 +231,11 @@ __device__ __forceinline__ void sm_read_values(SmSum<8>& acc, const __nv_bfloat1
 #pragma unroll
         for (int x = 0; x < 3; ++x) dec_ldsm4(a[x][0], a[x][1], a[x][2], a[x][3], sm_a_rows<SM_L>(pt + x * SM_L * SM_L, r0, k0, lane));
 #pragma unroll
-        for (int n = 0; n < 8; n += 2) {
-            unsigned b[4];
-            dec_ldsm4t(b[0], b[1], b[2], b[3], sm_b_cols<128>(vt, n0 + n * 8, k0, lane));
-            sm_mma3(acc, n, a, b);
+        for (int n = 0; n < 8; n += 4) {
+            unsigned b[2][4];
+#pragma unroll
+            for (int y = 0; y < 2; ++y) dec_ldsm4t(b[y][0], b[y][1], b[y][2], b[y][3], sm_b_cols<128>(vt, n0 + n * 8 + y * 16, k0, lane));
+            sm_mma3<2>(acc.v + n, a, b);
         }
     }
 }
@@ -228,6 +249,27 @@ __device__ __forceinline__ void sm_stage_values(__nv_bfloat16* vt, const __nv_bf
         else *(uint4*)dst = make_uint4(0, 0, 0, 0);
     }
     dec_commit();
+}
+// `dim` columns (up to 128) of the piece's rows, times a factor, into pieces [SM_L][128]; zeros beyond n rows
+__device__ __forceinline__ void sm_stage_rows(__nv_bfloat16* t, const __nv_bfloat16* p, size_t stride, int n, int dim, float scale, int tid) {
+    const int groups = dim >> 3;
+    uint4 u[4];                                       // (up to 16 groups of 64 rows: all of them on their way at once)
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+        const int x = tid + y * 256, l = x / groups, c = x - l * groups;
+        u[y] = make_uint4(0, 0, 0, 0);
+        if (l < n && ZLM_CHK(p + (size_t)l * stride + c * 8, 16)) u[y] = *(const uint4*)(p + (size_t)l * stride + c * 8);
+    }
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+        const int x = tid + y * 256, l = x / groups, c = x - l * groups;
+        if (l >= SM_L) continue;
+        float f[8];
+        widen8(u[y], f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] *= scale;
+        split8(t, SM_L * 128, tile_off<128>(l, c), f);
+    }
 }
 
 // ---------------------------------------------------------------------------- what leaves the kernels of a piece
@@ -275,26 +317,38 @@ __device__ __forceinline__ void sm_write(const SmSum<8>& acc, float f0, float f8
         ss += __shfl_xor_sync(0xffffffffu, ss, 2);
         if ((lane & 3) == 0) red[r0 + (lane >> 2) + 8 * e][half] = ss;
     }
+    // the weights, then (once they have arrived) the gate's logits of a row into registers before anything is written where
+    // they stand: otherwise every exponential waits for the one before it (9,200 cycles of a block's 45,000)
+    float2 w[8];
+    if (out.w.p) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int at = (out.w_rows ? h * V : 0) + c + i * 8;
+            w[i] = c + i * 8 < V ? make_float2(out.w[at], out.w[at + 1]) : make_float2(0.f, 0.f);
+        }
+    }
     dec_wait<0>();
     __syncthreads();
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
         const int j = r0 + (lane >> 2) + 8 * e;
         const float f = (e ? f8 : f0) / sqrtf((red[j][0] + red[j][1]) / (float)V + out.eps);
+        unsigned z[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) z[i] = *(const unsigned*)(gt + tile_off<128>(j, half * 8 + i) + (lane & 3) * 2);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            if (c + i * 8 >= V) continue;
-            unsigned* at = (unsigned*)(gt + tile_off<128>(j, half * 8 + i) + (lane & 3) * 2);
-            const unsigned z = *at;
             float v[2];
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
-                const float zz = __uint_as_float(x ? z & 0xffff0000u : z << 16), sg = 1.0f / (1.0f + expf(-zz));
-                const float w = out.w.p ? out.w[(out.w_rows ? h * V : 0) + c + i * 8 + x] : 1.0f;
-                v[x] = acc.get(i, 2 * e + x) * f * w * (out.act == 1 ? zz * sg : sg);
+                const float zz = __uint_as_float(x ? z[i] & 0xffff0000u : z[i] << 16), sg = 1.0f / (1.0f + expf(-zz));
+                v[x] = acc.get(i, 2 * e + x) * f * (out.act == 1 ? zz * sg : sg);
+                if (out.w.p) v[x] *= x ? w[i].y : w[i].x;
             }
-            *at = pack_bf16(v[0], v[1]);
+            z[i] = pack_bf16(v[0], v[1]);
         }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) *(unsigned*)(gt + tile_off<128>(j, half * 8 + i) + (lane & 3) * 2) = z[i];
     }
     __syncthreads();
     for (int x = threadIdx.x; x < n * 16; x += 256) {
