@@ -79,3 +79,58 @@ def test_retention(H, D, V, n_rot, news, starts, table):
     z = gate.double()
     close(y, unit(want).flatten(1) * z * torch.sigmoid(z), 4e-3)
     close(state, S, 1e-6)
+
+
+@pytest.mark.parametrize("H,D,V,cap", [(2, 128, 128, 15.0), (3, 64, 72, 0.0), (1, 16, 8, 15.0), (2, 96, 136, 15.0)])
+@pytest.mark.parametrize("news,starts", [([64], [0]), ([65, 1, 130], [0, 5, 300]), ([17, 2], [9, 0])])
+@pytest.mark.parametrize("spread", [1.0, 8.0])
+def test_matrix_memory(H, D, V, cap, news, starts, spread):
+    """``spread``: the gates' logits times that: forget gates near 0 and 1, running maxima that jump.  Outputs are quotients
+    whose denominator is a sum of either sign: one that is a hundredth of its terms carries their roundings a hundredfold, and a
+    few of a head's 19 to 200 rows are like that (4e-6 over all rows; with gates spread wide one token decides a row: 1e-4)."""
+    from zlm_b200.kernels import get_kernels
+    k, plan = get_kernels(), plan_of(news, starts)
+    T = plan.T
+    gen = torch.Generator(device="cuda").manual_seed(D + V + T)
+
+    def rand(*shape):
+        return torch.randn(shape, generator=gen, device="cuda")
+    proj, z = rand(T, 2 * H * D + 2 * H * V).bfloat16(), rand(T, 2 * H) * spread
+    b_i, b_f = rand(H), rand(H) + 2
+    first = (rand(plan.R, H, D, V) * 0.3, rand(plan.R, H, D), rand(plan.R, H).abs())
+    q, key = (proj[:, i * H * D:(i + 1) * H * D].double().view(T, H, D) for i in (0, 1))
+    q = q * D ** -0.5
+    v = proj[:, 2 * H * D:2 * H * D + H * V].double().view(T, H, V)
+
+    def capped(x):
+        return cap * torch.tanh(x / cap) if cap else x
+    gi = capped(z[:, :H].double() + b_i.double())
+    gf = torch.nn.functional.logsigmoid(capped(z[:, H:].double() + b_f.double()))
+    want = torch.empty((T, H, V), dtype=torch.float64, device="cuda")
+    S, N, M = (t.double() for t in first)
+    at = 0
+    for r, n in enumerate(news):
+        s, nv, m = (t[plan.R - 1 - r] for t in (S, N, M))
+        for t in range(at, at + n):
+            new = torch.maximum(gf[t] + m, gi[t])
+            a, b = torch.exp(gf[t] + m - new), torch.exp(gi[t] - new)
+            s = a[:, None, None] * s + b[:, None, None] * key[t][:, :, None] * v[t][:, None]
+            nv, m = a[:, None] * nv + b[:, None] * key[t], new
+            want[t] = (s * q[t][:, :, None]).sum(1) / (torch.maximum((nv * q[t]).sum(1).abs(), torch.exp(-m)) + 1e-6)[:, None]
+        S[plan.R - 1 - r], N[plan.R - 1 - r], M[plan.R - 1 - r] = s, nv, m
+        at += n
+    gate = proj[:, 2 * H * D + H * V:]
+    for gated in (False, True):
+        state = tuple(t.clone() for t in first)
+        args = (proj, 0, H * D, 2 * H * D, z, 0, H, b_i, b_f, cap, state, plan, H, D, V, D ** -0.5)
+        o = torch.full((T, H * V), float("nan"), device="cuda")
+        if gated:
+            y = torch.full((T, H * V), float("nan"), device="cuda", dtype=torch.bfloat16)
+            w = torch.rand((H * V,), generator=gen, device="cuda") + 0.5
+            k.mlstm_gated(y, gate, w, 1e-6, o, *args)
+            close(y, unit(want).flatten(1) * w.double() * torch.sigmoid(gate.double()), 4e-3)
+        else:
+            k.mlstm(o, *args)
+            close(o, want.flatten(1), 4e-6 if spread == 1.0 else 1e-4)
+        for got, exact in zip(state, (S, N, M)):
+            close(got, exact, 1e-6)

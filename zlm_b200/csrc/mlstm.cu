@@ -17,7 +17,7 @@
 //   2. mlstm_chain   the pieces' states and maxima in order: the state ahead of every piece, and the sequence's new state
 //   3. mlstm_out     with M_j = max(m ahead, max_(l <= j) e_l), so that m_j = b_j + M_j:
 //                    o_j = (sum_(l <= j) exp(e_l - M_j) (q_j . k_l) v_l + exp(m ahead - M_j) S^T q_j) / ...
-#include "common.cuh"
+#include "split_mma.cuh"
 #include <cooperative_groups.h>
 namespace cg = cooperative_groups;
 
@@ -186,9 +186,10 @@ mlstm_step_kernel(TO* __restrict__ out, int out_stride, const TA* __restrict__ p
 }
 
 // ---------------------------------------------------------------------------- pieces of many tokens
-// What one warp works out about a piece: b (sums of log forget gates, inclusive) and e = i - b per token, in 64-bit, into
-// shared memory [ML_L] each; tokens from n on have f = 0 and e = -infinity.  Returns (b of the whole piece, the largest e).
-__device__ __forceinline__ double2 ml_piece_gates(const MlstmGates& gates, size_t row0, int n, int h, double* sb, double* se) {
+// What one warp works out about a piece, in 64-bit: b (sums of log forget gates, inclusive) and e = i - b of tokens 2 lane and
+// 2 lane + 1, b of the whole piece and the largest e; tokens from n on have f = 0 and e = -infinity.
+struct MlPieceGates { double b0, b1, e0, e1, total, top; };
+__device__ __forceinline__ MlPieceGates ml_piece_gates(const MlstmGates& gates, size_t row0, int n, int h) {
     const int lane = threadIdx.x & 31;
     float2 g[2];
 #pragma unroll
@@ -200,14 +201,29 @@ __device__ __forceinline__ double2 ml_piece_gates(const MlstmGates& gates, size_
         const double up = __shfl_up_sync(0xffffffffu, sum, o);
         if (lane >= o) sum += up;
     }
-    const double b0 = sum - (double)g[1].y, b1 = sum;
-    const double e0 = (double)g[0].x - b0, e1 = (double)g[1].x - b1;
-    sb[2 * lane] = b0; sb[2 * lane + 1] = b1;
-    se[2 * lane] = e0; se[2 * lane + 1] = e1;
+    MlPieceGates r;
+    r.b0 = sum - (double)g[1].y;
+    r.b1 = sum;
+    r.e0 = (double)g[0].x - r.b0;
+    r.e1 = (double)g[1].x - r.b1;
+    r.top = fmax(r.e0, r.e1);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) r.top = fmax(r.top, __shfl_xor_sync(0xffffffffu, r.top, o));
+    r.total = __shfl_sync(0xffffffffu, sum, 31);
+    return r;
+}
+// the running maximum of e and of the maximum ahead, for the lane's two tokens
+__device__ __forceinline__ double2 ml_running_max(double e0, double e1, double ahead) {
+    const int lane = threadIdx.x & 31;
     double mx = fmax(e0, e1);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    return make_double2(__shfl_sync(0xffffffffu, sum, 31), mx);
+    for (int x = 1; x < 32; x <<= 1) {
+        const double up = __shfl_up_sync(0xffffffffu, mx, x);
+        if (lane >= x) mx = fmax(mx, up);
+    }
+    double before = __shfl_up_sync(0xffffffffu, mx, 1);
+    before = lane ? fmax(before, ahead) : ahead;
+    return make_double2(fmax(before, e0), fmax(before, fmax(e0, e1)));
 }
 
 // eight neighbouring elements of a row, zeros where `ok` is false or beyond `left` of them
@@ -303,7 +319,7 @@ mlstm_piece_kernel(float* __restrict__ part, float* __restrict__ part_n, float2*
     extern __shared__ __align__(16) float ml_smem[];
     float* X = ml_smem;                          // [ML_L][ML_LD]: w_l k_l
     float* Y = X + ML_L * ML_LD;                   // [ML_L][ML_COLS]: v_l
-    __shared__ double sb[ML_L], se[ML_L], top;
+    __shared__ double se[ML_L], top;
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int d0 = blockIdx.y * 64, c0 = blockIdx.z * ML_COLS;
@@ -318,10 +334,12 @@ mlstm_piece_kernel(float* __restrict__ part, float* __restrict__ part_n, float2*
         ml_load8<TA>(proj + (size_t)(pc.row0 + l) * stride + k_off + (size_t)pc.h * D + d0 + d, D - d0 - d, l < pc.n, vec, fk[y]);
     }
     if (warp == 0) {
-        const double2 g = ml_piece_gates(gates, pc.row0, pc.n, pc.h, sb, se);
+        const MlPieceGates g = ml_piece_gates(gates, pc.row0, pc.n, pc.h);
+        se[2 * lane] = g.e0;
+        se[2 * lane + 1] = g.e1;
         if (lane == 0) {
-            top = g.y;
-            if (blockIdx.y == 0 && blockIdx.z == 0 && ZLM_CHK(part_m + pc.at, 8)) part_m[pc.at] = make_float2((float)g.x, (float)(g.x + g.y));
+            top = g.top;
+            if (blockIdx.y == 0 && blockIdx.z == 0 && ZLM_CHK(part_m + pc.at, 8)) part_m[pc.at] = make_float2((float)g.total, (float)(g.total + g.top));
         }
     }
     for (int x = tid; x < ML_L * (ML_COLS / 8); x += ML_THREADS) {
@@ -494,20 +512,11 @@ mlstm_out_kernel(float* __restrict__ o, const TA* __restrict__ proj, int stride,
     };
     fetch(0, 0);
     if (warp == 0) {
-        ml_piece_gates(gates, pc.row0, pc.n, pc.h, sb, se);
-        __syncwarp();
-        // M: the running maximum of e and of the maximum ahead
-        const double e0 = se[2 * lane], e1 = fmax(e0, se[2 * lane + 1]);
-        double mx = e1;
-#pragma unroll
-        for (int x = 1; x < 32; x <<= 1) {
-            const double up = __shfl_up_sync(0xffffffffu, mx, x);
-            if (lane >= x) mx = fmax(mx, up);
-        }
-        double before = __shfl_up_sync(0xffffffffu, mx, 1);
-        before = lane ? fmax(before, (double)ma.x) : (double)ma.x;
-        sm[2 * lane] = fmax(before, e0);
-        sm[2 * lane + 1] = fmax(before, e1);
+        const MlPieceGates g = ml_piece_gates(gates, pc.row0, pc.n, pc.h);
+        const double2 m = ml_running_max(g.e0, g.e1, (double)ma.x);
+        sb[2 * lane] = g.b0; sb[2 * lane + 1] = g.b1;
+        se[2 * lane] = g.e0; se[2 * lane + 1] = g.e1;
+        sm[2 * lane] = m.x; sm[2 * lane + 1] = m.y;
         // the sequence's new maximum, from its last piece
         if (lane == 0 && blockIdx.y == 0 && (pc.p + 1) * ML_L >= cu_seqlens[pc.r + 1] - cu_seqlens[pc.r]) {
             float* dst = mmax + (size_t)pc.slot * H + pc.h;
@@ -622,6 +631,129 @@ mlstm_out_kernel(float* __restrict__ o, const TA* __restrict__ proj, int stride,
     }
 }
 
+// ---------------------------------------------------------------------------- the outputs as tensor-core products
+// The third pass for bfloat16 projections and heads of up to 128 coordinates, every fp32 operand cut into three bfloat16
+// pieces (split_mma.cuh), the heads' norm and gate along with it.  3,001 tokens of four sequences, 16 heads of 128 x 128: 108 us
+// on the FFMA pipe (three shared-memory reads for 48 FMAs) and 28 us norm and gate, 94 us so; outputs 3.7e-7 off 64-bit
+// sums before, 2.1e-7 now.  (The first pass stays an FFMA chain: as products it took 37 instead of 58 us, but its states, which
+// exponential weights make the sum of a few last tokens, were 7e-8 off instead of 6e-8.)
+// grid (R * maxp * H, ceil(V / 128)); a warp owns 16 tokens and 64 value columns
+__global__ void __launch_bounds__(ML_THREADS, 2)
+mlstm_out_products_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, int stride, int q_off, int k_off, int v_off,
+                          MlstmGates gates, const float* __restrict__ part, const float* __restrict__ part_n,
+                          const float2* __restrict__ ahead, float* __restrict__ mmax, const int* __restrict__ seq_slot,
+                          const int* __restrict__ cu_seqlens, int H, int D, int V, int maxp, float q_scale) {
+    extern __shared__ __align__(128) __nv_bfloat16 ml_tiles[];
+    __nv_bfloat16* qt = ml_tiles;                    // [3][SM_L][128], later the gate's columns
+    __nv_bfloat16* kt = qt + 3 * SM_L * 128;         // [3][SM_L][128], later the weights and the state's rows:
+    __nv_bfloat16* pt = kt;                          // [3][SM_L][SM_L]
+    __nv_bfloat16* st = pt + 3 * SM_L * SM_L;        // [3][32][128]
+    __nv_bfloat16* vt = kt + 3 * SM_L * 128;         // [SM_L][128]
+    // (with the tiles this is all that two blocks an SM have room for: what comes later takes the place of what is read)
+    __shared__ __align__(16) double se[SM_L], sm[SM_L];
+    float* m_of = (float*)se;                        // [SM_L], after the weights
+    float (*sums)[2] = (float (*)[2])sm;             // [SM_L][2], after the weights; once more for the heads' norms
+    pdl_launch_dependents();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c0 = blockIdx.y * 128;
+    MlPiece pc;
+    pdl_wait();
+    if (!ml_piece(pc, blockIdx.x, H, maxp, seq_slot, cu_seqlens)) return;         // block-uniform
+    if (!ZLM_CHK(ahead + pc.at, 8)) return;
+    const float2 ma = ahead[pc.at];
+    const __nv_bfloat16* rows = proj + (size_t)pc.row0 * stride;
+    sm_stage_values(vt, rows + v_off + (size_t)pc.h * V, stride, pc.n, c0, V, tid);
+    float m0 = 0.f, m1 = 0.f;
+    if (warp == 0) {
+        const MlPieceGates g = ml_piece_gates(gates, pc.row0, pc.n, pc.h);
+        const double2 m = ml_running_max(g.e0, g.e1, (double)ma.x);
+        se[2 * lane] = g.e0; se[2 * lane + 1] = g.e1;
+        sm[2 * lane] = m.x; sm[2 * lane + 1] = m.y;
+        m0 = (float)(g.b0 + m.x);
+        m1 = (float)(g.b1 + m.y);
+        // the sequence's new maximum, from its last piece
+        if (lane == 0 && blockIdx.y == 0 && (pc.p + 1) * SM_L >= cu_seqlens[pc.r + 1] - cu_seqlens[pc.r]) {
+            float* dst = mmax + (size_t)pc.slot * H + pc.h;
+            if (ZLM_CHK(dst, 4)) *dst = ma.y;
+        }
+    }
+    sm_stage_rows(qt, rows + q_off + (size_t)pc.h * D, stride, pc.n, D, q_scale, tid);
+    sm_stage_rows(kt, rows + k_off + (size_t)pc.h * D, stride, pc.n, D, 1.f, tid);
+    const float* S = part + pc.at * D * V;
+    SmRows next = sm_fetch_state(S, 0, D, V, c0, tid);
+    const float* np = part_n + pc.at * D + lane * 4;
+    const float4 n_ahead = lane * 4 < D && ZLM_CHK(np, 16) ? *(const float4*)np : make_float4(0.f, 0.f, 0.f, 0.f);
+    dec_wait<0>();
+    __syncthreads();
+    const int r0 = (warp >> 1) * 16, half = warp & 1, j0 = r0 + (lane >> 2);
+    float s[4][4], keep[2], sum[2] = {0.f, 0.f};
+    {
+        SmSum<4> dots;
+        sm_scores(dots, qt, kt, r0, half * 32, D, lane);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            const int j = j0 + 8 * x;
+            const double M = sm[j];
+            keep[x] = expf((float)((double)ma.x - M));
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int l = half * 32 + i * 8 + (lane & 3) * 2 + e;
+                    s[i][2 * x + e] = (l <= j && l < pc.n) ? dots.get(i, 2 * x + e) * expf((float)(se[l] - M)) : 0.f;
+                    sum[x] += s[i][2 * x + e];
+                }
+            sum[x] += __shfl_xor_sync(0xffffffffu, sum[x], 1);
+            sum[x] += __shfl_xor_sync(0xffffffffu, sum[x], 2);
+        }
+    }
+    if (half == 0) {
+        // n ahead . q, two lanes a token (n from the lanes that hold it); then to the lanes that hold the token's sums
+        const int row = r0 + (lane >> 1);
+        float nq = 0.f;
+        for (int c = 0; c < D >> 3; c += 2) {
+            float f[3][8];
+#pragma unroll
+            for (int x = 0; x < 3; ++x) widen8(*(const uint4*)(qt + x * SM_L * 128 + tile_off<128>(row, c + (lane & 1))), f[x]);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float mine = (e & 3) == 0 ? n_ahead.x : (e & 3) == 1 ? n_ahead.y : (e & 3) == 2 ? n_ahead.z : n_ahead.w;
+                const float nv = __shfl_sync(0xffffffffu, mine, 2 * (c + (lane & 1)) + (e >> 2));
+                nq = fmaf(nv, f[0][e] + (f[1][e] + f[2][e]), nq);
+            }
+        }
+        nq += __shfl_xor_sync(0xffffffffu, nq, 1);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) sum[x] = fmaf(keep[x], __shfl_sync(0xffffffffu, nq, 2 * (lane >> 2) + 16 * x), sum[x]);
+    }
+    __syncthreads();                                 // (the keys, e and the maxima are read)
+    sm_put_weights(pt, s, r0, half * 32, lane);
+    if (warp == 0) { m_of[2 * lane] = m0; m_of[2 * lane + 1] = m1; }
+    if ((lane & 3) == 0) { sums[j0][half] = sum[0]; sums[j0 + 8][half] = sum[1]; }
+    SmSum<8> acc;
+    acc.zero();
+    for (int d0 = 0; d0 < D; d0 += 32) {
+        sm_put_state(st, next, tid);
+        if (d0 + 32 < D) next = sm_fetch_state(S, d0 + 32, D, V, c0, tid);
+        __syncthreads();
+        sm_read_state(acc, qt, st, r0, half * 64, d0, D, lane);
+        __syncthreads();
+    }
+    if (out.y) sm_stage_values(qt, out.g + (size_t)pc.row0 * out.g_stride + (size_t)pc.h * V, out.g_stride, pc.n, 0, V, tid);      // (the queries are read)
+    acc.scale(keep[0], keep[1]);
+    sm_read_values(acc, pt, vt, r0, half * 64, lane);
+    float inv[2];
+#pragma unroll
+    for (int x = 0; x < 2; ++x) inv[x] = 1.0f / ml_denominator(sums[j0 + 8 * x][0] + sums[j0 + 8 * x][1], m_of[j0 + 8 * x]);
+    __syncthreads();                                 // (the sums are read)
+    sm_write(acc, inv[0], inv[1], out, qt, sums, pc.row0, pc.n, pc.h, H, V, c0, r0, half, lane);
+}
+
+// what the tensor-core form takes: 16-byte reads of 8 neighbouring coordinates
+extern "C" int zlm_mlstm_products(int dtype, int stride, int q_off, int k_off, int v_off, int D, int V) {
+    return dtype == ZLM_DTYPE_BF16 && D > 0 && D % 16 == 0 && D <= 128 && V > 0 && V % 8 == 0 && stride % 8 == 0 && q_off % 8 == 0 &&
+           k_off % 8 == 0 && v_off % 8 == 0;
+}
+
 // ---------------------------------------------------------------------------- entry points
 static int mlstm_check(const float* z, int H, int D, int V, int R) {
     ZLM_REQUIRE(H > 0 && H <= 65535 && D > 0 && D <= 4096 && V > 0 && R > 0 && z, "mlstm: %d heads of %d key and %d value columns, %d sequences", H, D, V, R);
@@ -705,17 +837,31 @@ extern "C" int zlm_mlstm_step(void* out, int out_stride, int out_dtype, const vo
     ZLM_REQUIRE(false, "mlstm_step: unsupported dtypes %d, %d", dtype, out_dtype);
 }
 
+static void launch_chain(float* part, float* part_n, const float2* part_m, float2* ahead, float* S, float* n, const float* m,
+                         const int* seq_slot, const int* cu_seqlens, int R, int H, int D, int V, int maxp, cudaStream_t st) {
+    const long long DV = (long long)D * V;
+    if (DV % 4 == 0 && (uintptr_t)S % 16 == 0)
+        zlm_launch(mlstm_chain_kernel<4>, dim3(R * H, (unsigned)((DV + 511) / 512)), dim3(128), 0, st, part, part_n, part_m, ahead, S, n, m,
+                   seq_slot, cu_seqlens, H, D, V, maxp);
+    else
+        zlm_launch(mlstm_chain_kernel<1>, dim3(R * H, (unsigned)((DV + 127) / 128)), dim3(128), 0, st, part, part_n, part_m, ahead, S, n, m,
+                   seq_slot, cu_seqlens, H, D, V, maxp);
+}
+
 // floats of scratch that zlm_mlstm wants
 extern "C" long long zlm_mlstm_scratch(int R, int H, int D, int V, int max_new) {
     const long long maxp = (max_new + ML_L - 1) / ML_L;
     return (long long)R * maxp * H * ((long long)D * V + D + 4);
 }
 
-// Any number of tokens a sequence: as zlm_mlstm_step, without the norm and the gate; o [T][H * V] fp32.
+// Any number of tokens a sequence: as zlm_mlstm_step, without the norm and the gate; o [T][H * V] fp32.  y (null: none; where
+// zlm_mlstm_products says yes, heads of up to 128 value columns): [T][y_stride] bfloat16 receives, in the place of o, what
+// zlm_mlstm_step gives, with the gate's logits g [T][g_stride].
 extern "C" int zlm_mlstm(float* o, const void* proj, int stride, int dtype, int q_off, int k_off, int v_off, const float* z,
                          int z_stride, int i_off, int f_off, const void* bi, const void* bf, int b_dtype, float cap, float* S, float* n,
                          float* m, const int* seq_slot, const int* cu_seqlens, int T, int R, int H, int D, int V, float q_scale,
-                         int max_new, float* scratch, cudaStream_t st) {
+                         int max_new, float* scratch, void* y, int y_stride, const void* g, int g_stride, const void* w_norm, int w_dtype,
+                         float eps, cudaStream_t st) {
     if (T == 0) return ZLM_OK;
     if (int rc = mlstm_check(z, H, D, V, R)) return rc;
     ZLM_REQUIRE(max_new > 0 && scratch && (uintptr_t)scratch % 16 == 0, "mlstm: longest sequence %d", max_new);
@@ -734,6 +880,30 @@ extern "C" int zlm_mlstm(float* o, const void* proj, int stride, int dtype, int 
     const size_t smem1 = (size_t)ML_L * (ML_LD + ML_COLS) * sizeof(float);
     const size_t smem3 = (size_t)(2 * ML_KC * ML_LD + ML_L * ML_LD + 2 * ML_KC * ML_COLS) * sizeof(float);
     const dim3 g1((unsigned)units, (D + 63) / 64, (V + ML_COLS - 1) / ML_COLS), g3((unsigned)units, (V + ML_COLS - 1) / ML_COLS);
+    const bool products = zlm_mlstm_products(dtype, stride, q_off, k_off, v_off, D, V) && (uintptr_t)proj % 16 == 0 && (uintptr_t)o % 8 == 0;
+    ZLM_REQUIRE(!y || (products && V <= 128 && y_stride % 8 == 0 && g_stride % 8 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)g % 16 == 0),
+                "mlstm: heads of %d x %d do not take their gate along", D, V);
+    if (products) {
+        const size_t t3 = (size_t)7 * SM_L * 128 * sizeof(__nv_bfloat16);
+        static bool attr_set_dev[64] = {};
+        bool& attr_set = attr_set_dev[zlm_device_index()];
+        if (!attr_set) {
+            cudaError_t e1 = cudaFuncSetAttribute(mlstm_piece_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
+            cudaError_t e3 = cudaFuncSetAttribute(mlstm_out_products_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t3);
+            if (e1 != cudaSuccess || e3 != cudaSuccess) {
+                zlm_set_error("mlstm: cannot reserve shared memory");
+                return ZLM_ERR_CUDA;
+            }
+            attr_set = true;
+        }
+        zlm_launch(mlstm_piece_kernel<__nv_bfloat16>, g1, dim3(ML_THREADS), smem1, st, part, part_n, part_m, (const __nv_bfloat16*)proj,
+                   stride, k_off, v_off, gates, seq_slot, cu_seqlens, H, D, V, maxp, vec);
+        launch_chain(part, part_n, part_m, ahead, S, n, m, seq_slot, cu_seqlens, R, H, D, V, maxp, st);
+        const SmOut out{o, (__nv_bfloat16*)y, y_stride, (const __nv_bfloat16*)g, g_stride, VecW{w_norm, w_dtype}, 1, eps, 0};
+        zlm_launch(mlstm_out_products_kernel, g3, dim3(ML_THREADS), t3, st, out, (const __nv_bfloat16*)proj, stride, q_off, k_off, v_off,
+                   gates, (const float*)part, (const float*)part_n, (const float2*)ahead, m, seq_slot, cu_seqlens, H, D, V, maxp, q_scale);
+        return zlm_check_launch("mlstm_products");
+    }
 #define ZLM_ML_RUN(TA)                                                                                                          \
     do {                                                                                                                        \
         static bool attr_set_dev[64] = {};                                                                                      \
@@ -749,12 +919,7 @@ extern "C" int zlm_mlstm(float* o, const void* proj, int stride, int dtype, int 
         }                                                                                                                       \
         zlm_launch(mlstm_piece_kernel<TA>, g1, dim3(ML_THREADS), smem1, st, part, part_n, part_m, (const TA*)proj, stride, k_off, v_off, \
                    gates, seq_slot, cu_seqlens, H, D, V, maxp, vec);                                                            \
-        if (DV % 4 == 0 && (uintptr_t)S % 16 == 0)                                                                              \
-            zlm_launch(mlstm_chain_kernel<4>, dim3(R * H, (unsigned)((DV + 511) / 512)), dim3(128), 0, st, part, part_n,        \
-                       (const float2*)part_m, ahead, S, n, (const float*)m, seq_slot, cu_seqlens, H, D, V, maxp);              \
-        else                                                                                                                    \
-            zlm_launch(mlstm_chain_kernel<1>, dim3(R * H, (unsigned)((DV + 127) / 128)), dim3(128), 0, st, part, part_n,        \
-                       (const float2*)part_m, ahead, S, n, (const float*)m, seq_slot, cu_seqlens, H, D, V, maxp);              \
+        launch_chain(part, part_n, part_m, ahead, S, n, m, seq_slot, cu_seqlens, R, H, D, V, maxp, st);                         \
         zlm_launch(mlstm_out_kernel<TA>, g3, dim3(ML_THREADS), smem3, st, o, (const TA*)proj, stride, q_off, k_off, v_off, gates, \
                    (const float*)part, (const float*)part_n, (const float2*)ahead, m, seq_slot, cu_seqlens, H, D, V, maxp, q_scale, vec); \
     } while (0)

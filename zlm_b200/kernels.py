@@ -1101,7 +1101,7 @@ class CudaKernels:
 
     def mlstm(self, o: torch.Tensor, proj: torch.Tensor, q_off: int, k_off: int, v_off: int, z: torch.Tensor, i_off: int,
               f_off: int, b_i: Optional[torch.Tensor], b_f: Optional[torch.Tensor], cap: float, state, plan, heads: int,
-              dim: int, v_dim: int, q_scale: float) -> None:
+              dim: int, v_dim: int, q_scale: float, _gate: Optional[tuple] = None) -> None:
         """o [T, heads*v_dim] fp32: per head, with i = cap tanh((zi + b_i) / cap), f = log sigmoid(cap tanh((zf + b_f) / cap)),
         m_t = max(f + m_(t-1), i), S_t = exp(f + m_(t-1) - m_t) S_(t-1) + exp(i - m_t) k v^T and n_t likewise with k alone,
         o = S_t^T q / (max(|n_t . q|, exp(-m_t)) + 1e-6).  q (times ``q_scale``), k, v are columns of ``proj`` from q_off,
@@ -1114,11 +1114,31 @@ class CudaKernels:
         self.lib.zlm_mlstm_scratch.restype = ctypes.c_longlong
         part = plan.scratch("mlstm.pieces", (int(self.lib.zlm_mlstm_scratch(plan.R, heads, dim, v_dim, max_new)),), torch.float32)
         b = b_i if b_i is not None else b_f
+        y, g, w, eps = _gate if _gate is not None else (None, None, None, 0.0)
         self._call("zlm_mlstm", self._p(o), self._p(proj), c_int(proj.stride(0)), c_int(_dt(proj)), c_int(q_off), c_int(k_off),
                    c_int(v_off), self._p(z), c_int(z.stride(0)), c_int(i_off), c_int(f_off), self._p(b_i), self._p(b_f),
                    c_int(_dt(b) if b is not None else F32), c_float(cap), self._p(S), self._p(n), self._p(m),
                    self._p(plan.seq_slot), self._p(plan.cu_seqlens), c_int(T), c_int(plan.R), c_int(heads), c_int(dim),
-                   c_int(v_dim), c_float(q_scale), c_int(max_new), self._p(part), self._stream())
+                   c_int(v_dim), c_float(q_scale), c_int(max_new), self._p(part), self._p(y), c_int(y.stride(0) if y is not None else 0),
+                   self._p(g), c_int(g.stride(0) if g is not None else 0), self._p(w), c_int(_dt(w) if w is not None else F32),
+                   c_float(eps), self._stream())
+
+    def mlstm_gated(self, y: torch.Tensor, g: torch.Tensor, w_norm: torch.Tensor, eps: float, o: torch.Tensor, proj: torch.Tensor,
+                    q_off: int, k_off: int, v_off: int, z: torch.Tensor, i_off: int, f_off: int, b_i: Optional[torch.Tensor],
+                    b_f: Optional[torch.Tensor], cap: float, state, plan, heads: int, dim: int, v_dim: int, q_scale: float) -> None:
+        """``mlstm``, then ``norm_gate``: y [T, heads*v_dim] = o / rms(o, per head) * w_norm * sigmoid(g).  ``o`` is scratch
+        that bfloat16 heads of up to 128 columns do not touch (their last kernel writes y)."""
+        args = (proj, q_off, k_off, v_off, z, i_off, f_off, b_i, b_f, cap, state, plan, heads, dim, v_dim, q_scale)
+        if (y.dtype == g.dtype == torch.bfloat16 and v_dim <= 128 and y.stride(1) == g.stride(1) == 1
+                and (y.stride(0) | g.stride(0)) % 8 == 0 and (proj.data_ptr() | y.data_ptr() | g.data_ptr()) % 16 == 0
+                and self.lib.zlm_mlstm_products(c_int(_dt(proj)), c_int(proj.stride(0)), c_int(q_off), c_int(k_off), c_int(v_off),
+                                                c_int(dim), c_int(v_dim))):
+            assert y.shape == g.shape == (proj.shape[0], heads * v_dim)
+            assert w_norm.is_contiguous() and w_norm.numel() == heads * v_dim
+            self.mlstm(o, *args, _gate=(y, g, w_norm, eps))
+            return
+        self.mlstm(o, *args)
+        self.norm_gate(y, o, g, heads, v_dim, "head", w_norm, eps, "sigmoid")
 
     @staticmethod
     def _check_mlstm(proj, z, b_i, b_f, state, heads, dim, v_dim):

@@ -284,6 +284,5 @@ class MatrixLSTM(Mixer):
             k.mlstm_step(y[:, :VV], proj, q_off, k_off, v_off, g_off, *gates, self.w_norm, self.eps)
         else:
             o = rt.ws.get("mlstm.o", (T, VV), torch.float32)
-            k.mlstm(o, proj, q_off, k_off, v_off, *gates)
-            k.norm_gate(y[:, :VV], o, proj[:, g_off:g_off + VV], H, V, "head", self.w_norm, self.eps, "sigmoid")
+            k.mlstm_gated(y[:, :VV], proj[:, g_off:g_off + VV], self.w_norm, self.eps, o, proj, q_off, k_off, v_off, *gates)
         k.linear(residual, y, self.w_o, accumulate=True, defer=True)       # a norm reads the stream next

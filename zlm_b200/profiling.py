@@ -304,6 +304,13 @@ class ProfilingKernels:
         return self._timed("matrix memory prefill", n, 4.0 * T * heads * dim * v_dim, self.k.mlstm, o, proj, q_off, k_off, v_off, z,
                            i_off, f_off, b_i, b_f, cap, state, plan, heads, dim, v_dim, *args)
 
+    def mlstm_gated(self, y, g, w_norm, eps, o, proj, q_off, k_off, v_off, z, i_off, f_off, b_i, b_f, cap, state, plan, heads, dim,
+                    v_dim, *args):
+        T, el = proj.shape[0], proj.element_size()
+        n = T * heads * (2 * dim + v_dim) * el + 2 * _nbytes(y) + 2 * plan.R * heads * dim * v_dim * 4
+        return self._timed("matrix memory prefill, heads norm*gate", n, 4.0 * T * heads * dim * v_dim, self.k.mlstm_gated, y, g, w_norm,
+                           eps, o, proj, q_off, k_off, v_off, z, i_off, f_off, b_i, b_f, cap, state, plan, heads, dim, v_dim, *args)
+
     def mlstm_step(self, out, proj, q_off, k_off, v_off, g_off, z, i_off, f_off, b_i, b_f, cap, state, plan, heads, dim, v_dim, *args):
         T, el = proj.shape[0], proj.element_size()
         n = T * heads * 2 * (dim + v_dim) * el + _nbytes(out) + 2 * plan.R * heads * dim * v_dim * 4
