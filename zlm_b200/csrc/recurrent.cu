@@ -12,6 +12,8 @@
 // the state, the read-out) is fp32 in both element types.  A sequence's state is [slots][...] fp32 and is read at
 // a step's start and written at its end; nothing is special about a sequence's first token: its state is zero.
 #include "common.cuh"
+#include <cooperative_groups.h>
+namespace cg = cooperative_groups;
 
 #define RC_MAX_TAPS 8
 
@@ -450,6 +452,315 @@ extern "C" int zlm_rglru(void* out, int out_stride, float* u, void* u16, float* 
     else
         ZLM_REQUIRE(false, "rglru: unsupported dtype %d", dtype);
     return zlm_check_launch("rglru");
+}
+
+// ---------------------------------------------------------------------------- long bfloat16 prompts: three launches
+// (1) the convolution, in bfloat16 and block by block: u16 [blocks][Tp][bs], Tp = T rounded up to 128, so that (2) all
+// diagonal blocks' gate logits are one grouped product, z [blocks][Tp][2][bs] fp32; (3) the recurrence on thread-block
+// clusters in one pass over z and the two branches, with u formed again from the x branch (the same sum: the same bits) instead
+// of stored in fp32.  1,999 tokens of 2,048 channels in 8 blocks: convolution 37, eight products 45, three passes of the
+// recurrence 88 us before (u, z and the pieces' decays written and read by each); RG_NOW us now.
+
+// A thread: 8 neighbouring channels of RC_RUN tokens, each token's row of x read once for all its taps.
+#define RC_RUN 8
+template <int TAPS>
+__global__ void __launch_bounds__(128)
+rglru_conv_blocks_kernel(__nv_bfloat16* __restrict__ u16, int* __restrict__ group_of_tile, const __nv_bfloat16* __restrict__ proj,
+                         int proj_stride, int x_off, const __nv_bfloat16* __restrict__ bx, const __nv_bfloat16* __restrict__ conv_w,
+                         const __nv_bfloat16* __restrict__ cb, const float* __restrict__ state, const int* __restrict__ token_pos,
+                         const int* __restrict__ token_slot, const int* __restrict__ token_seq, const int* __restrict__ seq_start,
+                         int T, int Tp, int W, int bs, int blocks) {
+    pdl_trigger();
+    const int c = (blockIdx.y * 128 + threadIdx.x) * 8, t0 = blockIdx.x * RC_RUN;
+    float w[8][TAPS], b[8], bias[8];
+    if (c < W) {
+#pragma unroll
+        for (int v = 0; v < 8; ++v) {
+            b[v] = bx ? to_f32(bx[c + v]) : 0.f;
+            bias[v] = cb ? to_f32(cb[c + v]) : 0.f;
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j)
+                w[v][j] = ZLM_CHK(conv_w + (size_t)(c + v) * TAPS + j, 2) ? to_f32(conv_w[(size_t)(c + v) * TAPS + j]) : 0.f;
+        }
+    }
+    pdl_wait();
+    if (blockIdx.x == 0)                              // (for the product: which diagonal block a tile of 128 rows belongs to)
+        for (int x = blockIdx.y * 128 + threadIdx.x; x < blocks * (Tp / 128); x += gridDim.y * 128)
+            if (ZLM_CHK(group_of_tile + x, 4)) group_of_tile[x] = x / (Tp / 128);
+    if (c >= W) return;
+    uint4 x[RC_RUN + TAPS - 1];
+#pragma unroll
+    for (int j = 0; j < RC_RUN + TAPS - 1; ++j) {
+        const int t = t0 - (TAPS - 1) + j;
+        const __nv_bfloat16* p = proj + (size_t)t * proj_stride + x_off + c;
+        x[j] = (t >= 0 && t < T && ZLM_CHK(p, 16)) ? *(const uint4*)p : make_uint4(0, 0, 0, 0);
+    }
+    __nv_bfloat16* dst = u16 + ((size_t)(c / bs) * Tp + t0) * bs + c % bs;
+#pragma unroll
+    for (int k = 0; k < RC_RUN; ++k) {
+        const int t = t0 + k;
+        if (t >= T || !ZLM_CHK(token_pos + t, 4) || !ZLM_CHK(token_seq + t, 4) || !ZLM_CHK(token_slot + t, 4)) break;
+        const int pos = token_pos[t], i = pos - seq_start[token_seq[t]];
+        float a[8];
+#pragma unroll
+        for (int v = 0; v < 8; ++v) a[v] = bias[v];
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {
+            const int s = i - (TAPS - 1) + j;         // the tap's token among the sequence's tokens of this step
+            if (pos - (TAPS - 1) + j < 0) continue;   // before the sequence's start
+            float f[8];
+            if (s >= 0) {
+                const uint4 q = x[k + j];
+                f[0] = __uint_as_float(q.x << 16); f[1] = __uint_as_float(q.x & 0xffff0000u);
+                f[2] = __uint_as_float(q.y << 16); f[3] = __uint_as_float(q.y & 0xffff0000u);
+                f[4] = __uint_as_float(q.z << 16); f[5] = __uint_as_float(q.z & 0xffff0000u);
+                f[6] = __uint_as_float(q.w << 16); f[7] = __uint_as_float(q.w & 0xffff0000u);
+#pragma unroll
+                for (int v = 0; v < 8; ++v) f[v] += b[v];
+            } else {
+                const float* p = state + ((size_t)token_slot[t] * TAPS + (TAPS + s)) * W + c;
+                const bool ok = ZLM_CHK(p, 32);
+#pragma unroll
+                for (int v = 0; v < 8; ++v) f[v] = ok ? p[v] : 0.f;
+            }
+#pragma unroll
+            for (int v = 0; v < 8; ++v) a[v] = fmaf(w[v][j], f[v], a[v]);
+        }
+        unsigned h[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            const __nv_bfloat162 p = __floats2bfloat162_rn(a[2 * v], a[2 * v + 1]);
+            h[v] = *(const unsigned*)&p;
+        }
+        if (ZLM_CHK(dst + (size_t)k * bs, 16)) *(uint4*)(dst + (size_t)k * bs) = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+}
+
+// The recurrence's functions without branches, so that the numbers of a thread's tokens are worked out side by side (the
+// library's division, square root, expm1f and tanhf each branch for arguments that do not occur here: 62 us of the kernel
+// below with them, 55 us without).  To the last places of fp32: a reciprocal and a square root are a Newton step from the
+// approximate one, 1 - e^y is a series where it would cancel.  NaN stays NaN.
+__device__ __forceinline__ float rl_sigmoid(float x) {
+    const float e = expf(-x > 80.f ? 80.f : -x), d = 1.0f + e, r = __fdividef(1.0f, d);
+    return fmaf(r, fmaf(-d, r, 1.0f), r);
+}
+// 1 - e^y for y <= 0, a = e^(y/2)
+__device__ __forceinline__ float rl_one_minus_exp(float y, float a) {
+    float p = 1.0f / 479001600.0f;                   // sum of y^k / k!, k = 1 .. 12; y^13 / 13! is below 2^-32 on [-1, 0]
+    constexpr float c[11] = {1.0f / 39916800.0f, 1.0f / 3628800.0f, 1.0f / 362880.0f, 1.0f / 40320.0f, 1.0f / 5040.0f, 1.0f / 720.0f,
+                             1.0f / 120.0f, 1.0f / 24.0f, 1.0f / 6.0f, 0.5f, 1.0f};
+#pragma unroll
+    for (int k = 0; k < 11; ++k) p = fmaf(p, y, c[k]);
+    return y < -1.0f ? fmaf(-a, a, 1.0f) : -y * p;
+}
+__device__ __forceinline__ float rl_sqrt(float x) {
+    const float r = rsqrtf(x), s = x * r, q = fmaf(fmaf(-s, s, x), 0.5f * r, s);
+    return x < 1e-30f ? 0.f : q;                     // (what it multiplies is of the order of one; NaN is not below)
+}
+__device__ __forceinline__ void rl_ab(float zr, float zi, float u, float sl, float& a, float& b) {
+    const float log_a = -rl_sigmoid(zr) * sl;
+    a = expf(log_a);
+    b = rl_sqrt(rl_one_minus_exp(2.0f * log_a, a)) * rl_sigmoid(zi) * u;
+}
+// gelu_tanh as z sigmoid(2 t): 1 + tanh(t) = 2 sigmoid(2 t)
+__device__ __forceinline__ float rl_gelu(float z) { return z * rl_sigmoid(1.5957691216057308f * (z + 0.044715f * z * z * z)); }
+
+// A cluster of RL_CLUSTER blocks owns 64 channels of one sequence, a warp RL_P neighbouring tokens of two channels a lane, whose
+// decays and inputs it keeps in registers.  What a warp's tokens do to a state, S_out = A S_in + B, is folded over the block in
+// shared memory and over the cluster in distributed shared memory; then every warp knows the state it starts from and walks
+// its tokens.  Longer sequences go round again.  Bound by its exponentials and divisions (about 110 instructions a number).
+#define RL_CLUSTER 8
+#define RL_WARPS 8
+#define RL_P 8
+template <int TAPS>
+__global__ void __cluster_dims__(RL_CLUSTER, 1, 1) __launch_bounds__(RL_WARPS * 32, 2)
+rglru_cluster_kernel(__nv_bfloat16* __restrict__ out, int out_stride, const float* __restrict__ z, const __nv_bfloat16* __restrict__ proj,
+                     int proj_stride, int x_off, int y_off, const __nv_bfloat16* __restrict__ bx, const __nv_bfloat16* __restrict__ by,
+                     const __nv_bfloat16* __restrict__ conv_w, const __nv_bfloat16* __restrict__ cb, const __nv_bfloat16* __restrict__ cr,
+                     const __nv_bfloat16* __restrict__ ci, const __nv_bfloat16* __restrict__ lam, float c_decay,
+                     float* __restrict__ state, const int* __restrict__ seq_slot, const int* __restrict__ seq_start,
+                     const int* __restrict__ cu_seqlens, int Tp, int W, int bs, float out_scale) {
+    // two sets, for rounds in turn: a block that is a round ahead does not overwrite what another still reads
+    __shared__ float2 piece[2][RL_WARPS][64];
+    __shared__ float2 total[2][64];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank(), r = blockIdx.x / RL_CLUSTER;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.y * 64 + lane * 2;
+    pdl_trigger();
+    bool live = c < W;                               // (no thread leaves early: the cluster meets at barriers)
+    float w[2][TAPS], xb[2], ub[2], yb[2], rb[2], ib[2], sl[2], S0[2] = {0.f, 0.f};
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+        xb[v] = (live && bx) ? to_f32(bx[c + v]) : 0.f;
+        ub[v] = (live && cb) ? to_f32(cb[c + v]) : 0.f;
+        yb[v] = (live && by) ? to_f32(by[c + v]) : 0.f;
+        rb[v] = (live && cr) ? to_f32(cr[c + v]) : 0.f;
+        ib[v] = (live && ci) ? to_f32(ci[c + v]) : 0.f;
+        sl[v] = live ? softplus_f(to_f32(lam[c + v])) * c_decay : 0.f;
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) w[v][j] = live ? to_f32(conv_w[(size_t)(c + v) * TAPS + j]) : 0.f;
+    }
+    pdl_wait();
+    int row0 = 0, n = 0, slot = 0, start = 0;
+    if (ZLM_CHK(seq_slot + r, 4) && ZLM_CHK(cu_seqlens + r, 8) && ZLM_CHK(seq_start + r, 4)) {
+        row0 = cu_seqlens[r];
+        n = cu_seqlens[r + 1] - row0;
+        slot = seq_slot[r];
+        start = seq_start[r];
+    }
+    float* sp = state + (size_t)slot * TAPS * W + c;
+    live = live && ZLM_CHK(sp, 8);
+    if (live) { S0[0] = sp[0]; S0[1] = sp[1]; }
+    const float* zp = z + ((size_t)(c / bs) * Tp + row0) * 2 * bs + c % bs;
+    int par = 0;
+    for (int base = 0; base < n; base += RL_CLUSTER * RL_WARPS * RL_P, par ^= 1) {
+        const int lo = base + (rank * RL_WARPS + warp) * RL_P, cnt = live ? min(n - lo, RL_P) : 0;
+        float2 zr[RL_P], zi[RL_P];
+        unsigned xr[RL_P + TAPS - 1], yr[RL_P];
+#pragma unroll
+        for (int j = 0; j < RL_P; ++j) {
+            const float* q = zp + (size_t)(lo + j) * 2 * bs;
+            const bool ok = j < cnt && ZLM_CHK(q, 8) && ZLM_CHK(q + bs, 8);
+            zr[j] = ok ? *(const float2*)q : make_float2(0.f, 0.f);
+            zi[j] = ok ? *(const float2*)(q + bs) : make_float2(0.f, 0.f);
+        }
+#pragma unroll
+        for (int j = 0; j < RL_P + TAPS - 1; ++j) {
+            const int i = lo - (TAPS - 1) + j;
+            const __nv_bfloat16* q = proj + (size_t)(row0 + i) * proj_stride + x_off + c;
+            xr[j] = (live && i >= 0 && i < n && ZLM_CHK(q, 4)) ? *(const unsigned*)q : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < RL_P; ++j) {
+            const __nv_bfloat16* q = proj + (size_t)(row0 + lo + j) * proj_stride + y_off + c;
+            yr[j] = (j < cnt && ZLM_CHK(q, 4)) ? *(const unsigned*)q : 0u;
+        }
+        float A[2] = {1.f, 1.f}, B[2] = {0.f, 0.f};
+#pragma unroll
+        for (int j = 0; j < RL_P; ++j) {
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                float u = ub[v];
+#pragma unroll
+                for (int k = 0; k < TAPS; ++k) {
+                    const int i = lo + j - (TAPS - 1) + k;
+                    if (start + i < 0) continue;
+                    float x;
+                    if (i >= 0) x = __uint_as_float(v ? xr[j + k] & 0xffff0000u : xr[j + k] << 16) + xb[v];
+                    else x = (j < cnt && ZLM_CHK(sp + (size_t)(TAPS + i) * W + v, 4)) ? sp[(size_t)(TAPS + i) * W + v] : 0.f;
+                    u = fmaf(w[v][k], x, u);
+                }
+                float a, b;
+                rl_ab((v ? zr[j].y : zr[j].x) + rb[v], (v ? zi[j].y : zi[j].x) + ib[v], u, sl[v], a, b);
+                if (v) { zr[j].y = a; zi[j].y = b; } else { zr[j].x = a; zi[j].x = b; }
+                if (j < cnt) {
+                    A[v] *= a;
+                    B[v] = fmaf(a, B[v], b);
+                }
+            }
+        }
+#pragma unroll
+        for (int v = 0; v < 2; ++v) piece[par][warp][lane * 2 + v] = make_float2(A[v], B[v]);
+        __syncthreads();
+        if (warp == 0)
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                float2 t = piece[par][0][lane * 2 + v];
+                for (int x = 1; x < RL_WARPS; ++x) {
+                    const float2 q = piece[par][x][lane * 2 + v];
+                    t = make_float2(q.x * t.x, fmaf(q.x, t.y, q.y));
+                }
+                total[par][lane * 2 + v] = t;
+            }
+        cluster.sync();
+        // the state this warp's tokens start from, and the one the whole round ends with
+        float S[2];
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+            float2 t[RL_CLUSTER];
+#pragma unroll
+            for (int k = 0; k < RL_CLUSTER; ++k) t[k] = cluster.map_shared_rank(&total[par][0], k)[lane * 2 + v];
+            float q = S0[v];
+            S[v] = q;
+#pragma unroll
+            for (int k = 0; k < RL_CLUSTER; ++k) {
+                q = fmaf(t[k].x, q, t[k].y);
+                if (k + 1 == rank) S[v] = q;
+            }
+            S0[v] = q;
+            for (int x = 0; x < warp; ++x) {
+                const float2 p = piece[par][x][lane * 2 + v];
+                S[v] = fmaf(p.x, S[v], p.y);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < RL_P; ++j) {
+            if (j >= cnt) break;
+            S[0] = fmaf(zr[j].x, S[0], zi[j].x);
+            S[1] = fmaf(zr[j].y, S[1], zi[j].y);
+            const float y0 = S[0] * rl_gelu(__uint_as_float(yr[j] << 16) + yb[0]) * out_scale;
+            const float y1 = S[1] * rl_gelu(__uint_as_float(yr[j] & 0xffff0000u) + yb[1]) * out_scale;
+            __nv_bfloat16* o = out + (size_t)(row0 + lo + j) * out_stride + c;
+            if (ZLM_CHK(o, 4)) *(__nv_bfloat162*)o = __floats2bfloat162_rn(y0, y1);
+        }
+    }
+    // (every block has read the old state ahead of the first barrier, and its older inputs only this warp has read)
+    if (live && rank == 0 && warp == 0)
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+            sp[v] = S0[v];
+            rglru_keep_inputs<__nv_bfloat16>(sp + v, proj, proj_stride, x_off, c + v, row0, n, W, TAPS, xb[v]);
+        }
+    cluster.sync();                                  // no block leaves while another may still read its shared memory
+}
+
+// bfloat16, with everything as in zlm_rglru: the first of the three launches.  u16 [blocks][Tp][W/blocks], Tp = T rounded up to
+// 128; group_of_tile [blocks * Tp / 128] for zlm_gemm_tc_grouped.
+extern "C" int zlm_rglru_conv_blocks(void* u16, int* group_of_tile, const void* proj, int proj_stride, int x_off, const void* bx,
+                                     const void* conv_w, const void* cb, const float* state, const int* token_pos,
+                                     const int* token_slot, const int* token_seq, const int* seq_start, int T, int W, int blocks, int taps,
+                                     cudaStream_t st) {
+    if (T == 0) return ZLM_OK;
+    ZLM_REQUIRE(W > 0 && blocks > 0 && W % blocks == 0 && (W / blocks) % 8 == 0, "rglru: %d channels in %d blocks", W, blocks);
+    ZLM_REQUIRE(taps >= 1 && taps <= RC_MAX_TAPS, "rglru: %d taps (at most %d)", taps, RC_MAX_TAPS);
+    ZLM_REQUIRE(proj_stride % 8 == 0 && x_off % 8 == 0 && (uintptr_t)proj % 16 == 0 && (uintptr_t)u16 % 16 == 0 && (W + 1023) / 1024 <= 65535,
+                "rglru: rows of %d from column %d", proj_stride, x_off);
+    const int Tp = (T + 127) / 128 * 128;
+    const dim3 grid((T + RC_RUN - 1) / RC_RUN, (W + 1023) / 1024);
+#define ZLM_RC(N)                                                                                                               \
+    case N:                                                                                                                     \
+        zlm_launch(rglru_conv_blocks_kernel<N>, grid, dim3(128), 0, st, (__nv_bfloat16*)u16, group_of_tile, (const __nv_bfloat16*)proj, \
+                   proj_stride, x_off, (const __nv_bfloat16*)bx, (const __nv_bfloat16*)conv_w, (const __nv_bfloat16*)cb, state, token_pos, \
+                   token_slot, token_seq, seq_start, T, Tp, W, W / blocks, blocks);                                            \
+        break;
+    switch (taps) { ZLM_RC(1) ZLM_RC(2) ZLM_RC(3) ZLM_RC(4) ZLM_RC(5) ZLM_RC(6) ZLM_RC(7) ZLM_RC(8) }
+#undef ZLM_RC
+    return zlm_check_launch("rglru_conv_blocks");
+}
+
+// The third: z [blocks][Tp][2][W/blocks] fp32 holds the gates' logits without their biases.
+extern "C" int zlm_rglru_cluster(void* out, int out_stride, const float* z, const void* proj, int proj_stride, int x_off, int y_off,
+                                 const void* bx, const void* by, const void* conv_w, const void* cb, const void* cr, const void* ci,
+                                 const void* lam, float c_decay, float* state, const int* seq_slot, const int* seq_start,
+                                 const int* cu_seqlens, int T, int R, int W, int blocks, int taps, float out_scale, cudaStream_t st) {
+    if (T == 0) return ZLM_OK;
+    ZLM_REQUIRE(W > 0 && blocks > 0 && W % blocks == 0 && (W / blocks) % 8 == 0, "rglru: %d channels in %d blocks", W, blocks);
+    ZLM_REQUIRE(taps >= 1 && taps <= RC_MAX_TAPS, "rglru: %d taps (at most %d)", taps, RC_MAX_TAPS);
+    ZLM_REQUIRE(proj_stride % 2 == 0 && x_off % 2 == 0 && y_off % 2 == 0 && out_stride % 2 == 0 && (uintptr_t)proj % 4 == 0 &&
+                    (uintptr_t)out % 4 == 0 && (uintptr_t)z % 8 == 0 && (W + 63) / 64 <= 65535 && R > 0 && R <= (1 << 27),
+                "rglru: rows of %d and %d, %d sequences", proj_stride, out_stride, R);
+    const int Tp = (T + 127) / 128 * 128;
+    const dim3 grid(R * RL_CLUSTER, (W + 63) / 64);
+#define ZLM_RL(N)                                                                                                               \
+    case N:                                                                                                                     \
+        zlm_launch(rglru_cluster_kernel<N>, grid, dim3(RL_WARPS * 32), 0, st, (__nv_bfloat16*)out, out_stride, z,               \
+                   (const __nv_bfloat16*)proj, proj_stride, x_off, y_off, (const __nv_bfloat16*)bx, (const __nv_bfloat16*)by,   \
+                   (const __nv_bfloat16*)conv_w, (const __nv_bfloat16*)cb, (const __nv_bfloat16*)cr, (const __nv_bfloat16*)ci,  \
+                   (const __nv_bfloat16*)lam, c_decay, state, seq_slot, seq_start, cu_seqlens, Tp, W, W / blocks, out_scale);   \
+        break;
+    switch (taps) { ZLM_RL(1) ZLM_RL(2) ZLM_RL(3) ZLM_RL(4) ZLM_RL(5) ZLM_RL(6) ZLM_RL(7) ZLM_RL(8) }
+#undef ZLM_RL
+    return zlm_check_launch("rglru_cluster");
 }
 
 // ---------------------------------------------------------------------------- decays from a low-rank projection

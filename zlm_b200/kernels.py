@@ -1021,11 +1021,32 @@ class CudaKernels:
             assert m.shape == (blocks, bs, bs) and m.is_contiguous() and m.dtype == dt
         for v in (bx, by, conv_b, c_r, c_i, lam):
             assert v is None or (v.numel() == W and v.is_contiguous() and v.dtype == dt)
-        u = plan.scratch("rglru.u", (T, W), torch.float32)
-        z = plan.scratch("rglru.z", (T, blocks, 2 * bs), torch.float32)
         max_new = int(getattr(plan, "max_new", 0) or 0)
         if pieces is None:
             pieces = max_new >= self.RECURRENT_PIECES_FROM
+        if (pieces and gates is not None and dt == torch.bfloat16 and T > 16 and bs % 8 == 0 and x_off % 8 == 0 and y_off % 2 == 0
+                and proj.stride(0) % 8 == 0 and out.stride(0) % 2 == 0 and proj.data_ptr() % 16 == 0 and gates.data_ptr() % 16 == 0
+                and out.data_ptr() % 4 == 0):
+            # three launches: the convolution, all blocks' gate logits as one grouped product, the recurrence on clusters
+            assert gates.shape == (blocks, 2 * bs, bs) and gates.is_contiguous() and gates.dtype == dt
+            Tp = -(-T // 128) * 128
+            u16 = plan.scratch("rglru.u16", (blocks, Tp, bs), dt)
+            z = plan.scratch("rglru.z", (blocks * Tp, 2 * bs), torch.float32)
+            tiles = plan.scratch("rglru.tiles", (blocks * Tp // 128,), torch.int32)
+            self._call("zlm_rglru_conv_blocks", self._p(u16), self._p(tiles), self._p(proj), c_int(proj.stride(0)), c_int(x_off),
+                       self._p(bx), self._p(conv_w), self._p(conv_b), self._p(state), self._p(plan.token_pos),
+                       self._p(plan.token_slot), self._p(plan.token_seq), self._p(plan.seq_start), c_int(T), c_int(W),
+                       c_int(blocks), c_int(taps), self._stream())
+            self._call("zlm_gemm_tc_grouped", self._p(z), self._p(u16), self._p(gates), self._p(tiles), c_int(blocks * Tp // 128),
+                       c_int(blocks), c_int(2 * bs), c_int(bs), c_int(2 * bs), c_int(STORE_F32), self._stream())
+            self._call("zlm_rglru_cluster", self._p(out), c_int(out.stride(0)), self._p(z), self._p(proj), c_int(proj.stride(0)),
+                       c_int(x_off), c_int(y_off), self._p(bx), self._p(by), self._p(conv_w), self._p(conv_b), self._p(c_r),
+                       self._p(c_i), self._p(lam), c_float(c_decay), self._p(state), self._p(plan.seq_slot),
+                       self._p(plan.seq_start), self._p(plan.cu_seqlens), c_int(T), c_int(plan.R), c_int(W), c_int(blocks),
+                       c_int(taps), c_float(out_scale), self._stream())
+            return
+        u = plan.scratch("rglru.u", (T, W), torch.float32)
+        z = plan.scratch("rglru.z", (T, blocks, 2 * bs), torch.float32)
         part = None
         if pieces:
             maxp = (max_new + self.RECURRENT_PIECE - 1) // self.RECURRENT_PIECE
