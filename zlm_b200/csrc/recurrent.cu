@@ -459,7 +459,7 @@ extern "C" int zlm_rglru(void* out, int out_stride, float* u, void* u16, float* 
 // diagonal blocks' gate logits are one grouped product, z [blocks][Tp][2][bs] fp32; (3) the recurrence on thread-block
 // clusters in one pass over z and the two branches, with u formed again from the x branch (the same sum: the same bits) instead
 // of stored in fp32.  1,999 tokens of 2,048 channels in 8 blocks: convolution 37, eight products 45, three passes of the
-// recurrence 88 us before (u, z and the pieces' decays written and read by each); RG_NOW us now.
+// recurrence 88 us before (u, z and the pieces' decays written and read by each); 11, 25 and 38 us now.
 
 // A thread: 8 neighbouring channels of RC_RUN tokens, each token's row of x read once for all its taps.
 #define RC_RUN 8
@@ -583,6 +583,7 @@ rglru_cluster_kernel(__nv_bfloat16* __restrict__ out, int out_stride, const floa
     // two sets, for rounds in turn: a block that is a round ahead does not overwrite what another still reads
     __shared__ float2 piece[2][RL_WARPS][64];
     __shared__ float2 total[2][64];
+    __shared__ float begin[RL_WARPS][64];
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank(), r = blockIdx.x / RL_CLUSTER;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.y * 64 + lane * 2;
@@ -635,23 +636,46 @@ rglru_cluster_kernel(__nv_bfloat16* __restrict__ out, int out_stride, const floa
             const __nv_bfloat16* q = proj + (size_t)(row0 + lo + j) * proj_stride + y_off + c;
             yr[j] = (j < cnt && ZLM_CHK(q, 4)) ? *(const unsigned*)q : 0u;
         }
+        float u[RL_P][2];
+        if (lo >= TAPS - 1) {                        // (every tap of every token is one of the step's)
+            float x[2][RL_P + TAPS - 1];
+#pragma unroll
+            for (int j = 0; j < RL_P + TAPS - 1; ++j) {
+                x[0][j] = __uint_as_float(xr[j] << 16) + xb[0];
+                x[1][j] = __uint_as_float(xr[j] & 0xffff0000u) + xb[1];
+            }
+#pragma unroll
+            for (int j = 0; j < RL_P; ++j)
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    u[j][v] = ub[v];
+#pragma unroll
+                    for (int k = 0; k < TAPS; ++k) u[j][v] = fmaf(w[v][k], x[v][j + k], u[j][v]);
+                }
+        } else {
+#pragma unroll
+            for (int j = 0; j < RL_P; ++j)
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    u[j][v] = ub[v];
+#pragma unroll
+                    for (int k = 0; k < TAPS; ++k) {
+                        const int i = lo + j - (TAPS - 1) + k;
+                        if (start + i < 0) continue;
+                        float x;
+                        if (i >= 0) x = __uint_as_float(v ? xr[j + k] & 0xffff0000u : xr[j + k] << 16) + xb[v];
+                        else x = (j < cnt && ZLM_CHK(sp + (size_t)(TAPS + i) * W + v, 4)) ? sp[(size_t)(TAPS + i) * W + v] : 0.f;
+                        u[j][v] = fmaf(w[v][k], x, u[j][v]);
+                    }
+                }
+        }
         float A[2] = {1.f, 1.f}, B[2] = {0.f, 0.f};
 #pragma unroll
         for (int j = 0; j < RL_P; ++j) {
 #pragma unroll
             for (int v = 0; v < 2; ++v) {
-                float u = ub[v];
-#pragma unroll
-                for (int k = 0; k < TAPS; ++k) {
-                    const int i = lo + j - (TAPS - 1) + k;
-                    if (start + i < 0) continue;
-                    float x;
-                    if (i >= 0) x = __uint_as_float(v ? xr[j + k] & 0xffff0000u : xr[j + k] << 16) + xb[v];
-                    else x = (j < cnt && ZLM_CHK(sp + (size_t)(TAPS + i) * W + v, 4)) ? sp[(size_t)(TAPS + i) * W + v] : 0.f;
-                    u = fmaf(w[v][k], x, u);
-                }
                 float a, b;
-                rl_ab((v ? zr[j].y : zr[j].x) + rb[v], (v ? zi[j].y : zi[j].x) + ib[v], u, sl[v], a, b);
+                rl_ab((v ? zr[j].y : zr[j].x) + rb[v], (v ? zi[j].y : zi[j].x) + ib[v], u[j][v], sl[v], a, b);
                 if (v) { zr[j].y = a; zi[j].y = b; } else { zr[j].x = a; zi[j].x = b; }
                 if (j < cnt) {
                     A[v] *= a;
@@ -673,26 +697,29 @@ rglru_cluster_kernel(__nv_bfloat16* __restrict__ out, int out_stride, const floa
                 total[par][lane * 2 + v] = t;
             }
         cluster.sync();
-        // the state this warp's tokens start from, and the one the whole round ends with
-        float S[2];
+        // the states that the block's warps start from, and the one the whole round ends with
+        if (warp == 0)
 #pragma unroll
-        for (int v = 0; v < 2; ++v) {
-            float2 t[RL_CLUSTER];
+            for (int v = 0; v < 2; ++v) {
+                float2 t[RL_CLUSTER];
 #pragma unroll
-            for (int k = 0; k < RL_CLUSTER; ++k) t[k] = cluster.map_shared_rank(&total[par][0], k)[lane * 2 + v];
-            float q = S0[v];
-            S[v] = q;
+                for (int k = 0; k < RL_CLUSTER; ++k) t[k] = cluster.map_shared_rank(&total[par][0], k)[lane * 2 + v];
+                float q = S0[v], s = q;
 #pragma unroll
-            for (int k = 0; k < RL_CLUSTER; ++k) {
-                q = fmaf(t[k].x, q, t[k].y);
-                if (k + 1 == rank) S[v] = q;
+                for (int k = 0; k < RL_CLUSTER; ++k) {
+                    q = fmaf(t[k].x, q, t[k].y);
+                    if (k + 1 == rank) s = q;
+                }
+                S0[v] = q;
+#pragma unroll
+                for (int x = 0; x < RL_WARPS; ++x) {
+                    begin[x][lane * 2 + v] = s;
+                    const float2 p = piece[par][x][lane * 2 + v];
+                    s = fmaf(p.x, s, p.y);
+                }
             }
-            S0[v] = q;
-            for (int x = 0; x < warp; ++x) {
-                const float2 p = piece[par][x][lane * 2 + v];
-                S[v] = fmaf(p.x, S[v], p.y);
-            }
-        }
+        __syncthreads();
+        float S[2] = {begin[warp][lane * 2], begin[warp][lane * 2 + 1]};
 #pragma unroll
         for (int j = 0; j < RL_P; ++j) {
             if (j >= cnt) break;
