@@ -124,6 +124,93 @@ conv_norm_write_kernel(TA* __restrict__ q_out, int q_out_stride, const TA* __res
     }
 }
 
+// The same for steps of many tokens and heads of up to 128 columns: a warp takes one head of SC_RUN neighbouring tokens, so that
+// a row of the projection is read once for all its taps and a lane's taps once for all its tokens (the kernel above reads
+// both for every token: 16 taps and four rows of 8 bytes for four outputs).  The same sums in the same order.  2,999 tokens of
+// 16 + 2 x 4 heads of 128 columns, 4 taps: 47 us above, 25 us here; 2,048 of 32 + 2 x 8: 62 and 31.
+#define SC_RUN 8
+template <typename TA, int TAPS>
+__global__ void __launch_bounds__(SC_WARPS * 32)
+conv_norm_write_run_kernel(TA* __restrict__ q_out, int q_out_stride, const TA* __restrict__ proj, int proj_stride,
+                           const TA* __restrict__ conv_w, const TA* __restrict__ state, const int* __restrict__ token_pos,
+                           const int* __restrict__ token_slot, const int* __restrict__ token_seq, const int* __restrict__ seq_start,
+                           const int* __restrict__ block_table, int table_stride, TA* __restrict__ pool, int T, int nq, int nkv,
+                           int dim, int vdim, int hdp, int norm, float eps) {
+    struct alignas(4 * sizeof(TA)) Raw { TA v[4]; };
+    pdl_trigger();
+    const int t0 = blockIdx.x * SC_RUN, lane = threadIdx.x & 31, unit = blockIdx.y * SC_WARPS + (threadIdx.x >> 5);
+    if (unit >= nq + 2 * nkv) return;
+    const int C = (nq + nkv) * dim + nkv * vdim;
+    const int kind = unit < nq ? 0 : (unit < nq + nkv ? 1 : 2);
+    const int width = kind == 2 ? vdim : dim, e = lane * 4;
+    const int c = (kind == 0 ? unit * dim : (kind == 1 ? nq * dim + (unit - nq) * dim : (nq + nkv) * dim + (unit - nq - nkv) * vdim)) + e;
+    float w[4][TAPS];
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j)
+            w[v][j] = (e < width && ZLM_CHK(conv_w + (size_t)(c + v) * TAPS + j, sizeof(TA))) ? to_f32(conv_w[(size_t)(c + v) * TAPS + j]) : 0.f;
+    pdl_wait();
+    Raw x[SC_RUN + TAPS - 1];
+#pragma unroll
+    for (int j = 0; j < SC_RUN + TAPS - 1; ++j) {
+        const int t = t0 - (TAPS - 1) + j;
+        const TA* p = proj + (size_t)t * proj_stride + c;
+        if (e < width && t >= 0 && t < T && ZLM_CHK(p, sizeof(Raw))) x[j] = *(const Raw*)p;
+        else memset(&x[j], 0, sizeof(Raw));
+    }
+#pragma unroll
+    for (int k = 0; k < SC_RUN; ++k) {
+        const int t = t0 + k;
+        if (t >= T || !ZLM_CHK(token_pos + t, 4) || !ZLM_CHK(token_slot + t, 4) || !ZLM_CHK(token_seq + t, 4)) break;
+        const int pos = token_pos[t], slot = token_slot[t], i = pos - seq_start[token_seq[t]];
+        float val[4] = {0.f, 0.f, 0.f, 0.f};
+        if (i >= TAPS - 1) {                         // (every tap is one of the step's tokens; the same answer for the whole warp)
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j)
+#pragma unroll
+                for (int v = 0; v < 4; ++v) val[v] = fmaf(w[v][j], to_f32(x[k + j].v[v]), val[v]);
+        } else if (e < width) {
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) {
+                const int s = i - (TAPS - 1) + j;
+                if (pos - (TAPS - 1) + j < 0) continue;               // before the sequence's start
+                const TA* up = state + ((size_t)slot * (TAPS - 1) + (TAPS - 1 + s)) * C + c;
+                float f[4];
+#pragma unroll
+                for (int v = 0; v < 4; ++v) f[v] = to_f32(x[k + j].v[v]);
+                if (s < 0) {
+                    if (!ZLM_CHK(up, sizeof(Raw))) continue;
+                    load_vec<TA, 4>(up, f);
+                }
+#pragma unroll
+                for (int v = 0; v < 4; ++v) val[v] = fmaf(w[v][j], f[v], val[v]);
+            }
+        }
+        float scale = 1.0f;
+        if (norm && kind != 2) {
+            float ss = 0.f;
+#pragma unroll
+            for (int v = 0; v < 4; ++v) ss = fmaf(val[v], val[v], ss);
+            scale = 1.0f / sqrtf(warp_sum(ss) / (float)width + eps);
+        }
+        TA* dst;
+        if (kind == 0) {
+            dst = q_out + (size_t)t * q_out_stride + (size_t)unit * hdp;
+        } else {
+            if (!ZLM_CHK(block_table + (size_t)slot * table_stride + pos / ZLM_PAGE, 4)) continue;
+            const int page = block_table[(size_t)slot * table_stride + pos / ZLM_PAGE];
+            const int kvh = kind == 1 ? unit - nq : unit - nq - nkv;
+            dst = pool + (((size_t)page * 2 + (kind - 1)) * nkv + kvh) * ZLM_PAGE * hdp + (size_t)(pos % ZLM_PAGE) * hdp;
+        }
+        if (e >= hdp || !ZLM_CHK(dst + e, sizeof(Raw))) continue;
+        float o[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) o[v] = e < width ? val[v] * scale : 0.f;
+        store_vec<TA, 4>(dst + e, o);
+    }
+}
+
 // state[slot][m] <- the (taps-1) newest projected values of the sequence after this step, m = taps-2 the newest
 template <typename TA>
 __global__ void __launch_bounds__(256)
@@ -160,7 +247,18 @@ static void launch_conv(void* q_out, int q_out_stride, const void* proj, int pro
     const bool vec = dim % 4 == 0 && vdim % 4 == 0 && hdp % 4 == 0 && proj_stride % 4 == 0 && q_out_stride % 4 == 0 && C0 % 4 == 0 &&
                      (uintptr_t)proj % al == 0 && (uintptr_t)q_out % al == 0 && (uintptr_t)pool % al == 0 &&
                      (state == nullptr || (uintptr_t)state % al == 0);
-    if (vec)
+    // (a run of tokens a warp from 256 tokens on: below that a token a warp leaves more of them to run: 16 + 2 x 4 heads at 256 tokens 9.4 us a token a warp, 8.4 so, at 128 7.0 and 7.1)
+    if (vec && hdp <= 128 && taps >= 2 && taps <= 5 && T >= 256) {
+        const dim3 grid((T + SC_RUN - 1) / SC_RUN, (units + SC_WARPS - 1) / SC_WARPS);
+#define ZLM_SC(N)                                                                                                               \
+    case N:                                                                                                                     \
+        zlm_launch(conv_norm_write_run_kernel<TA, N>, grid, dim3(SC_WARPS * 32), 0, st, (TA*)q_out, q_out_stride, (const TA*)proj, \
+                   proj_stride, (const TA*)conv_w, (const TA*)state, token_pos, token_slot, token_seq, seq_start, block_table,  \
+                   table_stride, (TA*)pool, T, nq, nkv, dim, vdim, hdp, norm, eps);                                             \
+        break;
+        switch (taps) { ZLM_SC(2) ZLM_SC(3) ZLM_SC(4) ZLM_SC(5) }
+#undef ZLM_SC
+    } else if (vec)
         zlm_launch(conv_norm_write_kernel<TA, 4>, dim3(T, (units + SC_WARPS - 1) / SC_WARPS), dim3(SC_WARPS * 32), 0, st,
                    (TA*)q_out, q_out_stride, (const TA*)proj, proj_stride, (const TA*)conv_w, (const TA*)state, token_pos,
                    token_slot, token_seq, seq_start, cu_seqlens, block_table, table_stride, (TA*)pool, nq, nkv, dim, vdim, hdp,
