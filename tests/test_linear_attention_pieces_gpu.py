@@ -1,0 +1,50 @@
+"""Linear attention with decays per channel or per head over prompts in pieces, alone and with the heads' norm and gate, beside
+a 64-bit walk: lengths around a piece's edges, key widths around the kernels' 32, 64 and 128 rows, value widths that are no
+multiple of four or wider than a block, states carried in.
+
+Bounds.  Sums of some ten to hundred fp32 products, 2^-24 of each: 1e-6 of the norm; gated outputs are rounded to their type."""
+import pytest
+import torch
+
+from test_piece_products_gpu import close, plan_of, unit
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,D,V", [(2, 64, 128), (3, 20, 72), (1, 128, 30), (2, 33, 136)])
+@pytest.mark.parametrize("news,starts", [([128], [0]), ([129, 1, 33], [0, 5, 300]), ([31, 200], [9, 0])])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("per_head", [False, True])
+def test_pieces(H, D, V, news, starts, dtype, per_head):
+    from zlm_b200.kernels import get_kernels
+    k, plan = get_kernels(), plan_of(news, starts)
+    T = plan.T
+    gen = torch.Generator(device="cuda").manual_seed(D + V + T)
+    proj = torch.randn((T, 2 * H * D + 2 * H * V + 3), generator=gen, device="cuda").to(dtype)
+    # decays from almost nothing kept to almost everything
+    alpha = torch.sigmoid(torch.randn((T, H * D), generator=gen, device="cuda") * 4)
+    head = torch.linspace(0.5, 0.99, H, device="cuda")
+    first = torch.randn((plan.R, H, D, V), generator=gen, device="cuda")
+    q, key = (proj[:, i * H * D:(i + 1) * H * D].double().view(T, H, D) for i in (0, 1))
+    v = proj[:, 2 * H * D:2 * H * D + H * V].double().view(T, H, V)
+    a = head.double()[:, None].expand(T, H, D) if per_head else alpha.double().view(T, H, D)
+    want, S = torch.empty((T, H, V), dtype=torch.float64, device="cuda"), first.double()
+    at = 0
+    for r, n in enumerate(news):
+        s = S[plan.R - 1 - r]
+        for t in range(at, at + n):
+            s = a[t][:, :, None] * s + key[t][:, :, None] * v[t][:, None]
+            want[t] = (s * q[t][:, :, None]).sum(1) * 0.3
+        S[plan.R - 1 - r] = s
+        at += n
+    args = (proj, 0, H * D, 2 * H * D, None if per_head else alpha, head if per_head else None)
+    state, o = first.clone(), torch.full((T, H * V), float("nan"), device="cuda")
+    k.linear_attention(o, *args, state, plan, H, D, V, 0.3)
+    close(o, want.flatten(1), 1e-6)
+    close(state, S, 1e-6)
+    gate, w = proj[:, 2 * H * D + H * V:2 * H * D + 2 * H * V], torch.rand((V,), generator=gen, device="cuda") + 0.5
+    state, y = first.clone(), torch.full((T, H * V), float("nan"), device="cuda", dtype=dtype)
+    k.linear_attention_gated(y, gate, w, 1e-6, "silu", o, *args, state, plan, H, D, V, 0.3)
+    z = gate.double()
+    close(y, (unit(want) * w.double()).flatten(1) * z * torch.sigmoid(z), 4e-3 if dtype == torch.bfloat16 else 2e-6)
+    close(state, S, 1e-6)

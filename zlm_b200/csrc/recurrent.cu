@@ -848,50 +848,64 @@ extern "C" int zlm_lowrank_decay(float* alpha, const void* proj, int proj_stride
 }
 
 // ---------------------------------------------------------------------------- linear attention with decays per channel
-// A block: one head of one sequence (or of one piece of a sequence) and up to 128 value columns; a thread owns one
-// column of the state, DR rows in registers (rows from `dim` on stay zero).  The tokens are staged LA_CH at a time in
-// shared memory as fp32: q (scaled), k, the decays, v.  o [T][H*V] fp32.
+// A block: one head of one sequence (or of one piece of a sequence) and 512 / DS value columns, DS = DR / DPT.  A thread owns
+// DPT rows of four columns of the state in registers (rows from `dim` on stay zero), two rows a packed instruction, so that a
+// number of q, k or the decays read from shared memory serves four columns; the DS lanes that share columns add their parts of
+// an output by shuffles, dealing the columns out.  Tokens are staged LA_CH at a time as fp32: q (scaled), k, the decays, v.
 //   MODE 0: a sequence's tokens in order, from and to the sequence's state.
 //   MODE 1: a piece of L tokens from a zero state; leaves the piece's outputs, the state it ends with (part) and the
-//           product of its decays per key channel (pdecay): S_out = diag(pdecay) S_in + part.
-//   MODE 2: the piece again from the state it really starts with (part, after the chain), without keys and values:
-//           o_t += (diag(alpha_lo .. alpha_t) S_in)^T q_t.
+//           product of its decays per key channel (pdecay): S_out = diag(pdecay) S_in + part.  o [T][H*V] fp32.
+// Bound by the packed FMAs and, with one column a thread, by shared-memory reads before: 2,048 tokens of 8 heads of 64 x 128 in
+// pieces 37 us with a column a thread (62 with two threads a column), 32 us so.
 #define LA_CH 16
-template <typename TA, int DR, int MODE>
-__global__ void __launch_bounds__(128)
+#define LA_CPT 4
+template <typename TA, int DR, int DPT, int MODE>
+__global__ void __launch_bounds__(128, DR == 128 ? 4 : 5)
 linear_attention_kernel(float* __restrict__ o, const TA* __restrict__ proj, int proj_stride, int q_off, int k_off, int v_off,
                         const float* __restrict__ alpha, const float* __restrict__ head_decay, float* __restrict__ state,
                         const int* __restrict__ seq_slot, const int* __restrict__ cu_seqlens, int H, int D, int V,
                         float q_scale, float* __restrict__ part, float* __restrict__ pdecay, int maxp, int L) {
-    __shared__ __align__(16) float sq[LA_CH][DR], sk[LA_CH][DR], sa[LA_CH][DR];
-    __shared__ float sv[LA_CH][128];
+    constexpr int DS = DR / DPT, COLS = 128 / DS * LA_CPT, SEG = DPT + 4, DP = DS * SEG;      // (segments in different banks)
+    static_assert(DS == 4 || DS == 8, "the sums below deal four columns out to four lanes or eight");
+    __shared__ __align__(16) float sq[LA_CH][DP], sk[LA_CH][DP], sa[LA_CH][DP];
+    __shared__ __align__(16) float sv[LA_CH][COLS];
     pdl_trigger();
-    const int unit = blockIdx.x / H, h = blockIdx.x % H, v0 = blockIdx.y * 128, tid = threadIdx.x;
+    const int unit = blockIdx.x / H, h = blockIdx.x % H, v0 = blockIdx.y * COLS, tid = threadIdx.x;
     const int r = MODE == 0 ? unit : unit / maxp, p = MODE == 0 ? 0 : unit % maxp;
-    const int v = v0 + tid;
+    const int grp = tid / DS, lane_d = tid % DS, v = v0 + grp * LA_CPT;
     pdl_wait();
     if (!ZLM_CHK(seq_slot + r, 4) || !ZLM_CHK(cu_seqlens + r, 8)) return;
     const int slot = seq_slot[r], row0 = cu_seqlens[r], n = cu_seqlens[r + 1] - row0;
     const int lo = MODE == 0 ? 0 : p * L, hi = MODE == 0 ? n : min(n, lo + L);
     if (lo >= hi) return;
-    float* sp = MODE == 0 ? state + (((size_t)slot * H + h) * D) * V + v
-                          : part + ((((size_t)r * maxp + p) * H + h) * D) * V + v;
-    float S[DR];
+    float* sp = (MODE == 0 ? state + (((size_t)slot * H + h) * D) * V : part + ((((size_t)r * maxp + p) * H + h) * D) * V) + v;
+    float2 S[DPT / 2][LA_CPT];
 #pragma unroll
-    for (int d = 0; d < DR; ++d)
-        S[d] = (MODE != 1 && d < D && v < V && ZLM_CHK(sp + (size_t)d * V, 4)) ? sp[(size_t)d * V] : 0.f;
+    for (int j = 0; j < DPT / 2; ++j)
+#pragma unroll
+        for (int c = 0; c < LA_CPT; ++c) {
+            float t[2] = {0.f, 0.f};
+            if (MODE == 0)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int d = lane_d * DPT + 2 * j + e;
+                    if (d < D && v + c < V && ZLM_CHK(sp + (size_t)d * V + c, 4)) t[e] = sp[(size_t)d * V + c];
+                }
+            S[j][c] = make_float2(t[0], t[1]);
+        }
     const float hd = head_decay ? head_decay[h] : 1.0f;
     float pd = 1.0f;                              // MODE 1: the product of the piece's decays of key channel `tid`
     for (int s0 = lo; s0 < hi; s0 += LA_CH) {
         const int m = min(LA_CH, hi - s0);
         __syncthreads();
+#pragma unroll 4
         for (int x = tid; x < LA_CH * DR; x += 128) {
-            const int j = x / DR, d = x % DR;
+            const int j = x / DR, d = x % DR, at = (d / DPT) * SEG + d % DPT;
             float fq = 0.f, fk = 0.f, fa = 1.f;
             if (j < m && d < D) {
                 const TA* row = proj + (size_t)(row0 + s0 + j) * proj_stride;
                 if (ZLM_CHK(row + q_off + h * D + d, sizeof(TA))) fq = to_f32(row[q_off + h * D + d]) * q_scale;
-                if (MODE != 2 && ZLM_CHK(row + k_off + h * D + d, sizeof(TA))) fk = to_f32(row[k_off + h * D + d]);
+                if (ZLM_CHK(row + k_off + h * D + d, sizeof(TA))) fk = to_f32(row[k_off + h * D + d]);
                 if (alpha) {
                     const float* ap = alpha + ((size_t)(row0 + s0 + j) * H + h) * D + d;
                     if (ZLM_CHK(ap, 4)) fa = *ap;
@@ -899,51 +913,71 @@ linear_attention_kernel(float* __restrict__ o, const TA* __restrict__ proj, int 
                     fa = hd;
                 }
             }
-            sq[j][d] = fq; sk[j][d] = fk; sa[j][d] = fa;
+            sq[j][at] = fq; sk[j][at] = fk; sa[j][at] = fa;
         }
-        if (MODE != 2) {
-            for (int x = tid; x < LA_CH * 128; x += 128) {
-                const int j = x / 128, e = x % 128;
-                float fv = 0.f;
-                if (j < m && v0 + e < V) {
-                    const TA* pv = proj + (size_t)(row0 + s0 + j) * proj_stride + v_off + h * V + v0 + e;
-                    if (ZLM_CHK(pv, sizeof(TA))) fv = to_f32(*pv);
-                }
-                sv[j][e] = fv;
+#pragma unroll 8
+        for (int x = tid; x < LA_CH * COLS; x += 128) {
+            const int j = x / COLS, e = x % COLS;
+            float fv = 0.f;
+            if (j < m && v0 + e < V) {
+                const TA* pv = proj + (size_t)(row0 + s0 + j) * proj_stride + v_off + h * V + v0 + e;
+                if (ZLM_CHK(pv, sizeof(TA))) fv = to_f32(*pv);
             }
+            sv[j][e] = fv;
         }
         __syncthreads();
         if (MODE == 1 && tid < DR)
-            for (int j = 0; j < m; ++j) pd *= sa[j][tid];
+            for (int j = 0; j < m; ++j) pd *= sa[j][(tid / DPT) * SEG + tid % DPT];
         for (int j = 0; j < m; ++j) {
-            const float vv = MODE == 2 ? 0.f : sv[j][tid];
-            float c0 = 0.f, c1 = 0.f, c2 = 0.f, c3 = 0.f;         // four sums side by side (always added in this order)
+            const float4 v4 = *(const float4*)&sv[j][grp * LA_CPT];
+            const float2 vv[LA_CPT] = {make_float2(v4.x, v4.x), make_float2(v4.y, v4.y), make_float2(v4.z, v4.z), make_float2(v4.w, v4.w)};
+            float2 acc2[LA_CPT];
 #pragma unroll
-            for (int d = 0; d < DR; d += 4) {
-                const float4 a4 = *(const float4*)&sa[j][d], q4 = *(const float4*)&sq[j][d];
-                if (MODE == 2) {
-                    S[d] *= a4.x;     c0 = fmaf(S[d], q4.x, c0);
-                    S[d + 1] *= a4.y; c1 = fmaf(S[d + 1], q4.y, c1);
-                    S[d + 2] *= a4.z; c2 = fmaf(S[d + 2], q4.z, c2);
-                    S[d + 3] *= a4.w; c3 = fmaf(S[d + 3], q4.w, c3);
-                } else {
-                    const float4 k4 = *(const float4*)&sk[j][d];
-                    S[d] = fmaf(a4.x, S[d], k4.x * vv);         c0 = fmaf(S[d], q4.x, c0);
-                    S[d + 1] = fmaf(a4.y, S[d + 1], k4.y * vv); c1 = fmaf(S[d + 1], q4.y, c1);
-                    S[d + 2] = fmaf(a4.z, S[d + 2], k4.z * vv); c2 = fmaf(S[d + 2], q4.z, c2);
-                    S[d + 3] = fmaf(a4.w, S[d + 3], k4.w * vv); c3 = fmaf(S[d + 3], q4.w, c3);
-                }
+            for (int c = 0; c < LA_CPT; ++c) acc2[c] = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int d = 0; d < DPT; d += 4) {
+                const int at = lane_d * SEG + d;
+                const float4 a4 = *(const float4*)&sa[j][at], q4 = *(const float4*)&sq[j][at], k4 = *(const float4*)&sk[j][at];
+                const float2 a2[2] = {make_float2(a4.x, a4.y), make_float2(a4.z, a4.w)}, q2[2] = {make_float2(q4.x, q4.y), make_float2(q4.z, q4.w)},
+                             k2[2] = {make_float2(k4.x, k4.y), make_float2(k4.z, k4.w)};
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+#pragma unroll
+                    for (int c = 0; c < LA_CPT; ++c) {
+                        S[d / 2 + e][c] = __ffma2_rn(a2[e], S[d / 2 + e][c], __fmul2_rn(k2[e], vv[c]));
+                        acc2[c] = __ffma2_rn(S[d / 2 + e][c], q2[e], acc2[c]);
+                    }
             }
-            const float acc = (c0 + c1) + (c2 + c3);
-            float* op = o + ((size_t)(row0 + s0 + j) * H + h) * V + v;
-            if (v < V && ZLM_CHK(op, 4)) *op = MODE == 2 ? *op + acc : acc;
+            float acc[LA_CPT];
+#pragma unroll
+            for (int c = 0; c < LA_CPT; ++c) acc[c] = acc2[c].x + acc2[c].y;
+            // half of the lanes go on with columns 0-1, half with 2-3, then one column each
+            const bool up = (lane_d & (DS >> 1)) != 0, up2 = (lane_d & (DS >> 2)) != 0;
+            const float r0 = __shfl_xor_sync(0xffffffffu, up ? acc[0] : acc[2], DS >> 1), r1 = __shfl_xor_sync(0xffffffffu, up ? acc[1] : acc[3], DS >> 1);
+            const float b0 = (up ? acc[2] : acc[0]) + r0, b1 = (up ? acc[3] : acc[1]) + r1;
+            float sum = (up2 ? b1 : b0) + __shfl_xor_sync(0xffffffffu, up2 ? b0 : b1, DS >> 2);
+            if (DS == 8) sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            const int mine = (up ? 2 : 0) + (up2 ? 1 : 0);
+            float* op = o + ((size_t)(row0 + s0 + j) * H + h) * V + v + mine;
+            if ((DS == 4 || (lane_d & 1) == 0) && v + mine < V && ZLM_CHK(op, 4)) *op = sum;
         }
     }
-    if (MODE != 2 && v < V) {
 #pragma unroll
-        for (int d = 0; d < DR; ++d)
-            if (d < D && ZLM_CHK(sp + (size_t)d * V, 4)) sp[(size_t)d * V] = S[d];
-    }
+    for (int j = 0; j < DPT / 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int d = lane_d * DPT + 2 * j + e;
+            float* dst = sp + (size_t)d * V;
+            if (d >= D) continue;
+            const float t[LA_CPT] = {e ? S[j][0].y : S[j][0].x, e ? S[j][1].y : S[j][1].x, e ? S[j][2].y : S[j][2].x, e ? S[j][3].y : S[j][3].x};
+            if (V % 4 == 0 && v < V && (uintptr_t)dst % 16 == 0 && ZLM_CHK(dst, 16)) {
+                *(float4*)dst = make_float4(t[0], t[1], t[2], t[3]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < LA_CPT; ++c)
+                    if (v + c < V && ZLM_CHK(dst + c, 4)) dst[c] = t[c];
+            }
+        }
     if (MODE == 1 && blockIdx.y == 0 && tid < D) {
         float* pp = pdecay + (((size_t)r * maxp + p) * H + h) * D + tid;
         if (ZLM_CHK(pp, 4)) *pp = pd;
@@ -951,73 +985,275 @@ linear_attention_kernel(float* __restrict__ o, const TA* __restrict__ proj, int 
 }
 
 // The pieces' states in order: part[piece] becomes the state the piece starts from, the sequence's state is left.
-// (a thread owns one number of the state; eight pieces' loads in flight)
+// (a thread owns VEC neighbouring numbers of one row of the state; eight pieces' loads in flight.)  grid (R * H, ceil(D * V / (128 VEC)))
 #define CHAIN_AHEAD 8
+template <int VEC>
 __global__ void __launch_bounds__(128)
 linear_attention_chain_kernel(float* __restrict__ part, const float* __restrict__ pdecay, float* __restrict__ state,
                               const int* __restrict__ seq_slot, const int* __restrict__ cu_seqlens, int H, int D, int V,
                               int maxp, int L) {
+    struct alignas(4 * VEC) Num { float v[VEC]; };
     pdl_trigger();
-    const int d = blockIdx.x % D, rh = blockIdx.x / D, r = rh / H, h = rh % H, v = blockIdx.y * 128 + threadIdx.x;
+    const int rh = blockIdx.x, r = rh / H, h = rh % H, e = (blockIdx.y * 128 + threadIdx.x) * VEC, d = e / V;
     pdl_wait();
-    if (v >= V || !ZLM_CHK(seq_slot + r, 4) || !ZLM_CHK(cu_seqlens + r, 8)) return;
+    if (e >= D * V || !ZLM_CHK(seq_slot + r, 4) || !ZLM_CHK(cu_seqlens + r, 8)) return;
     const int slot = seq_slot[r], n = cu_seqlens[r + 1] - cu_seqlens[r];
     const int np = (n + L - 1) / L;
-    float* sp = state + (((size_t)slot * H + h) * D + d) * V + v;
-    if (!ZLM_CHK(sp, 4)) return;
-    float S = *sp;
+    Num* sp = (Num*)(state + ((size_t)slot * H + h) * D * V + e);
+    if (!ZLM_CHK(sp, 4 * VEC)) return;
+    Num S = *sp;
     const size_t pstride = (size_t)H * D * V, dstride = (size_t)H * D;
-    float* pp = part + (((size_t)r * maxp * H + h) * D + d) * V + v;
+    float* pp = part + ((size_t)r * maxp * H + h) * D * V + e;
     const float* dp = pdecay + ((size_t)r * maxp * H + h) * D + d;
-    for (int p0 = 0; p0 < np; p0 += CHAIN_AHEAD) {
-        float A[CHAIN_AHEAD], g[CHAIN_AHEAD];
+    for (int p0 = 0; p0 < np; p0 += CHAIN_AHEAD, pp += CHAIN_AHEAD * pstride, dp += CHAIN_AHEAD * dstride) {
+        Num A[CHAIN_AHEAD];
+        float g[CHAIN_AHEAD];
 #pragma unroll
         for (int j = 0; j < CHAIN_AHEAD; ++j) {
-            const bool ok = p0 + j < np && ZLM_CHK(pp + (p0 + j) * pstride, 4) && ZLM_CHK(dp + (p0 + j) * dstride, 4);
-            A[j] = ok ? pp[(p0 + j) * pstride] : 0.f;
-            g[j] = ok ? dp[(p0 + j) * dstride] : 1.f;
+            g[j] = 1.f;
+            memset(&A[j], 0, sizeof(Num));
+            if (p0 + j < np && ZLM_CHK(pp + j * pstride, 4 * VEC) && ZLM_CHK(dp + j * dstride, 4)) {
+                A[j] = *(const Num*)(pp + j * pstride);
+                g[j] = dp[j * dstride];
+            }
         }
 #pragma unroll
         for (int j = 0; j < CHAIN_AHEAD; ++j) {
             if (p0 + j >= np) break;
-            if (ZLM_CHK(pp + (p0 + j) * pstride, 4)) pp[(p0 + j) * pstride] = S;
-            S = fmaf(g[j], S, A[j]);
+            if (ZLM_CHK(pp + j * pstride, 4 * VEC)) *(Num*)(pp + j * pstride) = S;
+#pragma unroll
+            for (int x = 0; x < VEC; ++x) S.v[x] = fmaf(g[j], S.v[x], A[j].v[x]);
         }
     }
     *sp = S;
 }
 
+// What the state ahead of a piece gives its tokens, as a product: o_t += S_in^T (diag(alpha_lo .. alpha_t) q_t), 32 tokens by 128
+// columns a block, a warp eight tokens, a lane four columns of each.  With y (heads of up to 128 columns) the outputs go on to
+// what follows them in the mixer: every head divided by its root mean square, times a weight, times the gate.
+// 2,048 tokens of 8 heads of 64 x 128: walked token by token 27 us, and 18 us for norm and gate; 19 us so, about 5 more with both.
 #define LA_PIECE 32
+#define LA_LD (LA_PIECE + 4)
+struct LaOut {
+    void* y;                         // null: o
+    int y_stride;
+    const void* g;
+    int g_stride;
+    VecW w;                          // [V]
+    float eps;
+    int act;                         // 1: silu, 0: sigmoid
+};
+template <typename TA, int DR>
+__global__ void __launch_bounds__(128, DR == 128 ? 2 : 4)
+linear_attention_out_kernel(float* __restrict__ o, const TA* __restrict__ proj, int proj_stride, int q_off,
+                            const float* __restrict__ alpha, const float* __restrict__ head_decay, const float* __restrict__ part,
+                            const int* __restrict__ cu_seqlens, int H, int D, int V, float q_scale, int maxp, LaOut out) {
+    struct alignas(4 * sizeof(TA)) Four { TA v[4]; };
+    extern __shared__ __align__(16) float la_smem[];
+    float* S = la_smem;                              // [DR][128]
+    float* Q = S + DR * 128;                         // [DR][LA_LD]: the decayed queries, tokens innermost
+    pdl_trigger();
+    const int unit = blockIdx.x / H, h = blockIdx.x % H, v0 = blockIdx.y * 128, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int r = unit / maxp, p = unit % maxp;
+    pdl_wait();
+    if (!ZLM_CHK(cu_seqlens + r, 8)) return;
+    const int row0 = cu_seqlens[r] + p * LA_PIECE, m = min(LA_PIECE, cu_seqlens[r + 1] - row0);
+    if (m <= 0) return;
+    const float* src = part + ((((size_t)r * maxp + p) * H + h) * D) * V + v0;
+    const bool vec = V % 4 == 0 && (uintptr_t)part % 16 == 0;
+    for (int x = tid; x < D * 32; x += 128) {
+        const int d = x >> 5, c = (x & 31) * 4;
+        const float* q = src + (size_t)d * V + c;
+        float* dst = S + d * 128 + c;
+        if (vec && v0 + c < V && ZLM_CHK(q, 16)) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(q));
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) dst[e] = (v0 + c + e < V && ZLM_CHK(q + e, 4)) ? q[e] : 0.f;
+        }
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+    if (tid < D) {
+        const float hd = head_decay ? head_decay[h] : 1.0f;
+        float pd = 1.0f;
+#pragma unroll 16
+        for (int j = 0; j < LA_PIECE; ++j) {
+            const TA* q = proj + (size_t)(row0 + j) * proj_stride + q_off + h * D + tid;
+            const float* a = alpha + ((size_t)(row0 + j) * H + h) * D + tid;
+            const bool ok = j < m && ZLM_CHK(q, sizeof(TA)) && (!alpha || ZLM_CHK(a, 4));
+            pd *= ok ? (alpha ? *a : hd) : 1.0f;
+            Q[tid * LA_LD + j] = ok ? to_f32(*q) * q_scale * pd : 0.f;
+        }
+    }
+    const int c = v0 + lane * 4;
+    const bool vo = V % 4 == 0 && c < V && (uintptr_t)o % 16 == 0;
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    float acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][e] = 0.f;
+    // sixteen coordinates at a time from zero, then added: the roundings of a short chain
+    for (int d0 = 0; d0 < D; d0 += 16) {
+        float t[8][4];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) t[i][e] = 0.f;
+#pragma unroll 8
+        for (int d = d0; d < min(D, d0 + 16); ++d) {
+            const float4 qa = *(const float4*)(Q + d * LA_LD + warp * 8), qb = *(const float4*)(Q + d * LA_LD + warp * 8 + 4);
+            const float4 s = *(const float4*)(S + d * 128 + lane * 4);
+            const float q[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                t[i][0] = fmaf(q[i], s.x, t[i][0]);
+                t[i][1] = fmaf(q[i], s.y, t[i][1]);
+                t[i][2] = fmaf(q[i], s.z, t[i][2]);
+                t[i][3] = fmaf(q[i], s.w, t[i][3]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[i][e] += t[i][e];
+    }
+    // the piece's own outputs and the gate's logits, all of them on their way before the first is used
+    float own[8][4];
+    Four z[8];
+    const bool yv = out.y && V % 4 == 0 && c < V && (out.y_stride | out.g_stride) % 4 == 0 &&
+                    ((uintptr_t)out.y | (uintptr_t)out.g) % sizeof(Four) == 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int j = warp * 8 + i;
+        const float* op = o + ((size_t)(row0 + j) * H + h) * V + c;
+        const TA* gp = (const TA*)out.g + (size_t)(row0 + j) * out.g_stride + (size_t)h * V + c;
+        memset(&z[i], 0, sizeof(Four));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) own[i][e] = 0.f;
+        if (j >= m) continue;
+        if (vo && ZLM_CHK(op, 16)) {
+            const float4 f = *(const float4*)op;
+            own[i][0] = f.x; own[i][1] = f.y; own[i][2] = f.z; own[i][3] = f.w;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (c + e < V && ZLM_CHK(op + e, 4)) own[i][e] = op[e];
+        }
+        if (!out.y) continue;
+        if (yv && ZLM_CHK(gp, sizeof(Four))) {
+            z[i] = *(const Four*)gp;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (c + e < V && ZLM_CHK(gp + e, sizeof(TA))) z[i].v[e] = gp[e];
+        }
+    }
+    float wn[4] = {0.f, 0.f, 0.f, 0.f};
+    if (out.y)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (c + e < V) wn[e] = out.w[c + e];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int j = warp * 8 + i;
+        if (j >= m) break;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][e] += own[i][e];
+        if (!out.y) {
+            float* op = o + ((size_t)(row0 + j) * H + h) * V + c;
+            if (vo && ZLM_CHK(op, 16)) *(float4*)op = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+            else
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (c + e < V && ZLM_CHK(op + e, 4)) op[e] = acc[i][e];
+            continue;
+        }
+        float ss = 0.f;                              // (columns beyond V are zero)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) ss = fmaf(acc[i][e], acc[i][e], ss);
+        const float f = 1.0f / sqrtf(warp_sum(ss) / (float)V + out.eps);
+        TA* yp = (TA*)out.y + (size_t)(row0 + j) * out.y_stride + (size_t)h * V + c;
+        Four y;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float zz = to_f32(z[i].v[e]), sg = 1.0f / (1.0f + expf(-zz));
+            y.v[e] = from_f32<TA>(acc[i][e] * f * wn[e] * (out.act == 1 ? zz * sg : sg));
+        }
+        if (yv && ZLM_CHK(yp, sizeof(Four))) {
+            *(Four*)yp = y;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (c + e < V && ZLM_CHK(yp + e, sizeof(TA))) yp[e] = y.v[e];
+        }
+    }
+}
+
+template <typename TA, int DR>
+static int launch_la_out(dim3 grid, cudaStream_t st, float* o, const void* proj, int proj_stride, int q_off, const float* alpha,
+                         const float* head_decay, const float* part, const int* cu_seqlens, int H, int D, int V, float q_scale,
+                         int maxp, const LaOut& out) {
+    const size_t smem = (size_t)DR * (128 + LA_LD) * sizeof(float);
+    auto kern = linear_attention_out_kernel<TA, DR>;
+    static bool attr_set_dev[64] = {};
+    bool& attr_set = attr_set_dev[zlm_device_index()];
+    if (!attr_set) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) {
+            zlm_set_error("linear_attention: cannot reserve shared memory: %s", cudaGetErrorString(e));
+            return ZLM_ERR_CUDA;
+        }
+        attr_set = true;
+    }
+    zlm_launch(kern, grid, dim3(128), smem, st, o, (const TA*)proj, proj_stride, q_off, alpha, head_decay, part, cu_seqlens, H, D, V,
+               q_scale, maxp, out);
+    return ZLM_OK;
+}
+
 // q, k [H*D], v [H*V]: columns of proj from q_off, k_off, v_off on (element type); alpha [T][H*D] fp32 decays per token
 // and key channel, or null with head_decay [H] fp32 (one decay a head); state [slots][H][D][V] fp32; o [T][H*V] fp32.
-// pieces: null, or R * ceil(max_new / 64) * H * D * (V + 1) floats: sequences run in pieces of 32 tokens side by side
-// (two passes and a chain between them).
+// pieces: null, or R * ceil(max_new / 32) * H * D * (V + 1) floats: sequences run in pieces of 32 tokens side by side
+// (a walk of every piece, a chain of their states, a product that adds what the state ahead of a piece gives).
+// y (null: none; with pieces, V <= 128): [T][y_stride] in the element type receives every head of o divided by its root mean
+// square, times w [V], times silu (act 1) or sigmoid (0) of g [T][g_stride]; o is then scratch.
 extern "C" int zlm_linear_attention(float* o, const void* proj, int proj_stride, int q_off, int k_off, int v_off,
                                     const float* alpha, const float* head_decay, float* state, int dtype, const int* seq_slot,
                                     const int* cu_seqlens, int T, int R, int H, int D, int V, float q_scale, int max_new,
-                                    float* pieces, cudaStream_t st) {
+                                    float* pieces, void* y, int y_stride, const void* g, int g_stride, const void* w, int w_dtype,
+                                    float eps, int act, cudaStream_t st) {
     if (T == 0) return ZLM_OK;
     ZLM_REQUIRE(H > 0 && D > 0 && V > 0 && D <= 128, "linear_attention: %d heads of %d key and %d value columns (keys up to 128)", H, D, V);
     ZLM_REQUIRE(alpha || head_decay, "linear_attention: neither decays per channel nor per head");
     ZLM_REQUIRE(!pieces || max_new > 0, "linear_attention: pieces without the longest sequence");
+    ZLM_REQUIRE(!y || (pieces && V <= 128 && g && w), "linear_attention: heads of %d columns do not take their gate along", V);
     const int L = LA_PIECE, maxp = pieces ? (max_new + L - 1) / L : 1;
-    ZLM_REQUIRE((long long)R * H * maxp <= 2147483647LL && (long long)R * H * D <= 2147483647LL && (V + 127) / 128 <= 65535, "linear_attention: too many sequences or columns");
-    const dim3 grid(R * H, (V + 127) / 128), pgrid(R * maxp * H, (V + 127) / 128), block(128);
+    ZLM_REQUIRE((long long)R * H * maxp <= 2147483647LL && (long long)R * H * D <= 2147483647LL && (V + 63) / 64 <= 65535 &&
+                    ((long long)D * V + 127) / 128 <= 65535, "linear_attention: too many sequences or columns");
+    const dim3 pgrid(R * maxp * H, (V + 127) / 128);
     float* part = pieces;
     float* pdecay = pieces ? pieces + (size_t)R * maxp * H * D * V : nullptr;
-#define ZLM_LA(TA, DR, MODE, G)                                                                                                \
-    zlm_launch(linear_attention_kernel<TA, DR, MODE>, G, block, 0, st, o, (const TA*)proj, proj_stride, q_off, k_off, v_off, alpha, \
-               head_decay, state, seq_slot, cu_seqlens, H, D, V, q_scale, part, pdecay, maxp, L)
-#define ZLM_LA_RUN(TA, DR)                                                                                                 \
+    const LaOut out{y, y_stride, g, g_stride, VecW{w, w_dtype}, eps, act};
+    int rc = ZLM_OK;
+#define ZLM_LA(TA, DR, SP, MODE, G)                                                                                            \
+    zlm_launch(linear_attention_kernel<TA, DR, SP, MODE>, dim3(G, (V + 512 * SP / DR - 1) / (512 * SP / DR)), dim3(128), 0, st, o, (const TA*)proj, proj_stride, q_off, k_off, v_off, \
+               alpha, head_decay, state, seq_slot, cu_seqlens, H, D, V, q_scale, part, pdecay, maxp, L)
+#define ZLM_LA_RUN(TA, DR, SP)                                                                                              \
     do {                                                                                                                   \
-        if (!pieces) { ZLM_LA(TA, DR, 0, grid); break; }                                                                   \
-        ZLM_LA(TA, DR, 1, pgrid);                                                                                          \
-        zlm_launch(linear_attention_chain_kernel, dim3(R * H * D, (V + 127) / 128), block, 0, st, part,                \
-                   (const float*)pdecay, state, seq_slot, cu_seqlens, H, D, V, maxp, L);                                                                          \
-        ZLM_LA(TA, DR, 2, pgrid);                                                                                          \
+        if (!pieces) { ZLM_LA(TA, DR, SP, 0, R * H); break; }                                                               \
+        ZLM_LA(TA, DR, SP, 1, R * maxp * H);                                                                                      \
+        if (V % 4 == 0 && (uintptr_t)state % 16 == 0 && (uintptr_t)part % 16 == 0)                                         \
+            zlm_launch(linear_attention_chain_kernel<4>, dim3(R * H, (D * V + 511) / 512), dim3(128), 0, st, part,         \
+                       (const float*)pdecay, state, seq_slot, cu_seqlens, H, D, V, maxp, L);                               \
+        else                                                                                                               \
+            zlm_launch(linear_attention_chain_kernel<1>, dim3(R * H, (D * V + 127) / 128), dim3(128), 0, st, part,         \
+                       (const float*)pdecay, state, seq_slot, cu_seqlens, H, D, V, maxp, L);                               \
+        rc = launch_la_out<TA, DR>(pgrid, st, o, proj, proj_stride, q_off, alpha, head_decay, part, cu_seqlens, H, D, V,   \
+                                   q_scale, maxp, out);                                                                    \
     } while (0)
 #define ZLM_LA_D(TA)                                                                     \
-    if (D <= 32) ZLM_LA_RUN(TA, 32); else if (D <= 64) ZLM_LA_RUN(TA, 64); else ZLM_LA_RUN(TA, 128)
+    if (D <= 32) ZLM_LA_RUN(TA, 32, 8); else if (D <= 64) ZLM_LA_RUN(TA, 64, 16); else ZLM_LA_RUN(TA, 128, 16)
     if (dtype == ZLM_DTYPE_F32) {
         ZLM_LA_D(float);
     } else if (dtype == ZLM_DTYPE_BF16) {
@@ -1028,6 +1264,7 @@ extern "C" int zlm_linear_attention(float* o, const void* proj, int proj_stride,
 #undef ZLM_LA_D
 #undef ZLM_LA_RUN
 #undef ZLM_LA
+    if (rc) return rc;
     return zlm_check_launch("linear_attention");
 }
 

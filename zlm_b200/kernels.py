@@ -1184,12 +1184,13 @@ class CudaKernels:
 
     def linear_attention(self, o: torch.Tensor, proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
                          alpha: Optional[torch.Tensor], head_decay: Optional[torch.Tensor], state: torch.Tensor, plan,
-                         heads: int, dim: int, v_dim: int, q_scale: float = 1.0, pieces: Optional[bool] = None) -> None:
+                         heads: int, dim: int, v_dim: int, q_scale: float = 1.0, pieces: Optional[bool] = None,
+                         _gate: Optional[tuple] = None) -> None:
         """o [T, heads*v_dim] fp32 = S_t^T q_t with S_t = diag(alpha_t) S_(t-1) + k_t v_t^T per head; q (times ``q_scale``),
         k, v are columns of ``proj`` from q_off, k_off, v_off on; ``alpha`` [T, heads*dim] fp32 gives a decay per token and
         key channel, or ``head_decay`` [heads] fp32 one per head; ``state`` [slots, heads, dim, v_dim] fp32.  Long prompts
-        run in pieces of 32 tokens side by side: every piece from a zero state, the pieces' states chained, and a second
-        pass that adds what the state before a piece gives its tokens (``pieces`` forces or forbids that)."""
+        run in pieces of 32 tokens side by side: every piece from a zero state, the pieces' states chained, and a
+        product that adds what the state before a piece gives its tokens (``pieces`` forces or forbids that)."""
         T = proj.shape[0]
         assert o.shape == (T, heads * v_dim) and o.dtype == torch.float32 and o.is_contiguous() and proj.stride(1) == 1
         assert state.dtype == torch.float32 and tuple(state.shape[1:]) == (heads, dim, v_dim) and state.is_contiguous()
@@ -1204,10 +1205,28 @@ class CudaKernels:
         if pieces:
             maxp = (max_new + self.RECURRENT_PIECE - 1) // self.RECURRENT_PIECE
             part = plan.scratch("linear_attention.pieces", (plan.R * maxp * heads * dim * (v_dim + 1),), torch.float32)
+        y, g, w, eps, act = _gate if _gate is not None else (None, None, None, 0.0, "silu")
         self._call("zlm_linear_attention", self._p(o), self._p(proj), c_int(proj.stride(0)), c_int(q_off), c_int(k_off),
                    c_int(v_off), self._p(alpha), self._p(head_decay if alpha is None else None), self._p(state), c_int(_dt(proj)),
                    self._p(plan.seq_slot), self._p(plan.cu_seqlens), c_int(T), c_int(plan.R), c_int(heads), c_int(dim),
-                   c_int(v_dim), c_float(q_scale), c_int(max_new), self._p(part), self._stream())
+                   c_int(v_dim), c_float(q_scale), c_int(max_new), self._p(part), self._p(y),
+                   c_int(y.stride(0) if y is not None else 0), self._p(g), c_int(g.stride(0) if g is not None else 0), self._p(w),
+                   c_int(_dt(w) if w is not None else F32), c_float(eps), c_int({"sigmoid": 0, "silu": 1}[act]), self._stream())
+
+    def linear_attention_gated(self, y: torch.Tensor, g: torch.Tensor, w_norm: torch.Tensor, eps: float, act: str, o: torch.Tensor,
+                               proj: torch.Tensor, q_off: int, k_off: int, v_off: int, alpha: Optional[torch.Tensor],
+                               head_decay: Optional[torch.Tensor], state: torch.Tensor, plan, heads: int, dim: int, v_dim: int,
+                               q_scale: float = 1.0) -> None:
+        """``linear_attention``, then ``norm_gate``: y [T, heads*v_dim] = o / rms(o, per head) * w_norm [v_dim] * act(g); a long
+        prompt's last kernel writes y itself.  ``o`` is scratch."""
+        args = (proj, q_off, k_off, v_off, alpha, head_decay, state, plan, heads, dim, v_dim, q_scale)
+        if (int(getattr(plan, "max_new", 0) or 0) >= self.RECURRENT_PIECES_FROM and v_dim <= 128 and w_norm.numel() == v_dim
+                and w_norm.is_contiguous() and y.dtype == g.dtype == proj.dtype and y.stride(1) == g.stride(1) == 1):
+            assert y.shape == g.shape == (proj.shape[0], heads * v_dim)
+            self.linear_attention(o, *args, _gate=(y, g, w_norm, eps, act))
+            return
+        self.linear_attention(o, *args)
+        self.norm_gate(y, o, g, heads, v_dim, "head", w_norm, eps, act)
 
     def scaled_sum(self, out: torch.Tensor, a: torch.Tensor, alpha: float, b: torch.Tensor, beta: float,
                    accumulate: bool = True) -> None:

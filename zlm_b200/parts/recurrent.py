@@ -160,9 +160,9 @@ class GatedLinearAttention(Mixer):
         alpha = rt.ws.get("gla.alpha", (T, QK), torch.float32)
         k.lowrank_decay(alpha, proj, 2 * QK + 2 * VV, self.a_up, self.a_bias, self.tau)
         o = rt.ws.get("gla.o", (T, VV), torch.float32)
-        k.linear_attention(o, proj, 0, QK, 2 * QK, alpha, None, io.state, ctx, self.H, self.D, self.V, self.D ** -0.5)
         y = rt.ws.get("gla.gated", (T, VV), rt.dtype)
-        k.norm_gate(y, o, proj[:, 2 * QK + VV: 2 * QK + 2 * VV], self.H, self.V, "head", self.w_norm, self.eps, self.gate)
+        k.linear_attention_gated(y, proj[:, 2 * QK + VV: 2 * QK + 2 * VV], self.w_norm, self.eps, self.gate, o, proj, 0, QK, 2 * QK,
+                                 alpha, None, io.state, ctx, self.H, self.D, self.V, self.D ** -0.5)
         k.linear(residual, y, self.w_o, accumulate=True, defer=True)       # a norm reads the stream next
 
 

@@ -297,6 +297,15 @@ class ProfilingKernels:
         return self._timed(kind, n, 6.0 * T * heads * dim * v_dim, self.k.linear_attention, o, proj, q_off, k_off, v_off,
                            alpha, head_decay, state, plan, heads, dim, v_dim, *args, **kw)
 
+    def linear_attention_gated(self, y, g, w_norm, eps, act, o, proj, q_off, k_off, v_off, alpha, head_decay, state, plan, heads, dim,
+                               v_dim, *args, **kw):
+        T, el = proj.shape[0], proj.element_size()
+        n = (T * heads * (2 * dim + v_dim) * el + 2 * _nbytes(y) + (0 if alpha is None else _nbytes(alpha))
+             + 2 * plan.R * heads * dim * v_dim * 4)
+        kind = "gated linear attention decode" if plan.is_decode else "gated linear attention prefill"
+        return self._timed(kind + ", heads norm*gate", n, 6.0 * T * heads * dim * v_dim, self.k.linear_attention_gated, y, g, w_norm,
+                           eps, act, o, proj, q_off, k_off, v_off, alpha, head_decay, state, plan, heads, dim, v_dim, *args, **kw)
+
     def mlstm(self, o, proj, q_off, k_off, v_off, z, i_off, f_off, b_i, b_f, cap, state, plan, heads, dim, v_dim, *args):
         T, el = proj.shape[0], proj.element_size()
         n = T * heads * (2 * dim + v_dim) * el + _nbytes(o) + 2 * plan.R * heads * dim * v_dim * 4
