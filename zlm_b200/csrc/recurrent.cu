@@ -860,7 +860,7 @@ extern "C" int zlm_lowrank_decay(float* alpha, const void* proj, int proj_stride
 #define LA_CH 16
 #define LA_CPT 4
 template <typename TA, int DR, int DPT, int MODE>
-__global__ void __launch_bounds__(128, DR == 128 ? 4 : 5)
+__global__ void __launch_bounds__(128, MODE == 0 || DR == 128 ? 4 : 5)
 linear_attention_kernel(float* __restrict__ o, const TA* __restrict__ proj, int proj_stride, int q_off, int k_off, int v_off,
                         const float* __restrict__ alpha, const float* __restrict__ head_decay, float* __restrict__ state,
                         const int* __restrict__ seq_slot, const int* __restrict__ cu_seqlens, int H, int D, int V,
