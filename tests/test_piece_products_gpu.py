@@ -134,3 +134,93 @@ def test_matrix_memory(H, D, V, cap, news, starts, spread):
             close(o, want.flatten(1), 4e-6 if spread == 1.0 else 1e-4)
         for got, exact in zip(state, (S, N, M)):
             close(got, exact, 1e-6)
+
+
+def kinds(x):
+    """0 where finite, 1 / -1 for infinities, 2 for NaN."""
+    x = x.double()
+    return torch.where(torch.isnan(x), 2.0, torch.where(torch.isinf(x), torch.sign(x), 0.0))
+
+
+# where a number that is not finite stands: the operand's columns of the projection (or the state), the token, the column
+@pytest.mark.parametrize("where", ["query", "key", "value", "state"])
+@pytest.mark.parametrize("number", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("token", [0, 8, 21, 63, 70, 255])
+@pytest.mark.parametrize("part", ["retention", "matrix memory"])
+def test_numbers_that_are_not_finite_reach_what_sees_them(part, where, number, token):
+    """Tokens ahead of such a number, and columns that it does not enter, keep their results to the bit; what it enters is not
+    finite, and behind a key or a state it is the infinity or NaN of a 64-bit walk over the tokens (behind a query or a value that
+    depends on the order of the sums: infinities of both signs meet where a state is read, or do not where scores are)."""
+    from zlm_b200.kernels import get_kernels
+    k, H, D, V, T = get_kernels(), 2, 64, 72, 256
+    plan = plan_of([T], [0])
+    g = torch.Generator(device="cuda").manual_seed(5)
+
+    def rand(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+    clean = (rand(T, 2 * H * D + 2 * H * V)).bfloat16()
+    # (forget gates near one: a weight that underflows times an infinity is NaN in any order of the sums)
+    z = torch.cat([rand(T, H), rand(T, H) + 7], 1)
+    first = [rand(1, H, D, V) * 0.3, rand(1, H, D), rand(1, H).abs()]
+    decay = torch.linspace(0.9, 0.99, H, device="cuda")
+    col = {"query": 5, "key": H * D + 5, "value": 2 * H * D + 5, "state": 0}[where]
+    spoilt, spoilt_first = clean.clone(), first[0].clone()
+    if where == "state":
+        spoilt_first[0, 0, 7, 5] = number
+    else:
+        spoilt[token, col] = number                  # (head 0)
+
+    def run(proj, S, gated):
+        state = [S.clone(), first[1].clone(), first[2].clone()]
+        o = torch.zeros((T, H * V), device="cuda")
+        y = torch.zeros((T, H * V), device="cuda", dtype=torch.bfloat16)
+        gate = proj[:, 2 * H * D + H * V:]
+        if part == "retention":
+            args = (o, proj, 0, H * D, 2 * H * D, None, 0, decay, state[0], plan, H, D, V, 0.125)
+            k.retention_gated(y, gate, 1e-6, "silu", *args) if gated else k.retention(*args)
+        else:
+            args = (o, proj, 0, H * D, 2 * H * D, z, 0, H, None, None, 15.0, state, plan, H, D, V, 0.125)
+            w = torch.ones((H * V,), device="cuda")
+            k.mlstm_gated(y, gate, w, 1e-6, *args) if gated else k.mlstm(*args)
+        return (y if gated else o).view(T, H, V), state[0]
+
+    def walk(proj, S0):
+        q, key = (proj[:, i * H * D:(i + 1) * H * D].double().view(T, H, D) for i in (0, 1))
+        v = proj[:, 2 * H * D:2 * H * D + H * V].double().view(T, H, V)
+        S, out = S0[0].double(), []
+        n, m = first[1][0].double(), first[2][0].double()
+        gi, gf = 15 * torch.tanh(z[:, :H].double() / 15), torch.nn.functional.logsigmoid(15 * torch.tanh(z[:, H:].double() / 15))
+        for t in range(T):
+            if part == "retention":
+                a, b, den = decay.double(), torch.full((H,), 0.125, dtype=torch.float64, device="cuda"), torch.ones(H, 1, device="cuda")
+            else:
+                new = torch.maximum(gf[t] + m, gi[t])
+                a, b, m = torch.exp(gf[t] + m - new), torch.exp(gi[t] - new), new
+                n = a[:, None] * n + b[:, None] * key[t]
+                den = torch.maximum((n * q[t] * 0.125).sum(1).abs(), torch.exp(-m))[:, None] + 1e-6
+            S = a[:, None, None] * S + b[:, None, None] * key[t][:, :, None] * v[t][:, None]
+            out.append((S * q[t][:, :, None] * (1.0 if part == "retention" else 0.125)).sum(1) / den)
+        return torch.stack(out), S[None]
+    sees = torch.zeros((T, H, V), dtype=torch.bool, device="cuda")       # outputs that the number enters
+    if where == "query":
+        sees[token, 0] = True
+    elif where == "key":
+        sees[token:, 0] = True
+    elif where == "value":
+        sees[token:, 0, 5] = True
+    else:
+        sees[:, 0, 5] = True
+    (o, S), (o_clean, S_clean) = run(spoilt, spoilt_first, False), run(clean, first[0], False)
+    want, S_want = walk(spoilt, spoilt_first)
+    assert torch.equal(o[~sees], o_clean[~sees])
+    if where in ("key", "state"):
+        assert torch.equal(kinds(o), kinds(want))
+    assert not torch.isfinite(o[sees]).any() and not torch.isfinite(want[sees]).any()
+    assert torch.equal(kinds(S), kinds(S_want))
+    fine = kinds(S_want) == 0
+    assert torch.equal(S[fine], S_clean[fine])
+    y, _ = run(spoilt, spoilt_first, True)
+    y_clean, _ = run(clean, first[0], True)
+    rows = ~sees.any(2)                                                   # (a head's norm takes all its columns along)
+    assert torch.equal(y[rows], y_clean[rows])
+    assert (kinds(y[~rows]) != 0).any(1).all()

@@ -644,10 +644,10 @@ mlstm_out_products_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, int
                           const float2* __restrict__ ahead, float* __restrict__ mmax, const int* __restrict__ seq_slot,
                           const int* __restrict__ cu_seqlens, int H, int D, int V, int maxp, float q_scale) {
     extern __shared__ __align__(128) __nv_bfloat16 ml_tiles[];
-    __nv_bfloat16* qt = ml_tiles;                    // [3][SM_L][128], later the gate's columns
+    __nv_bfloat16* qt = ml_tiles;                    // [3][SM_L][128]
     __nv_bfloat16* kt = qt + 3 * SM_L * 128;         // [3][SM_L][128], later the weights and the state's rows:
     __nv_bfloat16* pt = kt;                          // [3][SM_L][SM_L]
-    __nv_bfloat16* st = pt + 3 * SM_L * SM_L;        // [3][32][128]
+    __nv_bfloat16* st = pt + 3 * SM_L * SM_L;        // [3][32][128], later the gate's columns
     __nv_bfloat16* vt = kt + 3 * SM_L * 128;         // [SM_L][128]
     // (with the tiles this is all that two blocks an SM have room for: what comes later takes the place of what is read)
     __shared__ __align__(16) double se[SM_L], sm[SM_L];
@@ -683,7 +683,7 @@ mlstm_out_products_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, int
     const float* np = part_n + pc.at * D + lane * 4;
     const float4 n_ahead = lane * 4 < D && ZLM_CHK(np, 16) ? *(const float4*)np : make_float4(0.f, 0.f, 0.f, 0.f);
     dec_wait<0>();
-    __syncthreads();
+    const bool taken = __syncthreads_or(sm_clean_values(vt, tid));
     const int r0 = (warp >> 1) * 16, half = warp & 1, j0 = r0 + (lane >> 2);
     float s[4][4], keep[2], sum[2] = {0.f, 0.f};
     {
@@ -718,7 +718,7 @@ mlstm_out_products_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, int
             for (int e = 0; e < 8; ++e) {
                 const float mine = (e & 3) == 0 ? n_ahead.x : (e & 3) == 1 ? n_ahead.y : (e & 3) == 2 ? n_ahead.z : n_ahead.w;
                 const float nv = __shfl_sync(0xffffffffu, mine, 2 * (c + (lane & 1)) + (e >> 2));
-                nq = fmaf(nv, f[0][e] + (f[1][e] + f[2][e]), nq);
+                nq = fmaf(nv, sm_odd(f[0][e]) ? f[0][e] : f[0][e] + (f[1][e] + f[2][e]), nq);
             }
         }
         nq += __shfl_xor_sync(0xffffffffu, nq, 1);
@@ -738,14 +738,16 @@ mlstm_out_products_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, int
         sm_read_state(acc, qt, st, r0, half * 64, d0, D, lane);
         __syncthreads();
     }
-    if (out.y) sm_stage_values(qt, out.g + (size_t)pc.row0 * out.g_stride + (size_t)pc.h * V, out.g_stride, pc.n, 0, V, tid);      // (the queries are read)
+    if (out.y) sm_stage_values(st, out.g + (size_t)pc.row0 * out.g_stride + (size_t)pc.h * V, out.g_stride, pc.n, 0, V, tid);      // (the state is read)
     acc.scale(keep[0], keep[1]);
     sm_read_values(acc, pt, vt, r0, half * 64, lane);
+    sm_mend_out(acc, SmSeen{qt, pt, vt, S + c0, rows + v_off + (size_t)pc.h * V + c0, (size_t)stride, D, V}, keep[0], keep[1], taken, pc.n,
+                V - c0, r0, half * 64, lane);
     float inv[2];
 #pragma unroll
     for (int x = 0; x < 2; ++x) inv[x] = 1.0f / ml_denominator(sums[j0 + 8 * x][0] + sums[j0 + 8 * x][1], m_of[j0 + 8 * x]);
     __syncthreads();                                 // (the sums are read)
-    sm_write(acc, inv[0], inv[1], out, qt, sums, pc.row0, pc.n, pc.h, H, V, c0, r0, half, lane);
+    sm_write(acc, inv[0], inv[1], out, st, sums, pc.row0, pc.n, pc.h, H, V, c0, r0, half, lane);
 }
 
 // what the tensor-core form takes: 16-byte reads of 8 neighbouring coordinates

@@ -390,7 +390,7 @@ retention_piece_out_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, in
     __nv_bfloat16* qt = rm_smem;                     // [3][SM_L][128]
     __nv_bfloat16* kt = qt + 3 * SM_L * 128;         // [3][SM_L][128], later the weights and the state's rows:
     __nv_bfloat16* pt = kt;                          // [3][SM_L][SM_L]
-    __nv_bfloat16* st = pt + 3 * SM_L * SM_L;        // [3][32][128]
+    __nv_bfloat16* st = pt + 3 * SM_L * SM_L;        // [3][32][128], later the gate's columns
     __nv_bfloat16* vt = kt + 3 * SM_L * 128;         // [SM_L][128]
     __shared__ float pw[SM_L + 1], red[SM_L][2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y, c0 = blockIdx.z * 128;
@@ -408,7 +408,7 @@ retention_piece_out_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, in
     const float* S = before + ((size_t)blockIdx.x * H + h) * D * V;
     SmRows next = sm_fetch_state(S, 0, D, V, c0, tid);
     dec_wait<0>();
-    __syncthreads();
+    const bool taken = __syncthreads_or(sm_clean_values(vt, tid));
     const int r0 = (warp >> 1) * 16, part = warp & 1;
     SmSum<4> dots;
     sm_scores(dots, qt, kt, r0, part * 32, D, lane);
@@ -431,10 +431,13 @@ retention_piece_out_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, in
         sm_read_state(acc, qt, st, r0, part * 64, d0, D, lane);
         __syncthreads();
     }
-    if (out.y) sm_stage_values(qt, out.g + (size_t)row0 * out.g_stride + (size_t)h * V, out.g_stride, n, 0, V, tid);      // (the queries are read)
-    acc.scale(pw[r0 + (lane >> 2) + 1], pw[r0 + (lane >> 2) + 9]);
+    if (out.y) sm_stage_values(st, out.g + (size_t)row0 * out.g_stride + (size_t)h * V, out.g_stride, n, 0, V, tid);      // (the state is read)
+    const float keep0 = pw[r0 + (lane >> 2) + 1], keep8 = pw[r0 + (lane >> 2) + 9];
+    acc.scale(keep0, keep8);
     sm_read_values(acc, pt, vt, r0, part * 64, lane);
-    sm_write(acc, 1.f, 1.f, out, qt, red, row0, n, h, H, V, c0, r0, part, lane);
+    sm_mend_out(acc, SmSeen{qt, pt, vt, S + c0, rows + v_off + (size_t)h * V + c0, (size_t)ld, D, V}, keep0, keep8, taken, n, V - c0, r0,
+                part * 64, lane);
+    sm_write(acc, 1.f, 1.f, out, st, red, row0, n, h, H, V, c0, r0, part, lane);
 }
 
 // what the tensor-core form takes: 16-byte reads of 8 neighbouring coordinates (also of the halves of a rotation)

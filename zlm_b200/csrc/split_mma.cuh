@@ -120,6 +120,116 @@ template <int NT> struct SmSum {
     __device__ __forceinline__ float get(int n, int e) const { return v[n][e]; }
 };
 
+// ---------------------------------------------------------------------------- numbers that are not finite
+// Cut into pieces, an infinity leaves infinity - infinity = NaN behind, and a tile's zero weights make NaN of it in rows that do
+// not see it (0 x infinity).  So what is not finite among the values is taken out of their tile before the products (one
+// pass over the thread's own copies; a later token's values then leave the rows of earlier ones alone, to the bit), and sums
+// that still come out not finite (keys, queries, states) are formed again as FFMA chains of the whole numbers, with the
+// values that were taken out: infinities keep their signs and reach what sees them, as in a walk over the tokens.  Chosen
+// over a second kernel that a flag would wake: that costs every call a launch.
+__device__ __forceinline__ bool sm_odd(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
+// whether one of a thread's sums is not finite (zero times it is not zero)
+template <int NT> __device__ __forceinline__ bool sm_any_odd(const SmSum<NT>& s) {
+    float t[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) t[e] = fmaf(s.v[n][e], 0.f, t[e]);
+    return (t[0] + t[1]) + (t[2] + t[3]) != 0.f;
+}
+// the thread's copies of sm_stage_values, between dec_wait<0>() and the barrier; true where something was taken out
+__device__ __forceinline__ bool sm_clean_values(__nv_bfloat16* vt, int tid) {
+    unsigned top = 0;
+#pragma unroll
+    for (int y = 0; y < SM_L * 16 / 256; ++y) {
+        const int x = tid + y * 256;
+        const uint4 u = *(const uint4*)(vt + tile_off<128>(x >> 4, x & 15));
+        top = __vmaxu2(__vmaxu2(__vmaxu2(top, u.x & 0x7fff7fffu), __vmaxu2(u.y & 0x7fff7fffu, u.z & 0x7fff7fffu)), u.w & 0x7fff7fffu);
+    }
+    if ((top & 0xffffu) < 0x7f80u && (top >> 16) < 0x7f80u) return false;
+    for (int x = tid; x < SM_L * 16; x += 256) {
+        unsigned* p = (unsigned*)(vt + tile_off<128>(x >> 4, x & 15));
+        for (int e = 0; e < 4; ++e) {
+            if ((p[e] & 0x7f80u) == 0x7f80u) p[e] &= 0xffff0000u;
+            if ((p[e] & 0x7f800000u) == 0x7f800000u) p[e] &= 0xffffu;
+        }
+    }
+    return true;
+}
+// number c of a row of a tile in pieces of `elems` elements
+template <int HD> __device__ __forceinline__ float sm_whole(const __nv_bfloat16* t, int elems, int row, int c) {
+    const __nv_bfloat16* p = t + tile_off<HD>(row, c >> 3) + (c & 7);
+    const float hi = to_f32(p[0]);
+    return sm_odd(hi) ? hi : hi + (to_f32(p[elems]) + to_f32(p[2 * elems]));
+}
+// (calls, so that the kernels' own code stays short: their loops are unrolled, and inlined chains cost them 3 to 6 %)
+// scores that are not finite: row by row of both tiles, in pieces [SM_L][128]
+static __device__ __noinline__ void sm_mend_scores(float (*s)[4], const __nv_bfloat16* qt, const __nv_bfloat16* kt, int r0, int n0, int dim,
+                                                   int lane) {
+    for (int i = 0; i < 4; ++i)
+        for (int e = 0; e < 4; ++e) {
+            const int j = r0 + (lane >> 2) + 8 * (e >> 1), l = n0 + i * 8 + (lane & 3) * 2 + (e & 1);
+            if (!sm_odd(s[i][e])) continue;
+            float t = 0.f;
+            for (int c = 0; c < dim; ++c) t = fmaf(sm_whole<128>(qt, SM_L * 128, j, c), sm_whole<128>(kt, SM_L * 128, l, c), t);
+            s[i][e] = t;
+        }
+}
+// numbers of a state that are not finite: columns of the weighted keys times columns of the values
+static __device__ __noinline__ void sm_mend_state(float (*s)[4], const __nv_bfloat16* kt, const __nv_bfloat16* vt, int d0, int n0, int lane) {
+    for (int i = 0; i < 8; ++i)
+        for (int e = 0; e < 4; ++e) {
+            const int d = d0 + (lane >> 2) + 8 * (e >> 1), c = n0 + i * 8 + (lane & 3) * 2 + (e & 1);
+            if (!sm_odd(s[i][e])) continue;
+            float t = 0.f;
+            for (int l = 0; l < SM_L; ++l)
+                t = fmaf(sm_whole<128>(kt, SM_L * 128, l, d), to_f32(vt[tile_off<128>(l, c >> 3) + (c & 7)]), t);
+            s[i][e] = t;
+        }
+}
+// what an output is made of: S the state's column of the head's value column c0 + c, v the piece's values of that column
+struct SmSeen {
+    const __nv_bfloat16 *qt, *pt, *vt;
+    const float* S;
+    const __nv_bfloat16* v;
+    size_t stride;
+    int D, V;
+};
+static __device__ __noinline__ void sm_mend_outputs(float (*acc)[4], const SmSeen& s, float keep0, float keep8, bool taken, int n, int cols,
+                                                    int r0, int n0, int lane) {
+    for (int i = 0; i < 8; ++i)
+        for (int e = 0; e < 4; ++e) {
+            const int j = r0 + (lane >> 2) + 8 * (e >> 1), c = n0 + i * 8 + (lane & 3) * 2 + (e & 1);
+            if (j >= n || c >= cols) continue;
+            float x = acc[i][e];
+            if (sm_odd(x)) {
+                x = 0.f;
+                for (int d = 0; d < s.D; ++d) {
+                    const float* p = s.S + (size_t)d * s.V + c;
+                    if (ZLM_CHK(p, 4)) x = fmaf(sm_whole<128>(s.qt, SM_L * 128, j, d), *p, x);
+                }
+                x *= e < 2 ? keep0 : keep8;
+                for (int l = 0; l <= j; ++l)
+                    x = fmaf(sm_whole<SM_L>(s.pt, SM_L * SM_L, j, l), to_f32(s.vt[tile_off<128>(l, c >> 3) + (c & 7)]), x);
+            }
+            for (int l = 0; taken && l <= j; ++l) {
+                const __nv_bfloat16* p = s.v + (size_t)l * s.stride + c;
+                const float v = ZLM_CHK(p, 2) ? to_f32(*p) : 0.f;
+                if (sm_odd(v)) x = fmaf(sm_whole<SM_L>(s.pt, SM_L * SM_L, j, l), v, x);
+            }
+            acc[i][e] = x;
+        }
+}
+// a warp's outputs (16 rows of the piece's n from r0, 64 columns from n0 of the block's `cols`); queries, weights and the cleaned
+// values still in their tiles; taken: sm_clean_values took something out somewhere in the block
+__device__ __forceinline__ void sm_mend_out(SmSum<8>& acc, const SmSeen& s, float keep0, float keep8, bool taken, int n, int cols, int r0,
+                                            int n0, int lane) {
+    if (!taken && !sm_any_odd(acc)) return;
+    SmSum<8> t = acc;                                // (a copy, so that the sums themselves stay in registers)
+    sm_mend_outputs(t.v, s, keep0, keep8, taken, n, cols, r0, n0, lane);
+    acc = t;
+}
+
 // ---------------------------------------------------------------------------- a piece of 64 tokens, one head, 128 value columns
 // Blocks of 256 threads.  What a piece adds to a state:
 //   acc += (keys)^T (values): the warp's 16 rows of the state from d0 on, 64 columns from n0 on;
@@ -138,6 +248,10 @@ __device__ __forceinline__ void sm_piece_state(SmSum<8>& acc, const __nv_bfloat1
             sm_mma3<2>(acc.v + n, a, b);
         }
     }
+    if (!sm_any_odd(acc)) return;
+    SmSum<8> t = acc;
+    sm_mend_state(t.v, kt, vt, d0, n0, lane);
+    acc = t;
 }
 // 16 rows from d0, 64 columns from c of a state [..][V]
 __device__ __forceinline__ void sm_write_state(float* S, const SmSum<8>& acc, int d0, int c, int V, int lane) {
@@ -167,6 +281,10 @@ __device__ __forceinline__ void sm_scores(SmSum<4>& s, const __nv_bfloat16* qt, 
                 dec_ldsm4(b[y][x][0], b[y][x][1], b[y][x][2], b[y][x][3], sm_b_rows<128>(kt + x * SM_L * 128, n0 + y * 16, k0, lane));
         sm_mma6<2>(s.v, a, b);
     }
+    if (!sm_any_odd(s)) return;
+    SmSum<4> t = s;
+    sm_mend_scores(t.v, qt, kt, r0, n0, dim, lane);
+    s = t;
 }
 // 32 rows of the state, 128 columns: fetched into registers (a thread's four float4), then cut into pieces [32][128]
 struct SmRows { float4 f[4]; };
