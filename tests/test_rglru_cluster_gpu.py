@@ -58,3 +58,51 @@ def test_prompts(W, blocks, taps, news, starts):
     close(out, want * gelu * 0.7, 6e-3)
     close(state[:, 0], S[:, 0], 4e-3)
     assert torch.equal(state[:, 1:], S[:, 1:].float())
+
+
+def _function(which, x):
+    import ctypes
+
+    from zlm_b200.kernels import get_kernels
+    k, out = get_kernels(), torch.empty_like(x)
+    k._call("zlm_rglru_functions", k._p(out), k._p(x), ctypes.c_int(x.numel()), ctypes.c_int(which), k._stream())
+    return out
+
+
+def _spread(lo, hi, n=20001):
+    """``n`` numbers of [lo, hi], and as many spread over the logarithm towards zero, of either sign where the range has both."""
+    x = torch.linspace(lo, hi, n, dtype=torch.float64)
+    small = torch.pow(10.0, torch.linspace(-44, 0, n, dtype=torch.float64))
+    x = torch.cat([x, small[small <= hi], -small[small <= -lo]])
+    return x.float().cuda()
+
+
+# Units in the last place are 2^-23 of a number at most.  The exponential is off by up to two of them, the reciprocal after its step
+# by one, every product and sum by half: five for sigmoid; four for 1 - e^y (e^(y/2) twice over, of at most 0.6 of the result,
+# or a Horner chain whose terms shrink); the approximate root by two, and by half for its product.
+@pytest.mark.parametrize("which,lo,hi,ulps,want", [
+    (0, -100.0, 100.0, 5, torch.sigmoid), (1, -200.0, 0.0, 4, lambda y: -torch.expm1(y)), (2, 0.0, 1.0, 3, torch.sqrt)])
+def test_functions_to_the_last_places(which, lo, hi, ulps, want):
+    x = _spread(lo, hi)
+    x = torch.cat([x, torch.tensor([-1.0, -1.0 - 2.0 ** -23, -1.0 + 2.0 ** -24, 1e-30, 9.9e-31, 2.0 ** -126, 0.0], device="cuda").clamp(lo, hi)])
+    got, exact = _function(which, x).double(), want(x.double())
+    # (below 2^-126 a unit is 2^-149 whatever the number is)
+    assert ((got - exact).abs() <= ulps * torch.clamp(exact.abs() * 2.0 ** -23, min=2.0 ** -149)).all()
+    assert torch.isnan(_function(which, torch.tensor([float("nan")], device="cuda"))).all()
+
+
+def test_gelu_over_the_whole_range():
+    """z sigmoid(2 t), t = c (z + 0.044715 z^3): as sigmoid, and its argument's three roundings times its slope, |2 t| relative to
+    the result where that is small; nothing is left of the tail, however large the number, and what is not finite is what
+    0.5 z (1 + tanh t) makes of it."""
+    z = _spread(-12.0, 12.0)
+    got, x = _function(3, z).double(), z.double()
+    t2 = 1.5957691216057308 * (x + 0.044715 * x ** 3)
+    exact = x * torch.sigmoid(t2)
+    assert ((got - exact).abs() <= (6 + 4 * t2.abs()) * 2.0 ** -23 * exact.abs() + 2.0 ** -149 * (1 + x.abs())).all()
+    far = torch.tensor([-1e4, -1e13, -1e30, -3.3895e38, 1e13, 3.3895e38], device="cuda")
+    assert torch.equal(_function(3, far), torch.where(far < 0, torch.zeros_like(far), far))
+    edge = _function(3, torch.tensor([float("inf"), float("-inf"), float("nan")], device="cuda"))
+    assert edge[0] == float("inf") and torch.isnan(edge[1:]).all()
+    edge = _function(0, torch.tensor([float("inf"), float("-inf"), -200.0], device="cuda"))
+    assert edge.tolist() == [1.0, 0.0, 0.0]

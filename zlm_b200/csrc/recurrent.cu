@@ -538,13 +538,17 @@ rglru_conv_blocks_kernel(__nv_bfloat16* __restrict__ u16, int* __restrict__ grou
 
 // The recurrence's functions without branches, so that the numbers of a thread's tokens are worked out side by side (the
 // library's division, square root, expm1f and tanhf each branch for arguments that do not occur here: 62 us of the kernel
-// below with them, 55 us without).  To the last places of fp32: a reciprocal and a square root are a Newton step from the
-// approximate one, 1 - e^y is a series where it would cancel.  NaN stays NaN.
+// below with them, 55 us without).  Each is an approximation and one step of Newton's rule x - f(x) / f'(x) (Abramowitz and Stegun,
+// Handbook of Mathematical Functions, 3.9.5), or the exponential's series (4.2.1): a few units in the last place of fp32 over
+// the whole range, which a test compares with 64-bit values (zlm_rglru_functions).  NaN stays NaN.
+// 1 / (1 + e^-x).  With e = e^-|x| the denominator is in [1, 2], where neither it nor its reciprocal can overflow or vanish:
+// 1/d from r by f(r) = 1/r - d.  Below zero e / (1 + e): what underflows is the result itself (a clamped argument instead would
+// leave 1.8e-35 there, which gelu multiplies with numbers as large as the type has).
 __device__ __forceinline__ float rl_sigmoid(float x) {
-    const float e = expf(-x > 80.f ? 80.f : -x), d = 1.0f + e, r = __fdividef(1.0f, d);
-    return fmaf(r, fmaf(-d, r, 1.0f), r);
+    const float e = expf(-fabsf(x)), d = 1.0f + e, r0 = __fdividef(1.0f, d), r = fmaf(r0, fmaf(-d, r0, 1.0f), r0);
+    return x < 0.f ? e * r : r;
 }
-// 1 - e^y for y <= 0, a = e^(y/2)
+// 1 - e^y for y <= 0, a = e^(y/2): above -1, where the difference would cancel, the series of (e^y - 1) / y, Horner's form
 __device__ __forceinline__ float rl_one_minus_exp(float y, float a) {
     float p = 1.0f / 479001600.0f;                   // sum of y^k / k!, k = 1 .. 12; y^13 / 13! is below 2^-32 on [-1, 0]
     constexpr float c[11] = {1.0f / 39916800.0f, 1.0f / 3628800.0f, 1.0f / 362880.0f, 1.0f / 40320.0f, 1.0f / 5040.0f, 1.0f / 720.0f,
@@ -553,9 +557,10 @@ __device__ __forceinline__ float rl_one_minus_exp(float y, float a) {
     for (int k = 0; k < 11; ++k) p = fmaf(p, y, c[k]);
     return y < -1.0f ? fmaf(-a, a, 1.0f) : -y * p;
 }
+// sqrt x from s = x rsqrt x by f(s) = s^2 - x; where the difference would be of the order of the smallest fp32 numbers, s as it is
 __device__ __forceinline__ float rl_sqrt(float x) {
     const float r = rsqrtf(x), s = x * r, q = fmaf(fmaf(-s, s, x), 0.5f * r, s);
-    return x < 1e-30f ? 0.f : q;                     // (what it multiplies is of the order of one; NaN is not below)
+    return x < 1e-30f ? (x == 0.f ? 0.f : s) : q;
 }
 __device__ __forceinline__ void rl_ab(float zr, float zi, float u, float sl, float& a, float& b) {
     const float log_a = -rl_sigmoid(zr) * sl;
@@ -564,6 +569,20 @@ __device__ __forceinline__ void rl_ab(float zr, float zi, float u, float sl, flo
 }
 // gelu_tanh as z sigmoid(2 t): 1 + tanh(t) = 2 sigmoid(2 t)
 __device__ __forceinline__ float rl_gelu(float z) { return z * rl_sigmoid(1.5957691216057308f * (z + 0.044715f * z * z * z)); }
+
+// The four of them on n numbers, for their test: which 0 sigmoid, 1 one_minus_exp (of y, with e^(y/2) formed here), 2 sqrt, 3 gelu.
+__global__ void rglru_functions_kernel(float* __restrict__ out, const float* __restrict__ in, int n, int which) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n || !ZLM_CHK(in + i, 4) || !ZLM_CHK(out + i, 4)) return;
+    const float x = in[i];
+    out[i] = which == 0 ? rl_sigmoid(x) : which == 1 ? rl_one_minus_exp(x, expf(0.5f * x)) : which == 2 ? rl_sqrt(x) : rl_gelu(x);
+}
+extern "C" int zlm_rglru_functions(float* out, const float* in, int n, int which, cudaStream_t st) {
+    ZLM_REQUIRE(n > 0 && which >= 0 && which < 4, "rglru_functions: %d numbers, function %d", n, which);
+    zlm_count_launch();
+    rglru_functions_kernel<<<(n + 255) / 256, 256, 0, st>>>(out, in, n, which);
+    return zlm_check_launch("rglru_functions");
+}
 
 // A cluster of RL_CLUSTER blocks owns 64 channels of one sequence, a warp RL_P neighbouring tokens of two channels a lane, whose
 // decays and inputs it keeps in registers.  What a warp's tokens do to a state, S_out = A S_in + B, is folded over the block in
