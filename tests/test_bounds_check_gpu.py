@@ -30,6 +30,15 @@ def test_kernels_and_a_tiny_engine_stay_inside_their_tensors():
     assert " passed" in out and "failed" not in out, out
 
 
+def test_recurrences_over_prompts_and_32_bit_kernels_stay_inside_their_tensors():
+    """The kernels whose own tests walk along the edges of tiles, pieces, heads and sequences."""
+    rc, out = _run(["-m", "pytest", "-x", "-q", "--zlm-bounds-check", "-m", "gpu", "-p", "no:cacheprovider",
+                    "tests/test_piece_products_gpu.py", "tests/test_rglru_cluster_gpu.py", "tests/test_linear_attention_pieces_gpu.py",
+                    "tests/test_conv_runs_gpu.py", "tests/test_f32_tiles_gpu.py"])
+    assert rc == 0, out
+    assert " passed" in out and "failed" not in out, out
+
+
 STRAY = r"""
 import ctypes, sys, torch
 sys.path.insert(0, "tests")

@@ -139,6 +139,10 @@ struct VecW {
         return dtype == ZLM_DTYPE_F32 ? ((const float*)p)[i]
                                       : __bfloat162float(((const __nv_bfloat16*)p)[i]);
     }
+    // whether n elements from i on may be read (the bounds-check build asks; otherwise always)
+    __device__ __forceinline__ bool ok(int i, int n) const {
+        return ZLM_CHK((const char*)p + (size_t)i * (dtype == ZLM_DTYPE_F32 ? 4 : 2), (size_t)n * (dtype == ZLM_DTYPE_F32 ? 4 : 2));
+    }
     // elements i .. i + 3, i a multiple of 4 (the vector starts 16-byte aligned)
     __device__ __forceinline__ float4 load4(int i) const {
         if (dtype == ZLM_DTYPE_F32) return *(const float4*)((const float*)p + i);

@@ -476,8 +476,8 @@ rglru_conv_blocks_kernel(__nv_bfloat16* __restrict__ u16, int* __restrict__ grou
     if (c < W) {
 #pragma unroll
         for (int v = 0; v < 8; ++v) {
-            b[v] = bx ? to_f32(bx[c + v]) : 0.f;
-            bias[v] = cb ? to_f32(cb[c + v]) : 0.f;
+            b[v] = bx && ZLM_CHK(bx + c + v, 2) ? to_f32(bx[c + v]) : 0.f;
+            bias[v] = cb && ZLM_CHK(cb + c + v, 2) ? to_f32(cb[c + v]) : 0.f;
 #pragma unroll
             for (int j = 0; j < TAPS; ++j)
                 w[v][j] = ZLM_CHK(conv_w + (size_t)(c + v) * TAPS + j, 2) ? to_f32(conv_w[(size_t)(c + v) * TAPS + j]) : 0.f;
@@ -611,14 +611,15 @@ rglru_cluster_kernel(__nv_bfloat16* __restrict__ out, int out_stride, const floa
     float w[2][TAPS], xb[2], ub[2], yb[2], rb[2], ib[2], sl[2], S0[2] = {0.f, 0.f};
 #pragma unroll
     for (int v = 0; v < 2; ++v) {
-        xb[v] = (live && bx) ? to_f32(bx[c + v]) : 0.f;
-        ub[v] = (live && cb) ? to_f32(cb[c + v]) : 0.f;
-        yb[v] = (live && by) ? to_f32(by[c + v]) : 0.f;
-        rb[v] = (live && cr) ? to_f32(cr[c + v]) : 0.f;
-        ib[v] = (live && ci) ? to_f32(ci[c + v]) : 0.f;
-        sl[v] = live ? softplus_f(to_f32(lam[c + v])) * c_decay : 0.f;
+        xb[v] = (live && bx && ZLM_CHK(bx + c + v, 2)) ? to_f32(bx[c + v]) : 0.f;
+        ub[v] = (live && cb && ZLM_CHK(cb + c + v, 2)) ? to_f32(cb[c + v]) : 0.f;
+        yb[v] = (live && by && ZLM_CHK(by + c + v, 2)) ? to_f32(by[c + v]) : 0.f;
+        rb[v] = (live && cr && ZLM_CHK(cr + c + v, 2)) ? to_f32(cr[c + v]) : 0.f;
+        ib[v] = (live && ci && ZLM_CHK(ci + c + v, 2)) ? to_f32(ci[c + v]) : 0.f;
+        sl[v] = live && ZLM_CHK(lam + c + v, 2) ? softplus_f(to_f32(lam[c + v])) * c_decay : 0.f;
 #pragma unroll
-        for (int j = 0; j < TAPS; ++j) w[v][j] = live ? to_f32(conv_w[(size_t)(c + v) * TAPS + j]) : 0.f;
+        for (int j = 0; j < TAPS; ++j)
+            w[v][j] = live && ZLM_CHK(conv_w + (size_t)(c + v) * TAPS + j, 2) ? to_f32(conv_w[(size_t)(c + v) * TAPS + j]) : 0.f;
     }
     pdl_wait();
     int row0 = 0, n = 0, slot = 0, start = 0;
@@ -1173,7 +1174,7 @@ linear_attention_out_kernel(float* __restrict__ o, const TA* __restrict__ proj, 
     if (out.y)
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-            if (c + e < V) wn[e] = out.w[c + e];
+            if (c + e < V && out.w.ok(c + e, 1)) wn[e] = out.w[c + e];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const int j = warp * 8 + i;

@@ -300,7 +300,7 @@ __device__ __forceinline__ void rm_stage(__nv_bfloat16* qt, __nv_bfloat16* kt, c
                 if (ZLM_CHK(c, 4)) t.cs[e] = *c;
                 if (ZLM_CHK(s, 4)) t.sn[e] = *s;
             } else {
-                sincosf((float)(pos0 + l) * rot.inv_freq[f0 + e], &t.sn[e], &t.cs[e]);
+                if (ZLM_CHK(rot.inv_freq + f0 + e, 4)) sincosf((float)(pos0 + l) * rot.inv_freq[f0 + e], &t.sn[e], &t.cs[e]);
             }
         }
     };
@@ -355,6 +355,8 @@ retention_piece_state_kernel(float* __restrict__ part, const __nv_bfloat16* __re
     __shared__ float pw[SM_L + 1], kw[SM_L];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y, c0 = blockIdx.z * 128;
     const int r = blockIdx.x / maxp, first = (blockIdx.x % maxp) * SM_L;
+    // (ahead of pdl_wait(): the decays are weights, and the step's integer arrays are copied in ahead of its first kernel; no
+    // kernel of a step may write them)
     if (!ZLM_CHK(cu_seqlens + r, 8) || !ZLM_CHK(seq_start + r, 4) || !ZLM_CHK(decay + h, 4)) return;
     const int n = min(SM_L, cu_seqlens[r + 1] - cu_seqlens[r] - first);
     if (n <= 0) return;
@@ -395,6 +397,8 @@ retention_piece_out_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, in
     __shared__ float pw[SM_L + 1], red[SM_L][2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y, c0 = blockIdx.z * 128;
     const int r = blockIdx.x / maxp, first = (blockIdx.x % maxp) * SM_L;
+    // (ahead of pdl_wait(): the decays are weights, and the step's integer arrays are copied in ahead of its first kernel; no
+    // kernel of a step may write them)
     if (!ZLM_CHK(cu_seqlens + r, 8) || !ZLM_CHK(seq_start + r, 4) || !ZLM_CHK(decay + h, 4)) return;
     const int n = min(SM_L, cu_seqlens[r + 1] - cu_seqlens[r] - first);
     if (n <= 0) return;

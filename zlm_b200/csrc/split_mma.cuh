@@ -442,7 +442,7 @@ __device__ __forceinline__ void sm_write(const SmSum<8>& acc, float f0, float f8
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int at = (out.w_rows ? h * V : 0) + c + i * 8;
-            w[i] = c + i * 8 < V ? make_float2(out.w[at], out.w[at + 1]) : make_float2(0.f, 0.f);
+            w[i] = c + i * 8 < V && out.w.ok(at, 2) ? make_float2(out.w[at], out.w[at + 1]) : make_float2(0.f, 0.f);
         }
     }
     dec_wait<0>();
