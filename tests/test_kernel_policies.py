@@ -135,3 +135,16 @@ def test_latent_decode_splits_cover_the_pages():
                         assert per >= 2
                     if bucket * rows * tiles > 2 * wave and splits < 1024:
                         assert splits * rows * tiles <= wave + rows * tiles
+
+
+@pytest.mark.parametrize("R,H,D,V,maxp,fits", [
+    (1, 1, 128, 65536, 1, 1), (1, 2, 64, 128 * 65535, 2, 1), (1, 1, 1, 128 * 65535 + 1, 1, 0),        # 128 columns by 65,535
+    (1 << 20, 16, 64, 128, 1, 1), (1 << 20, 32, 64, 128, 1, 0)])                                       # sequences x heads x rows
+def test_linear_attention_takes_wide_heads(lib, R, H, D, V, maxp, fits):
+    assert lib.zlm_linear_attention_fits(R, H, D, V, maxp) == fits
+
+
+@pytest.mark.parametrize("R,max_new,takes", [(1, 1, 1), (65535, 1, 1), (65536, 1, 0), (1, 32 * 65535, 1), (1, 32 * 65535 + 1, 0)])
+def test_32_bit_attention_leaves_what_its_tiles_cannot_number_to_single_queries(lib, R, max_new, takes):
+    from ctypes import c_float
+    assert lib.zlm_attention_f32_tile_supported(16, 4, 128, 2048, 2048, c_float(0.0), 1, 0, 0, R, max_new) == takes

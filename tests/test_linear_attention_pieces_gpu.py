@@ -48,3 +48,23 @@ def test_pieces(H, D, V, news, starts, dtype, per_head):
     z = gate.double()
     close(y, (unit(want) * w.double()).flatten(1) * z * torch.sigmoid(z), 4e-3 if dtype == torch.bfloat16 else 2e-6)
     close(state, S, 1e-6)
+
+
+def test_states_of_more_blocks_than_a_grids_second_dimension():
+    """A head of 600,008 value columns over 64 rows: its state's chain has 75,001 blocks.  Columns know nothing of each other: its
+    first and last ones are those of narrow heads, to the bit."""
+    from zlm_b200.kernels import get_kernels
+    k, T, D, V, n = get_kernels(), 128, 64, 600_008, 136
+    g = torch.Generator(device="cuda").manual_seed(3)
+    qk, v = (torch.randn((T, w), generator=g, device="cuda").bfloat16() for w in (2 * D, V))
+    alpha, first = torch.rand((T, D), generator=g, device="cuda"), torch.randn((1, 1, D, V), generator=g, device="cuda")
+
+    def run(columns):
+        w = len(range(V)[columns])
+        state, o = first[..., columns].clone(), torch.empty((T, w), device="cuda")
+        k.linear_attention(o, torch.cat([qk, v[:, columns]], 1), 0, D, 2 * D, alpha, None, state, plan_of([T], [0]), 1, D, w, 0.3)
+        return o, state
+    o, state = run(slice(None))
+    for columns in (slice(n), slice(V - n, None)):
+        for a, b in zip((o[:, columns], state[..., columns]), run(columns)):
+            assert torch.equal(a, b)

@@ -378,7 +378,9 @@ attention_f32_tile_kernel(float* __restrict__ out, int out_stride, const float* 
 // head sizes that the tile kernel is built for, and rows it can read 16 bytes at a time; no cap, no bias, no kept first
 // keys, every key head with its own value head (the kernel above takes those, and everything else)
 extern "C" int zlm_attention_f32_tile_supported(int nq, int nkv, int hd, int q_stride, int out_stride, float softcap, int v_share,
-                                                int keep, int has_bias) {
+                                                int keep, int has_bias, int R, int max_new) {
+    // (a grid's second and third dimension end at 65,535: two million tokens of one sequence, and as many sequences)
+    if (R > 65535 || (max_new - 1) / AT_Q >= 65535) return 0;
     return (hd == 64 || hd == 96 || hd == 128) && nq > 0 && nkv > 0 && nq % nkv == 0 && q_stride % 4 == 0 && out_stride % 4 == 0 &&
            softcap == 0.f && v_share == 1 && keep == 0 && !has_bias;
 }
@@ -410,11 +412,11 @@ extern "C" int zlm_attention_f32_tile(float* out, int out_stride, const float* q
                                       const int* seq_start, int R, int max_new, int nq, int nkv, int hd, float scale, int window,
                                       int sink, int chunk, const float* sinks, cudaStream_t st) {
     if (R == 0 || max_new == 0) return ZLM_OK;
-    ZLM_REQUIRE(zlm_attention_f32_tile_supported(nq, nkv, hd, q_stride, out_stride, 0.f, 1, 0, 0) && (uintptr_t)q % 16 == 0 &&
+    ZLM_REQUIRE(zlm_attention_f32_tile_supported(nq, nkv, hd, q_stride, out_stride, 0.f, 1, 0, 0, R, max_new) && (uintptr_t)q % 16 == 0 &&
                     (uintptr_t)out % 16 == 0 && (uintptr_t)pool % 16 == 0,
-                "attention: %d query heads over %d kv heads of %d, rows of %d and %d floats", nq, nkv, hd, q_stride, out_stride);
-    ZLM_REQUIRE(window >= 0 && chunk >= 0 && R <= 65535 && (max_new + AT_Q - 1) / AT_Q <= 65535,
-                "attention: window=%d, %d sequences of up to %d tokens", window, R, max_new);
+                "attention: %d query heads over %d kv heads of %d, rows of %d and %d floats, %d sequences of up to %d tokens", nq, nkv, hd,
+                q_stride, out_stride, R, max_new);
+    ZLM_REQUIRE(window >= 0 && chunk >= 0, "attention: window=%d, chunk=%d", window, chunk);
     const dim3 grid(nq, (max_new + AT_Q - 1) / AT_Q, R);
 #define ZLM_AT(HD) launch_f32_tile<HD>(grid, st, out, out_stride, q, q_stride, pool, block_table, table_stride, cu_seqlens, seq_slot, \
                                        seq_start, nq, nkv, scale, window, sink, chunk, sinks)

@@ -890,14 +890,14 @@ linear_attention_kernel(float* __restrict__ o, const TA* __restrict__ proj, int 
     __shared__ __align__(16) float sq[LA_CH][DP], sk[LA_CH][DP], sa[LA_CH][DP];
     __shared__ __align__(16) float sv[LA_CH][COLS];
     pdl_trigger();
-    const int unit = blockIdx.x / H, h = blockIdx.x % H, v0 = blockIdx.y * COLS, tid = threadIdx.x;
+    const int unit = blockIdx.x / H, h = blockIdx.x % H, v0 = (blockIdx.y + blockIdx.z * gridDim.y) * COLS, tid = threadIdx.x;
     const int r = MODE == 0 ? unit : unit / maxp, p = MODE == 0 ? 0 : unit % maxp;
     const int grp = tid / DS, lane_d = tid % DS, v = v0 + grp * LA_CPT;
     pdl_wait();
     if (!ZLM_CHK(seq_slot + r, 4) || !ZLM_CHK(cu_seqlens + r, 8)) return;
     const int slot = seq_slot[r], row0 = cu_seqlens[r], n = cu_seqlens[r + 1] - row0;
     const int lo = MODE == 0 ? 0 : p * L, hi = MODE == 0 ? n : min(n, lo + L);
-    if (lo >= hi) return;
+    if (lo >= hi || v0 >= V) return;
     float* sp = (MODE == 0 ? state + (((size_t)slot * H + h) * D) * V : part + ((((size_t)r * maxp + p) * H + h) * D) * V) + v;
     float2 S[DPT / 2][LA_CPT];
 #pragma unroll
@@ -998,14 +998,14 @@ linear_attention_kernel(float* __restrict__ o, const TA* __restrict__ proj, int 
                     if (v + c < V && ZLM_CHK(dst + c, 4)) dst[c] = t[c];
             }
         }
-    if (MODE == 1 && blockIdx.y == 0 && tid < D) {
+    if (MODE == 1 && v0 == 0 && tid < D) {
         float* pp = pdecay + (((size_t)r * maxp + p) * H + h) * D + tid;
         if (ZLM_CHK(pp, 4)) *pp = pd;
     }
 }
 
 // The pieces' states in order: part[piece] becomes the state the piece starts from, the sequence's state is left.
-// (a thread owns VEC neighbouring numbers of one row of the state; eight pieces' loads in flight.)  grid (R * H, ceil(D * V / (128 VEC)))
+// (a thread owns VEC neighbouring numbers of one row of the state; eight pieces' loads in flight.)  grid la_grid(R * H, ceil(D * V / (128 VEC)))
 #define CHAIN_AHEAD 8
 template <int VEC>
 __global__ void __launch_bounds__(128)
@@ -1014,7 +1014,7 @@ linear_attention_chain_kernel(float* __restrict__ part, const float* __restrict_
                               int maxp, int L) {
     struct alignas(4 * VEC) Num { float v[VEC]; };
     pdl_trigger();
-    const int rh = blockIdx.x, r = rh / H, h = rh % H, e = (blockIdx.y * 128 + threadIdx.x) * VEC, d = e / V;
+    const int rh = blockIdx.x, r = rh / H, h = rh % H, e = ((blockIdx.y + blockIdx.z * gridDim.y) * 128 + threadIdx.x) * VEC, d = e / V;
     pdl_wait();
     if (e >= D * V || !ZLM_CHK(seq_slot + r, 4) || !ZLM_CHK(cu_seqlens + r, 8)) return;
     const int slot = seq_slot[r], n = cu_seqlens[r + 1] - cu_seqlens[r];
@@ -1232,6 +1232,13 @@ static int launch_la_out(dim3 grid, cudaStream_t st, float* o, const void* proj,
     return ZLM_OK;
 }
 
+// blocks `n` of a unit over a grid's second and third dimension, which end at 65,535
+static dim3 la_grid(int units, int n) { return n <= 65535 ? dim3(units, n) : dim3(units, 65535, (n + 65534) / 65535); }
+// R sequences in maxp pieces each (1: whole)
+extern "C" int zlm_linear_attention_fits(int R, int H, int D, int V, int maxp) {
+    return (long long)R * H * maxp <= 2147483647LL && (long long)R * H * D <= 2147483647LL && (V + 127) / 128 <= 65535;
+}
+
 // q, k [H*D], v [H*V]: columns of proj from q_off, k_off, v_off on (element type); alpha [T][H*D] fp32 decays per token
 // and key channel, or null with head_decay [H] fp32 (one decay a head); state [slots][H][D][V] fp32; o [T][H*V] fp32.
 // pieces: null, or R * ceil(max_new / 32) * H * D * (V + 1) floats: sequences run in pieces of 32 tokens side by side
@@ -1249,25 +1256,24 @@ extern "C" int zlm_linear_attention(float* o, const void* proj, int proj_stride,
     ZLM_REQUIRE(!pieces || max_new > 0, "linear_attention: pieces without the longest sequence");
     ZLM_REQUIRE(!y || (pieces && V <= 128 && g && w), "linear_attention: heads of %d columns do not take their gate along", V);
     const int L = LA_PIECE, maxp = pieces ? (max_new + L - 1) / L : 1;
-    ZLM_REQUIRE((long long)R * H * maxp <= 2147483647LL && (long long)R * H * D <= 2147483647LL && (V + 63) / 64 <= 65535 &&
-                    ((long long)D * V + 127) / 128 <= 65535, "linear_attention: too many sequences or columns");
+    ZLM_REQUIRE(zlm_linear_attention_fits(R, H, D, V, maxp), "linear_attention: too many sequences or columns");
     const dim3 pgrid(R * maxp * H, (V + 127) / 128);
     float* part = pieces;
     float* pdecay = pieces ? pieces + (size_t)R * maxp * H * D * V : nullptr;
     const LaOut out{y, y_stride, g, g_stride, VecW{w, w_dtype}, eps, act};
     int rc = ZLM_OK;
 #define ZLM_LA(TA, DR, SP, MODE, G)                                                                                            \
-    zlm_launch(linear_attention_kernel<TA, DR, SP, MODE>, dim3(G, (V + 512 * SP / DR - 1) / (512 * SP / DR)), dim3(128), 0, st, o, (const TA*)proj, proj_stride, q_off, k_off, v_off, \
+    zlm_launch(linear_attention_kernel<TA, DR, SP, MODE>, la_grid(G, (V + 512 * SP / DR - 1) / (512 * SP / DR)), dim3(128), 0, st, o, (const TA*)proj, proj_stride, q_off, k_off, v_off, \
                alpha, head_decay, state, seq_slot, cu_seqlens, H, D, V, q_scale, part, pdecay, maxp, L)
 #define ZLM_LA_RUN(TA, DR, SP)                                                                                              \
     do {                                                                                                                   \
         if (!pieces) { ZLM_LA(TA, DR, SP, 0, R * H); break; }                                                               \
         ZLM_LA(TA, DR, SP, 1, R * maxp * H);                                                                                      \
         if (V % 4 == 0 && (uintptr_t)state % 16 == 0 && (uintptr_t)part % 16 == 0)                                         \
-            zlm_launch(linear_attention_chain_kernel<4>, dim3(R * H, (D * V + 511) / 512), dim3(128), 0, st, part,         \
+            zlm_launch(linear_attention_chain_kernel<4>, la_grid(R * H, (D * V + 511) / 512), dim3(128), 0, st, part,         \
                        (const float*)pdecay, state, seq_slot, cu_seqlens, H, D, V, maxp, L);                               \
         else                                                                                                               \
-            zlm_launch(linear_attention_chain_kernel<1>, dim3(R * H, (D * V + 127) / 128), dim3(128), 0, st, part,         \
+            zlm_launch(linear_attention_chain_kernel<1>, la_grid(R * H, (D * V + 127) / 128), dim3(128), 0, st, part,         \
                        (const float*)pdecay, state, seq_slot, cu_seqlens, H, D, V, maxp, L);                               \
         rc = launch_la_out<TA, DR>(pgrid, st, o, proj, proj_stride, q_off, alpha, head_decay, part, cu_seqlens, H, D, V,   \
                                    q_scale, maxp, out);                                                                    \

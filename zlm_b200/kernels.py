@@ -808,10 +808,10 @@ class CudaKernels:
         # behind 62 cached ones 20 / 12, behind 4,000 650 / 343; 64 sequences' tokens behind 64 47 / 73, behind 1,000 621 / 519
         if (q.dtype == torch.float32 and plan is not None and getattr(plan, "cu_seqlens", None) is not None
                 and int(getattr(plan, "max_len", 0) or plan.max_new) >= (32 if int(plan.max_new) > 1 else 512)
-                and plan.R <= 65535 and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
+                and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
                 and self.lib.zlm_attention_f32_tile_supported(c_int(nq), c_int(nkv), c_int(hd), c_int(q.stride(0)),
                                                               c_int(out.stride(0)), c_float(softcap), c_int(v_share), c_int(keep),
-                                                              c_int(bias is not None))):
+                                                              c_int(bias is not None), c_int(plan.R), c_int(int(plan.max_new)))):
             self._call("zlm_attention_f32_tile", self._p(out), c_int(out.stride(0)), self._p(q), c_int(q.stride(0)), self._p(pool),
                        self._p(block_table), c_int(block_table.stride(0)), self._p(plan.cu_seqlens), self._p(plan.seq_slot),
                        self._p(plan.seq_start), c_int(plan.R), c_int(plan.max_new), c_int(nq), c_int(nkv), c_int(hd), c_float(scale),
