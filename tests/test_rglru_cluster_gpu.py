@@ -106,3 +106,30 @@ def test_gelu_over_the_whole_range():
     assert edge[0] == float("inf") and torch.isnan(edge[1:]).all()
     edge = _function(0, torch.tensor([float("inf"), float("-inf"), -200.0], device="cuda"))
     assert edge.tolist() == [1.0, 0.0, 0.0]
+
+
+@pytest.mark.parametrize("taps", [1, 4, 8])
+def test_every_cluster_size_gives_the_same_bits(taps, monkeypatch):
+    """Sequences from one token to more than two rounds of the largest cluster, side by side: blocks without a token leave, and the
+    blocks' parts are folded one after the other whatever shares them."""
+    from zlm_b200.kernels import get_kernels
+    k, W, blocks = get_kernels(), 96, 2
+    news, starts = [1, 128, 2, 1100, 64, 65, 1, 513, 9], [5, 0, 1, 300, 0, 2, 0, 7, 40]
+    plan, T, bs = plan_of(news, starts), sum(news), W // blocks
+    g = torch.Generator(device="cuda").manual_seed(taps)
+
+    def rand(*shape, scale=1.0):
+        return (torch.randn(shape, generator=g, device="cuda") * scale).bfloat16()
+    proj, gates = rand(T, 2 * W), rand(blocks, 2 * bs, bs, scale=bs ** -0.5)
+    bx, by, cb, cr, ci, lam = (rand(W, scale=0.3) for _ in range(6))
+    conv_w, first = rand(W, taps, scale=0.5), torch.randn((plan.R, taps, W), generator=g, device="cuda")
+    ar, ai = (gates[:, i * bs:(i + 1) * bs].contiguous() for i in (0, 1))
+    results = []
+    for size in (8, 4, 2, 1):
+        monkeypatch.setattr(k.lib, "zlm_rglru_cluster_size", lambda *a: size)
+        state, out = first.clone(), torch.full((T, W), float("nan"), device="cuda", dtype=torch.bfloat16)
+        k.rglru(out, proj, W, 0, bx, by, conv_w, cb, ar, ai, cr, ci, lam, 8.0, state, plan, W, blocks, taps, gates=gates)
+        results.append((out, state))
+    assert not torch.isnan(results[0][0]).any()
+    for out, state in results[1:]:
+        assert torch.equal(out, results[0][0]) and torch.equal(state, results[0][1])

@@ -584,15 +584,16 @@ extern "C" int zlm_rglru_functions(float* out, const float* in, int n, int which
     return zlm_check_launch("rglru_functions");
 }
 
-// A cluster of RL_CLUSTER blocks owns 64 channels of one sequence, a warp RL_P neighbouring tokens of two channels a lane, whose
+// A cluster of up to RL_CLUSTER blocks owns 64 channels of one sequence, a warp RL_P neighbouring tokens of two channels a lane, whose
 // decays and inputs it keeps in registers.  What a warp's tokens do to a state, S_out = A S_in + B, is folded over the block in
 // shared memory and over the cluster in distributed shared memory; then every warp knows the state it starts from and walks
-// its tokens.  Longer sequences go round again.  Bound by its exponentials and divisions (about 110 instructions a number).
+// its tokens.  Longer sequences go round again; of a shorter one the warps without a token only meet the barriers, and the
+// blocks without one leave at once (a barrier waits for the threads that are left).  Bound by its exponentials and divisions (about 110 instructions a number).
 #define RL_CLUSTER 8
 #define RL_WARPS 8
 #define RL_P 8
 template <int TAPS>
-__global__ void __cluster_dims__(RL_CLUSTER, 1, 1) __launch_bounds__(RL_WARPS * 32, 2)
+__global__ void __launch_bounds__(RL_WARPS * 32, 2)
 rglru_cluster_kernel(__nv_bfloat16* __restrict__ out, int out_stride, const float* __restrict__ z, const __nv_bfloat16* __restrict__ proj,
                      int proj_stride, int x_off, int y_off, const __nv_bfloat16* __restrict__ bx, const __nv_bfloat16* __restrict__ by,
                      const __nv_bfloat16* __restrict__ conv_w, const __nv_bfloat16* __restrict__ cb, const __nv_bfloat16* __restrict__ cr,
@@ -604,10 +605,10 @@ rglru_cluster_kernel(__nv_bfloat16* __restrict__ out, int out_stride, const floa
     __shared__ float2 total[2][64];
     __shared__ float begin[RL_WARPS][64];
     cg::cluster_group cluster = cg::this_cluster();
-    const int rank = (int)cluster.block_rank(), r = blockIdx.x / RL_CLUSTER;
+    const int rank = (int)cluster.block_rank(), r = blockIdx.x / (int)cluster.num_blocks();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.y * 64 + lane * 2;
     pdl_trigger();
-    bool live = c < W;                               // (no thread leaves early: the cluster meets at barriers)
+    bool live = c < W;                               // (no thread leaves its block: the block's others wait for it)
     float w[2][TAPS], xb[2], ub[2], yb[2], rb[2], ib[2], sl[2], S0[2] = {0.f, 0.f};
 #pragma unroll
     for (int v = 0; v < 2; ++v) {
@@ -629,77 +630,82 @@ rglru_cluster_kernel(__nv_bfloat16* __restrict__ out, int out_stride, const floa
         slot = seq_slot[r];
         start = seq_start[r];
     }
+    // the blocks of the cluster that the sequence has tokens for
+    const int ranks = min((int)cluster.num_blocks(), max(1, (n + RL_WARPS * RL_P - 1) / (RL_WARPS * RL_P)));
+    if (rank >= ranks) return;
     float* sp = state + (size_t)slot * TAPS * W + c;
     live = live && ZLM_CHK(sp, 8);
     if (live) { S0[0] = sp[0]; S0[1] = sp[1]; }
     const float* zp = z + ((size_t)(c / bs) * Tp + row0) * 2 * bs + c % bs;
     int par = 0;
-    for (int base = 0; base < n; base += RL_CLUSTER * RL_WARPS * RL_P, par ^= 1) {
+    for (int base = 0; base < n; base += ranks * RL_WARPS * RL_P, par ^= 1) {
         const int lo = base + (rank * RL_WARPS + warp) * RL_P, cnt = live ? min(n - lo, RL_P) : 0;
         float2 zr[RL_P], zi[RL_P];
         unsigned xr[RL_P + TAPS - 1], yr[RL_P];
+        float A[2] = {1.f, 1.f}, B[2] = {0.f, 0.f};
+        if (lo < n) {
 #pragma unroll
-        for (int j = 0; j < RL_P; ++j) {
-            const float* q = zp + (size_t)(lo + j) * 2 * bs;
-            const bool ok = j < cnt && ZLM_CHK(q, 8) && ZLM_CHK(q + bs, 8);
-            zr[j] = ok ? *(const float2*)q : make_float2(0.f, 0.f);
-            zi[j] = ok ? *(const float2*)(q + bs) : make_float2(0.f, 0.f);
-        }
-#pragma unroll
-        for (int j = 0; j < RL_P + TAPS - 1; ++j) {
-            const int i = lo - (TAPS - 1) + j;
-            const __nv_bfloat16* q = proj + (size_t)(row0 + i) * proj_stride + x_off + c;
-            xr[j] = (live && i >= 0 && i < n && ZLM_CHK(q, 4)) ? *(const unsigned*)q : 0u;
-        }
-#pragma unroll
-        for (int j = 0; j < RL_P; ++j) {
-            const __nv_bfloat16* q = proj + (size_t)(row0 + lo + j) * proj_stride + y_off + c;
-            yr[j] = (j < cnt && ZLM_CHK(q, 4)) ? *(const unsigned*)q : 0u;
-        }
-        float u[RL_P][2];
-        if (lo >= TAPS - 1) {                        // (every tap of every token is one of the step's)
-            float x[2][RL_P + TAPS - 1];
-#pragma unroll
-            for (int j = 0; j < RL_P + TAPS - 1; ++j) {
-                x[0][j] = __uint_as_float(xr[j] << 16) + xb[0];
-                x[1][j] = __uint_as_float(xr[j] & 0xffff0000u) + xb[1];
+            for (int j = 0; j < RL_P; ++j) {
+                const float* q = zp + (size_t)(lo + j) * 2 * bs;
+                const bool ok = j < cnt && ZLM_CHK(q, 8) && ZLM_CHK(q + bs, 8);
+                zr[j] = ok ? *(const float2*)q : make_float2(0.f, 0.f);
+                zi[j] = ok ? *(const float2*)(q + bs) : make_float2(0.f, 0.f);
             }
 #pragma unroll
-            for (int j = 0; j < RL_P; ++j)
+            for (int j = 0; j < RL_P + TAPS - 1; ++j) {
+                const int i = lo - (TAPS - 1) + j;
+                const __nv_bfloat16* q = proj + (size_t)(row0 + i) * proj_stride + x_off + c;
+                xr[j] = (live && i >= 0 && i < n && ZLM_CHK(q, 4)) ? *(const unsigned*)q : 0u;
+            }
 #pragma unroll
-                for (int v = 0; v < 2; ++v) {
-                    u[j][v] = ub[v];
+            for (int j = 0; j < RL_P; ++j) {
+                const __nv_bfloat16* q = proj + (size_t)(row0 + lo + j) * proj_stride + y_off + c;
+                yr[j] = (j < cnt && ZLM_CHK(q, 4)) ? *(const unsigned*)q : 0u;
+            }
+            float u[RL_P][2];
+            if (lo >= TAPS - 1) {                        // (every tap of every token is one of the step's)
+                float x[2][RL_P + TAPS - 1];
 #pragma unroll
-                    for (int k = 0; k < TAPS; ++k) u[j][v] = fmaf(w[v][k], x[v][j + k], u[j][v]);
+                for (int j = 0; j < RL_P + TAPS - 1; ++j) {
+                    x[0][j] = __uint_as_float(xr[j] << 16) + xb[0];
+                    x[1][j] = __uint_as_float(xr[j] & 0xffff0000u) + xb[1];
                 }
-        } else {
 #pragma unroll
-            for (int j = 0; j < RL_P; ++j)
+                for (int j = 0; j < RL_P; ++j)
 #pragma unroll
-                for (int v = 0; v < 2; ++v) {
-                    u[j][v] = ub[v];
+                    for (int v = 0; v < 2; ++v) {
+                        u[j][v] = ub[v];
 #pragma unroll
-                    for (int k = 0; k < TAPS; ++k) {
-                        const int i = lo + j - (TAPS - 1) + k;
-                        if (start + i < 0) continue;
-                        float x;
-                        if (i >= 0) x = __uint_as_float(v ? xr[j + k] & 0xffff0000u : xr[j + k] << 16) + xb[v];
-                        else x = (j < cnt && ZLM_CHK(sp + (size_t)(TAPS + i) * W + v, 4)) ? sp[(size_t)(TAPS + i) * W + v] : 0.f;
-                        u[j][v] = fmaf(w[v][k], x, u[j][v]);
+                        for (int k = 0; k < TAPS; ++k) u[j][v] = fmaf(w[v][k], x[v][j + k], u[j][v]);
                     }
-                }
-        }
-        float A[2] = {1.f, 1.f}, B[2] = {0.f, 0.f};
+            } else {
 #pragma unroll
-        for (int j = 0; j < RL_P; ++j) {
+                for (int j = 0; j < RL_P; ++j)
 #pragma unroll
-            for (int v = 0; v < 2; ++v) {
-                float a, b;
-                rl_ab((v ? zr[j].y : zr[j].x) + rb[v], (v ? zi[j].y : zi[j].x) + ib[v], u[j][v], sl[v], a, b);
-                if (v) { zr[j].y = a; zi[j].y = b; } else { zr[j].x = a; zi[j].x = b; }
-                if (j < cnt) {
-                    A[v] *= a;
-                    B[v] = fmaf(a, B[v], b);
+                    for (int v = 0; v < 2; ++v) {
+                        u[j][v] = ub[v];
+#pragma unroll
+                        for (int k = 0; k < TAPS; ++k) {
+                            const int i = lo + j - (TAPS - 1) + k;
+                            if (start + i < 0) continue;
+                            float x;
+                            if (i >= 0) x = __uint_as_float(v ? xr[j + k] & 0xffff0000u : xr[j + k] << 16) + xb[v];
+                            else x = (j < cnt && ZLM_CHK(sp + (size_t)(TAPS + i) * W + v, 4)) ? sp[(size_t)(TAPS + i) * W + v] : 0.f;
+                            u[j][v] = fmaf(w[v][k], x, u[j][v]);
+                        }
+                    }
+            }
+#pragma unroll
+            for (int j = 0; j < RL_P; ++j) {
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    float a, b;
+                    rl_ab((v ? zr[j].y : zr[j].x) + rb[v], (v ? zi[j].y : zi[j].x) + ib[v], u[j][v], sl[v], a, b);
+                    if (v) { zr[j].y = a; zi[j].y = b; } else { zr[j].x = a; zi[j].x = b; }
+                    if (j < cnt) {
+                        A[v] *= a;
+                        B[v] = fmaf(a, B[v], b);
+                    }
                 }
             }
         }
@@ -723,7 +729,7 @@ rglru_cluster_kernel(__nv_bfloat16* __restrict__ out, int out_stride, const floa
             for (int v = 0; v < 2; ++v) {
                 float2 t[RL_CLUSTER];
 #pragma unroll
-                for (int k = 0; k < RL_CLUSTER; ++k) t[k] = cluster.map_shared_rank(&total[par][0], k)[lane * 2 + v];
+                for (int k = 0; k < RL_CLUSTER; ++k) t[k] = k < ranks ? cluster.map_shared_rank(&total[par][0], k)[lane * 2 + v] : make_float2(1.f, 0.f);
                 float q = S0[v], s = q;
 #pragma unroll
                 for (int k = 0; k < RL_CLUSTER; ++k) {
@@ -785,25 +791,56 @@ extern "C" int zlm_rglru_conv_blocks(void* u16, int* group_of_tile, const void* 
     return zlm_check_launch("rglru_conv_blocks");
 }
 
-// The third: z [blocks][Tp][2][W/blocks] fp32 holds the gates' logits without their biases.
+// Blocks of a sequence's cluster: the size of the least estimate.  Every round of a cluster takes RL_ROUND, one after the other
+// (loads, exponentials, two barriers); all blocks of the step, most of them of short sequences where one is long, take
+// RL_LEAVE for each time that the GPU is full of them.
+#define RL_ROUND 4.0f
+#define RL_LEAVE 1.5f
+extern "C" int zlm_rglru_cluster_size(int R, int max_new, int W) {
+    int best = RL_CLUSTER;
+    float least = 0.f;
+    for (int c = RL_CLUSTER; c; c >>= 1) {
+        const float rounds = (float)((max_new + RL_WARPS * RL_P * c - 1) / (RL_WARPS * RL_P * c));
+        const float est = rounds * RL_ROUND + (float)R * c * ((W + 63) / 64) / 296.f * RL_LEAVE;
+        if (c == RL_CLUSTER || est < least) { best = c; least = est; }
+    }
+    return best;
+}
+
+// The third: z [blocks][Tp][2][W/blocks] fp32 holds the gates' logits without their biases; `cluster` blocks a sequence.
 extern "C" int zlm_rglru_cluster(void* out, int out_stride, const float* z, const void* proj, int proj_stride, int x_off, int y_off,
                                  const void* bx, const void* by, const void* conv_w, const void* cb, const void* cr, const void* ci,
                                  const void* lam, float c_decay, float* state, const int* seq_slot, const int* seq_start,
-                                 const int* cu_seqlens, int T, int R, int W, int blocks, int taps, float out_scale, cudaStream_t st) {
+                                 const int* cu_seqlens, int T, int R, int W, int blocks, int taps, float out_scale, int cluster,
+                                 cudaStream_t st) {
     if (T == 0) return ZLM_OK;
     ZLM_REQUIRE(W > 0 && blocks > 0 && W % blocks == 0 && (W / blocks) % 8 == 0, "rglru: %d channels in %d blocks", W, blocks);
     ZLM_REQUIRE(taps >= 1 && taps <= RC_MAX_TAPS, "rglru: %d taps (at most %d)", taps, RC_MAX_TAPS);
+    ZLM_REQUIRE(cluster == 1 || cluster == 2 || cluster == 4 || cluster == 8, "rglru: clusters of %d blocks", cluster);
     ZLM_REQUIRE(proj_stride % 2 == 0 && x_off % 2 == 0 && y_off % 2 == 0 && out_stride % 2 == 0 && (uintptr_t)proj % 4 == 0 &&
                     (uintptr_t)out % 4 == 0 && (uintptr_t)z % 8 == 0 && (W + 63) / 64 <= 65535 && R > 0 && R <= (1 << 27),
                 "rglru: rows of %d and %d, %d sequences", proj_stride, out_stride, R);
     const int Tp = (T + 127) / 128 * 128;
-    const dim3 grid(R * RL_CLUSTER, (W + 63) / 64);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(R * cluster, (W + 63) / 64);
+    cfg.blockDim = dim3(RL_WARPS * 32);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = zlm_pdl_enabled() ? 2 : 1;
+    zlm_count_launch();
 #define ZLM_RL(N)                                                                                                               \
     case N:                                                                                                                     \
-        zlm_launch(rglru_cluster_kernel<N>, grid, dim3(RL_WARPS * 32), 0, st, (__nv_bfloat16*)out, out_stride, z,               \
-                   (const __nv_bfloat16*)proj, proj_stride, x_off, y_off, (const __nv_bfloat16*)bx, (const __nv_bfloat16*)by,   \
-                   (const __nv_bfloat16*)conv_w, (const __nv_bfloat16*)cb, (const __nv_bfloat16*)cr, (const __nv_bfloat16*)ci,  \
-                   (const __nv_bfloat16*)lam, c_decay, state, seq_slot, seq_start, cu_seqlens, Tp, W, W / blocks, out_scale);   \
+        cudaLaunchKernelEx(&cfg, rglru_cluster_kernel<N>, (__nv_bfloat16*)out, out_stride, z, (const __nv_bfloat16*)proj,       \
+                           proj_stride, x_off, y_off, (const __nv_bfloat16*)bx, (const __nv_bfloat16*)by, (const __nv_bfloat16*)conv_w, \
+                           (const __nv_bfloat16*)cb, (const __nv_bfloat16*)cr, (const __nv_bfloat16*)ci, (const __nv_bfloat16*)lam, \
+                           c_decay, state, seq_slot, seq_start, cu_seqlens, Tp, W, W / blocks, out_scale);                      \
         break;
     switch (taps) { ZLM_RL(1) ZLM_RL(2) ZLM_RL(3) ZLM_RL(4) ZLM_RL(5) ZLM_RL(6) ZLM_RL(7) ZLM_RL(8) }
 #undef ZLM_RL
