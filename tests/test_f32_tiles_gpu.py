@@ -68,3 +68,22 @@ def test_product_at_the_edges_of_its_tiles(T, N, K, accumulate):
     # a token's result does not depend on the tokens beside it
     get_kernels().linear(bits[T // 2:T // 2 + 1], x[T // 2:T // 2 + 1], w, accumulate=accumulate)
     assert torch.equal(bits[T // 2], y[T // 2])
+
+
+@pytest.mark.parametrize("T,N,K", [(1, 64, 32), (65, 130, 100), (64, 64, 2048)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_products_of_operands_off_their_alignment_are_the_same_bits(T, N, K, accumulate):
+    """An operand that starts 4 bytes late takes the kernel of single columns: the same sums in the same order."""
+    from zlm_b200.kernels import get_kernels
+    k = get_kernels()
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x, w = torch.randn((T, K), generator=g, device="cuda"), torch.randn((N, K), generator=g, device="cuda")
+    y = torch.randn((T, N), generator=g, device="cuda")
+    want = y.clone()
+    k.linear(want, x, w, accumulate=accumulate)
+    for late in ("x", "w"):
+        a, b = (torch.empty(t.numel() + 1, device="cuda")[1:].view_as(t).copy_(t) if n == late else t for n, t in (("x", x), ("w", w)))
+        assert (a.data_ptr() | b.data_ptr()) % 16 == 4
+        got = y.clone()
+        k.linear(got, a, b, accumulate=accumulate)
+        assert torch.equal(got.view(torch.int32), want.view(torch.int32))

@@ -21,8 +21,8 @@
 // scalar loads and one stage, 174 and 126 us so.  Tried: operands transposed through registers one step ahead, packed FMAs
 // (253 and 182 us: a step of 16 columns waits 1,400 of its 1,900 cycles for memory); 8 x 8 outputs on 64 threads, which halves
 // the reads an FMA (213 and 208: one warp or two a scheduler do not cover their own latencies).
-// mode 0: Y = acc (fp32); mode 1: Y += acc (fp32 residual stream)
-template <int MODE, bool VEC>
+// mode 0: Y = acc (fp32); mode 1: Y += acc (fp32 residual stream).  Rows of 16-byte pieces: the next kernel takes the others.
+template <int MODE>
 __global__ void __launch_bounds__(F32_THREADS)
 gemm_f32_kernel(float* __restrict__ Y, const float* __restrict__ X, const float* __restrict__ W,
                 int T, int N, int K, int ldy) {
@@ -38,19 +38,17 @@ gemm_f32_kernel(float* __restrict__ Y, const float* __restrict__ X, const float*
     auto stage = [&](int step) {
         if (step < steps) {
             float* base = f32_smem + (size_t)(step % F32_STAGES) * (F32_BM + F32_BN) * F32_LD;
-            constexpr int E = VEC ? 4 : 1;
-#pragma unroll 16
-            for (int x = tid; x < (F32_BM + F32_BN) * (F32_BK / E); x += F32_THREADS) {
-                const int row = x / (F32_BK / E), k = step * F32_BK + (x % (F32_BK / E)) * E;
+#pragma unroll
+            for (int x = tid; x < (F32_BM + F32_BN) * (F32_BK / 4); x += F32_THREADS) {
+                const int row = x / (F32_BK / 4), k = step * F32_BK + (x % (F32_BK / 4)) * 4;
                 const bool w = row >= F32_BM;
                 const int g = w ? n0 + row - F32_BM : m0 + row;
                 const float* src = (w ? W : X) + (size_t)g * K + k;
-                const bool in = g < (w ? N : T) && k < K && ZLM_CHK(src, 4 * E);
-                const unsigned dst = (unsigned)__cvta_generic_to_shared(base + row * F32_LD + (x % (F32_BK / E)) * E);
-                const int bytes = in ? 4 * E : 0;              // (the rest of the copy is zeros)
+                const bool in = g < (w ? N : T) && k < K && ZLM_CHK(src, 16);
+                const unsigned dst = (unsigned)__cvta_generic_to_shared(base + row * F32_LD + (x % (F32_BK / 4)) * 4);
+                const int bytes = in ? 16 : 0;                 // (the rest of the copy is zeros)
                 if (!in) src = X;
-                if (VEC) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
-                else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
             }
         }
         asm volatile("cp.async.commit_group;\n" ::);
@@ -92,13 +90,65 @@ gemm_f32_kernel(float* __restrict__ Y, const float* __restrict__ X, const float*
     }
 }
 
-template <int MODE, bool VEC>
-static int launch_f32(dim3 grid, cudaStream_t st, float* Y, const float* X, const float* W, int T, int N, int K, int ldy) {
+// The same for rows whose columns come one at a time (K no multiple of four, or an operand off its 16 bytes): 4 x 4 outputs a
+// thread, operands through registers and transposed, one stage.  Copies of 4 bytes are as many as the columns, and issuing
+// them costs more than they hide: 1 and 2,048 tokens of 2,049 columns by 2,048 outputs take 98 and 536 us here, 110 and 622
+// with the stages above.  The sums' order is the same, and so are the bits.
+#define F32P_BK 16
+template <int MODE>
+__global__ void __launch_bounds__(256)
+gemm_f32_plain_kernel(float* __restrict__ Y, const float* __restrict__ X, const float* __restrict__ W, int T, int N, int K, int ldy) {
+    __shared__ float xs[F32P_BK][F32_BM + 4], ws[F32P_BK][F32_BN + 4];
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, m0 = blockIdx.y * F32_BM, n0 = blockIdx.x * F32_BN;
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    for (int k0 = 0; k0 < K; k0 += F32P_BK) {
+        const int k = k0 + tx;                       // a thread loads column k of rows ty, ty + 16, ...
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const int r = ty + 16 * p;
+            const float *x = X + (size_t)(m0 + r) * K + k, *w = W + (size_t)(n0 + r) * K + k;
+            xs[tx][r] = (m0 + r < T && k < K && ZLM_CHK(x, 4)) ? *x : 0.f;
+            ws[tx][r] = (n0 + r < N && k < K && ZLM_CHK(w, 4)) ? *w : 0.f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int kk = 0; kk < F32P_BK; ++kk) {
+            float a[4], b[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { a[i] = xs[kk][ty * 4 + i]; b[i] = ws[kk][tx * 4 + i]; }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int gm = m0 + ty * 4 + i, gn = n0 + tx * 4 + j;
+            float* y = Y + (size_t)gm * ldy + gn;
+            if (gm < T && gn < N && ZLM_CHK(y, 4)) *y = MODE == 0 ? acc[i][j] : *y + acc[i][j];
+        }
+}
+
+template <int MODE>
+static int launch_f32(dim3 grid, cudaStream_t st, bool vec, float* Y, const float* X, const float* W, int T, int N, int K, int ldy) {
+    if (!vec) {
+        zlm_count_launch();
+        gemm_f32_plain_kernel<MODE><<<grid, 256, 0, st>>>(Y, X, W, T, N, K, ldy);
+        return zlm_check_launch("gemm_f32");
+    }
     const size_t smem = (size_t)F32_STAGES * (F32_BM + F32_BN) * F32_LD * sizeof(float);
     static bool attr_set_dev[64] = {};
     bool& attr_set = attr_set_dev[zlm_device_index()];
     if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<MODE, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) {
             zlm_set_error("gemm_f32: cannot reserve shared memory: %s", cudaGetErrorString(e));
             return ZLM_ERR_CUDA;
@@ -106,7 +156,7 @@ static int launch_f32(dim3 grid, cudaStream_t st, float* Y, const float* X, cons
         attr_set = true;
     }
     zlm_count_launch();
-    gemm_f32_kernel<MODE, VEC><<<grid, F32_THREADS, smem, st>>>(Y, X, W, T, N, K, ldy);
+    gemm_f32_kernel<MODE><<<grid, F32_THREADS, smem, st>>>(Y, X, W, T, N, K, ldy);
     return zlm_check_launch("gemm_f32");
 }
 
@@ -117,8 +167,7 @@ extern "C" int zlm_gemm_f32(float* Y, const float* X, const float* W, int T, int
     dim3 grid((N + F32_BN - 1) / F32_BN, (T + F32_BM - 1) / F32_BM);
     ZLM_REQUIRE(grid.y <= 65535, "gemm_f32: more than %d tokens in one step", 65535 * F32_BM);
     const bool vec = K % 4 == 0 && (uintptr_t)X % 16 == 0 && (uintptr_t)W % 16 == 0;
-    if (accumulate) return vec ? launch_f32<1, true>(grid, st, Y, X, W, T, N, K, ldy) : launch_f32<1, false>(grid, st, Y, X, W, T, N, K, ldy);
-    return vec ? launch_f32<0, true>(grid, st, Y, X, W, T, N, K, ldy) : launch_f32<0, false>(grid, st, Y, X, W, T, N, K, ldy);
+    return accumulate ? launch_f32<1>(grid, st, vec, Y, X, W, T, N, K, ldy) : launch_f32<0>(grid, st, vec, Y, X, W, T, N, K, ldy);
 }
 
 ZLM_TRANSLATION_UNIT(gemm_f32)
