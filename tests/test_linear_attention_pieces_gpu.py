@@ -68,3 +68,33 @@ def test_states_of_more_blocks_than_a_grids_second_dimension():
     for columns in (slice(n), slice(V - n, None)):
         for a, b in zip((o[:, columns], state[..., columns]), run(columns)):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("H,D,V,R", [(16, 32, 72, 40), (16, 20, 30, 40), (8, 64, 128, 16), (8, 48, 136, 16), (4, 128, 72, 16), (4, 100, 128, 16)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("per_head", [False, True])
+def test_a_batch_gives_the_bits_of_its_sequences_alone(H, D, V, R, dtype, per_head):
+    """Many sequences of a token or two: a column a thread; each of them alone: four columns a thread.  The same sums in the same order."""
+    from zlm_b200.kernels import get_kernels
+    k = get_kernels()
+    news = [1 + (r % 3 == 1) for r in range(R)]
+    T = sum(news)
+    assert k.lib.zlm_linear_attention_by_columns(T, R, H, D, V) and not k.lib.zlm_linear_attention_by_columns(2, 1, H, D, V)
+    g = torch.Generator(device="cuda").manual_seed(D + V)
+    proj = torch.randn((T, 2 * H * D + H * V + 3), generator=g, device="cuda").to(dtype)
+    alpha, head = torch.rand((T, H * D), generator=g, device="cuda"), torch.linspace(0.5, 0.99, H, device="cuda")
+    first = torch.randn((R, H, D, V), generator=g, device="cuda")
+
+    def run(rows, states, n):
+        state, o = states.clone(), torch.full((rows.stop - rows.start, H * V), float("nan"), device="cuda")
+        k.linear_attention(o, proj[rows], 0, H * D, 2 * H * D, None if per_head else alpha[rows], head if per_head else None, state,
+                           plan_of(n, [5] * len(n)), H, D, V, 0.3)
+        return o, state
+    o, state = run(slice(0, T), first, news)
+    assert not torch.isnan(o).any()
+    at = 0
+    for r, n in enumerate(news):
+        slot = R - 1 - r                              # (plan_of hands the slots out in reverse)
+        a, b = run(slice(at, at + n), first[slot:slot + 1], [n])
+        assert torch.equal(a, o[at:at + n]) and torch.equal(b[0], state[slot])
+        at += n

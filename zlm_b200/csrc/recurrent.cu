@@ -1041,6 +1041,93 @@ linear_attention_kernel(float* __restrict__ o, const TA* __restrict__ proj, int 
     }
 }
 
+// The walk of steps that bring one token or two a sequence, where many heads and sequences fill the GPU (la_by_columns): a block is
+// one head of one sequence and up to 128 value columns, a thread owns one column of the state, DR rows in registers, so that
+// a warp reads and writes a row of the state 128 bytes at a time.  Bound by the state's way through memory then; the four columns
+// by sixteen rows a thread above read and write it in pieces.  Every sum is in the order of the kernel above (segments of DPT
+// rows, even and odd rows apart, the segments' sums as its shuffles pair them): a token's bits do not tell which of them ran.
+template <typename TA, int DR, int DPT>
+__global__ void __launch_bounds__(128)
+linear_attention_columns_kernel(float* __restrict__ o, const TA* __restrict__ proj, int proj_stride, int q_off, int k_off, int v_off,
+                                const float* __restrict__ alpha, const float* __restrict__ head_decay, float* __restrict__ state,
+                                const int* __restrict__ seq_slot, const int* __restrict__ cu_seqlens, int H, int D, int V,
+                                float q_scale) {
+    constexpr int DS = DR / DPT;
+    __shared__ __align__(16) float sq[LA_CH][DR], sk[LA_CH][DR], sa[LA_CH][DR];
+    __shared__ float sv[LA_CH][128];
+    pdl_trigger();
+    const int r = blockIdx.x / H, h = blockIdx.x % H, v0 = blockIdx.y * 128, tid = threadIdx.x, v = v0 + tid;
+    pdl_wait();
+    if (!ZLM_CHK(seq_slot + r, 4) || !ZLM_CHK(cu_seqlens + r, 8)) return;
+    const int slot = seq_slot[r], row0 = cu_seqlens[r], n = cu_seqlens[r + 1] - row0;
+    if (n <= 0) return;
+    float* sp = state + (((size_t)slot * H + h) * D) * V + v;
+    float S[DR];
+#pragma unroll
+    for (int d = 0; d < DR; ++d) S[d] = (d < D && v < V && ZLM_CHK(sp + (size_t)d * V, 4)) ? sp[(size_t)d * V] : 0.f;
+    const float hd = head_decay ? head_decay[h] : 1.0f;
+    for (int s0 = 0; s0 < n; s0 += LA_CH) {
+        const int m = min(LA_CH, n - s0);
+        __syncthreads();
+        for (int x = tid; x < LA_CH * DR; x += 128) {
+            const int j = x / DR, d = x % DR;
+            float fq = 0.f, fk = 0.f, fa = 1.f;
+            if (j < m && d < D) {
+                const TA* row = proj + (size_t)(row0 + s0 + j) * proj_stride;
+                if (ZLM_CHK(row + q_off + h * D + d, sizeof(TA))) fq = to_f32(row[q_off + h * D + d]) * q_scale;
+                if (ZLM_CHK(row + k_off + h * D + d, sizeof(TA))) fk = to_f32(row[k_off + h * D + d]);
+                if (alpha) {
+                    const float* ap = alpha + ((size_t)(row0 + s0 + j) * H + h) * D + d;
+                    if (ZLM_CHK(ap, 4)) fa = *ap;
+                } else {
+                    fa = hd;
+                }
+            }
+            sq[j][d] = fq; sk[j][d] = fk; sa[j][d] = fa;
+        }
+        for (int x = tid; x < LA_CH * 128; x += 128) {
+            const int j = x / 128, e = x % 128;
+            float fv = 0.f;
+            if (j < m && v0 + e < V) {
+                const TA* pv = proj + (size_t)(row0 + s0 + j) * proj_stride + v_off + h * V + v0 + e;
+                if (ZLM_CHK(pv, sizeof(TA))) fv = to_f32(*pv);
+            }
+            sv[j][e] = fv;
+        }
+        __syncthreads();
+        for (int j = 0; j < m; ++j) {
+            const float vv = sv[j][tid];
+            float sum[DS], odd[DS];
+#pragma unroll
+            for (int g = 0; g < DS; ++g) sum[g] = odd[g] = 0.f;
+#pragma unroll
+            for (int e = 0; e < DPT; e += 4)
+#pragma unroll
+                for (int g = 0; g < DS; ++g) {
+                    const int d = g * DPT + e;
+                    const float4 a4 = *(const float4*)&sa[j][d], q4 = *(const float4*)&sq[j][d], k4 = *(const float4*)&sk[j][d];
+                    S[d] = fmaf(a4.x, S[d], __fmul_rn(k4.x, vv));         sum[g] = fmaf(S[d], q4.x, sum[g]);
+                    S[d + 1] = fmaf(a4.y, S[d + 1], __fmul_rn(k4.y, vv)); odd[g] = fmaf(S[d + 1], q4.y, odd[g]);
+                    S[d + 2] = fmaf(a4.z, S[d + 2], __fmul_rn(k4.z, vv)); sum[g] = fmaf(S[d + 2], q4.z, sum[g]);
+                    S[d + 3] = fmaf(a4.w, S[d + 3], __fmul_rn(k4.w, vv)); odd[g] = fmaf(S[d + 3], q4.w, odd[g]);
+                }
+#pragma unroll
+            for (int g = 0; g < DS; ++g) sum[g] += odd[g];
+#pragma unroll
+            for (int x = DS / 2; x; x >>= 1)
+#pragma unroll
+                for (int g = 0; g < x; ++g) sum[g] += sum[g + x];
+            float* op = o + ((size_t)(row0 + s0 + j) * H + h) * V + v;
+            if (v < V && ZLM_CHK(op, 4)) *op = sum[0];
+        }
+    }
+    if (v < V) {                                     // (a branch of its own: as part of the next test it kept every row's address in registers)
+#pragma unroll
+        for (int d = 0; d < DR; ++d)
+            if (d < D && ZLM_CHK(sp + (size_t)d * V, 4)) sp[(size_t)d * V] = S[d];
+    }
+}
+
 // The pieces' states in order: part[piece] becomes the state the piece starts from, the sequence's state is left.
 // (a thread owns VEC neighbouring numbers of one row of the state; eight pieces' loads in flight.)  grid la_grid(R * H, ceil(D * V / (128 VEC)))
 #define CHAIN_AHEAD 8
@@ -1276,6 +1363,12 @@ extern "C" int zlm_linear_attention_fits(int R, int H, int D, int V, int maxp) {
     return (long long)R * H * maxp <= 2147483647LL && (long long)R * H * D <= 2147483647LL && (V + 127) / 128 <= 65535;
 }
 
+// A step of T tokens of R sequences: by columns, or four columns a thread.  LA_RULE
+extern "C" int zlm_linear_attention_by_columns(int T, int R, int H, int D, int V) {
+    const long long blocks = (long long)R * H * ((V + 127) / 128);
+    return T <= 2LL * R && blocks >= (D <= 32 ? 640 : D <= 64 ? 112 : 64);
+}
+
 // q, k [H*D], v [H*V]: columns of proj from q_off, k_off, v_off on (element type); alpha [T][H*D] fp32 decays per token
 // and key channel, or null with head_decay [H] fp32 (one decay a head); state [slots][H][D][V] fp32; o [T][H*V] fp32.
 // pieces: null, or R * ceil(max_new / 32) * H * D * (V + 1) floats: sequences run in pieces of 32 tokens side by side
@@ -1299,11 +1392,17 @@ extern "C" int zlm_linear_attention(float* o, const void* proj, int proj_stride,
     float* pdecay = pieces ? pieces + (size_t)R * maxp * H * D * V : nullptr;
     const LaOut out{y, y_stride, g, g_stride, VecW{w, w_dtype}, eps, act};
     int rc = ZLM_OK;
+    const bool columns = !pieces && zlm_linear_attention_by_columns(T, R, H, D, V);
 #define ZLM_LA(TA, DR, SP, MODE, G)                                                                                            \
     zlm_launch(linear_attention_kernel<TA, DR, SP, MODE>, la_grid(G, (V + 512 * SP / DR - 1) / (512 * SP / DR)), dim3(128), 0, st, o, (const TA*)proj, proj_stride, q_off, k_off, v_off, \
                alpha, head_decay, state, seq_slot, cu_seqlens, H, D, V, q_scale, part, pdecay, maxp, L)
 #define ZLM_LA_RUN(TA, DR, SP)                                                                                              \
     do {                                                                                                                   \
+        if (columns) {                                                                                                      \
+            zlm_launch(linear_attention_columns_kernel<TA, DR, SP>, dim3(R * H, (V + 127) / 128), dim3(128), 0, st, o, (const TA*)proj,  \
+                       proj_stride, q_off, k_off, v_off, alpha, head_decay, state, seq_slot, cu_seqlens, H, D, V, q_scale); \
+            break;                                                                                                          \
+        }                                                                                                                   \
         if (!pieces) { ZLM_LA(TA, DR, SP, 0, R * H); break; }                                                               \
         ZLM_LA(TA, DR, SP, 1, R * maxp * H);                                                                                      \
         if (V % 4 == 0 && (uintptr_t)state % 16 == 0 && (uintptr_t)part % 16 == 0)                                         \
