@@ -927,14 +927,14 @@ linear_attention_kernel(float* __restrict__ o, const TA* __restrict__ proj, int 
     __shared__ __align__(16) float sq[LA_CH][DP], sk[LA_CH][DP], sa[LA_CH][DP];
     __shared__ __align__(16) float sv[LA_CH][COLS];
     pdl_trigger();
-    const int unit = blockIdx.x / H, h = blockIdx.x % H, v0 = (blockIdx.y + blockIdx.z * gridDim.y) * COLS, tid = threadIdx.x;
+    const int unit = blockIdx.x / H, h = blockIdx.x % H, v0 = blockIdx.y * COLS, tid = threadIdx.x;
     const int r = MODE == 0 ? unit : unit / maxp, p = MODE == 0 ? 0 : unit % maxp;
     const int grp = tid / DS, lane_d = tid % DS, v = v0 + grp * LA_CPT;
     pdl_wait();
     if (!ZLM_CHK(seq_slot + r, 4) || !ZLM_CHK(cu_seqlens + r, 8)) return;
     const int slot = seq_slot[r], row0 = cu_seqlens[r], n = cu_seqlens[r + 1] - row0;
     const int lo = MODE == 0 ? 0 : p * L, hi = MODE == 0 ? n : min(n, lo + L);
-    if (lo >= hi || v0 >= V) return;
+    if (lo >= hi) return;
     float* sp = (MODE == 0 ? state + (((size_t)slot * H + h) * D) * V : part + ((((size_t)r * maxp + p) * H + h) * D) * V) + v;
     float2 S[DPT / 2][LA_CPT];
 #pragma unroll
@@ -1035,7 +1035,7 @@ linear_attention_kernel(float* __restrict__ o, const TA* __restrict__ proj, int 
                     if (v + c < V && ZLM_CHK(dst + c, 4)) dst[c] = t[c];
             }
         }
-    if (MODE == 1 && v0 == 0 && tid < D) {
+    if (MODE == 1 && blockIdx.y == 0 && tid < D) {
         float* pp = pdecay + (((size_t)r * maxp + p) * H + h) * D + tid;
         if (ZLM_CHK(pp, 4)) *pp = pd;
     }
@@ -1129,7 +1129,7 @@ linear_attention_columns_kernel(float* __restrict__ o, const TA* __restrict__ pr
 }
 
 // The pieces' states in order: part[piece] becomes the state the piece starts from, the sequence's state is left.
-// (a thread owns VEC neighbouring numbers of one row of the state; eight pieces' loads in flight.)  grid la_grid(R * H, ceil(D * V / (128 VEC)))
+// (a thread owns VEC neighbouring numbers of one row of the state; eight pieces' loads in flight.)  grid (R * H, ceil(D * V / (128 VEC)))
 #define CHAIN_AHEAD 8
 template <int VEC>
 __global__ void __launch_bounds__(128)
@@ -1138,7 +1138,7 @@ linear_attention_chain_kernel(float* __restrict__ part, const float* __restrict_
                               int maxp, int L) {
     struct alignas(4 * VEC) Num { float v[VEC]; };
     pdl_trigger();
-    const int rh = blockIdx.x, r = rh / H, h = rh % H, e = ((blockIdx.y + blockIdx.z * gridDim.y) * 128 + threadIdx.x) * VEC, d = e / V;
+    const int rh = blockIdx.x, r = rh / H, h = rh % H, e = (blockIdx.y * 128 + threadIdx.x) * VEC, d = e / V;
     pdl_wait();
     if (e >= D * V || !ZLM_CHK(seq_slot + r, 4) || !ZLM_CHK(cu_seqlens + r, 8)) return;
     const int slot = seq_slot[r], n = cu_seqlens[r + 1] - cu_seqlens[r];
@@ -1356,17 +1356,19 @@ static int launch_la_out(dim3 grid, cudaStream_t st, float* o, const void* proj,
     return ZLM_OK;
 }
 
-// blocks `n` of a unit over a grid's second and third dimension, which end at 65,535
-static dim3 la_grid(int units, int n) { return n <= 65535 ? dim3(units, n) : dim3(units, 65535, (n + 65534) / 65535); }
 // R sequences in maxp pieces each (1: whole)
 extern "C" int zlm_linear_attention_fits(int R, int H, int D, int V, int maxp) {
     return (long long)R * H * maxp <= 2147483647LL && (long long)R * H * D <= 2147483647LL && (V + 127) / 128 <= 65535;
 }
 
-// A step of T tokens of R sequences: by columns, or four columns a thread.  LA_RULE
+// A step of T tokens of R sequences: by columns, or four columns a thread?  By columns from so many blocks on, where a sequence
+// brings up to three tokens: with more of them the arithmetic counts, with fewer blocks the depth of a thread's chain does.  Us by
+// columns / with four a thread, 8 heads, one token a sequence: 64 x 128, 8 sequences 4.6 / 4.3, 16 5.5 / 5.7, 64 7.1 / 7.8; 128 x
+// 128, 4 sequences 7.3 / 5.1, 16 8.8 / 11.0, 64 16 / 22; 32 x 128, 64 sequences 4 to 5, a fifth less with four, 96 a fifth more.
+// Heads of up to 64 columns leave half of a block of columns idle (64 x 64, 80 sequences 9.7 / 9.1).
 extern "C" int zlm_linear_attention_by_columns(int T, int R, int H, int D, int V) {
     const long long blocks = (long long)R * H * ((V + 127) / 128);
-    return T <= 2LL * R && blocks >= (D <= 32 ? 640 : D <= 64 ? 112 : 64);
+    return T <= 3LL * R && blocks >= (D <= 32 ? 600 : D <= 64 ? 112 : 64) && (V > 64 || D <= 32 || D > 64);
 }
 
 // q, k [H*D], v [H*V]: columns of proj from q_off, k_off, v_off on (element type); alpha [T][H*D] fp32 decays per token
@@ -1392,9 +1394,13 @@ extern "C" int zlm_linear_attention(float* o, const void* proj, int proj_stride,
     float* pdecay = pieces ? pieces + (size_t)R * maxp * H * D * V : nullptr;
     const LaOut out{y, y_stride, g, g_stride, VecW{w, w_dtype}, eps, act};
     int rc = ZLM_OK;
-    const bool columns = !pieces && zlm_linear_attention_by_columns(T, R, H, D, V);
+    // a grid's second dimension ends at 65,535.  Heads with more blocks of 64 columns, or more blocks of the chain, than that (four
+    // million columns, or 33 million numbers of state) walk by columns whatever their tokens: one head fills the GPU.  (Carrying on
+    // in the third dimension cost every walk 5 to 25 %: the column's range is no longer known to the compiler.)
+    const bool wide = (D > 64 && (V + 63) / 64 > 65535) || (pieces && (D * V + (V % 4 ? 127 : 511)) / (V % 4 ? 128 : 512) > 65535);
+    const bool columns = wide || (!pieces && zlm_linear_attention_by_columns(T, R, H, D, V));
 #define ZLM_LA(TA, DR, SP, MODE, G)                                                                                            \
-    zlm_launch(linear_attention_kernel<TA, DR, SP, MODE>, la_grid(G, (V + 512 * SP / DR - 1) / (512 * SP / DR)), dim3(128), 0, st, o, (const TA*)proj, proj_stride, q_off, k_off, v_off, \
+    zlm_launch(linear_attention_kernel<TA, DR, SP, MODE>, dim3(G, (V + 512 * SP / DR - 1) / (512 * SP / DR)), dim3(128), 0, st, o, (const TA*)proj, proj_stride, q_off, k_off, v_off, \
                alpha, head_decay, state, seq_slot, cu_seqlens, H, D, V, q_scale, part, pdecay, maxp, L)
 #define ZLM_LA_RUN(TA, DR, SP)                                                                                              \
     do {                                                                                                                   \
@@ -1406,10 +1412,10 @@ extern "C" int zlm_linear_attention(float* o, const void* proj, int proj_stride,
         if (!pieces) { ZLM_LA(TA, DR, SP, 0, R * H); break; }                                                               \
         ZLM_LA(TA, DR, SP, 1, R * maxp * H);                                                                                      \
         if (V % 4 == 0 && (uintptr_t)state % 16 == 0 && (uintptr_t)part % 16 == 0)                                         \
-            zlm_launch(linear_attention_chain_kernel<4>, la_grid(R * H, (D * V + 511) / 512), dim3(128), 0, st, part,         \
+            zlm_launch(linear_attention_chain_kernel<4>, dim3(R * H, (D * V + 511) / 512), dim3(128), 0, st, part,         \
                        (const float*)pdecay, state, seq_slot, cu_seqlens, H, D, V, maxp, L);                               \
         else                                                                                                               \
-            zlm_launch(linear_attention_chain_kernel<1>, la_grid(R * H, (D * V + 127) / 128), dim3(128), 0, st, part,         \
+            zlm_launch(linear_attention_chain_kernel<1>, dim3(R * H, (D * V + 127) / 128), dim3(128), 0, st, part,         \
                        (const float*)pdecay, state, seq_slot, cu_seqlens, H, D, V, maxp, L);                               \
         rc = launch_la_out<TA, DR>(pgrid, st, o, proj, proj_stride, q_off, alpha, head_decay, part, cu_seqlens, H, D, V,   \
                                    q_scale, maxp, out);                                                                    \
