@@ -1,5 +1,5 @@
 """Convolution, heads' norm and cache write in runs of tokens: bit for bit what the kernel of a token a warp gives (the same
-step cut into chunks of fewer tokens than a run's rule wants), over unequal sequences, carried inputs, padded heads, 2 to 5 taps."""
+step cut into chunks of fewer tokens than a run's rule wants, which is asked), over unequal sequences, carried inputs, padded heads, 2 to 5 taps."""
 import pytest
 import torch
 
@@ -17,7 +17,7 @@ def test_runs_give_the_bits_of_single_tokens(nq, nkv, dim, vdim, hdp, taps, dtyp
     k = get_kernels()
     g = torch.Generator(device="cuda").manual_seed(dim + taps)
     C = (nq + nkv) * dim + nkv * vdim
-    news, starts = [255, 1, 3, 131], [0, 70, 1, 64]
+    news, starts = [1791, 1, 3, 131], [0, 70, 1, 64]
     proj = torch.randn((sum(news), C + 8), generator=g, device="cuda").to(dtype)
     w = torch.randn((C, taps), generator=g, device="cuda").to(dtype)
     R = len(news)
@@ -44,7 +44,9 @@ def test_runs_give_the_bits_of_single_tokens(nq, nkv, dim, vdim, hdp, taps, dtyp
         assert done == news
         return out, state, pool
     whole = run([news])
-    cut = [[min(97, max(0, n - 97 * i)) for n in news] for i in range(3)]
-    assert sum(cut[0]) < 256
+    cut = [[min(97, max(0, n - 97 * i)) for n in news] for i in range(19)]
+    units = nq + 2 * nkv
+    assert k.lib.zlm_conv_runs(sum(news), R, units, hdp, taps)
+    assert not any(k.lib.zlm_conv_runs(sum(step), sum(n > 0 for n in step), units, hdp, taps) for step in cut)
     for a, b in zip(whole, run(cut)):
         assert torch.equal(a, b)

@@ -155,3 +155,13 @@ def test_32_bit_attention_leaves_what_its_tiles_cannot_number_to_single_queries(
 def test_recurrent_units_clusters_by_rounds_and_blocks(lib, R, max_new, W, least, most):
     """One long sequence: the whole cluster; many short ones: no more blocks than they have tokens for."""
     assert least <= lib.zlm_rglru_cluster_size(R, max_new, W) <= most
+
+
+@pytest.mark.parametrize("T,R,units,hdp,taps,runs", [
+    (2999, 3, 24, 128, 4, 1), (256, 1, 48, 128, 4, 1), (255, 1, 48, 128, 4, 0),
+    (512, 1, 8, 128, 4, 0), (1152, 1, 8, 128, 4, 1), (256, 1, 24, 128, 4, 0),                  # warps of eight tokens that fill the GPU
+    (4096, 4096, 48, 128, 4, 0), (320, 64, 24, 128, 4, 0), (512, 64, 24, 128, 4, 1),            # decode steps, and a prompt beside them
+    (512, 256, 48, 128, 4, 0), (2048, 1024, 48, 128, 4, 1),                                     # two tokens a sequence
+    (2999, 3, 24, 256, 4, 0), (2999, 3, 24, 128, 1, 0), (2999, 3, 24, 128, 6, 0)])
+def test_convolution_in_runs_where_they_win(lib, T, R, units, hdp, taps, runs):
+    assert lib.zlm_conv_runs(T, R, units, hdp, taps) == runs

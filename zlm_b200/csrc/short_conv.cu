@@ -234,6 +234,16 @@ conv_state_update_kernel(TA* __restrict__ state, const TA* __restrict__ proj, in
     }
 }
 
+// Runs of SC_RUN tokens a warp, or a token a warp?  Runs from about 9,200 heads' tokens on (fewer warps of eight tokens do not
+// fill the GPU), and more where sequences bring under eight tokens, whose taps reach into the carried inputs one token after the
+// other.  Us by tokens / by runs, 4 taps: 1 sequence of 256 tokens, 8 heads 6.8 / 8.2, 24 heads 9.2 / 9.2, 48 heads 13.0 / 10.4; of
+// 1,024, 8 heads 10.3 / 9.2, 24 heads 20.0 / 12.7; 256 sequences' single tokens, 24 heads 13.1 / 19.4; 128 of 2 10.8 / 14.7; 64 of 8
+// 13.9 / 12.7; 1,024 of 2 51 / 46; a prompt of 257 beside 63 single tokens 11.1 / 16.0.
+extern "C" int zlm_conv_runs(int T, int R, int units, int hdp, int taps) {
+    const long long work = (long long)T * units;
+    return hdp <= 128 && taps >= 2 && taps <= 5 && T >= 256 && work >= 9216 && T >= 2LL * R && work * T >= 73728LL * R;
+}
+
 template <typename TA>
 static void launch_conv(void* q_out, int q_out_stride, const void* proj, int proj_stride, const void* conv_w, void* state,
                         const int* token_pos, const int* token_slot, const int* token_seq, const int* seq_start,
@@ -247,8 +257,7 @@ static void launch_conv(void* q_out, int q_out_stride, const void* proj, int pro
     const bool vec = dim % 4 == 0 && vdim % 4 == 0 && hdp % 4 == 0 && proj_stride % 4 == 0 && q_out_stride % 4 == 0 && C0 % 4 == 0 &&
                      (uintptr_t)proj % al == 0 && (uintptr_t)q_out % al == 0 && (uintptr_t)pool % al == 0 &&
                      (state == nullptr || (uintptr_t)state % al == 0);
-    // (a run of tokens a warp from 256 tokens on: below that a token a warp leaves more of them to run: 16 + 2 x 4 heads at 256 tokens 9.4 us a token a warp, 8.4 so, at 128 7.0 and 7.1)
-    if (vec && hdp <= 128 && taps >= 2 && taps <= 5 && T >= 256) {
+    if (vec && zlm_conv_runs(T, R, units, hdp, taps)) {
         const dim3 grid((T + SC_RUN - 1) / SC_RUN, (units + SC_WARPS - 1) / SC_WARPS);
 #define ZLM_SC(N)                                                                                                               \
     case N:                                                                                                                     \
