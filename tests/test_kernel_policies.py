@@ -150,11 +150,12 @@ def test_32_bit_attention_leaves_what_its_tiles_cannot_number_to_single_queries(
     assert lib.zlm_attention_f32_tile_supported(16, 4, 128, 2048, 2048, c_float(0.0), 1, 0, 0, R, max_new) == takes
 
 
-@pytest.mark.parametrize("R,max_new,W,least,most", [(1, 2048, 2048, 8, 8), (2, 1000, 2048, 8, 8), (64, 128, 2048, 1, 2), (64, 128, 4096, 1, 2),
-                                                    (1, 128, 64, 2, 8), (1, 1, 64, 1, 8), (65535, 2000, 8192, 1, 1)])
-def test_recurrent_units_clusters_by_rounds_and_blocks(lib, R, max_new, W, least, most):
-    """One long sequence: the whole cluster; many short ones: no more blocks than they have tokens for."""
-    assert least <= lib.zlm_rglru_cluster_size(R, max_new, W) <= most
+@pytest.mark.parametrize("R,T,max_new,W,size", [
+    (1, 2048, 2048, 2048, 8), (1, 8192, 8192, 4096, 8), (2, 1999, 1000, 1024, 8),           # one long sequence: the whole cluster
+    (64, 8192, 128, 2048, 1), (16, 2048, 128, 4096, 1), (64, 191, 128, 2048, 1),             # many short ones: as few blocks as can be
+    (64, 2111, 2048, 1024, 4), (21, 1824, 1024, 4096, 2), (1, 1, 1, 64, 1), (65535, 65535, 1, 8192, 1)])
+def test_recurrent_units_clusters_by_rounds_and_blocks(lib, R, T, max_new, W, size):
+    assert lib.zlm_rglru_cluster_size(R, T, max_new, W) == size
 
 
 @pytest.mark.parametrize("T,R,units,hdp,taps,runs", [

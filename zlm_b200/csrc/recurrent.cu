@@ -608,21 +608,7 @@ rglru_cluster_kernel(__nv_bfloat16* __restrict__ out, int out_stride, const floa
     const int rank = (int)cluster.block_rank(), r = blockIdx.x / (int)cluster.num_blocks();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.y * 64 + lane * 2;
     pdl_trigger();
-    bool live = c < W;                               // (no thread leaves its block: the block's others wait for it)
-    float w[2][TAPS], xb[2], ub[2], yb[2], rb[2], ib[2], sl[2], S0[2] = {0.f, 0.f};
-#pragma unroll
-    for (int v = 0; v < 2; ++v) {
-        xb[v] = (live && bx && ZLM_CHK(bx + c + v, 2)) ? to_f32(bx[c + v]) : 0.f;
-        ub[v] = (live && cb && ZLM_CHK(cb + c + v, 2)) ? to_f32(cb[c + v]) : 0.f;
-        yb[v] = (live && by && ZLM_CHK(by + c + v, 2)) ? to_f32(by[c + v]) : 0.f;
-        rb[v] = (live && cr && ZLM_CHK(cr + c + v, 2)) ? to_f32(cr[c + v]) : 0.f;
-        ib[v] = (live && ci && ZLM_CHK(ci + c + v, 2)) ? to_f32(ci[c + v]) : 0.f;
-        sl[v] = live && ZLM_CHK(lam + c + v, 2) ? softplus_f(to_f32(lam[c + v])) * c_decay : 0.f;
-#pragma unroll
-        for (int j = 0; j < TAPS; ++j)
-            w[v][j] = live && ZLM_CHK(conv_w + (size_t)(c + v) * TAPS + j, 2) ? to_f32(conv_w[(size_t)(c + v) * TAPS + j]) : 0.f;
-    }
-    pdl_wait();
+    // (the step's integer arrays are copied in ahead of its first kernel: they may be read before pdl_wait())
     int row0 = 0, n = 0, slot = 0, start = 0;
     if (ZLM_CHK(seq_slot + r, 4) && ZLM_CHK(cu_seqlens + r, 8) && ZLM_CHK(seq_start + r, 4)) {
         row0 = cu_seqlens[r];
@@ -633,6 +619,22 @@ rglru_cluster_kernel(__nv_bfloat16* __restrict__ out, int out_stride, const floa
     // the blocks of the cluster that the sequence has tokens for
     const int ranks = min((int)cluster.num_blocks(), max(1, (n + RL_WARPS * RL_P - 1) / (RL_WARPS * RL_P)));
     if (rank >= ranks) return;
+    bool live = c < W;                               // (no thread leaves its block: the block's others wait for it)
+    const bool own = live && ((rank * RL_WARPS + warp) * RL_P < n || warp == 0);      // (a warp without a token needs nothing of these)
+    float w[2][TAPS], xb[2], ub[2], yb[2], rb[2], ib[2], sl[2], S0[2] = {0.f, 0.f};
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+        xb[v] = (own && bx && ZLM_CHK(bx + c + v, 2)) ? to_f32(bx[c + v]) : 0.f;
+        ub[v] = (own && cb && ZLM_CHK(cb + c + v, 2)) ? to_f32(cb[c + v]) : 0.f;
+        yb[v] = (own && by && ZLM_CHK(by + c + v, 2)) ? to_f32(by[c + v]) : 0.f;
+        rb[v] = (own && cr && ZLM_CHK(cr + c + v, 2)) ? to_f32(cr[c + v]) : 0.f;
+        ib[v] = (own && ci && ZLM_CHK(ci + c + v, 2)) ? to_f32(ci[c + v]) : 0.f;
+        sl[v] = own && ZLM_CHK(lam + c + v, 2) ? softplus_f(to_f32(lam[c + v])) * c_decay : 0.f;
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j)
+            w[v][j] = own && ZLM_CHK(conv_w + (size_t)(c + v) * TAPS + j, 2) ? to_f32(conv_w[(size_t)(c + v) * TAPS + j]) : 0.f;
+    }
+    pdl_wait();
     float* sp = state + (size_t)slot * TAPS * W + c;
     live = live && ZLM_CHK(sp, 8);
     if (live) { S0[0] = sp[0]; S0[1] = sp[1]; }
@@ -722,7 +724,7 @@ rglru_cluster_kernel(__nv_bfloat16* __restrict__ out, int out_stride, const floa
                 }
                 total[par][lane * 2 + v] = t;
             }
-        cluster.sync();
+        if (ranks > 1) cluster.sync();               // (one block: the totals are this warp's own lanes')
         // the states that the block's warps start from, and the one the whole round ends with
         if (warp == 0)
 #pragma unroll
@@ -764,7 +766,7 @@ rglru_cluster_kernel(__nv_bfloat16* __restrict__ out, int out_stride, const floa
             sp[v] = S0[v];
             rglru_keep_inputs<__nv_bfloat16>(sp + v, proj, proj_stride, x_off, c + v, row0, n, W, TAPS, xb[v]);
         }
-    cluster.sync();                                  // no block leaves while another may still read its shared memory
+    if (ranks > 1) cluster.sync();                   // no block leaves while another may still read its shared memory
 }
 
 // bfloat16, with everything as in zlm_rglru: the first of the three launches.  u16 [blocks][Tp][W/blocks], Tp = T rounded up to
@@ -791,18 +793,21 @@ extern "C" int zlm_rglru_conv_blocks(void* u16, int* group_of_tile, const void* 
     return zlm_check_launch("rglru_conv_blocks");
 }
 
-// Blocks of a sequence's cluster: the size of the least estimate.  Every round of a cluster takes RL_ROUND, one after the other
-// (loads, exponentials, two barriers); all blocks of the step, most of them of short sequences where one is long, take
-// RL_LEAVE for each time that the GPU is full of them.
-#define RL_ROUND 4.0f
-#define RL_LEAVE 1.5f
-extern "C" int zlm_rglru_cluster_size(int R, int max_new, int W) {
-    int best = RL_CLUSTER;
+// Blocks of a sequence's cluster, in a step of T tokens: the size of the least estimate.  In rounds of the longest sequence, which
+// follow one another (4 us each), the GPU takes three for as many blocks with tokens as fit on it (two an SM) and one for as many
+// that leave at once.  What the other sequences bring is taken as their mean.  Us of the three launches in clusters of 1 / 2 / 4 / 8,
+// and of the passes over pieces, 2,048 channels: 1 sequence of 2,048 tokens 182 / 120 / 79 / 67 and 147; 64 of 128 239 / 278 / 308 /
+// 372 and 394; 1 of 128 beside 63 single tokens 76 / 123 / 142 / 183 and 83 (665 in full clusters that neither left nor skipped); 1
+// of 1,024 beside 20 of 40 148 / 123 / 109 / 113 and 151.
+extern "C" int zlm_rglru_cluster_size(int R, int T, int max_new, int W) {
+    constexpr int ROUND = RL_WARPS * RL_P;
+    const int longest = (max_new + ROUND - 1) / ROUND, mean = R > 1 ? (T - max_new) / (R - 1) : 0, other = mean > ROUND ? (mean + ROUND - 1) / ROUND : 1;
+    int best = 1;
     float least = 0.f;
-    for (int c = RL_CLUSTER; c; c >>= 1) {
-        const float rounds = (float)((max_new + RL_WARPS * RL_P * c - 1) / (RL_WARPS * RL_P * c));
-        const float est = rounds * RL_ROUND + (float)R * c * ((W + 63) / 64) / 296.f * RL_LEAVE;
-        if (c == RL_CLUSTER || est < least) { best = c; least = est; }
+    for (int c = 1; c <= RL_CLUSTER; c <<= 1) {
+        const float with = (float)(longest < c ? longest : c) + (R - 1.f) * (float)(other < c ? other : c), leave = (float)R * c - with;
+        const float est = (float)((longest + c - 1) / c) + (3.f * with + leave) * (float)((W + 63) / 64) / 296.f;
+        if (c == 1 || est < least) { best = c; least = est; }
     }
     return best;
 }

@@ -1043,7 +1043,7 @@ class CudaKernels:
                        c_int(x_off), c_int(y_off), self._p(bx), self._p(by), self._p(conv_w), self._p(conv_b), self._p(c_r),
                        self._p(c_i), self._p(lam), c_float(c_decay), self._p(state), self._p(plan.seq_slot),
                        self._p(plan.seq_start), self._p(plan.cu_seqlens), c_int(T), c_int(plan.R), c_int(W), c_int(blocks),
-                       c_int(taps), c_float(out_scale), c_int(self.lib.zlm_rglru_cluster_size(c_int(plan.R), c_int(max_new), c_int(W))),
+                       c_int(taps), c_float(out_scale), c_int(self.lib.zlm_rglru_cluster_size(c_int(plan.R), c_int(T), c_int(max_new), c_int(W))),
                        self._stream())
             return
         u = plan.scratch("rglru.u", (T, W), torch.float32)
