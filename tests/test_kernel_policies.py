@@ -166,3 +166,10 @@ def test_recurrent_units_clusters_by_rounds_and_blocks(lib, R, T, max_new, W, si
     (2999, 3, 24, 256, 4, 0), (2999, 3, 24, 128, 1, 0), (2999, 3, 24, 128, 6, 0)])
 def test_convolution_in_runs_where_they_win(lib, T, R, units, hdp, taps, runs):
     assert lib.zlm_conv_runs(T, R, units, hdp, taps) == runs
+
+
+@pytest.mark.parametrize("longest,R,H,D,V,columns", [
+    (1, 16, 8, 64, 128, 1), (1, 8, 8, 64, 128, 0), (3, 64, 8, 64, 128, 1), (4, 64, 8, 64, 128, 0), (1, 64, 8, 64, 64, 0),
+    (1, 8, 8, 128, 128, 1), (1, 4, 8, 128, 128, 0), (1, 4, 8, 128, 256, 1), (1, 64, 8, 32, 128, 0), (1, 96, 8, 32, 64, 1)])
+def test_linear_attention_by_columns_where_sequences_and_heads_fill_the_gpu(lib, longest, R, H, D, V, columns):
+    assert lib.zlm_linear_attention_by_columns(longest, R, H, D, V) == columns

@@ -74,12 +74,12 @@ def test_heads_of_more_columns_than_a_grid_numbers():
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("per_head", [False, True])
 def test_a_batch_gives_the_bits_of_its_sequences_alone(H, D, V, R, dtype, per_head):
-    """Many sequences of a token or two: a column a thread; each of them alone: four columns a thread.  The same sums in the same order."""
+    """Many sequences of up to three tokens: a column a thread; each of them alone: four columns a thread.  The same sums in the same order."""
     from zlm_b200.kernels import get_kernels
     k = get_kernels()
     news = [1 + r % 3 for r in range(R)]
     T = sum(news)
-    assert k.lib.zlm_linear_attention_by_columns(T, R, H, D, V) and not k.lib.zlm_linear_attention_by_columns(3, 1, H, D, V)
+    assert k.lib.zlm_linear_attention_by_columns(3, R, H, D, V) and not k.lib.zlm_linear_attention_by_columns(3, 1, H, D, V)
     g = torch.Generator(device="cuda").manual_seed(D + V)
     proj = torch.randn((T, 2 * H * D + H * V + 3), generator=g, device="cuda").to(dtype)
     alpha, head = torch.rand((T, H * D), generator=g, device="cuda"), torch.linspace(0.5, 0.99, H, device="cuda")

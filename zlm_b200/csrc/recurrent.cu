@@ -1366,14 +1366,14 @@ extern "C" int zlm_linear_attention_fits(int R, int H, int D, int V, int maxp) {
     return (long long)R * H * maxp <= 2147483647LL && (long long)R * H * D <= 2147483647LL && (V + 127) / 128 <= 65535;
 }
 
-// A step of T tokens of R sequences: by columns, or four columns a thread?  By columns from so many blocks on, where a sequence
-// brings up to three tokens: with more of them the arithmetic counts, with fewer blocks the depth of a thread's chain does.  Us by
+// A step of R sequences of up to `longest` tokens: by columns, or four columns a thread?  By columns from so many blocks on, where no
+// sequence brings more than three tokens: with more of them the arithmetic counts, with fewer blocks the depth of a thread's chain does.  Us by
 // columns / with four a thread, 8 heads, one token a sequence: 64 x 128, 8 sequences 4.6 / 4.3, 16 5.5 / 5.7, 64 7.1 / 7.8; 128 x
 // 128, 4 sequences 7.3 / 5.1, 16 8.8 / 11.0, 64 16 / 22; 32 x 128, 64 sequences 4 to 5, a fifth less with four, 96 a fifth more.
 // Heads of up to 64 columns leave half of a block of columns idle (64 x 64, 80 sequences 9.7 / 9.1).
-extern "C" int zlm_linear_attention_by_columns(int T, int R, int H, int D, int V) {
+extern "C" int zlm_linear_attention_by_columns(int longest, int R, int H, int D, int V) {
     const long long blocks = (long long)R * H * ((V + 127) / 128);
-    return T <= 3LL * R && blocks >= (D <= 32 ? 600 : D <= 64 ? 112 : 64) && (V > 64 || D <= 32 || D > 64);
+    return longest <= 3 && blocks >= (D <= 32 ? 600 : D <= 64 ? 112 : 64) && (V > 64 || D <= 32 || D > 64);
 }
 
 // q, k [H*D], v [H*V]: columns of proj from q_off, k_off, v_off on (element type); alpha [T][H*D] fp32 decays per token
@@ -1403,7 +1403,7 @@ extern "C" int zlm_linear_attention(float* o, const void* proj, int proj_stride,
     // million columns, or 33 million numbers of state) walk by columns whatever their tokens: one head fills the GPU.  (Carrying on
     // in the third dimension cost every walk 5 to 25 %: the column's range is no longer known to the compiler.)
     const bool wide = (D > 64 && (V + 63) / 64 > 65535) || (pieces && (D * V + (V % 4 ? 127 : 511)) / (V % 4 ? 128 : 512) > 65535);
-    const bool columns = wide || (!pieces && zlm_linear_attention_by_columns(T, R, H, D, V));
+    const bool columns = wide || (!pieces && zlm_linear_attention_by_columns(max_new > 0 ? max_new : T, R, H, D, V));
 #define ZLM_LA(TA, DR, SP, MODE, G)                                                                                            \
     zlm_launch(linear_attention_kernel<TA, DR, SP, MODE>, dim3(G, (V + 512 * SP / DR - 1) / (512 * SP / DR)), dim3(128), 0, st, o, (const TA*)proj, proj_stride, q_off, k_off, v_off, \
                alpha, head_decay, state, seq_slot, cu_seqlens, H, D, V, q_scale, part, pdecay, maxp, L)
