@@ -5,6 +5,8 @@ import types
 import pytest
 import torch
 
+from test_piece_products_gpu import calls
+
 pytestmark = pytest.mark.gpu
 
 
@@ -39,16 +41,17 @@ def _case(nq, nkv, hd, news, starts, seed=0):
 @pytest.mark.parametrize("nq,nkv,hd", [(4, 2, 128), (3, 1, 64), (2, 2, 96)])
 @pytest.mark.parametrize("news,starts", [([8], [0]), ([31, 1, 33], [0, 200, 31]), ([129], [515]), ([40, 64], [1, 64]), ([1, 1], [700, 3])])
 @pytest.mark.parametrize("window,chunk,sink", [(0, 0, None), (40, 0, True), (1, 0, "numbers"), (0, 48, None), (100, 0, None)])
-def test_tiles_give_the_bits_of_single_queries(nq, nkv, hd, news, starts, window, chunk, sink):
+def test_tiles_give_the_bits_of_single_queries(nq, nkv, hd, news, starts, window, chunk, sink, monkeypatch):
     from zlm_b200.kernels import get_kernels
     k = get_kernels()
     q, pool, table, pos, slot, plan = _case(nq, nkv, hd, news, starts)
     sinks = torch.linspace(-2, 2, nq, device="cuda") if sink == "numbers" else None
-    outs = []
+    outs, names = [], calls(k, monkeypatch)
     for p in (None, plan):
         out = torch.full((q.shape[0], nq * hd), float("nan"), device="cuda")
         k.attention(out, q, pool, table, pos, slot, nq, nkv, hd, hd ** -0.5, window, p, sink=bool(sink), sinks=sinks, chunk=chunk)
         outs.append(out)
+    assert names == ["zlm_attention_generic", "zlm_attention_f32_tile"]
     assert not torch.isnan(outs[0]).any()
     assert torch.equal(outs[0].view(torch.int32), outs[1].view(torch.int32))
 

@@ -6,7 +6,7 @@ Bounds.  Sums of some ten to hundred fp32 products, 2^-24 of each: 1e-6 of the n
 import pytest
 import torch
 
-from test_piece_products_gpu import close, plan_of, unit
+from test_piece_products_gpu import calls, close, plan_of, unit
 
 pytestmark = pytest.mark.gpu
 
@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("news,starts", [([128], [0]), ([129, 1, 33], [0, 5, 300]), ([31, 200], [9, 0])])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("per_head", [False, True])
-def test_pieces(H, D, V, news, starts, dtype, per_head):
+def test_pieces(H, D, V, news, starts, dtype, per_head, monkeypatch):
     from zlm_b200.kernels import get_kernels
     k, plan = get_kernels(), plan_of(news, starts)
     T = plan.T
@@ -44,7 +44,9 @@ def test_pieces(H, D, V, news, starts, dtype, per_head):
     close(state, S, 1e-6)
     gate, w = proj[:, 2 * H * D + H * V:2 * H * D + 2 * H * V], torch.rand((V,), generator=gen, device="cuda") + 0.5
     state, y = first.clone(), torch.full((T, H * V), float("nan"), device="cuda", dtype=dtype)
+    names = calls(k, monkeypatch)
     k.linear_attention_gated(y, gate, w, 1e-6, "silu", o, *args, state, plan, H, D, V, 0.3)
+    assert names == ["zlm_linear_attention"] + ["zlm_norm_gate"] * (V > 128)
     z = gate.double()
     close(y, (unit(want) * w.double()).flatten(1) * z * torch.sigmoid(z), 4e-3 if dtype == torch.bfloat16 else 2e-6)
     close(state, S, 1e-6)

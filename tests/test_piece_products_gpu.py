@@ -30,6 +30,17 @@ def close(got, want, rel):
     assert (got.double() - want).norm() <= rel * want.norm(), f"{((got.double() - want).norm() / want.norm()).item():.2e}"
 
 
+def calls(k, monkeypatch):
+    """The names of the library's entry points, as ``k`` calls them from here on."""
+    names, call = [], k._call
+
+    def noted(name, *args):
+        names.append(name)
+        return call(name, *args)
+    monkeypatch.setattr(k, "_call", noted)
+    return names
+
+
 def unit(o):
     return o / torch.sqrt((o * o).mean(-1, keepdim=True) + 1e-6)
 
@@ -37,9 +48,10 @@ def unit(o):
 @pytest.mark.parametrize("H,D,V,n_rot", [(2, 128, 128, 128), (3, 64, 72, 32), (1, 16, 8, 0), (2, 96, 136, 96), (1, 112, 64, 16)])
 @pytest.mark.parametrize("news,starts", [([256], [0]), ([257, 1, 64], [0, 5, 300]), ([63, 321], [9, 0])])
 @pytest.mark.parametrize("table", [True, False])
-def test_retention(H, D, V, n_rot, news, starts, table):
+def test_retention(H, D, V, n_rot, news, starts, table, monkeypatch):
     from zlm_b200.kernels import get_kernels
     k, plan = get_kernels(), plan_of(news, starts)
+    assert k.lib.zlm_retention_products(1, 2 * H * (D + V), 0, H * D, 2 * H * D, n_rot, D, V)
     T = plan.T
     g = torch.Generator(device="cuda").manual_seed(D + V + T)
     proj = torch.randn((T, 2 * H * D + 2 * H * V), generator=g, device="cuda").bfloat16()
@@ -75,7 +87,9 @@ def test_retention(H, D, V, n_rot, news, starts, table):
     close(o, want.flatten(1), 1e-6)
     close(state, S, 1e-6)
     state, y = first.clone(), torch.full((T, H * V), float("nan"), device="cuda", dtype=torch.bfloat16)
+    names = calls(k, monkeypatch)
     k.retention_gated(y, gate, 1e-6, "silu", o, *args, state, plan, H, D, V, D ** -0.5, cos_sin=cos_sin)
+    assert names == ["zlm_retention_parts"] + ["zlm_head_gate"] * (V > 128)        # (a head wider than a block norms elsewhere)
     z = gate.double()
     close(y, unit(want).flatten(1) * z * torch.sigmoid(z), 4e-3)
     close(state, S, 1e-6)
@@ -84,7 +98,7 @@ def test_retention(H, D, V, n_rot, news, starts, table):
 @pytest.mark.parametrize("H,D,V,cap", [(2, 128, 128, 15.0), (3, 64, 72, 0.0), (1, 16, 8, 15.0), (2, 96, 136, 15.0)])
 @pytest.mark.parametrize("news,starts", [([64], [0]), ([65, 1, 130], [0, 5, 300]), ([17, 2], [9, 0])])
 @pytest.mark.parametrize("spread", [1.0, 8.0])
-def test_matrix_memory(H, D, V, cap, news, starts, spread):
+def test_matrix_memory(H, D, V, cap, news, starts, spread, monkeypatch):
     """``spread``: the gates' logits times that: forget gates near 0 and 1, running maxima that jump.  Outputs are quotients
     whose denominator is a sum of either sign: one that is a hundredth of its terms carries their roundings a hundredfold, and a
     few of a head's 19 to 200 rows are like that (4e-6 over all rows; with gates spread wide one token decides a row: 1e-4)."""
@@ -92,6 +106,8 @@ def test_matrix_memory(H, D, V, cap, news, starts, spread):
     k, plan = get_kernels(), plan_of(news, starts)
     T = plan.T
     gen = torch.Generator(device="cuda").manual_seed(D + V + T)
+    assert k.lib.zlm_mlstm_products(1, 2 * H * (D + V), 0, H * D, 2 * H * D, D, V)
+    names = calls(k, monkeypatch)
 
     def rand(*shape):
         return torch.randn(shape, generator=gen, device="cuda")
@@ -127,7 +143,9 @@ def test_matrix_memory(H, D, V, cap, news, starts, spread):
         if gated:
             y = torch.full((T, H * V), float("nan"), device="cuda", dtype=torch.bfloat16)
             w = torch.rand((H * V,), generator=gen, device="cuda") + 0.5
+            names.clear()
             k.mlstm_gated(y, gate, w, 1e-6, o, *args)
+            assert names == ["zlm_mlstm"] + ["zlm_norm_gate"] * (V > 128)
             close(y, unit(want).flatten(1) * w.double() * torch.sigmoid(gate.double()), 4e-3)
         else:
             k.mlstm(o, *args)

@@ -8,22 +8,25 @@ carried inputs are the projection's own numbers plus a bias: the bits of a 32-bi
 import pytest
 import torch
 
-from test_piece_products_gpu import close, plan_of
+from test_piece_products_gpu import calls, close, plan_of
 
 pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("W,blocks,taps", [(256, 1, 4), (72, 3, 1), (320, 5, 8), (1056, 4, 3), (16, 2, 2)])
 @pytest.mark.parametrize("news,starts", [([128], [0]), ([513, 1, 7], [0, 2, 300]), ([5, 1029], [1, 9])])
-def test_prompts(W, blocks, taps, news, starts):
+@pytest.mark.parametrize("pad", [0, 2])
+def test_prompts(W, blocks, taps, news, starts, pad, monkeypatch):
+    """``pad``: columns behind the projection's; with two of them its rows are off 16 bytes, and the passes over pieces take the step."""
     from zlm_b200.kernels import get_kernels
     k, plan = get_kernels(), plan_of(news, starts)
+    names = calls(k, monkeypatch)
     T, bs = plan.T, W // blocks
     g = torch.Generator(device="cuda").manual_seed(W + taps + T)
 
     def rand(*shape, scale=1.0):
         return (torch.randn(shape, generator=g, device="cuda") * scale).bfloat16()
-    proj = rand(T, 2 * W)
+    proj = rand(T, 2 * W + pad)
     bx, by, cb, cr, ci, lam = (rand(W, scale=0.3) for _ in range(6))
     conv_w, ar, ai = rand(W, taps, scale=0.5), rand(blocks, bs, bs, scale=bs ** -0.5), rand(blocks, bs, bs, scale=bs ** -0.5)
     first = torch.randn((plan.R, taps, W), generator=g, device="cuda")
@@ -33,6 +36,7 @@ def test_prompts(W, blocks, taps, news, starts):
     state, out = first.clone(), torch.full((T, W), float("nan"), device="cuda", dtype=torch.bfloat16)
     k.rglru(out, proj, W, 0, bx, by, conv_w, cb, ar, ai, cr, ci, lam, 8.0, state, plan, W, blocks, taps, 0.7,
             gates=torch.cat([ar, ai], dim=1).contiguous())
+    assert ("zlm_rglru_cluster" in names, "zlm_rglru" in names) == (not pad, bool(pad))
     want, S = torch.empty((T, W), dtype=torch.float64, device="cuda"), first.double()
     gelu = torch.nn.functional.gelu(proj[:, :W].double() + by.double(), approximate="tanh")
     at = 0
@@ -41,7 +45,7 @@ def test_prompts(W, blocks, taps, news, starts):
         before = S[slot, 1:].clone()
         if starts[r] < taps - 1:
             before[:taps - 1 - starts[r]] = 0         # positions ahead of the sequence's first count as zeros
-        ext = torch.cat([before, (proj[at:at + n, W:].float() + bx.float()).double()])
+        ext = torch.cat([before, (proj[at:at + n, W:2 * W].float() + bx.float()).double()])
         u = sum(ext[j:j + n] * conv_w[:, j].double() for j in range(taps)) + cb.double()
         ub = u.view(n, blocks, bs)
         rg, ig = (torch.sigmoid(torch.einsum("nbi,boi->nbo", ub, m.double()).flatten(1) + b.double()) for m, b in ((ar, cr), (ai, ci)))
