@@ -178,7 +178,7 @@ extern "C" int zlm_attention_generic(void* out, int out_stride, const void* q, i
 // that is followed by a sum is written as fmaf or as a rounded product in both kernels: nothing is left to contraction.)
 // Bound by shared-memory reads (4 x 4 scores a thread: 8 reads of 16 bytes for 64 FMAs) and the FFMA pipe.  509 queries
 // behind 515 cached tokens, 16 heads of 128: 3,498 us a query a block (every query reads all its keys from L2, a row a
-// lane), 132 us here.
+// lane), 132 us here (two blocks an SM leave heads of 96 and 128 with 150 to 160 bytes of spills).
 #define AT_Q 32                  // queries of a block
 #define AT_GROUPS ATT_WARPS      // running softmaxes, a group of threads each
 #define AT_GT 64                 // threads of a group

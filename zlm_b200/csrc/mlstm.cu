@@ -634,7 +634,7 @@ mlstm_out_kernel(float* __restrict__ o, const TA* __restrict__ proj, int stride,
 // ---------------------------------------------------------------------------- the outputs as tensor-core products
 // The third pass for bfloat16 projections and heads of up to 128 coordinates, every fp32 operand cut into three bfloat16
 // pieces (split_mma.cuh), the heads' norm and gate along with it.  3,001 tokens of four sequences, 16 heads of 128 x 128: 108 us
-// on the FFMA pipe (three shared-memory reads for 48 FMAs) and 28 us norm and gate, 94 us so; outputs 3.7e-7 off 64-bit
+// on the FFMA pipe (three shared-memory reads for 48 FMAs) and 28 us norm and gate, 99 us so (56 bytes of spills); outputs 3.7e-7 off 64-bit
 // sums before, 2.1e-7 now.  (The first pass stays an FFMA chain: as products it took 37 instead of 58 us, but its states, which
 // exponential weights make the sum of a few last tokens, were 7e-8 off instead of 6e-8.)
 // grid (R * maxp * H, ceil(V / 128)); a warp owns 16 tokens and 64 value columns

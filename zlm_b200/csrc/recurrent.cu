@@ -459,7 +459,8 @@ extern "C" int zlm_rglru(void* out, int out_stride, float* u, void* u16, float* 
 // diagonal blocks' gate logits are one grouped product, z [blocks][Tp][2][bs] fp32; (3) the recurrence on thread-block
 // clusters in one pass over z and the two branches, with u formed again from the x branch (the same sum: the same bits) instead
 // of stored in fp32.  1,999 tokens of 2,048 channels in 8 blocks: convolution 37, eight products 45, three passes of the
-// recurrence 88 us before (u, z and the pieces' decays written and read by each); 11, 25 and 38 us now.
+// recurrence 88 us before (u, z and the pieces' decays written and read by each); 11, 25 and 53 us now, one by one in a layer, and
+// 67 for the three where they follow each other as dependent launches (144 before).
 
 // A thread: 8 neighbouring channels of RC_RUN tokens, each token's row of x read once for all its taps.
 #define RC_RUN 8
@@ -588,7 +589,9 @@ extern "C" int zlm_rglru_functions(float* out, const float* in, int n, int which
 // decays and inputs it keeps in registers.  What a warp's tokens do to a state, S_out = A S_in + B, is folded over the block in
 // shared memory and over the cluster in distributed shared memory; then every warp knows the state it starts from and walks
 // its tokens.  Longer sequences go round again; of a shorter one the warps without a token only meet the barriers, and the
-// blocks without one leave at once (a barrier waits for the threads that are left).  Bound by its exponentials and divisions (about 110 instructions a number).
+// blocks without one leave at once (a barrier waits for the threads that are left).  Bound by its exponentials and divisions: about
+// 150 instructions a number, half of the issue slots busy with 16 warps an SM (128 registers; 16 to 20 bytes of spills up to 4
+// taps, up to 132 beyond).
 #define RL_CLUSTER 8
 #define RL_WARPS 8
 #define RL_P 8

@@ -260,8 +260,9 @@ retention_kernel(float* __restrict__ o, const TA* __restrict__ proj, int ld, int
 //   outputs  o_j = sum_(l <= j) w_(j-l) (q_j . k_l) v_l + w_(j+1) S^T q_j            scores, weights times values, queries times state
 // All of it stays fp32: rotated queries and keys, weights and states are cut into three bfloat16 pieces (split_mma.cuh).
 // The token-by-token walk of the same pieces issues two packed FMAs and two shared-memory reads for 8 numbers of the state and
-// waits for itself: 287 us with the chain for 2,048 tokens of 16 heads of 128 x 128, 78 us as products (22 states, 11 chain, 45
-// outputs; the tensor pipe 41 % busy in the outputs, bound by a block's phases between barriers at 16 warps an SM), and no
+// waits for itself: 303 us with the chain, the heads' norm and gate for 2,048 tokens of 16 heads of 128 x 128, 87 us as products
+// (states 22, chain 11, outputs 58 one by one; the tensor pipe 32 % and the issue slots 35 % busy in the outputs, bound by a block's
+// phases between barriers at 16 warps an SM; 20 bytes of spills), and no
 // further from 64-bit sums (outputs 2.4e-7 of their norm before, 1.7e-7 now; states 2.4e-7 and 2.0e-7).  Pieces of 64 tokens:
 // the states of longer ones are fewer, but scores and weights grow with the square.
 #define RM_THREADS 256
