@@ -311,12 +311,7 @@ static int tile_group(int bm, int K) {
 template <int BN, int STAGES, int MODE>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                          void* __restrict__ Y, int T, int N, int K, int ldy, int gm,
-                          const int* __restrict__ m_tile_group, int group_rows) {
-    // A grouped product (m_tile_group given): token tile tm multiplies the matrix of group m_tile_group[tm],
-    // whose N rows start at row group * group_rows of the second operand; tiles of group -1 are not needed in
-    // this step and every role passes over them.  The table is written by a kernel of the same step and is
-    // read after the wait for it.
+                          void* __restrict__ Y, int T, int N, int K, int ldy, int gm) {
     constexpr unsigned A_BYTES = TC_BM * TC_BK * 2, B_BYTES = BN * TC_BK * 2;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -359,12 +354,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
                 int tm, tn;
                 tile_of(tile, m_tiles, n_tiles, gm, tm, tn);
-                int group = 0;
-                if (m_tile_group) {
-                    group = m_tile_group[tm];
-                    if (group < 0) continue;
-                }
-                const int a0row = tm * TC_BM, b0row = group * group_rows + tn * BN;
+                const int a0row = tm * TC_BM, b0row = tn * BN;
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     const int s = it % STAGES;
                     if (!mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, abort_flag, 1)) { ok = false; break; }
@@ -386,11 +376,6 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             unsigned it = 0, local = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-                if (m_tile_group) {
-                    int tm, tn;
-                    tile_of(tile, m_tiles, n_tiles, gm, tm, tn);
-                    if (m_tile_group[tm] < 0) continue;
-                }
                 const unsigned buf = local & 1;
                 // the epilogue must have drained this accumulator (two tiles ago)
                 ok = mbar_wait(&acc_empty[buf], ((local >> 1) & 1) ^ 1, abort_flag, 4);
@@ -419,7 +404,6 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             const unsigned buf = local & 1;
             int tm, tn;
             tile_of(tile, m_tiles, n_tiles, gm, tm, tn);
-            if (m_tile_group && m_tile_group[tm] < 0) continue;
             const int a0row = tm * TC_BM, b0row = tn * BN;
             const bool ok = mbar_wait_warp(&acc_full[buf], (local >> 1) & 1, abort_flag, 3);
             tc_fence_after();
@@ -821,6 +805,204 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 }
 
 // ---------------------------------------------------------------------------
+// Routed experts' products, on pairs of blocks with the operands swapped: an expert's matrix is the
+// 256-row operand (128 rows a block), its sorted rows are the product's N, as wide as they are many
+// (a multiple of 32, up to 256; a run-time field of the instruction descriptor).  What bounds it is the
+// experts' weights: with 192 rows an expert each tile of W crosses from L2 once (tiles of 128 rows x 256
+// outputs on stand-alone blocks pulled it twice, 48 KB a stage of 512 cycles of products: 165 and 106 us
+// for 2,048 tokens x 6 of 60 experts of 2,048 x 768), and a block that gets few rows spends few cycles on
+// them.  The table of row tiles is written by a kernel of the same step: all roles read it after the wait
+// and fetch a tile's entry one tile ahead.  Each block loads half of the rows; a box of 32, 64, 96 or 128
+// rows, whatever the rows' number: what a box holds beyond them is another expert's or zeros and its
+// columns are not stored.
+// ---------------------------------------------------------------------------
+struct ExpertMaps { CUtensorMap m[4]; };       // boxes of 32, 64, 96 and 128 rows x 64
+struct ExpertTile { int expert, row0, rows, n0; };
+__device__ __forceinline__ ExpertTile expert_tile(int tile, int n_tiles, int max_tiles, const int* __restrict__ tile_expert,
+                                                  const int* __restrict__ tile_row0, const int* __restrict__ tile_rows) {
+    const int tt = tile / n_tiles;
+    ExpertTile r{-1, 0, 0, (tile - tt * n_tiles) * 256};
+    if (tt >= max_tiles || !ZLM_CHK(tile_expert + tt, 4) || !ZLM_CHK(tile_row0 + tt, 4) || !ZLM_CHK(tile_rows + tt, 4)) return r;
+    r.expert = tile_expert[tt];
+    r.row0 = tile_row0[tt];
+    r.rows = min(tile_rows[tt], 256);
+    return r;
+}
+
+// Eight epilogue warps, two for every quarter of the accumulators' lanes, which take 32 columns in turn: with four, an SM's
+// scheduler had one warp whose loads, shuffles and stores wait for one another, and the product into fp32 rows ran at the
+// epilogue's pace (84 us; 21 % of the tensor cores' time, 3 of the memory's 6.5 TB/s).
+#define TCE_THREADS 320
+template <int STAGES, int MODE>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCE_THREADS, 1)
+gemm_tc_experts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ ExpertMaps map_x, void* __restrict__ Y,
+                       int N, int K, int ldy, int max_tiles, const int* __restrict__ tile_expert,
+                       const int* __restrict__ tile_row0, const int* __restrict__ tile_rows) {
+    constexpr unsigned A_BYTES = TC_BM * TC_BK * 2, B_BYTES = 128 * TC_BK * 2;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* sA = smem;
+    unsigned char* sB = smem + STAGES * A_BYTES;
+    uint64_t* full = (uint64_t*)(sB + STAGES * B_BYTES);
+    uint64_t* empty = full + STAGES;
+    uint64_t* acc_full = empty + STAGES;       // [2]
+    uint64_t* acc_empty = acc_full + 2;        // [2]
+    unsigned* tmem_slot = (unsigned*)(acc_empty + 2);
+    volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned rank = cluster_rank();
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int KB = (K + TC_BK - 1) / TC_BK;
+    const int n_tiles = (N + TCQ_BM - 1) / TCQ_BM;
+#define ZLM_TILE_AT(t) expert_tile(t, n_tiles, max_tiles, tile_expert, tile_row0, tile_rows)
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 16); }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n"
+                     ::"r"(smem_u32(tmem_slot)), "r"((unsigned)(2 * TCP_ACC)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();          // the other block's barriers are initialised before anything arrives there
+    tc_fence_after();
+    const unsigned tmem_base = *tmem_slot;
+    pdl_launch_dependents();
+    pdl_wait();
+
+    if (warp == 0) {
+        if (lane == 0) {
+            unsigned it = 0;
+            bool ok = true;
+            ExpertTile next = ZLM_TILE_AT(pair);
+            for (int tile = pair; next.expert >= 0 && ok; tile += pairs) {
+                const ExpertTile t = next;
+                next = ZLM_TILE_AT(tile + pairs);
+                const int half = (t.rows + 31) / 32 * 16, box = (half + 31) / 32;      // box: in 32 rows
+                const CUtensorMap* mx = &map_x.m[box - 1];
+                const unsigned bytes = 2 * (A_BYTES + (unsigned)box * 32 * TC_BK * 2);
+                const int w0 = t.expert * N + t.n0 + rank * TC_BM, x0 = t.row0 + rank * half;
+                for (int kb = 0; kb < KB; ++kb, ++it) {
+                    const int s = it % STAGES;
+                    const unsigned bar0 = cluster_addr(&full[s], 0);
+                    if (!mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, abort_flag, 1)) { ok = false; break; }
+                    if (rank == 0) mbar_expect_tx(&full[s], bytes);
+                    tma_load_2d_pair(sA + s * A_BYTES, &map_w, kb * TC_BK, w0, bar0);
+                    tma_load_2d_pair(sB + s * B_BYTES, mx, kb * TC_BK, x0, bar0);
+                }
+            }
+            if (*abort_flag && rank == 0) {
+                for (unsigned j = it > (unsigned)STAGES ? it - STAGES : 0; j < it; ++j)
+                    mbar_drain(&full[j % STAGES], (j / STAGES) & 1);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && rank == 0) {
+            unsigned it = 0, local = 0;
+            bool ok = true;
+            ExpertTile next = ZLM_TILE_AT(pair);
+            for (int tile = pair; next.expert >= 0 && ok; tile += pairs, ++local) {
+                const ExpertTile t = next;
+                next = ZLM_TILE_AT(tile + pairs);
+                // fp32 accumulate, bf16 x bf16, both K-major, N the rows rounded up to 32, M = 256 over the two blocks
+                const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((t.rows + 31) / 32 * 4) << 17) |
+                                       ((unsigned)(TCQ_BM >> 4) << 24);
+                const unsigned buf = local & 1;
+                ok = mbar_wait_pair(&acc_empty[buf], ((local >> 1) & 1) ^ 1, abort_flag, 4);
+                if (!ok) break;
+                tc_fence_after();
+                for (int kb = 0; kb < KB; ++kb, ++it) {
+                    const int s = it % STAGES;
+                    ok = mbar_wait(&full[s], (it / STAGES) & 1, abort_flag, 2);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint64_t ad = make_desc(smem_u32(sA + s * A_BYTES)), bd = make_desc(smem_u32(sB + s * B_BYTES));
+#pragma unroll
+                    for (int k = 0; k < TC_BK / 16; ++k)
+                        tc_mma_pair(tmem_base + buf * TCP_ACC, ad + ((k * 32) >> 4), bd + ((k * 32) >> 4), idesc, (kb | k) != 0);
+                    tc_commit_pair(&empty[s]);
+                }
+                tc_commit_pair(&acc_full[buf]);
+            }
+            if (!ok) { tc_commit_pair(&acc_full[0]); tc_commit_pair(&acc_full[1]); }     // let the epilogues out
+        }
+    } else {
+        const int lg = warp & 3, turn = (warp - 2) >> 2;
+        unsigned local = 0;
+        const unsigned empty0[2] = {cluster_addr(&acc_empty[0], 0), cluster_addr(&acc_empty[1], 0)};
+        ExpertTile next = ZLM_TILE_AT(pair);
+        for (int tile = pair; next.expert >= 0; tile += pairs, ++local) {
+            const ExpertTile t = next;
+            next = ZLM_TILE_AT(tile + pairs);
+            const unsigned buf = local & 1;
+            const bool ok = mbar_wait_warp(&acc_full[buf], (local >> 1) & 1, abort_flag, 3);
+            tc_fence_after();
+            if (!ok || *abort_flag) break;
+            const int out = t.n0 + (int)rank * TC_BM + lg * 32 + lane;        // this lane's row of the expert's matrix
+            const unsigned taddr = tmem_base + ((unsigned)(lg * 32) << 16) + buf * TCP_ACC;
+#pragma unroll 1
+            for (int c = turn * 32; c < t.rows; c += 64) {
+                const bool whole = c + 32 <= t.rows;
+                float v[32];
+                tc_ld16_nowait(taddr + (unsigned)c, v);
+                tc_ld16_nowait(taddr + (unsigned)c + 16, v + 16);
+                tc_wait_ld();
+                if (MODE == 2) {
+                    // a warp's 32 lanes are 32 neighbouring outputs of one row: whole lines
+                    float* y = (float*)Y + (size_t)(t.row0 + c) * ldy + out;
+                    if (out < N) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i, y += ldy)
+                            if ((whole || c + i < t.rows) && ZLM_CHK(y, 4)) *y = v[i];
+                    }
+                } else if (MODE == 6) {
+                    // neighbouring lanes trade: the even one stores row 2 i's pair of outputs, the odd one row 2 i + 1's
+                    const bool odd = lane & 1;
+                    __nv_bfloat16* y = (__nv_bfloat16*)Y + (size_t)(t.row0 + c + odd) * ldy + (out & ~1);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i, y += 2 * ldy) {
+                        const float got = __shfl_xor_sync(0xffffffffu, odd ? v[2 * i] : v[2 * i + 1], 1);
+                        const float a = fmaxf(odd ? got : v[2 * i], 0.f), b = fmaxf(odd ? v[2 * i + 1] : got, 0.f);
+                        if ((whole || c + 2 * i + odd < t.rows) && out < N && ZLM_CHK(y, 4))
+                            *(__nv_bfloat162*)y = __floats2bfloat162_rn(a * a, b * b);
+                    }
+                } else {
+                    // lanes 0-7 and 16-23 hold gate rows, lanes 8-15 and 24-31 the matching up rows: they trade halves of
+                    // the 32 columns, so that every lane finishes one channel of 16 rows
+                    const bool up = lane & 8;
+                    const int ch = (out >> 4) * 8 + (out & 7), first = c + (up ? 16 : 0);
+                    __nv_bfloat16* y = (__nv_bfloat16*)Y + (size_t)(t.row0 + first) * ldy + ch;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i, y += ldy) {
+                        const float got = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[16 + i], 8);
+                        const float z = gated_mul<MODE>(up ? got : v[i], up ? v[16 + i] : got);
+                        if ((whole || first + i < t.rows) && out < N && ZLM_CHK(y, 2)) *y = __float2bfloat16_rn(z);
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_at(empty0[buf]);
+        }
+    }
+#undef ZLM_TILE_AT
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();          // neither block leaves while the other may still read its memory or signal it
+    if (warp == 1) {
+        __syncwarp();
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"((unsigned)(2 * TCP_ACC)) : "memory");
+    }
+}
+
+// ---------------------------------------------------------------------------
 // The few-token form (17 to 384 tokens) as a persistent kernel.  W is the 128-row operand,
 // the tokens are the product's N (a tile of BN = 32, 64 or 128).  A work item is a tile of
 // 128 outputs x BN tokens and one of `ks` shares of K; one block per SM walks the items, its
@@ -1188,8 +1370,7 @@ static int launch_tc_persistent(void* Y, const void* X, const void* W, int T, in
             }                                                                                              \
             attr_set = true;                                                                               \
         }                                                                                                  \
-        zlm_launch(kern, dim3(blocks), dim3(TC_THREADS), smem, st, mx, mw, Y, T, N, K, ldy, tile_group(TC_BM, K), \
-                   (const int*)nullptr, 0); \
+        zlm_launch(kern, dim3(blocks), dim3(TC_THREADS), smem, st, mx, mw, Y, T, N, K, ldy, tile_group(TC_BM, K)); \
     }
     if (mode == 0) ZLM_TCP_LAUNCH(0)
     else if (mode == 1) ZLM_TCP_LAUNCH(1)
@@ -1321,54 +1502,57 @@ static int launch_tc_few(void* Y, const void* X, const void* W, int T, int N, in
     return launch_reduce(Y, scratch, T, N, ldy, mode, plan.ks, plan.whole / plan.t_tiles * TC_BM, st);
 }
 
-// A grouped product for routed experts: the rows of X come in tiles of 128, tile tm belongs to group
-// tile_group[tm] (-1: not used in this step), and multiplies that group's matrix, rows
-// [group * N, group * N + N) of W [groups * N, K]; Y [m_tiles * 128, N]; group_of_tile[tm] is tile tm's group.  The persistent single-block
-// form with its tiles' second operand looked up per token tile.
-// mode 0: Y bf16; mode 2: Y fp32; mode 6: Y bf16 = relu(.)^2; mode 3: Y bf16 [.., N / 2] = silu(gate) * up, a group's rows in
-// sixteens of 8 gate rows and the 8 matching up rows; mode 8: the same with the clamped activation, whose constants
+// The products of routed experts.  X [rows, K]: the (token, choice) rows sorted by expert; tile tt of the table holds
+// rows tile_row0[tt] .. + tile_rows[tt] (at most 256) of expert tile_expert[tt] (-1: the table ends), which multiply that
+// expert's matrix, rows [e * N, e * N + N) of W [experts * N, K]; Y [rows, ldy].
+// mode 2: Y fp32; mode 6: Y bf16 = relu(.)^2; mode 3: Y bf16 [.., N / 2] = silu(gate) * up, an expert's rows in sixteens
+// of 8 gate rows and the 8 matching up rows; mode 8: the same with the clamped activation, whose constants
 // zlm_set_gate_gemm_tcgen05 has set before.
-extern "C" int zlm_gemm_tc_grouped(void* Y, const void* X, const void* W, const int* group_of_tile, int m_tiles, int groups,
-                                   int N, int K, int ldy, int mode, cudaStream_t st) {
-    if (m_tiles == 0 || N == 0) return ZLM_OK;
-    const int T = m_tiles * TC_BM;
-    ZLM_REQUIRE(m_tiles > 0 && groups > 0 && N >= 8 && K >= 8 && K % 8 == 0, "gemm_tc_grouped: tiles=%d groups=%d N=%d K=%d",
-                m_tiles, groups, N, K);
-    ZLM_REQUIRE((long long)groups * N < (1ll << 31), "gemm_tc_grouped: %d groups of %d rows", groups, N);
-    ZLM_REQUIRE(((uintptr_t)X % 16 == 0) && ((uintptr_t)W % 16 == 0) && group_of_tile, "gemm_tc_grouped: operands must be 16-byte aligned");
-    ZLM_REQUIRE(mode == 0 || mode == 2 || mode == 3 || mode == 6 || mode == 8, "gemm_tc_grouped: mode %d", mode);
-    ZLM_REQUIRE(!ZLM_GATED(mode) || N % 16 == 0, "gemm_tc_grouped: gated rows come in groups of 16, N=%d", N);
-    constexpr int BN = 256, STAGES = 4;
-    CUtensorMap mx, mw;
-    int rc = make_map(&mx, X, T, K, K, TC_BM);
+extern "C" int zlm_gemm_tc_experts(void* Y, const void* X, const void* W, const int* table, int max_tiles, int rows,
+                                   int experts, int N, int K, int ldy, int mode, cudaStream_t st) {
+    if (max_tiles == 0 || rows == 0 || N == 0) return ZLM_OK;
+    ZLM_REQUIRE(max_tiles > 0 && rows > 0 && experts > 0 && N >= 8 && K >= 8 && K % 8 == 0 && N % 2 == 0,
+                "gemm_tc_experts: tiles=%d rows=%d experts=%d N=%d K=%d", max_tiles, rows, experts, N, K);
+    ZLM_REQUIRE((long long)experts * N < (1ll << 31), "gemm_tc_experts: %d experts of %d rows", experts, N);
+    ZLM_REQUIRE(((uintptr_t)X % 16 == 0) && ((uintptr_t)W % 16 == 0) && table && (uintptr_t)Y % 4 == 0,
+                "gemm_tc_experts: operands must be 16-byte aligned");
+    ZLM_REQUIRE(mode == 2 || mode == 3 || mode == 6 || mode == 8, "gemm_tc_experts: mode %d", mode);
+    ZLM_REQUIRE(!ZLM_GATED(mode) || N % 16 == 0, "gemm_tc_experts: gated rows come in groups of 16, N=%d", N);
+    ZLM_REQUIRE(mode != 6 || ldy % 2 == 0, "gemm_tc_experts: rows of %d outputs", ldy);
+    constexpr int STAGES = 6;
+    CUtensorMap mw;
+    ExpertMaps mx;
+    int rc = make_map(&mw, W, experts * N, K, K, TC_BM);
     if (rc) return rc;
-    rc = make_map(&mw, W, groups * N, K, K, BN);
-    if (rc) return rc;
-    const size_t smem = (size_t)STAGES * (TC_BM + BN) * TC_BK * 2 + 1024 + 256;
-    const long long tiles = (long long)m_tiles * ((N + BN - 1) / BN);
-    const int blocks = (int)(tiles < sm_count() ? tiles : sm_count());
-#define ZLM_TCG_LAUNCH(M)                                                                                  \
+    for (int i = 0; i < 4; ++i) {
+        rc = make_map(&mx.m[i], X, rows, K, K, 32 * (i + 1));
+        if (rc) return rc;
+    }
+    const size_t smem = (size_t)STAGES * 2 * TC_BM * TC_BK * 2 + 1024 + 256;
+    const long long tiles = (long long)max_tiles * ((N + TCQ_BM - 1) / TCQ_BM);
+    ZLM_REQUIRE(tiles < (1ll << 30), "gemm_tc_experts: too many tiles (%lld)", tiles);
+    const int pairs = (int)(tiles < sm_count() / 2 ? tiles : sm_count() / 2);
+#define ZLM_TCE_LAUNCH(M)                                                                                  \
     {                                                                                                      \
-        auto kern = gemm_tc_persistent_kernel<BN, STAGES, M>;                                              \
+        auto kern = gemm_tc_experts_kernel<STAGES, M>;                                                     \
         static bool attr_set_dev[64] = {}; bool& attr_set = attr_set_dev[zlm_device_index()];              \
         if (!attr_set) {                                                                                   \
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
             if (e != cudaSuccess) {                                                                        \
-                zlm_set_error("gemm_tc_grouped: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e)); \
+                zlm_set_error("gemm_tc_experts: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e)); \
                 return ZLM_ERR_CUDA;                                                                       \
             }                                                                                              \
             attr_set = true;                                                                               \
         }                                                                                                  \
-        zlm_launch(kern, dim3(blocks), dim3(TC_THREADS), smem, st, mx, mw, Y, T, N, K, ldy, tile_group(TC_BM, K), \
-                   group_of_tile, N);                                                                       \
+        zlm_launch(kern, dim3(2 * pairs), dim3(TCE_THREADS), smem, st, mw, mx, Y, N, K, ldy, max_tiles, table, \
+                   table + max_tiles, table + 2 * max_tiles);                                              \
     }
-    if (mode == 0) ZLM_TCG_LAUNCH(0)
-    else if (mode == 2) ZLM_TCG_LAUNCH(2)
-    else if (mode == 3) ZLM_TCG_LAUNCH(3)
-    else if (mode == 8) ZLM_TCG_LAUNCH(8)
-    else ZLM_TCG_LAUNCH(6)
-#undef ZLM_TCG_LAUNCH
-    return zlm_check_launch("gemm_tc_grouped");
+    if (mode == 2) ZLM_TCE_LAUNCH(2)
+    else if (mode == 3) ZLM_TCE_LAUNCH(3)
+    else if (mode == 8) ZLM_TCE_LAUNCH(8)
+    else ZLM_TCE_LAUNCH(6)
+#undef ZLM_TCE_LAUNCH
+    return zlm_check_launch("gemm_tc_experts");
 }
 
 // 1 if the tensor-memory kernel takes this product (else use zlm_gemm_bf16_mma)

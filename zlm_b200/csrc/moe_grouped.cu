@@ -24,69 +24,113 @@ __device__ __forceinline__ void mg_cp_async16(void* smem, const void* gmem, bool
 }
 
 // ---------------------------------------------------------------------------- sort
-// One block.  counts and cursors in shared memory (E entries each); tile table: tile -> (expert, first
-// sorted row, rows), expert -1 for the tiles a step does not need.
-__global__ void __launch_bounds__(1024)
-moe_sort_kernel(const int* __restrict__ idx, int P, int E, int BM, int max_tiles, int padded, int drop, int* __restrict__ perm,
+// A cluster of MS_BLOCKS blocks, each with a share of the pairs: it counts its share's pairs by expert, reads the
+// other blocks' counts through their shared memory, and from the sums over experts and over the blocks before it knows
+// where its own pairs go.  (One block alone took 17 to 24 us for 12,288 pairs: its thread that walked the experts and
+// the atomics of all pairs on one SM.)  An expert's n rows come in ceil(n / BM) tiles of equal height (but the last);
+// the tile table: tile -> (expert, first sorted row, rows), expert -1 for the tiles a step does not need.
+#define MS_BLOCKS 8
+__device__ __forceinline__ int ms_remote(const int* p, unsigned rank) {
+    unsigned a;
+    int v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.s32 %0, [%1];\n" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void ms_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+__global__ void __cluster_dims__(MS_BLOCKS, 1, 1) __launch_bounds__(1024)
+moe_sort_kernel(const int* __restrict__ idx, int P, int E, int BM, int max_tiles, int drop, int* __restrict__ perm,
                 int* __restrict__ inv, int* __restrict__ tile_expert, int* __restrict__ tile_row0,
                 int* __restrict__ tile_rows) {
     extern __shared__ int sh[];
-    int* count = sh;              // [E]
-    int* start = sh + E;          // [E + 1] first sorted row of each expert
-    int* tstart = start + E + 1;  // [E + 1] first tile of each expert
+    int* count = sh;              // [E] this block's pairs
+    int* total = sh + E;          // [E] all blocks' pairs
+    int* cursor = total + E;      // [E] where this block's next pair of the expert goes
+    int* tstart = cursor + E;     // [E + 1] first tile of each expert
+    const int rank = blockIdx.x, tid = threadIdx.x;
     pdl_trigger();
-    for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
+    for (int e = tid; e < E; e += blockDim.x) count[e] = 0;
     pdl_wait();
-    // padded: every expert's rows start at a tile's first row, and the rows between are marked empty
-    if (padded)
-        for (int i = threadIdx.x; i < max_tiles * BM; i += blockDim.x)
-            if (ZLM_CHK(perm + i, 4)) perm[i] = -1;
     __syncthreads();
+    const int per = (P + MS_BLOCKS - 1) / MS_BLOCKS, lo = min(P, rank * per), hi = min(P, lo + per);
     // drop: a pair whose index is E or more (an expert without matrices) gets no row; its inv is -1
-    for (int i = threadIdx.x; i < P; i += blockDim.x)
-        if (ZLM_CHK(idx + i, 4) && !(drop && idx[i] >= E)) atomicAdd(&count[min(max(idx[i], 0), E - 1)], 1);
+    for (int i = lo + tid; i < hi; i += blockDim.x) {
+        if (!ZLM_CHK(idx + i, 4)) continue;
+        const int e = idx[i];
+        if (!(drop && e >= E)) atomicAdd(&count[min(max(e, 0), E - 1)], 1);
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int s = 0, t = 0;
-        for (int e = 0; e < E; ++e) {
-            start[e] = padded ? t * BM : s;
-            tstart[e] = t;
-            s += count[e];
-            t += (count[e] + BM - 1) / BM;
+    ms_cluster_sync();
+    for (int e = tid; e < E; e += blockDim.x) {
+        int all = 0, before = 0;
+#pragma unroll
+        for (int r = 0; r < MS_BLOCKS; ++r) {
+            const int c = ms_remote(count + e, r);
+            if (r < rank) before += c;
+            all += c;
         }
-        start[E] = padded ? t * BM : s;
-        tstart[E] = t;
+        total[e] = all;
+        cursor[e] = before;
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < E; e += blockDim.x) {
-        const int n = count[e];
-        for (int j = 0, t = tstart[e]; j * BM < n; ++j, ++t)
-            if (t < max_tiles && ZLM_CHK(tile_expert + t, 4) && ZLM_CHK(tile_row0 + t, 4) && ZLM_CHK(tile_rows + t, 4)) {
-                tile_expert[t] = e;
-                tile_row0[t] = start[e] + j * BM;
-                tile_rows[t] = min(BM, n - j * BM);
+    ms_cluster_sync();            // the counts have been read: any block may leave from here on
+    if (tid < 32) {               // running sums over the experts, 32 at a time
+        int rows = 0, tiles = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + tid, n = e < E ? total[e] : 0, t = (n + BM - 1) / BM;
+            int sn = n, stl = t;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int a = __shfl_up_sync(0xffffffffu, sn, o), b = __shfl_up_sync(0xffffffffu, stl, o);
+                if (tid >= o) { sn += a; stl += b; }
             }
-        count[e] = 0;            // from here on: the expert's cursor
+            if (e < E) {
+                cursor[e] += rows + sn - n;
+                tstart[e] = tiles + stl - t;
+            }
+            rows += __shfl_sync(0xffffffffu, sn, 31);
+            tiles += __shfl_sync(0xffffffffu, stl, 31);
+        }
+        if (tid == 0) tstart[E] = tiles;
     }
-    for (int t = tstart[E] + threadIdx.x; t < max_tiles; t += blockDim.x)
-        if (ZLM_CHK(tile_expert + t, 4)) tile_expert[t] = -1;
     __syncthreads();
+    if (rank == 0) {              // (no block before it: its cursors are the experts' first rows)
+        for (int e = tid; e < E; e += blockDim.x) {
+            const int n = total[e], tiles = tstart[e + 1] - tstart[e], high = tiles ? (n + tiles - 1) / tiles : 0;
+            for (int j = 0, t = tstart[e]; j < tiles; ++j, ++t)
+                if (t < max_tiles && ZLM_CHK(tile_expert + t, 4) && ZLM_CHK(tile_row0 + t, 4) && ZLM_CHK(tile_rows + t, 4)) {
+                    tile_expert[t] = e;
+                    tile_row0[t] = cursor[e] + j * high;
+                    tile_rows[t] = min(high, n - j * high);
+                }
+        }
+        for (int t = tstart[E] + tid; t < max_tiles; t += blockDim.x)
+            if (ZLM_CHK(tile_expert + t, 4)) tile_expert[t] = -1;
+        __syncthreads();
+    }
     // a pair's place among its expert's rows is whatever the cursor gives it: a row's result does not depend
     // on its place, and the combine step finds it through inv
     // (lanes that hold the same expert adding once through their first lane was measured: twice as slow)
-    for (int i = threadIdx.x; i < P; i += blockDim.x) {
+    for (int i = lo + tid; i < hi; i += blockDim.x) {
         if (!ZLM_CHK(idx + i, 4)) continue;
-        if (drop && idx[i] >= E) {
+        int e = idx[i];
+        if (drop && e >= E) {
             if (ZLM_CHK(inv + i, 4)) inv[i] = -1;
             continue;
         }
-        const int e = min(max(idx[i], 0), E - 1);
-        const int place = start[e] + atomicAdd(&count[e], 1);
-        if (ZLM_CHK(perm + place, 4) && ZLM_CHK(inv + i, 4)) {
-            perm[place] = i;
-            inv[i] = place;
-        }
+        e = min(max(e, 0), E - 1);
+        const int place = atomicAdd(&cursor[e], 1);
+        if (!ZLM_CHK(inv + i, 4)) continue;
+        inv[i] = place;
+        if (perm && ZLM_CHK(perm + place, 4)) perm[place] = i;
     }
+}
+static int launch_sort(const int* idx, int P, int E, int BM, int max_tiles, int drop, int* perm, int* inv, int* tiles, cudaStream_t st) {
+    zlm_launch(moe_sort_kernel, dim3(MS_BLOCKS), dim3(1024), (size_t)(4 * E + 1) * sizeof(int), st, idx, P, E, BM, max_tiles, drop, perm,
+               inv, tiles, tiles + max_tiles, tiles + 2 * max_tiles);
+    return zlm_check_launch("moe_sort");
 }
 
 // ---------------------------------------------------------------------------- grouped products
@@ -370,9 +414,7 @@ extern "C" int zlm_moe_grouped(float* stream, const void* x, int x_stride, const
     int* perm = ints;
     int* inv = ints + P;
     int* tiles = ints + 2 * P;
-    zlm_launch(moe_sort_kernel, dim3(1), dim3(1024), (size_t)(3 * E + 2) * sizeof(int), st, idx, P, E, BM, max_tiles, 0, 0, perm,
-               inv, tiles, tiles + max_tiles, tiles + 2 * max_tiles);
-    int rc = zlm_check_launch("moe_sort");
+    int rc = launch_sort(idx, P, E, BM, max_tiles, 0, perm, inv, tiles, st);
     if (rc) return rc;
 #define ZLM_MG(BM_, WM_, WN_)                                                                                         \
     do {                                                                                                              \
@@ -392,54 +434,62 @@ extern "C" int zlm_moe_grouped(float* stream, const void* x, int x_stride, const
     return zlm_check_launch("moe_combine");
 }
 
-// ---------------------------------------------------------------------------- the pieces, for the tcgen05 grouped product
-// Rows in tiles of 128 with every expert's rows starting at a tile (padded): ints = perm [max_tiles * 128] (-1: an
-// empty row) | inv [P] | tile table [3 * max_tiles]; the table's first part is what zlm_gemm_tc_grouped reads.
-extern "C" int zlm_moe_sort_padded(const int* idx, int P, int E, int max_tiles, int* ints, cudaStream_t st) {
-    ZLM_REQUIRE(P > 0 && E > 0 && E <= 2048 && max_tiles > 0, "moe_sort: pairs=%d experts=%d tiles=%d", P, E, max_tiles);
-    int* perm = ints;
-    int* inv = ints + (size_t)max_tiles * 128;
-    int* tiles = inv + P;
-    zlm_launch(moe_sort_kernel, dim3(1), dim3(1024), (size_t)(3 * E + 2) * sizeof(int), st, idx, P, E, 128, max_tiles, 1, 1, perm,
-               inv, tiles, tiles + max_tiles, tiles + 2 * max_tiles);
-    return zlm_check_launch("moe_sort");
+// ---------------------------------------------------------------------------- the pieces, for the tcgen05 products
+// Rows sorted by expert, tiles of at most 256 of them: inv [P] and the tile table [3 * max_tiles] that zlm_gemm_tc_experts
+// reads; pairs of an index from E on take no row (inv -1).
+extern "C" int zlm_moe_sort(const int* idx, int P, int E, int max_tiles, int* inv, int* table, cudaStream_t st) {
+    ZLM_REQUIRE(P > 0 && E > 0 && E <= 2048 && max_tiles >= (P + 255) / 256 + min(E, P), "moe_sort: pairs=%d experts=%d tiles=%d",
+                P, E, max_tiles);
+    return launch_sort(idx, P, E, 256, max_tiles, 1, nullptr, inv, table, st);
 }
 
-// xs[row, :] = bf16(w * x[token(row), :]) for the sorted, padded rows (empty rows are left alone); w the pair's weight
-// if scale (the weight on the expert's input), else 1
+// xs[inv[t, j], :] = bf16(w * x[t, :]); w the pair's weight if scale (the weight on the expert's input), else 1.  A block
+// reads its token once and writes the rows of all its choices, whose places are in registers before the first store: the
+// stores are what bounds it (47 MB for 2,048 tokens of 2,048 channels and 6 choices).
+#define MO_KEEP 8
 __global__ void __launch_bounds__(256)
 moe_gather_kernel(__nv_bfloat16* __restrict__ xs, const __nv_bfloat16* __restrict__ x, int x_stride,
-                  const int* __restrict__ perm, const float* __restrict__ wgt, int top, int K, int scale) {
+                  const int* __restrict__ inv, const float* __restrict__ wgt, int top, int K, int scale) {
     pdl_launch_dependents();
     pdl_wait();
-    const int row = blockIdx.x;
-    if (!ZLM_CHK(perm + row, 4)) return;
-    const int pair = perm[row];
-    __nv_bfloat16* dst = xs + (size_t)row * K;
-    // (an empty row's products are rows that nobody reads, whatever stands in it: of 2,048 tokens with 6 choices among 60 experts
-    // 20,000 rows were written for 11,500 that count, 21.3 us; 17.9 us without the others)
-    if (pair < 0) return;
-    const __nv_bfloat16* src = x + (size_t)(pair / top) * x_stride;
-    const float w = (scale && ZLM_CHK(wgt + pair, 4)) ? wgt[pair] : 1.0f;
-    for (int c = threadIdx.x; c < K / 8; c += blockDim.x) {
-        if (!ZLM_CHK(src + c * 8, 16) || !ZLM_CHK(dst + c * 8, 16)) continue;
-        uint4 v = *(const uint4*)(src + c * 8);
-        if (scale) {
-            unsigned* u = (unsigned*)&v;
+    const int token = blockIdx.x;
+    const __nv_bfloat16* src = x + (size_t)token * x_stride;
+    for (int j0 = 0; j0 < top; j0 += MO_KEEP) {
+        int row[MO_KEEP];
+        float w[MO_KEEP];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                u[i] = pack_bf16(__uint_as_float(u[i] << 16) * w, __uint_as_float(u[i] & 0xffff0000u) * w);
+        for (int j = 0; j < MO_KEEP; ++j) {
+            const int pair = token * top + j0 + j;
+            row[j] = j0 + j < top && ZLM_CHK(inv + pair, 4) ? inv[pair] : -1;
+            w[j] = scale && j0 + j < top && ZLM_CHK(wgt + pair, 4) ? wgt[pair] : 1.0f;
         }
-        *(uint4*)(dst + c * 8) = v;
+        for (int c = threadIdx.x; c < K / 8; c += blockDim.x) {
+            if (!ZLM_CHK(src + c * 8, 16)) continue;
+            const uint4 v = *(const uint4*)(src + c * 8);
+#pragma unroll
+            for (int j = 0; j < MO_KEEP; ++j) {
+                __nv_bfloat16* dst = xs + (size_t)row[j] * K + c * 8;
+                if (row[j] < 0 || !ZLM_CHK(dst, 16)) continue;
+                uint4 o = v;
+                if (scale) {
+                    unsigned* u = (unsigned*)&o;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        u[i] = pack_bf16(__uint_as_float(u[i] << 16) * w[j], __uint_as_float(u[i] & 0xffff0000u) * w[j]);
+                }
+                *(uint4*)dst = o;
+            }
+        }
     }
 }
 
-extern "C" int zlm_moe_gather(void* xs, const void* x, int x_stride, const int* perm, const float* wgt, int rows, int top,
+extern "C" int zlm_moe_gather(void* xs, const void* x, int x_stride, const int* inv, const float* wgt, int T, int top,
                               int K, int scale, cudaStream_t st) {
-    if (rows == 0) return ZLM_OK;
+    if (T == 0) return ZLM_OK;
     ZLM_REQUIRE(K % 8 == 0 && x_stride % 8 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)xs % 16 == 0,
                 "moe_gather: K=%d and the row stride must be multiples of 8, operands 16-byte aligned", K);
-    zlm_launch(moe_gather_kernel, dim3(rows), dim3(256), 0, st, (__nv_bfloat16*)xs, (const __nv_bfloat16*)x, x_stride, perm, wgt,
+    ZLM_REQUIRE((long long)T * top < (1ll << 31), "moe_gather: %d tokens of %d choices", T, top);
+    zlm_launch(moe_gather_kernel, dim3(T), dim3(K > 1024 ? 256 : 128), 0, st, (__nv_bfloat16*)xs, (const __nv_bfloat16*)x, x_stride, inv, wgt,
                top, K, scale);
     return zlm_check_launch("moe_gather");
 }

@@ -466,7 +466,7 @@ extern "C" int zlm_rglru(void* out, int out_stride, float* u, void* u16, float* 
 #define RC_RUN 8
 template <int TAPS>
 __global__ void __launch_bounds__(128)
-rglru_conv_blocks_kernel(__nv_bfloat16* __restrict__ u16, int* __restrict__ group_of_tile, const __nv_bfloat16* __restrict__ proj,
+rglru_conv_blocks_kernel(__nv_bfloat16* __restrict__ u16, int* __restrict__ table, const __nv_bfloat16* __restrict__ proj,
                          int proj_stride, int x_off, const __nv_bfloat16* __restrict__ bx, const __nv_bfloat16* __restrict__ conv_w,
                          const __nv_bfloat16* __restrict__ cb, const float* __restrict__ state, const int* __restrict__ token_pos,
                          const int* __restrict__ token_slot, const int* __restrict__ token_seq, const int* __restrict__ seq_start,
@@ -485,9 +485,14 @@ rglru_conv_blocks_kernel(__nv_bfloat16* __restrict__ u16, int* __restrict__ grou
         }
     }
     pdl_wait();
-    if (blockIdx.x == 0)                              // (for the product: which diagonal block a tile of 128 rows belongs to)
-        for (int x = blockIdx.y * 128 + threadIdx.x; x < blocks * (Tp / 128); x += gridDim.y * 128)
-            if (ZLM_CHK(group_of_tile + x, 4)) group_of_tile[x] = x / (Tp / 128);
+    const int per = (T + 255) / 256, tiles = blocks * per;       // (for the product: tiles of up to 256 rows of one diagonal block)
+    if (blockIdx.x == 0)
+        for (int x = blockIdx.y * 128 + threadIdx.x; x < tiles; x += gridDim.y * 128)
+            if (ZLM_CHK(table + x, 4) && ZLM_CHK(table + tiles + x, 4) && ZLM_CHK(table + 2 * tiles + x, 4)) {
+                table[x] = x / per;
+                table[tiles + x] = x / per * Tp + x % per * 256;
+                table[2 * tiles + x] = min(256, T - x % per * 256);
+            }
     if (c >= W) return;
     uint4 x[RC_RUN + TAPS - 1];
 #pragma unroll
@@ -773,8 +778,8 @@ rglru_cluster_kernel(__nv_bfloat16* __restrict__ out, int out_stride, const floa
 }
 
 // bfloat16, with everything as in zlm_rglru: the first of the three launches.  u16 [blocks][Tp][W/blocks], Tp = T rounded up to
-// 128; group_of_tile [blocks * Tp / 128] for zlm_gemm_tc_grouped.
-extern "C" int zlm_rglru_conv_blocks(void* u16, int* group_of_tile, const void* proj, int proj_stride, int x_off, const void* bx,
+// 128; table [3][blocks * ceil(T / 256)] for zlm_gemm_tc_experts.
+extern "C" int zlm_rglru_conv_blocks(void* u16, int* table, const void* proj, int proj_stride, int x_off, const void* bx,
                                      const void* conv_w, const void* cb, const float* state, const int* token_pos,
                                      const int* token_slot, const int* token_seq, const int* seq_start, int T, int W, int blocks, int taps,
                                      cudaStream_t st) {
@@ -787,7 +792,7 @@ extern "C" int zlm_rglru_conv_blocks(void* u16, int* group_of_tile, const void* 
     const dim3 grid((T + RC_RUN - 1) / RC_RUN, (W + 1023) / 1024);
 #define ZLM_RC(N)                                                                                                               \
     case N:                                                                                                                     \
-        zlm_launch(rglru_conv_blocks_kernel<N>, grid, dim3(128), 0, st, (__nv_bfloat16*)u16, group_of_tile, (const __nv_bfloat16*)proj, \
+        zlm_launch(rglru_conv_blocks_kernel<N>, grid, dim3(128), 0, st, (__nv_bfloat16*)u16, table, (const __nv_bfloat16*)proj, \
                    proj_stride, x_off, (const __nv_bfloat16*)bx, (const __nv_bfloat16*)conv_w, (const __nv_bfloat16*)cb, state, token_pos, \
                    token_slot, token_seq, seq_start, T, Tp, W, W / blocks, blocks);                                            \
         break;

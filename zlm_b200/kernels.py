@@ -1032,13 +1032,14 @@ class CudaKernels:
             Tp = -(-T // 128) * 128
             u16 = plan.scratch("rglru.u16", (blocks, Tp, bs), dt)
             z = plan.scratch("rglru.z", (blocks * Tp, 2 * bs), torch.float32)
-            tiles = plan.scratch("rglru.tiles", (blocks * Tp // 128,), torch.int32)
-            self._call("zlm_rglru_conv_blocks", self._p(u16), self._p(tiles), self._p(proj), c_int(proj.stride(0)), c_int(x_off),
+            tiles = blocks * (-(-T // 256))
+            table = plan.scratch("rglru.tiles", (3 * tiles,), torch.int32)
+            self._call("zlm_rglru_conv_blocks", self._p(u16), self._p(table), self._p(proj), c_int(proj.stride(0)), c_int(x_off),
                        self._p(bx), self._p(conv_w), self._p(conv_b), self._p(state), self._p(plan.token_pos),
                        self._p(plan.token_slot), self._p(plan.token_seq), self._p(plan.seq_start), c_int(T), c_int(W),
                        c_int(blocks), c_int(taps), self._stream())
-            self._call("zlm_gemm_tc_grouped", self._p(z), self._p(u16), self._p(gates), self._p(tiles), c_int(blocks * Tp // 128),
-                       c_int(blocks), c_int(2 * bs), c_int(bs), c_int(2 * bs), c_int(STORE_F32), self._stream())
+            self._call("zlm_gemm_tc_experts", self._p(z), self._p(u16), self._p(gates), self._p(table), c_int(tiles),
+                       c_int(blocks * Tp), c_int(blocks), c_int(2 * bs), c_int(bs), c_int(2 * bs), c_int(STORE_F32), self._stream())
             self._call("zlm_rglru_cluster", self._p(out), c_int(out.stride(0)), self._p(z), self._p(proj), c_int(proj.stride(0)),
                        c_int(x_off), c_int(y_off), self._p(bx), self._p(by), self._p(conv_w), self._p(conv_b), self._p(c_r),
                        self._p(c_i), self._p(lam), c_float(c_decay), self._p(state), self._p(plan.seq_slot),
@@ -1696,8 +1697,8 @@ class CudaKernels:
         """What ``moe_up`` and ``moe_down`` compute, for steps of many tokens (bf16): the (token, choice) pairs
         are sorted by expert on the device and every expert's rows go through its matrices as tiles of one
         grouped tensor-core product, so an expert's weights are read once per tile, not once per token.  Two
-        forms (``impl`` forces one): "tc", TMA + tcgen05 on tiles of 128 rows, where an expert gets about half
-        a tile or more; "mma", mma.sync on tiles of 16 to 128 rows, for fewer rows an expert.  ``activation``
+        forms (``impl`` forces one): "tc", TMA + tcgen05 on pairs of blocks, 256 rows of a matrix against up to 256
+        sorted rows; "mma", mma.sync on tiles of 16 to 128 rows, for fewer rows an expert.  ``activation``
         "swiglu_interleaved": w_up is [E, 2F, K], an expert's rows in sixteens of 8 gate and 8 up rows, and the first
         product's epilogue writes silu(gate) * up ("tc" only); "swish_limit_interleaved": the same layout with ``moe_up``'s
         clamped activation.  ``identity``: a choice of an index from E on adds
@@ -1713,32 +1714,34 @@ class CudaKernels:
         assert idx.shape == (T, top) and wgt.shape == (T, top) and idx.is_contiguous() and wgt.is_contiguous()
         P = T * top
         if impl is None:
-            # rows an expert gets on average: from about half a tile of 128 on, the tcgen05 grouped product
-            impl = "tc" if ((P >= 64 * E or gated or identity) and K % 8 == 0 and F % 8 == 0 and x.stride(0) % 8 == 0) else "mma"
+            # by the rows an expert gets on average.  Us, "mma" / "tc", 60 experts of 2,048 x 768, 6 choices: 99 / 100 at 6 rows,
+            # 116 / 100 at 13, 152 / 111 at 51; 64 of 1,024 x 512: 52 / 55 at 6, 56 / 56 at 12, 71 / 56 at 24.  Where the weight
+            # scales the expert's input, "tc" rounds the scaled input and "mma" does not: there it stays with the rows of before.
+            least = 64 if scale_input else 12
+            impl = "tc" if ((P >= least * E or gated or identity) and K % 8 == 0 and F % 8 == 0 and x.stride(0) % 8 == 0) else "mma"
         if impl != "tc" and (gated or identity):
             raise KernelError("moe_grouped: gated or identity experts run on the tcgen05 form only (sizes multiples of 8)")
         if impl == "tc":
-            # pairs sorted into tiles of 128 rows that start at an expert's first row; the inputs gathered (with the
-            # pair's weight, which scales the expert's input) into that order; both products as grouped tcgen05
-            # products that look up each token tile's expert; the choices' rows added into the stream in order
-            tiles = (P + 127) // 128 + min(E, P)
-            rows = tiles * 128
-            ints = self.scratch("moe.padded", rows + P + 3 * tiles, torch.int32, x.device)
-            xs = self.scratch("moe.padded_x", rows * K, torch.bfloat16, x.device)
-            act = self.scratch("moe.padded_act", rows * F, torch.bfloat16, x.device)
-            y = self.scratch("moe.padded_out", rows * K, torch.float32, x.device)
-            perm, inv, table = ints[:rows], ints[rows:rows + P], ints[rows + P:]
-            self._call("zlm_moe_sort_padded", self._p(idx), c_int(P), c_int(E), c_int(tiles), self._p(ints), self._stream())
-            self._call("zlm_moe_gather", self._p(xs), self._p(x), c_int(x.stride(0)), self._p(perm), self._p(wgt), c_int(rows),
+            # pairs sorted by expert, up to 256 rows a tile; the inputs gathered (with the pair's weight, which scales the
+            # expert's input) into that order; both products look up each tile's expert and rows in the sort's table;
+            # the choices' rows added into the stream in order
+            tiles = (P + 255) // 256 + min(E, P)
+            ints = self.scratch("moe.sorted", P + 3 * tiles, torch.int32, x.device)
+            xs = self.scratch("moe.sorted_x", P * K, torch.bfloat16, x.device)
+            act = self.scratch("moe.sorted_act", P * F, torch.bfloat16, x.device)
+            y = self.scratch("moe.sorted_out", P * K, torch.float32, x.device)
+            inv, table = ints[:P], ints[P:P + 3 * tiles]
+            self._call("zlm_moe_sort", self._p(idx), c_int(P), c_int(E), c_int(tiles), self._p(inv), self._p(table), self._stream())
+            self._call("zlm_moe_gather", self._p(xs), self._p(x), c_int(x.stride(0)), self._p(inv), self._p(wgt), c_int(T),
                        c_int(top), c_int(K), c_int(1 if scale_input else 0), self._stream())
             if activation == "swish_limit_interleaved":
                 assert limit > 0
                 self._call("zlm_set_gate_gemm_tcgen05", c_float(limit), c_float(alpha), self._stream())
-            self._call("zlm_gemm_tc_grouped", self._p(act), self._p(xs), self._p(w_up), self._p(table), c_int(tiles), c_int(E),
-                       c_int(2 * F if gated else F), c_int(K), c_int(F),
+            self._call("zlm_gemm_tc_experts", self._p(act), self._p(xs), self._p(w_up), self._p(table), c_int(tiles), c_int(P),
+                       c_int(E), c_int(2 * F if gated else F), c_int(K), c_int(F),
                        c_int({"relu2": 6, "swiglu_interleaved": 3, "swish_limit_interleaved": GATED_LIMIT}[activation]), self._stream())
-            self._call("zlm_gemm_tc_grouped", self._p(y), self._p(act), self._p(w_down), self._p(table), c_int(tiles), c_int(E),
-                       c_int(K), c_int(F), c_int(K), c_int(2), self._stream())
+            self._call("zlm_gemm_tc_experts", self._p(y), self._p(act), self._p(w_down), self._p(table), c_int(tiles), c_int(P),
+                       c_int(E), c_int(K), c_int(F), c_int(K), c_int(2), self._stream())
             self._call("zlm_moe_combine", self._p(stream), self._p(y), self._p(inv), self._p(None if scale_input else wgt),
                        c_int(T), c_int(top), c_int(K), self._p(x if identity else None), c_int(x.stride(0)),
                        self._p(wgt if identity else None), self._stream())
