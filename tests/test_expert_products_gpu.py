@@ -1,5 +1,5 @@
 """The routed experts' sorted products at the edges of their tiles (256 rows of W, up to 256 sorted rows, 32 columns an
-epilogue turn, 64 of K)."""
+epilogue turn, 64 of K), and products of few outputs over many tokens, which are cut along K."""
 import pytest
 import torch
 
@@ -66,3 +66,21 @@ def test_sorted_experts_against_64_bits(case, activation):
     # missing choice or a column out of place would be of the order of the row itself
     rel = ((got.cpu().double() - want).norm(dim=1) / want.norm(dim=1)).max()
     assert rel < 2e-3, f"case {case} {activation}: a token is {rel:.2e} off"
+
+
+@pytest.mark.parametrize("T, N, K", [(385, 8, 512), (2048, 64, 2048), (2047, 33, 1032), (4097, 128, 1024), (9472, 16, 1024), (9473, 16, 1024)])
+def test_few_outputs_over_many_tokens(T, N, K):
+    k = get_kernels()
+    assert (k.lib.zlm_gemm_tc_ksplit(T, N, K) > 1) == (T <= 9472 and K >= 1024)
+    g = torch.Generator().manual_seed(T + N)
+    x, w = torch.randn(T, K, generator=g).bfloat16(), (torch.randn(N, K, generator=g) / K ** 0.5).bfloat16()
+    want = x.double() @ w.double().T
+    first = torch.randn(T, N, generator=g)
+    got, acc = torch.empty(T, N, device="cuda"), first.cuda()
+    k.linear(got, x.cuda(), w.cuda())
+    k.linear(acc, x.cuda(), w.cuda(), accumulate=True)
+    k.flush_shares()
+    k.check_status(sync=True)
+    # sums of K products of the order of 1 / sqrt(K) in 32 bits
+    assert (got.cpu().double() - want).abs().max() < 2e-5
+    assert (acc.cpu().double() - first.double() - want).abs().max() < 2e-5

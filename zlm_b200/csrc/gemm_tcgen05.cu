@@ -1560,13 +1560,23 @@ extern "C" int zlm_gemm_tc_supported(int T, int N, int K, int ldx) {
     return (T >= 1 && N >= 8 && K >= 8 && K % 8 == 0 && ldx % 8 == 0) ? 1 : 0;
 }
 
+// Whether a product runs in a few-token form: up to 384 tokens; and with more where it has one tile of outputs and all its
+// tiles, cut along K, are one round of the GPU (a router's logits, a mixer's gates: 2,048 tokens x 64 outputs x 2,048 is 8 tiles
+// for 74 pairs of blocks, and 64 blocks of a quarter of K each here: 15.5 us and 13.3 with the shares' sum).
+static bool few_form(int T, int N, int K) {
+    if (T <= 384) return true;
+    if (N > TC_BM || g_tc_form) return false;
+    const FewPlan plan = few_plan(T, N, K);
+    return plan.ks > 1 && plan.whole == 0;
+}
+
 // shares of K whose fp32 partial products need scratch memory (T * N floats each)
 extern "C" int zlm_gemm_tc_ksplit(int T, int N, int K) {
-    if (T > 384) return 1;
+    if (!few_form(T, N, K)) return 1;
     return few_plan(T, N, K).ks;
 }
 
-// The width of the many-token forms' tiles (0 for the few-token forms, up to 384 tokens).  Tiles run
+// The width of the many-token forms' tiles (0 for the few-token forms).  Tiles run
 // in rounds of one per SM (or pair of SMs), and a round costs its width: N = 4096 at 2,048 tokens
 // is 128 tiles of 256 columns on 74 pairs (2 rounds, the second 73 % full) or 144 of 240 (2 rounds,
 // 97 % full).  A narrower tile re-reads the activations more often, so it has to win by more than
@@ -1575,8 +1585,7 @@ extern "C" int zlm_gemm_tc_ksplit(int T, int N, int K) {
 // the reuse of the activations per product, so only where the wider tiles would leave a third of
 // the pairs idle (N = 1024 at 2,048 tokens: 32 tiles on 74 pairs).
 extern "C" int zlm_gemm_tc_tile_width(int T, int N, int K) {
-    (void)K;
-    if (T <= 384) return 0;
+    if (few_form(T, N, K)) return 0;
     if (g_tc_width) return g_tc_width;
     const bool pairs = g_tc_form != 1;
     const long long m_tiles = pairs ? (T + TCQ_BM - 1) / TCQ_BM : (T + TC_BM - 1) / TC_BM;
@@ -1603,7 +1612,7 @@ extern "C" int zlm_gemm_tc(void* Y, const void* X, const void* W, int T, int N, 
     const int ks = zlm_gemm_tc_ksplit(T, N, K);
     ZLM_REQUIRE(ks == 1 || scratch, "gemm_tc: scratch for %d shares of K is missing", ks);
     // few tokens: W is the 128-row operand so that it streams at full height
-    if (T <= 384) {
+    if (few_form(T, N, K)) {
         const FewPlan plan = few_plan(T, N, K);
         const long long tiles = (long long)((N + TC_BM - 1) / TC_BM) * plan.t_tiles;
         if (plan.whole + (tiles - plan.whole) * plan.ks <= sm_count()) {
