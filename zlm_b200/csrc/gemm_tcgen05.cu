@@ -459,43 +459,55 @@ struct QkvEpilogue {
     int nq, nkv, hd;
 };
 
-__device__ __forceinline__ void qkv_store16(__nv_bfloat16* dst, const float* v) {
-    if (!ZLM_CHK(dst, 32)) return;
-    __nv_bfloat162 t;
-    uint4 a, b;
-#define ZLM_PK2(x, y) (t = __floats2bfloat162_rn(x, y), *(unsigned*)&t)
-    a.x = ZLM_PK2(v[0], v[1]); a.y = ZLM_PK2(v[2], v[3]); a.z = ZLM_PK2(v[4], v[5]); a.w = ZLM_PK2(v[6], v[7]);
-    b.x = ZLM_PK2(v[8], v[9]); b.y = ZLM_PK2(v[10], v[11]); b.z = ZLM_PK2(v[12], v[13]); b.w = ZLM_PK2(v[14], v[15]);
-#undef ZLM_PK2
-    *(uint4*)dst = a;
-    *(uint4*)(dst + 8) = b;
-}
-
-// one token row (this thread's lane of tensor memory at `taddr`, tile columns [n0, n0 + BN))
-template <int BN>
-__device__ __forceinline__ void qkv_epilogue_row(const QkvEpilogue& ep, unsigned taddr, __nv_bfloat16* Y, int row, int n0,
-                                                 int T, int N, int ldy) {
-    const int hd = ep.hd, half = hd >> 1;
-    int pos = 0, page = 0;
-    // a row beyond the step's tokens (or, in the bounds-check build, one whose integers lie outside
-    // the tensors passed) still walks tensor memory with its warp, and stores nothing
-    bool live = row < T && ZLM_CHK(ep.token_pos + row, 4);
-    if (live) {
-        pos = ep.token_pos[row];
-        if (ep.nkv > 0) {
-            live = ZLM_CHK(ep.token_slot + row, 4);
-            if (live) {
-                const int* entry = ep.block_table + (size_t)ep.token_slot[row] * ep.table_stride + pos / ZLM_PAGE;
-                live = ZLM_CHK(entry, 4);
-                if (live) page = *entry;
-            }
+// A token row's place: what a thread needs of its row, fetched before it waits for the row's sums (three reads that
+// depend on one another).  A row beyond the step's tokens (or, in the bounds-check build, one whose integers lie outside
+// the tensors passed) still walks tensor memory with its warp, and stores nothing.
+struct QkvRow { int pos, page; bool live; };
+__device__ __forceinline__ QkvRow qkv_row(const QkvEpilogue& ep, int row, int T) {
+    QkvRow r{0, 0, row < T && ZLM_CHK(ep.token_pos + row, 4)};
+    if (!r.live) return r;
+    r.pos = ep.token_pos[row];
+    if (ep.nkv > 0) {
+        r.live = ZLM_CHK(ep.token_slot + row, 4);
+        if (r.live) {
+            const int* entry = ep.block_table + (size_t)ep.token_slot[row] * ep.table_stride + r.pos / ZLM_PAGE;
+            r.live = ZLM_CHK(entry, 4);
+            if (r.live) r.page = *entry;
         }
     }
-    const VecW qw{ep.q_w, ep.w_dtype}, kw{ep.k_w, ep.w_dtype};
+    return r;
+}
+
+// Results go out through `stage`, 32 rows x 128 bytes of the warp's own in shared memory: the 16 to 32 columns of a head's
+// first half in a row's first 64 bytes and their partners half a head further in the others, 16-byte pieces swizzled by the
+// row, so that eight lanes write eight rows, and read one, without bank conflicts.  Then eight lanes store one row's two
+// runs of up to 64 bytes.  (A thread that stored its own row's columns touched 32 rows and half a sector of each per
+// instruction.)  dst: this lane's row's head (null: not stored); n16: sixteens staged.
+__device__ __forceinline__ void qkv_flush(const unsigned char* stage, __nv_bfloat16* dst, int c, int half, int n16, int lane) {
+    __syncwarp();
+    const int piece = lane & 7, col = c + (piece & 4 ? half : 0) + (piece & 3) * 8;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = 4 * i + (lane >> 3);
+        __nv_bfloat16* p = (__nv_bfloat16*)__shfl_sync(0xffffffffu, (unsigned long long)dst, r);
+        const uint4 v = *(const uint4*)(stage + r * 128 + ((piece ^ (r & 7)) << 4));
+        if (p && (piece & 3) < 2 * n16 && ZLM_CHK(p + col, 16)) *(uint4*)(p + col) = v;
+    }
+    __syncwarp();
+}
+
+// the heads first, first + step, .. of one warp's 32 token rows (this thread's: lane `taddr` of tensor memory, tile columns
+// [n0, n0 + BN)); ws: the norm weights of q and of k, widened, in shared memory (null: read them where they are)
+template <int BN>
+__device__ __forceinline__ void qkv_epilogue_rows(const QkvEpilogue& ep, const QkvRow& at, unsigned taddr, __nv_bfloat16* Y, int row,
+                                                  int n0, int T, int N, int ldy, int first, int step, unsigned char* stage,
+                                                  const float* ws, int lane) {
+    const int hd = ep.hd, half = hd >> 1;
     // the table is [2][hd/2][T]: the warp's 32 rows read 32 neighbouring floats of one angle
     const float* cs_row = ep.cos_sin ? ep.cos_sin + min(row, T - 1) : nullptr;
     const float* sn_row = ep.cos_sin ? ep.cos_sin + (size_t)half * T + min(row, T - 1) : nullptr;
-    for (int c0 = 0; c0 < BN; c0 += hd) {                 // the tile's heads; warp-uniform
+    unsigned char* const mine = stage + lane * 128;
+    for (int c0 = first * hd; c0 < BN; c0 += step * hd) { // the tile's heads; warp-uniform
         const int n = n0 + c0;
         if (n >= N) break;
         const int j = n / hd;                             // head among q heads, then k heads, then v heads
@@ -505,64 +517,74 @@ __device__ __forceinline__ void qkv_epilogue_row(const QkvEpilogue& ep, unsigned
             dst = Y + (size_t)row * ldy + n;
         } else {
             const int kvh = kind == 1 ? j - ep.nq : j - ep.nq - ep.nkv;
-            dst = ep.pool + ((((size_t)page * 2 + (kind - 1)) * ep.nkv + kvh) * ZLM_PAGE + (pos % ZLM_PAGE)) * hd;
+            dst = ep.pool + ((((size_t)at.page * 2 + (kind - 1)) * ep.nkv + kvh) * ZLM_PAGE + (at.pos % ZLM_PAGE)) * hd;
         }
-        if (kind == 2) {
-#pragma unroll 1
-            for (int c = 0; c < hd; c += 16) {
-                float v[16];
-                tc_ld16(taddr + (unsigned)(c0 + c), v);
-                if (live) qkv_store16(dst + c, v);
+        if (!at.live) dst = nullptr;
+        const bool norm = kind < 2 && ep.q_w, turn = kind < 2 && cs_row;
+        const VecW w{kind == 0 ? ep.q_w : ep.k_w, ep.w_dtype};
+        const float* wk = ws + (kind == 1 ? hd : 0);
+        float cc[16], sn[16];
+        if (turn) {                                       // (on their way while the squares are summed)
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+                cc[e] = __ldg(cs_row + (size_t)e * T);
+                sn[e] = __ldg(sn_row + (size_t)e * T);
             }
-            continue;
         }
-        const VecW& w = kind == 0 ? qw : kw;
         float inv = 1.f;
-        if (w.p) {
+        if (norm) {
             float ss = 0.f;
 #pragma unroll 1
-            for (int c = 0; c < hd; c += 16) {
-                float v[16];
-                tc_ld16(taddr + (unsigned)(c0 + c), v);
+            for (int c = 0; c < hd; c += 32) {
+                float v[32];
+                tc_ld16_nowait(taddr + (unsigned)(c0 + c), v);
+                tc_ld16_nowait(taddr + (unsigned)(c0 + c) + 16, v + 16);
+                tc_wait_ld();
 #pragma unroll
-                for (int i = 0; i < 16; ++i) ss = fmaf(v[i], v[i], ss);
+                for (int i = 0; i < 32; ++i) ss = fmaf(v[i], v[i], ss);
             }
             inv = 1.0f / sqrtf(ss / (float)hd + ep.eps);
         }
 #pragma unroll 1
-        for (int c = 0; c < half; c += 16) {
+        for (int c = 0, k = 0; c < half; c += 16, k ^= 1) {
             float lo[16], hi[16];
             tc_ld16_nowait(taddr + (unsigned)(c0 + c), lo);
             tc_ld16_nowait(taddr + (unsigned)(c0 + half + c), hi);
             tc_wait_ld();
-            if (w.p) {
+            if (norm) {
 #pragma unroll
                 for (int i = 0; i < 16; i += 4) {
-                    const float4 wl = w.load4(c + i), wh = w.load4(half + c + i);
+                    const float4 wl = ws ? *(const float4*)(wk + c + i) : w.load4(c + i);
+                    const float4 wh = ws ? *(const float4*)(wk + half + c + i) : w.load4(half + c + i);
                     lo[i] = (lo[i] * inv) * wl.x; lo[i + 1] = (lo[i + 1] * inv) * wl.y;
                     lo[i + 2] = (lo[i + 2] * inv) * wl.z; lo[i + 3] = (lo[i + 3] * inv) * wl.w;
                     hi[i] = (hi[i] * inv) * wh.x; hi[i + 1] = (hi[i + 1] * inv) * wh.y;
                     hi[i + 2] = (hi[i + 2] * inv) * wh.z; hi[i + 3] = (hi[i + 3] * inv) * wh.w;
                 }
             }
-            if (cs_row && live) {
-                float cc[16], sn[16];
-#pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                    cc[e] = __ldg(cs_row + (size_t)(c + e) * T);
-                    sn[e] = __ldg(sn_row + (size_t)(c + e) * T);
-                }
+            if (turn) {
 #pragma unroll
                 for (int e = 0; e < 16; ++e) {
                     const float x0 = lo[e], x1 = hi[e];
                     lo[e] = x0 * cc[e] - x1 * sn[e];
                     hi[e] = x0 * sn[e] + x1 * cc[e];
                 }
+                if (c + 16 < half)                        // the next sixteen angles, while these results go out
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) {
+                        cc[e] = __ldg(cs_row + (size_t)(c + 16 + e) * T);
+                        sn[e] = __ldg(sn_row + (size_t)(c + 16 + e) * T);
+                    }
             }
-            if (live) {
-                qkv_store16(dst + c, lo);
-                qkv_store16(dst + half + c, hi);
-            }
+#define ZLM_PK8(v) make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]))
+            auto pack2 = [](float a, float b) { __nv_bfloat162 t = __floats2bfloat162_rn(a, b); return *(unsigned*)&t; };
+            const int sw = lane & 7;
+            *(uint4*)(mine + (((2 * k) ^ sw) << 4)) = ZLM_PK8(lo);
+            *(uint4*)(mine + (((2 * k + 1) ^ sw) << 4)) = ZLM_PK8((lo + 8));
+            *(uint4*)(mine + (((2 * k + 4) ^ sw) << 4)) = ZLM_PK8(hi);
+            *(uint4*)(mine + (((2 * k + 5) ^ sw) << 4)) = ZLM_PK8((hi + 8));
+#undef ZLM_PK8
+            if (k == 1 || c + 16 >= half) qkv_flush(stage, dst, c - 16 * k, half, k + 1, lane);
         }
     }
 }
@@ -593,8 +615,13 @@ __device__ __forceinline__ void qkv_epilogue_row(const QkvEpilogue& ep, unsigned
 #define TCQ_BOX_BYTES (32 * 64)
 #define TCQ_BOX_ACC(MODE) (ZLM_GATED(MODE) ? 64 : (MODE) == 0 ? 32 : 16)
 #define TCQ_OUT_BYTES (4 * TCQ_RING * TCQ_BOX_BYTES)
+// MODE 5 has eight epilogue warps, two for every quarter of the accumulators' lanes: they share a tile's heads, or take the
+// tiles in turn where a tile is one head.  At K = 1,024 a tile's products take 8,200 cycles, and four warps' epilogue took
+// 25,000 (61,037 tokens, 16 + 2 x 8 heads of 128: 772 us); the other modes lose 3 to 5 % with eight.
+#define TCQ_THREADS(MODE) ((MODE) == 5 ? 320 : TC_THREADS)
+#define TCQ_NORM_BYTES 1024          // MODE 5: the norm weights of q and k as fp32, heads of up to 128
 template <int BN, int STAGES, int MODE>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCQ_THREADS(MODE), 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_y, void* __restrict__ Y, int T, int N, int K, int ldy, int gm,
                     int y_tma, const QkvEpilogue ep) {
@@ -610,6 +637,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     uint64_t* acc_empty = acc_full + 2;        // [2]
     unsigned* tmem_slot = (unsigned*)(acc_empty + 2);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    float* norm_w = (float*)(((uintptr_t)(tmem_slot + 2) + 15) & ~(uintptr_t)15);       // MODE 5
+    const bool share_tile = MODE == 5 && BN / ep.hd >= 2;       // both sets of epilogue warps work on every tile
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned rank = cluster_rank();
@@ -620,7 +649,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], share_tile ? 16 : 8); }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -628,6 +657,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n"
                      ::"r"(smem_u32(tmem_slot)), "r"((unsigned)(2 * TCP_ACC)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
+    }
+    if (MODE == 5 && ep.q_w && 8 * ep.hd <= TCQ_NORM_BYTES) {
+        const VecW qw{ep.q_w, ep.w_dtype}, kw{ep.k_w, ep.w_dtype};
+        for (int i = threadIdx.x; i < 2 * ep.hd; i += blockDim.x) {
+            if (i < ep.hd) norm_w[i] = qw.ok(i, 1) ? qw[i] : 0.f;
+            else if (ep.k_w) norm_w[i] = kw.ok(i - ep.hd, 1) ? kw[i - ep.hd] : 0.f;
+        }
     }
     tc_fence_before();
     __syncthreads();
@@ -714,13 +750,19 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             int tm, tn;
             tile_of(tile, m_tiles, n_tiles, gm, tm, tn);
             const int a0row = tm * TCQ_BM + rank * TC_BM, b0row = tn * BN;
+            const int arow = a0row + lg * 32 + lane;
+            const int set = (warp - 2) >> 2;
+            if (MODE == 5 && !share_tile && (int)buf != set) continue;
+            QkvRow at{};
+            if constexpr (MODE == 5) at = qkv_row(ep, arow, T);
             const bool ok = mbar_wait_warp(&acc_full[buf], (local >> 1) & 1, abort_flag, 3);
             tc_fence_after();
             if (!ok || *abort_flag) break;
-            const int arow = a0row + lg * 32 + lane;
             if constexpr (MODE == 5) {
-                qkv_epilogue_row<BN>(ep, tmem_base + ((unsigned)(lg * 32) << 16) + buf * TCP_ACC, (__nv_bfloat16*)Y, arow,
-                                     b0row, T, N, ldy);
+                qkv_epilogue_rows<BN>(ep, at, tmem_base + ((unsigned)(lg * 32) << 16) + buf * TCP_ACC, (__nv_bfloat16*)Y, arow,
+                                      b0row, T, N, ldy, share_tile ? set : 0, share_tile ? 2 : 1,
+                                      sOut + (warp - 2) * (TCQ_OUT_BYTES / 8),
+                                      8 * ep.hd <= TCQ_NORM_BYTES ? norm_w : nullptr, lane);
             } else if (y_tma && BN % TCQ_BOX_ACC(MODE) == 0) {
                 // a box is 32 rows x 64 bytes of output: 16 fp32 sums, 32 bf16 values, or the 32 bf16
                 // results of 64 gate/up sums; a thread writes its row's four 16-byte pieces
@@ -1401,7 +1443,7 @@ static int launch_tc_pair(void* Y, const void* X, const void* W, int T, int N, i
         rc = zlm_make_map_out(&my, Y, T, ZLM_GATED(mode) ? N / 2 : N, ldy, ybytes, 32, 64 / ybytes);
         if (rc) return rc;
     }
-    const size_t smem = (size_t)STAGES * (TC_BM + BN / 2) * TC_BK * 2 + TCQ_OUT_BYTES + 1024 + 256;
+    const size_t smem = (size_t)STAGES * (TC_BM + BN / 2) * TC_BK * 2 + TCQ_OUT_BYTES + 1024 + 256 + (mode == 5 ? TCQ_NORM_BYTES : 0);
     const long long tiles = (long long)((T + TCQ_BM - 1) / TCQ_BM) * ((N + BN - 1) / BN);
     const int pairs = (int)(tiles < sm_count() / 2 ? tiles : sm_count() / 2);
 #define ZLM_TCQ_LAUNCH(M)                                                                                  \
@@ -1416,7 +1458,7 @@ static int launch_tc_pair(void* Y, const void* X, const void* W, int T, int N, i
             }                                                                                              \
             attr_set = true;                                                                               \
         }                                                                                                  \
-        zlm_launch(kern, dim3(2 * pairs), dim3(TC_THREADS), smem, st, mx, mw, my, Y, T, N, K, ldy, tile_group(TCQ_BM, K), y_tma, ep); \
+        zlm_launch(kern, dim3(2 * pairs), dim3(TCQ_THREADS(M)), smem, st, mx, mw, my, Y, T, N, K, ldy, tile_group(TCQ_BM, K), y_tma, ep); \
     }
     if (mode == 0) ZLM_TCQ_LAUNCH(0)
     else if (mode == 1) ZLM_TCQ_LAUNCH(1)
