@@ -14,11 +14,15 @@ builds it, ``CudaKernels(variant="check")`` loads it.
 """
 from __future__ import annotations
 
+import ctypes
 import hashlib
+import importlib.util
+import operator
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import time
 from concurrent.futures import ThreadPoolExecutor, as_completed
@@ -141,6 +145,45 @@ def build(out_dir: str, lib: str, verbose: bool = True, obj_name: str = "_build"
     os.replace(tmp, lib)
     if verbose:
         _say(f"built {lib} in {time.time() - t0:.0f}s")
+
+
+def _through_ctypes(address: int, *args) -> int:
+    """What ``host_call.c`` does, where it cannot be built: one argument after the other as an object of ctypes."""
+    fn = ctypes.CFUNCTYPE(ctypes.c_int)(address)
+    return fn(*(a if isinstance(a, ctypes._SimpleCData) else ctypes.c_void_p(a if a is None else operator.index(a) or None) for a in args))
+
+
+def host_call(verbose: bool = True):
+    """``call(address, *arguments) -> int`` of ``host_call.c`` (built in-tree at first use, seconds), else through ctypes."""
+    src = os.path.join(HERE, "host_call.c")
+    include, cc = sysconfig.get_paths()["include"], shutil.which("gcc") or shutil.which("cc")
+    with open(src, "rb") as f:
+        want = hashlib.sha256(f.read() + (sysconfig.get_config_var("SOABI") or "").encode()).hexdigest()
+    out_dir = HERE if _writable(HERE) else os.path.join(tempfile.gettempdir(), f"zlm_b200_{os.getuid()}_{want[:16]}")
+    path = os.path.join(out_dir, "zlm_host_call.so")
+    stamp = path + ".hash"
+    fresh = False
+    if os.path.isfile(path) and os.path.isfile(stamp):
+        with open(stamp) as f:
+            fresh = f.read().strip() == want
+    try:
+        if not fresh:
+            os.makedirs(out_dir, exist_ok=True)
+            tmp = path + f".tmp{os.getpid()}"
+            r = subprocess.run([cc or "gcc", "-O2", "-shared", "-fPIC", "-I", include, src, "-o", tmp], capture_output=True, text=True)
+            if r.returncode != 0:
+                raise OSError(r.stderr[-500:])
+            os.replace(tmp, path)
+            with open(stamp, "w") as f:
+                f.write(want)
+        spec = importlib.util.spec_from_file_location("zlm_host_call", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        return module.call
+    except (OSError, ImportError) as e:
+        if verbose:
+            _say(f"launches go through ctypes: {e}")
+        return _through_ctypes
 
 
 if __name__ == "__main__":

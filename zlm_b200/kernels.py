@@ -161,12 +161,13 @@ class CudaKernels:
     name = "cuda"
 
     def __init__(self, verbose_build: bool = True, variant: str = ""):
-        from .csrc.build import library_path
+        from .csrc.build import host_call, library_path
         self.variant = variant
         self.lib_path = library_path(verbose=verbose_build, variant=variant)
         self.lib = ctypes.CDLL(self.lib_path)
+        self._invoke = host_call(verbose=verbose_build)
         self.lib.zlm_last_error.restype = ctypes.c_char_p
-        self.lib.zlm_launch_count.restype = ctypes.c_longlong
+        self.lib.zlm_launch_count.restype = self.lib.zlm_mlstm_scratch.restype = ctypes.c_longlong
         if self.lib.zlm_page_tokens() != PAGE_TOKENS:
             raise KernelError("kernel library and Python disagree on the cache page size")
         if not torch.cuda.is_available():
@@ -218,15 +219,22 @@ class CudaKernels:
         return int(self.lib.zlm_launch_count())
 
     # -- plumbing ---------------------------------------------------------
+    def _entry(self, name: str) -> int:
+        at = self._fn.get(name)
+        if at is None:
+            at = self._fn[name] = ctypes.cast(getattr(self.lib, name), c_void_p).value
+        return at
+
+    def _ask(self, name: str, *args) -> int:
+        """What an entry point that launches nothing says of its (integer) arguments."""
+        return self._invoke(self._entry(name), *args)
+
     def _call(self, name: str, *args):
-        fn = self._fn.get(name)
-        if fn is None:
-            fn = getattr(self.lib, name)
-            fn.restype = c_int
-            self._fn[name] = fn
+        """An entry point that launches kernels.  Integers and addresses go as plain numbers, floats as ``c_float``."""
+        at = self._fn.get(name) or self._entry(name)
         if self.bounds_check:
             self._register_ranges()
-        rc = fn(*args)
+        rc = self._invoke(at, *args)
         self._launches += 1
         if rc != 0:
             raise KernelError(self.lib.zlm_last_error().decode())
@@ -234,10 +242,14 @@ class CudaKernels:
             self.check_bounds(name)
 
     def _p(self, t: Optional[torch.Tensor]) -> c_void_p:
+        """``_at`` as an object of ctypes, for calls of other libraries."""
+        return c_void_p(self._at(t))
+
+    def _at(self, t: Optional[torch.Tensor]) -> int:
         """The tensor's address as a kernel argument.  In the bounds-check build the bytes it
         spans are also noted as memory the next call may touch."""
         if t is None:
-            return c_void_p(0)
+            return 0
         if self._join is not None and self._overlap(t, self._join[0]):
             self.join()
         if self._shares is not None:
@@ -254,7 +266,7 @@ class CudaKernels:
             blank.zero_()           # somebody other than the expected product comes first: the zeros are made real
         if self.bounds_check:
             self._ranges.append((t.data_ptr(), _span_bytes(t)))
-        return c_void_p(t.data_ptr())
+        return t.data_ptr()
 
     @staticmethod
     def _overlap(a: torch.Tensor, b: torch.Tensor) -> bool:
@@ -336,8 +348,8 @@ class CudaKernels:
         out, x, w, eps = self._lazy[:4]
         self._lazy = None
         R, H = out.shape
-        self._call("zlm_rmsnorm", self._p(out), c_int(_dt(out)), self._p(x), self._p(w), c_int(_dt(w)),
-                   self._p(None), c_int(R), c_int(H), c_float(eps), self._stream())
+        self._call("zlm_rmsnorm", self._at(out), _dt(out), self._at(x), self._at(w), _dt(w),
+                   self._at(None), R, H, c_float(eps), self._queue())
 
     def _register_ranges(self) -> None:
         lib = self.lib
@@ -385,9 +397,13 @@ class CudaKernels:
                               f"status {code:#x}): results since the last check are not valid")
 
     @staticmethod
-    def _stream() -> c_void_p:
+    def _queue() -> int:
         # (the handle alone: a Stream object for every launch would cost as much host time as the rest of a call)
-        return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+    @staticmethod
+    def _stream() -> c_void_p:
+        return c_void_p(CudaKernels._queue())
 
     def check_linear(self, what: str, w: torch.Tensor) -> None:
         """Raises at once, with the weight's name, if no kernel takes a product with this
@@ -402,8 +418,8 @@ class CudaKernels:
         T, H = out.shape
         assert out.dtype == torch.float32 and ids.dtype == torch.int32 and table.shape[1] == H
         assert out.is_contiguous() and table.is_contiguous()
-        self._call("zlm_embed", self._p(out), self._p(table), c_int(_dt(table)),
-                   self._p(ids), c_int(T), c_int(H), c_int(table.shape[0]), self._stream())
+        self._call("zlm_embed", self._at(out), self._at(table), _dt(table),
+                   self._at(ids), T, H, table.shape[0], self._queue())
 
     def rmsnorm(self, out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, eps: float,
                 rows: Optional[torch.Tensor] = None) -> None:
@@ -423,12 +439,12 @@ class CudaKernels:
         self._lazy = None
         taken = self._takes_shares(x, ACCUM) if (rows is None and x.shape[0] == R) else None
         if taken is not None:
-            self._call("zlm_rmsnorm_shares", self._p(out), c_int(_dt(out)), self._p(x), self._p(w), c_int(_dt(w)),
-                       c_int(R), c_int(H), c_float(eps), self._p(taken[0]), c_int(taken[1]), self._stream())
+            self._call("zlm_rmsnorm_shares", self._at(out), _dt(out), self._at(x), self._at(w), _dt(w),
+                       R, H, c_float(eps), self._at(taken[0]), taken[1], self._queue())
             return
-        self._call("zlm_rmsnorm", self._p(out), c_int(_dt(out)), self._p(x),
-                   self._p(w), c_int(_dt(w)), self._p(rows), c_int(R), c_int(H),
-                   c_float(eps), self._stream())
+        self._call("zlm_rmsnorm", self._at(out), _dt(out), self._at(x),
+                   self._at(w), _dt(w), self._at(rows), R, H,
+                   c_float(eps), self._queue())
 
     def layernorm(self, out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, eps: float,
                   rows: Optional[torch.Tensor] = None) -> None:
@@ -437,16 +453,16 @@ class CudaKernels:
         assert x.dtype == torch.float32 and x.shape[1] == H and w.shape == (H,)
         assert out.is_contiguous() and x.is_contiguous() and w.is_contiguous()
         assert rows is None or (rows.dtype == torch.int32 and rows.numel() >= R)
-        self._call("zlm_layernorm", self._p(out), c_int(_dt(out)), self._p(x), self._p(w), c_int(_dt(w)), self._p(rows),
-                   c_int(R), c_int(H), c_float(eps), self._stream())
+        self._call("zlm_layernorm", self._at(out), _dt(out), self._at(x), self._at(w), _dt(w), self._at(rows),
+                   R, H, c_float(eps), self._queue())
 
     def swiglu(self, out: torch.Tensor, gu: torch.Tensor) -> None:
         """out[t, i] = silu(gu[t, i]) * gu[t, I + i]."""
         T, I = out.shape
         assert gu.shape == (T, 2 * I) and gu.dtype == out.dtype
         assert out.is_contiguous() and gu.is_contiguous()
-        self._call("zlm_swiglu", self._p(out), self._p(gu), c_int(_dt(out)),
-                   c_int(T), c_int(I), self._stream())
+        self._call("zlm_swiglu", self._at(out), self._at(gu), _dt(out),
+                   T, I, self._queue())
 
     def linear(self, out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, accumulate: bool = False,
                impl: Optional[str] = None, defer: bool = False) -> None:
@@ -479,9 +495,9 @@ class CudaKernels:
                 accumulate = defer = False       # adding to zeros: a plain store of the fp32 sums
         if x.dtype == torch.float32:
             assert out.dtype == torch.float32 and ldx == K
-            self._call("zlm_gemm_f32", self._p(out), self._p(x),
-                       self._p(w), c_int(T), c_int(N), c_int(K), c_int(ldy),
-                       c_int(1 if accumulate else 0), self._stream())
+            self._call("zlm_gemm_f32", self._at(out), self._at(x),
+                       self._at(w), T, N, K, ldy,
+                       1 if accumulate else 0, self._queue())
             return
         if x.dtype != torch.bfloat16:
             raise KernelError(f"linear: unsupported dtype {x.dtype}")
@@ -496,12 +512,12 @@ class CudaKernels:
                 return
         if (defer and self.defer_shares and impl is None and mode in (ACCUM, STORE) and T > 16 and out.is_contiguous()
                 and not self.streams_weights(T, N)):
-            ks = int(self.lib.zlm_gemm_tc_shares_plan(c_int(T), c_int(N), c_int(K), c_int(ldx)))
+            ks = self._ask("zlm_gemm_tc_shares_plan", T, N, K, ldx)
             if ks > 1:
                 self.flush_shares()
                 scratch = self.scratch("gemm_tc.partials", ks * T * N, torch.float32, out.device)
-                self._call("zlm_gemm_tc_shares", self._p(x), self._p(w), c_int(T), c_int(N), c_int(K), c_int(ldx),
-                           self._p(scratch), self._stream())
+                self._call("zlm_gemm_tc_shares", self._at(x), self._at(w), T, N, K, ldx,
+                           self._at(scratch), self._queue())
                 self._shares = (out, scratch, ks, mode)
                 return
         self._bf16_product(out, x, w, T, N, K, ldx, ldy, mode, impl)
@@ -516,8 +532,8 @@ class CudaKernels:
         out, scratch, ks, mode = self._shares
         self._shares = None
         T, N = out.shape
-        self._call("zlm_gemm_tc_add_shares", self._p(out), self._p(scratch), c_int(T), c_int(N), c_int(out.stride(0)),
-                   c_int(mode), c_int(ks), self._stream())
+        self._call("zlm_gemm_tc_add_shares", self._at(out), self._at(scratch), T, N, out.stride(0),
+                   mode, ks, self._queue())
 
     def _takes_shares(self, t: torch.Tensor, mode: int):
         """The pending shares if they are those of ``t`` (whole, in this mode), else None after finishing them."""
@@ -543,22 +559,22 @@ class CudaKernels:
     def _bf16_product(self, out, x, w, T, N, K, ldx, ldy, mode, impl) -> None:
         if impl is None:
             # few tokens: the streaming product; from 17 tokens on the tcgen05 forms
-            tc_ok = self.lib.zlm_gemm_tc_supported(T, N, K, ldx)
+            tc_ok = self._ask("zlm_gemm_tc_supported", T, N, K, ldx)
             small = self.streams_weights(T, N)
             impl = "gemv" if (small or (T <= 16 and not tc_ok)) else ("tc" if tc_ok else "mma")
         if impl == "tc":
             self.flush_shares()             # the shares' scratch is about to be written again
-            ks = self.lib.zlm_gemm_tc_ksplit(T, N, K)
+            ks = self._ask("zlm_gemm_tc_ksplit", T, N, K)
             scratch = self.scratch("gemm_tc.partials", ks * T * N, torch.float32, out.device) if ks > 1 else None
-            self._call("zlm_gemm_tc", self._p(out), self._p(x), self._p(w),
-                       c_int(T), c_int(N), c_int(K), c_int(ldx), c_int(ldy), c_int(mode), self._p(scratch),
-                       self._stream())
+            self._call("zlm_gemm_tc", self._at(out), self._at(x), self._at(w),
+                       T, N, K, ldx, ldy, mode, self._at(scratch),
+                       self._queue())
             return
         if impl == "gemv":
             self._gemv(out, x, w, T, N, K, ldx, ldy, mode)
             return
-        self._call("zlm_gemm_bf16_mma", self._p(out), self._p(x), self._p(w),
-                   c_int(T), c_int(N), c_int(K), c_int(ldx), c_int(ldy), c_int(mode), self._stream())
+        self._call("zlm_gemm_bf16_mma", self._at(out), self._at(x), self._at(w),
+                   T, N, K, ldx, ldy, mode, self._queue())
 
     def _gemv(self, out, x, w, T, N, K, ldx, ldy, mode, norm_weight: Optional[torch.Tensor] = None) -> None:
         """The streaming product, with what it may carry beside its sums: candidates for the argmax of
@@ -567,7 +583,7 @@ class CudaKernels:
         lazy = self._lazy
         if not (lazy is not None and lazy[0].data_ptr() == x.data_ptr() and tuple(lazy[0].shape) == (T, K) and ldx == K):
             lazy = None
-        nb = int(self.lib.zlm_gemv_blocks(c_int(N)))
+        nb = self._ask("zlm_gemv_blocks", N)
         cv = ci = nxt = sq = None
         if mode == STORE_F32 and out.is_contiguous():
             # fp32 outputs of a few-token product are logits: the product also leaves, for every
@@ -579,12 +595,12 @@ class CudaKernels:
             nxt = self.scratch("gemv.norm_rows", T * N, torch.bfloat16, out.device)
             sq = self.scratch("gemv.norm_squares", T * nb, torch.float32, out.device)
         # a norm not run: its rows times weight stand in for x, the scale comes from the sums of squares
-        px = self._p(lazy[4]) if lazy is not None else self._p(x)
-        self._call("zlm_gemv_bf16_norms", self._p(out), px, self._p(w), c_int(T), c_int(N), c_int(K),
-                   c_int(ldx), c_int(ldy), c_int(mode), self._p(cv), self._p(ci),
-                   self._p(lazy[5]) if lazy is not None else c_void_p(0), c_int(lazy[6] if lazy is not None else 0),
-                   c_float(lazy[3] if lazy is not None else 0.0), self._p(norm_weight),
-                   c_int(_dt(norm_weight) if norm_weight is not None else 0), self._p(nxt), self._p(sq), self._stream())
+        px = self._at(lazy[4]) if lazy is not None else self._at(x)
+        self._call("zlm_gemv_bf16_norms", self._at(out), px, self._at(w), T, N, K,
+                   ldx, ldy, mode, self._at(cv), self._at(ci),
+                   self._at(lazy[5]) if lazy is not None else (0), lazy[6] if lazy is not None else 0,
+                   c_float(lazy[3] if lazy is not None else 0.0), self._at(norm_weight),
+                   _dt(norm_weight) if norm_weight is not None else 0, self._at(nxt), self._at(sq), self._queue())
         if cv is not None:
             self._candidates = (out.data_ptr(), T, N, nb, cv, ci)
         if norm_weight is not None:
@@ -618,11 +634,11 @@ class CudaKernels:
         if act == "swish_limit":
             assert limit > 0
             if impl is None:
-                tc_ok = self.lib.zlm_gemm_tc_supported(T, N, K, x.stride(0))
+                tc_ok = self._ask("zlm_gemm_tc_supported", T, N, K, x.stride(0))
                 impl = "gemv" if (self.streams_weights(T, N) or (T <= 16 and not tc_ok)) else ("tc" if tc_ok else "mma")
             unit = {"gemv": "gemv_bf16", "tc": "gemm_tcgen05", "mma": "gemm_bf16_mma"}[impl]
             self.flush_shares()
-            self._call("zlm_set_gate_" + unit, c_float(limit), c_float(alpha), self._stream())
+            self._call("zlm_set_gate_" + unit, c_float(limit), c_float(alpha), self._queue())
             self._bf16_product(out, x, w, T, N, K, x.stride(0), out.stride(0), GATED_LIMIT, impl)
             return
         self._bf16_product(out, x, w, T, N, K, x.stride(0), out.stride(0),
@@ -635,15 +651,15 @@ class CudaKernels:
         T = token_pos.shape[0]
         assert out.dtype == torch.float32 and out.is_contiguous() and out.numel() == T * n_rot
         assert inv_freq.dtype == torch.float32 and inv_freq.numel() * 2 == n_rot and token_pos.dtype == torch.int32
-        self._call("zlm_rope_table", self._p(out), self._p(inv_freq), c_int(n_rot), self._p(token_pos), c_int(T),
-                   self._stream())
+        self._call("zlm_rope_table", self._at(out), self._at(inv_freq), n_rot, self._at(token_pos), T,
+                   self._queue())
 
     def qkv_rope_supported(self, x: torch.Tensor, w: torch.Tensor, nq: int, nkv: int, hd: int, n_rot: int) -> bool:
         """Whether ``linear_qkv_rope`` takes this step: bf16, many tokens, heads that divide a tile."""
         if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
             return False
-        return bool(self.lib.zlm_gemm_tc_qkv_supported(c_int(x.shape[0]), c_int(w.shape[0]), c_int(w.shape[1]),
-                                                       c_int(x.stride(0)), c_int(nq), c_int(nkv), c_int(hd), c_int(n_rot)))
+        return bool(self._ask("zlm_gemm_tc_qkv_supported", x.shape[0], w.shape[0], w.shape[1],
+                                                       x.stride(0), nq, nkv, hd, n_rot))
 
     def linear_qkv_rope(self, q_out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, q_w: Optional[torch.Tensor],
                         k_w: Optional[torch.Tensor], eps: float, cos_sin: Optional[torch.Tensor],
@@ -664,12 +680,12 @@ class CudaKernels:
             assert q_w.shape == (hd,) and (nkv == 0 or (k_w is not None and k_w.dtype == q_w.dtype))
         if cos_sin is not None:
             assert cos_sin.dtype == torch.float32 and cos_sin.numel() == T * hd and cos_sin.is_contiguous()
-        self._call("zlm_gemm_tc_qkv", self._p(q_out), self._p(x), self._p(w), c_int(T), c_int(N), c_int(K),
-                   c_int(x.stride(0)), c_int(q_out.stride(0)), self._p(q_w), self._p(k_w),
-                   c_int(_dt(q_w) if q_w is not None else F32), c_float(eps), self._p(cos_sin),
-                   self._p(token_pos), self._p(token_slot), self._p(block_table),
-                   c_int(block_table.stride(0) if block_table is not None else 0), self._p(pool), c_int(nq), c_int(nkv),
-                   c_int(hd), self._stream())
+        self._call("zlm_gemm_tc_qkv", self._at(q_out), self._at(x), self._at(w), T, N, K,
+                   x.stride(0), q_out.stride(0), self._at(q_w), self._at(k_w),
+                   _dt(q_w) if q_w is not None else F32, c_float(eps), self._at(cos_sin),
+                   self._at(token_pos), self._at(token_slot), self._at(block_table),
+                   block_table.stride(0) if block_table is not None else 0, self._at(pool), nq, nkv,
+                   hd, self._queue())
 
     def qk_norm_rope_write(self, qkv: torch.Tensor, q_w: Optional[torch.Tensor],
                            k_w: Optional[torch.Tensor], eps: float,
@@ -697,16 +713,16 @@ class CudaKernels:
             assert tuple(pool.shape[1:]) == (2, nkv, PAGE_TOKENS, hd)
             assert block_table is not None and block_table.dtype == torch.int32
         taken = self._takes_shares(qkv, STORE) if T < 512 else None
-        args = (self._p(qkv), c_int(_dt(qkv)), c_int(qkv.stride(0)),
-                self._p(q_w), self._p(k_w), c_int(_dt(q_w) if has_norm else F32),
-                c_int(1 if has_norm else 0), c_float(eps), self._p(inv_freq), c_int(n_rot),
-                self._p(token_pos), self._p(token_slot),
-                self._p(block_table), c_int(block_table.stride(0) if block_table is not None else 0),
-                self._p(pool), c_int(nq), c_int(nkv), c_int(hd), c_int(1 if write else 0), c_int(T))
+        args = (self._at(qkv), _dt(qkv), qkv.stride(0),
+                self._at(q_w), self._at(k_w), _dt(q_w) if has_norm else F32,
+                1 if has_norm else 0, c_float(eps), self._at(inv_freq), n_rot,
+                self._at(token_pos), self._at(token_slot),
+                self._at(block_table), block_table.stride(0) if block_table is not None else 0,
+                self._at(pool), nq, nkv, hd, 1 if write else 0, T)
         if taken is not None:
-            self._call("zlm_qk_norm_rope_write_shares", *args, self._p(taken[0]), c_int(taken[1]), self._stream())
+            self._call("zlm_qk_norm_rope_write_shares", *args, self._at(taken[0]), taken[1], self._queue())
         else:
-            self._call("zlm_qk_norm_rope_write", *args, self._stream())
+            self._call("zlm_qk_norm_rope_write", *args, self._queue())
 
     def attention(self, out: torch.Tensor, q: torch.Tensor, pool: torch.Tensor, block_table: torch.Tensor,
                   token_pos: torch.Tensor, token_slot: torch.Tensor, nq: int, nkv: int, hd: int,
@@ -737,14 +753,14 @@ class CudaKernels:
         if sinks is not None:
             assert sinks.dtype == torch.float32 and sinks.shape == (nq,) and sinks.is_contiguous()
             sink = True
-        sk = c_int(1 if sink else 0)
+        sk = 1 if sink else 0
         assert out.shape == (T, nq * hd) and q.shape[1] == nq * hd and q.dtype == out.dtype == pool.dtype
         assert q.stride(1) == 1 and out.stride(1) == 1 and pool.is_contiguous()
         assert v_share >= 1 and nkv % v_share == 0 and chunk >= 0 and softcap >= 0
         assert pool[0].numel() == (nkv + nkv // v_share) * PAGE_TOKENS * hd and pool.shape[-1] == hd
-        extra = (c_int(chunk), c_float(softcap), self._p(sinks), c_int(v_share), c_int(keep), self._p(bias), c_int(bias_n))
+        extra = (chunk, c_float(softcap), self._at(sinks), v_share, keep, self._at(bias), bias_n)
         if (plan is not None and plan.is_decode and q.dtype == torch.bfloat16
-                and self.lib.zlm_attention_decode_supported(nq, nkv, hd)):
+                and self._ask("zlm_attention_decode_supported", nq, nkv, hd)):
             if len_bucket is None:
                 len_bucket = attention_len_bucket(plan.max_len)
             splits, per = decode_splits(T, nkv, len_bucket, self.decode_blocks or self.sm_count * DECODE_BLOCKS_PER_SM)
@@ -754,53 +770,53 @@ class CudaKernels:
                 part_ml = plan.scratch("attn.part_ml", (T * nq * splits * 2,), torch.float32)
             # (a decode step writes one position per sequence: every page below that one is from earlier
             # steps, and its load need not wait for the kernel that wrote this step's keys and values)
-            self._call("zlm_attention_decode_fresh", self._p(out), c_int(out.stride(0)),
-                       self._p(q), c_int(q.stride(0)), self._p(pool),
-                       self._p(block_table), c_int(block_table.stride(0)),
-                       self._p(token_pos), self._p(token_slot), c_int(T), c_int(nq),
-                       c_int(nkv), c_int(hd), c_float(scale), c_int(window), c_int(splits), c_int(per),
-                       self._p(part_o), self._p(part_ml), c_int(max(1, int(getattr(plan, "max_new", 1) or 1))),
-                       sk, *extra, self._stream())
+            self._call("zlm_attention_decode_fresh", self._at(out), out.stride(0),
+                       self._at(q), q.stride(0), self._at(pool),
+                       self._at(block_table), block_table.stride(0),
+                       self._at(token_pos), self._at(token_slot), T, nq,
+                       nkv, hd, c_float(scale), window, splits, per,
+                       self._at(part_o), self._at(part_ml), max(1, int(getattr(plan, "max_new", 1) or 1)),
+                       sk, *extra, self._queue())
             return
         if (plan is not None and not plan.is_decode and q.dtype == torch.bfloat16
                 and getattr(plan, "cu_seqlens", None) is not None
-                and self.lib.zlm_attention_prefill_supported(nq, nkv, hd)):
+                and self._ask("zlm_attention_prefill_supported", nq, nkv, hd)):
             impl = getattr(plan, "attention_impl", None)
             if (impl != "mma" and not (keep and bias is not None)
-                    and self.lib.zlm_attention_prefill_tc_supported(nq, nkv, hd, q.stride(0), out.stride(0))):
-                self._call("zlm_attention_prefill_tc", self._p(out), c_int(out.stride(0)),
-                           self._p(q), c_int(q.stride(0)), c_int(T), self._p(pool),
-                           ctypes.c_longlong(pool.shape[0]), self._p(block_table),
-                           c_int(block_table.stride(0)), self._p(plan.cu_seqlens),
-                           self._p(plan.seq_slot), self._p(plan.seq_start), c_int(plan.R),
-                           c_int(plan.max_new), c_int(nq), c_int(nkv), c_int(hd), c_float(scale), c_int(window),
-                           sk, *extra, self._stream())
+                    and self._ask("zlm_attention_prefill_tc_supported", nq, nkv, hd, q.stride(0), out.stride(0))):
+                self._call("zlm_attention_prefill_tc", self._at(out), out.stride(0),
+                           self._at(q), q.stride(0), T, self._at(pool),
+                           pool.shape[0], self._at(block_table),
+                           block_table.stride(0), self._at(plan.cu_seqlens),
+                           self._at(plan.seq_slot), self._at(plan.seq_start), plan.R,
+                           plan.max_new, nq, nkv, hd, c_float(scale), window,
+                           sk, *extra, self._queue())
                 return
             if (impl != "mma" and v_dim is not None and v_dim < hd and not keep and bias is None
-                    and self.lib.zlm_attention_prefill_tc_vd_supported(nq, nkv, hd, v_dim, q.stride(0), out.stride(0))):
+                    and self._ask("zlm_attention_prefill_tc_vd_supported", nq, nkv, hd, v_dim, q.stride(0), out.stride(0))):
                 # keys of 192 over values of 128 on the tcgen05 kernel (out's columns from v_dim on become zeros)
-                self._call("zlm_attention_prefill_tc_vd", self._p(out), c_int(out.stride(0)),
-                           self._p(q), c_int(q.stride(0)), c_int(T), self._p(pool),
-                           ctypes.c_longlong(pool.shape[0]), self._p(block_table),
-                           c_int(block_table.stride(0)), self._p(plan.cu_seqlens),
-                           self._p(plan.seq_slot), self._p(plan.seq_start), c_int(plan.R),
-                           c_int(plan.max_new), c_int(nq), c_int(nkv), c_int(hd), c_int(v_dim), c_float(scale),
-                           c_int(window), sk, *extra, self._stream())
+                self._call("zlm_attention_prefill_tc_vd", self._at(out), out.stride(0),
+                           self._at(q), q.stride(0), T, self._at(pool),
+                           pool.shape[0], self._at(block_table),
+                           block_table.stride(0), self._at(plan.cu_seqlens),
+                           self._at(plan.seq_slot), self._at(plan.seq_start), plan.R,
+                           plan.max_new, nq, nkv, hd, v_dim, c_float(scale),
+                           window, sk, *extra, self._queue())
                 return
-            if v_dim is not None and v_dim < hd and self.lib.zlm_attention_prefill_vd_supported(nq, nkv, hd, v_dim):
+            if v_dim is not None and v_dim < hd and self._ask("zlm_attention_prefill_vd_supported", nq, nkv, hd, v_dim):
                 # values narrower than keys (their rows in the pool are padded to the keys' width): the padding is
                 # neither loaded nor multiplied, and out's columns from v_dim on become zeros
-                self._call("zlm_attention_prefill_vd", self._p(out), c_int(out.stride(0)), self._p(q), c_int(q.stride(0)),
-                           self._p(pool), self._p(block_table), c_int(block_table.stride(0)), self._p(plan.cu_seqlens),
-                           self._p(plan.seq_slot), self._p(plan.seq_start), c_int(plan.R), c_int(plan.max_new), c_int(nq),
-                           c_int(nkv), c_int(hd), c_int(v_dim), c_float(scale), c_int(window), sk, *extra, self._stream())
+                self._call("zlm_attention_prefill_vd", self._at(out), out.stride(0), self._at(q), q.stride(0),
+                           self._at(pool), self._at(block_table), block_table.stride(0), self._at(plan.cu_seqlens),
+                           self._at(plan.seq_slot), self._at(plan.seq_start), plan.R, plan.max_new, nq,
+                           nkv, hd, v_dim, c_float(scale), window, sk, *extra, self._queue())
                 return
-            self._call("zlm_attention_prefill", self._p(out), c_int(out.stride(0)),
-                       self._p(q), c_int(q.stride(0)), self._p(pool),
-                       self._p(block_table), c_int(block_table.stride(0)),
-                       self._p(plan.cu_seqlens), self._p(plan.seq_slot),
-                       self._p(plan.seq_start), c_int(plan.R), c_int(plan.max_new), c_int(nq),
-                       c_int(nkv), c_int(hd), c_float(scale), c_int(window), sk, *extra, self._stream())
+            self._call("zlm_attention_prefill", self._at(out), out.stride(0),
+                       self._at(q), q.stride(0), self._at(pool),
+                       self._at(block_table), block_table.stride(0),
+                       self._at(plan.cu_seqlens), self._at(plan.seq_slot),
+                       self._at(plan.seq_start), plan.R, plan.max_new, nq,
+                       nkv, hd, c_float(scale), window, sk, *extra, self._queue())
             return
         # 32-bit attention in tiles of 32 queries, the same bits as a query a block, from 32 tokens of the longest sequence on
         # (512 where a step brings one token a sequence).  Measured at 16 heads of 128, a query a block / tiles: 509 new tokens
@@ -809,19 +825,19 @@ class CudaKernels:
         if (q.dtype == torch.float32 and plan is not None and getattr(plan, "cu_seqlens", None) is not None
                 and int(getattr(plan, "max_len", 0) or plan.max_new) >= (32 if int(plan.max_new) > 1 else 512)
                 and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
-                and self.lib.zlm_attention_f32_tile_supported(c_int(nq), c_int(nkv), c_int(hd), c_int(q.stride(0)),
-                                                              c_int(out.stride(0)), c_float(softcap), c_int(v_share), c_int(keep),
-                                                              c_int(bias is not None), c_int(plan.R), c_int(int(plan.max_new)))):
-            self._call("zlm_attention_f32_tile", self._p(out), c_int(out.stride(0)), self._p(q), c_int(q.stride(0)), self._p(pool),
-                       self._p(block_table), c_int(block_table.stride(0)), self._p(plan.cu_seqlens), self._p(plan.seq_slot),
-                       self._p(plan.seq_start), c_int(plan.R), c_int(plan.max_new), c_int(nq), c_int(nkv), c_int(hd), c_float(scale),
-                       c_int(window), sk, c_int(chunk), self._p(sinks), self._stream())
+                and self._ask("zlm_attention_f32_tile_supported", nq, nkv, hd, q.stride(0),
+                                                              out.stride(0), c_float(softcap), v_share, keep,
+                                                              bias is not None, plan.R, int(plan.max_new))):
+            self._call("zlm_attention_f32_tile", self._at(out), out.stride(0), self._at(q), q.stride(0), self._at(pool),
+                       self._at(block_table), block_table.stride(0), self._at(plan.cu_seqlens), self._at(plan.seq_slot),
+                       self._at(plan.seq_start), plan.R, plan.max_new, nq, nkv, hd, c_float(scale),
+                       window, sk, chunk, self._at(sinks), self._queue())
             return
-        self._call("zlm_attention_generic", self._p(out), c_int(out.stride(0)),
-                   self._p(q), c_int(q.stride(0)), c_int(_dt(q)), self._p(pool),
-                   self._p(block_table), c_int(block_table.stride(0)),
-                   self._p(token_pos), self._p(token_slot), c_int(T), c_int(nq),
-                   c_int(nkv), c_int(hd), c_float(scale), c_int(window), sk, *extra, self._stream())
+        self._call("zlm_attention_generic", self._at(out), out.stride(0),
+                   self._at(q), q.stride(0), _dt(q), self._at(pool),
+                   self._at(block_table), block_table.stride(0),
+                   self._at(token_pos), self._at(token_slot), T, nq,
+                   nkv, hd, c_float(scale), window, sk, *extra, self._queue())
 
     # -- short convolution, retention, gated heads (see csrc/short_conv.cu, csrc/retention.cu) --------------
     def conv_norm_write(self, q_out: torch.Tensor, proj: torch.Tensor, conv_w: torch.Tensor, state: Optional[torch.Tensor],
@@ -841,12 +857,12 @@ class CudaKernels:
         assert proj.dtype == conv_w.dtype == q_out.dtype == pool.dtype
         if taps > 1:
             assert state is not None and tuple(state.shape[1:]) == (taps - 1, C) and state.is_contiguous() and state.dtype == proj.dtype
-        self._call("zlm_conv_norm_write", self._p(q_out), c_int(q_out.stride(0)), self._p(proj), c_int(proj.stride(0)),
-                   self._p(conv_w), self._p(state if taps > 1 else None), c_int(_dt(proj)), self._p(plan.token_pos),
-                   self._p(plan.token_slot), self._p(plan.token_seq), self._p(plan.seq_start), self._p(plan.cu_seqlens),
-                   self._p(plan.seq_slot), self._p(block_table), c_int(block_table.stride(0)), self._p(pool), c_int(T),
-                   c_int(plan.R), c_int(nq), c_int(nkv), c_int(dim), c_int(vdim), c_int(hdp), c_int(taps),
-                   c_int(1 if norm else 0), c_float(eps), self._stream())
+        self._call("zlm_conv_norm_write", self._at(q_out), q_out.stride(0), self._at(proj), proj.stride(0),
+                   self._at(conv_w), self._at(state if taps > 1 else None), _dt(proj), self._at(plan.token_pos),
+                   self._at(plan.token_slot), self._at(plan.token_seq), self._at(plan.seq_start), self._at(plan.cu_seqlens),
+                   self._at(plan.seq_slot), self._at(block_table), block_table.stride(0), self._at(pool), T,
+                   plan.R, nq, nkv, dim, vdim, hdp, taps,
+                   1 if norm else 0, c_float(eps), self._queue())
 
     def head_gate(self, out: torch.Tensor, o: torch.Tensor, g: torch.Tensor, heads: int, v_dim: int, norm: bool,
                   eps: float, act: str) -> None:
@@ -857,10 +873,10 @@ class CudaKernels:
         assert o.dim() == 3 and o.shape[1] == heads and o.shape[2] >= v_dim and o.stride(2) == 1
         assert out.shape == (T, heads * v_dim) and out.stride(1) == 1 and g.shape == (T, heads * v_dim) and g.stride(1) == 1
         assert out.dtype == g.dtype and o.dtype in (out.dtype, torch.float32)
-        self._call("zlm_head_gate", self._p(out), c_int(out.stride(0)), self._p(o), c_int(1 if o.dtype == torch.float32 else 0),
-                   c_int(o.stride(0)), c_int(o.stride(1)), self._p(g), c_int(g.stride(0)), c_int(_dt(out)), c_int(T),
-                   c_int(heads), c_int(v_dim), c_int(1 if norm else 0), c_float(eps), c_int({"sigmoid": 0, "silu": 1}[act]),
-                   self._stream())
+        self._call("zlm_head_gate", self._at(out), out.stride(0), self._at(o), 1 if o.dtype == torch.float32 else 0,
+                   o.stride(0), o.stride(1), self._at(g), g.stride(0), _dt(out), T,
+                   heads, v_dim, 1 if norm else 0, c_float(eps), {"sigmoid": 0, "silu": 1}[act],
+                   self._queue())
 
     # tokens of a sequence from which a step's retention runs in pieces side by side, and the pieces' length
     RETENTION_PIECES_FROM = 256
@@ -886,10 +902,10 @@ class CudaKernels:
             n_rot = 0
         if cos_sin is not None:
             assert n_rot and cos_sin.dtype == torch.float32 and cos_sin.is_contiguous() and cos_sin.numel() == T * n_rot
-        tail = (c_int(heads), c_int(dim), c_int(v_dim), c_float(k_scale), self._p(cos_sin), c_int(T), self._stream())
-        head = (self._p(o), self._p(proj), c_int(proj.stride(0)), c_int(q_off), c_int(k_off), c_int(v_off), c_int(_dt(proj)),
-                self._p(inv_freq if n_rot else None), c_int(n_rot), self._p(decay), self._p(state), self._p(plan.cu_seqlens),
-                self._p(plan.seq_slot), self._p(plan.seq_start), c_int(plan.R))
+        tail = (heads, dim, v_dim, c_float(k_scale), self._at(cos_sin), T, self._queue())
+        head = (self._at(o), self._at(proj), proj.stride(0), q_off, k_off, v_off, _dt(proj),
+                self._at(inv_freq if n_rot else None), n_rot, self._at(decay), self._at(state), self._at(plan.cu_seqlens),
+                self._at(plan.seq_slot), self._at(plan.seq_start), plan.R)
         if pieces is None:
             pieces = plan.max_new >= self.RETENTION_PIECES_FROM
         if pieces:
@@ -900,11 +916,11 @@ class CudaKernels:
             part = plan.scratch("retention.part_state", (plan.R * maxp * heads * dim * v_dim,), torch.float32)
             # (the gate rides in the last kernel where the pieces run as products)
             y, g, eps, act = (_gate[0], _gate[1], _gate[2], _gate[3]) if _gate is not None else (None, None, 0.0, "silu")
-            self._call("zlm_retention_parts", *head, c_int(maxp), c_int(L), self._p(part), *tail[:-1], self._p(y),
-                       c_int(y.stride(0) if y is not None else 0), self._p(g), c_int(g.stride(0) if g is not None else 0),
-                       c_float(eps), c_int({"sigmoid": 0, "silu": 1}[act]), tail[-1])
+            self._call("zlm_retention_parts", *head, maxp, L, self._at(part), *tail[:-1], self._at(y),
+                       y.stride(0) if y is not None else 0, self._at(g), g.stride(0) if g is not None else 0,
+                       c_float(eps), {"sigmoid": 0, "silu": 1}[act], tail[-1])
             return
-        self._call("zlm_retention", *head, *tail[:-1], c_int(int(getattr(plan, "max_new", 0) or 0)), tail[-1])
+        self._call("zlm_retention", *head, *tail[:-1], int(getattr(plan, "max_new", 0) or 0), tail[-1])
 
     def retention_gated(self, y: torch.Tensor, g: torch.Tensor, eps: float, act: str, o: torch.Tensor, proj: torch.Tensor,
                         q_off: int, k_off: int, v_off: int, inv_freq: Optional[torch.Tensor], n_rot: int, decay: torch.Tensor,
@@ -916,8 +932,8 @@ class CudaKernels:
         if (y.dtype == g.dtype == torch.bfloat16 and plan.max_new >= self.RETENTION_PIECES_FROM and v_dim <= 128
                 and y.stride(1) == g.stride(1) == 1 and (y.stride(0) | g.stride(0)) % 8 == 0
                 and (proj.data_ptr() | y.data_ptr() | g.data_ptr()) % 16 == 0
-                and self.lib.zlm_retention_products(c_int(_dt(proj)), c_int(proj.stride(0)), c_int(q_off), c_int(k_off), c_int(v_off),
-                                                    c_int(n_rot if inv_freq is not None else 0), c_int(dim), c_int(v_dim))):
+                and self._ask("zlm_retention_products", _dt(proj), proj.stride(0), q_off, k_off, v_off,
+                                                    n_rot if inv_freq is not None else 0, dim, v_dim)):
             assert y.shape == g.shape == (proj.shape[0], heads * v_dim)
             self.retention(o, *args, cos_sin=cos_sin, _gate=(y, g, eps, act))
             return
@@ -961,15 +977,15 @@ class CudaKernels:
             assert inv_freq.dtype == torch.float32 and inv_freq.numel() * 2 == n_rot and n_rot <= dim
         else:
             n_rot = 0
-        self._call("zlm_attn_prep", self._p(q_out), c_int(q_out.stride(0)), self._p(proj), c_int(proj.stride(0)),
-                   self._p(conv_w), self._p(state if (conv_w is not None and taps > 1) else None), c_int(_dt(proj)),
-                   self._p(plan.token_pos), self._p(plan.token_slot), self._p(plan.token_seq), self._p(plan.seq_start),
-                   self._p(plan.cu_seqlens), self._p(plan.seq_slot), self._p(block_table), c_int(block_table.stride(0)),
-                   self._p(pool), c_int(T), c_int(plan.R), c_int(nq), c_int(nkv), c_int(dim), c_int(vdim), c_int(hdp),
-                   c_int(taps), c_int(mode), self._p(q_w if mode >= 2 else None), self._p(k_w if mode >= 2 else None),
-                   c_int(_dt(q_w) if mode >= 2 else F32), c_float(eps), self._p(inv_freq if n_rot else None), c_int(n_rot),
-                   c_float(rot_scale), c_int(1 if interleaved else 0), c_float(coef), c_int(every), self._p(v_first),
-                   c_float(v_lambda), self._p(v_keep), self._stream())
+        self._call("zlm_attn_prep", self._at(q_out), q_out.stride(0), self._at(proj), proj.stride(0),
+                   self._at(conv_w), self._at(state if (conv_w is not None and taps > 1) else None), _dt(proj),
+                   self._at(plan.token_pos), self._at(plan.token_slot), self._at(plan.token_seq), self._at(plan.seq_start),
+                   self._at(plan.cu_seqlens), self._at(plan.seq_slot), self._at(block_table), block_table.stride(0),
+                   self._at(pool), T, plan.R, nq, nkv, dim, vdim, hdp,
+                   taps, mode, self._at(q_w if mode >= 2 else None), self._at(k_w if mode >= 2 else None),
+                   _dt(q_w) if mode >= 2 else F32, c_float(eps), self._at(inv_freq if n_rot else None), n_rot,
+                   c_float(rot_scale), 1 if interleaved else 0, c_float(coef), every, self._at(v_first),
+                   c_float(v_lambda), self._at(v_keep), self._queue())
 
     def norm_gate(self, out: torch.Tensor, o: torch.Tensor, g: Optional[torch.Tensor], heads: int, v_dim: int, group: str,
                   weight: Optional[torch.Tensor], eps: float, act: str, out_scale: float = 1.0) -> None:
@@ -986,11 +1002,11 @@ class CudaKernels:
         if weight is not None:
             assert weight.is_contiguous() and weight.numel() in (v_dim, N)
             w_rows = 1 if (weight.numel() == N and heads > 1) else 0
-        self._call("zlm_norm_gate", self._p(out), c_int(out.stride(0)), self._p(o), self._p(g if a != 2 else None),
-                   c_int(g.stride(0) if a != 2 else 0), c_int(_dt(out)), c_int(T), c_int(heads), c_int(v_dim),
-                   c_int({"none": 0, "head": 1, "row": 2}[group]), self._p(weight),
-                   c_int(_dt(weight) if weight is not None else F32), c_int(w_rows), c_float(eps), c_int(a),
-                   c_float(out_scale), self._stream())
+        self._call("zlm_norm_gate", self._at(out), out.stride(0), self._at(o), self._at(g if a != 2 else None),
+                   g.stride(0) if a != 2 else 0, _dt(out), T, heads, v_dim,
+                   {"none": 0, "head": 1, "row": 2}[group], self._at(weight),
+                   _dt(weight) if weight is not None else F32, w_rows, c_float(eps), a,
+                   c_float(out_scale), self._queue())
 
     # -- recurrent mixers (see csrc/recurrent.cu) ---------------------------------------------------------------
     # tokens of a sequence from which a step's recurrences run in pieces side by side, and the pieces' length
@@ -1034,18 +1050,18 @@ class CudaKernels:
             z = plan.scratch("rglru.z", (blocks * Tp, 2 * bs), torch.float32)
             tiles = blocks * (-(-T // 256))
             table = plan.scratch("rglru.tiles", (3 * tiles,), torch.int32)
-            self._call("zlm_rglru_conv_blocks", self._p(u16), self._p(table), self._p(proj), c_int(proj.stride(0)), c_int(x_off),
-                       self._p(bx), self._p(conv_w), self._p(conv_b), self._p(state), self._p(plan.token_pos),
-                       self._p(plan.token_slot), self._p(plan.token_seq), self._p(plan.seq_start), c_int(T), c_int(W),
-                       c_int(blocks), c_int(taps), self._stream())
-            self._call("zlm_gemm_tc_experts", self._p(z), self._p(u16), self._p(gates), self._p(table), c_int(tiles),
-                       c_int(blocks * Tp), c_int(blocks), c_int(2 * bs), c_int(bs), c_int(2 * bs), c_int(STORE_F32), self._stream())
-            self._call("zlm_rglru_cluster", self._p(out), c_int(out.stride(0)), self._p(z), self._p(proj), c_int(proj.stride(0)),
-                       c_int(x_off), c_int(y_off), self._p(bx), self._p(by), self._p(conv_w), self._p(conv_b), self._p(c_r),
-                       self._p(c_i), self._p(lam), c_float(c_decay), self._p(state), self._p(plan.seq_slot),
-                       self._p(plan.seq_start), self._p(plan.cu_seqlens), c_int(T), c_int(plan.R), c_int(W), c_int(blocks),
-                       c_int(taps), c_float(out_scale), c_int(self.lib.zlm_rglru_cluster_size(c_int(plan.R), c_int(T), c_int(max_new), c_int(W))),
-                       self._stream())
+            self._call("zlm_rglru_conv_blocks", self._at(u16), self._at(table), self._at(proj), proj.stride(0), x_off,
+                       self._at(bx), self._at(conv_w), self._at(conv_b), self._at(state), self._at(plan.token_pos),
+                       self._at(plan.token_slot), self._at(plan.token_seq), self._at(plan.seq_start), T, W,
+                       blocks, taps, self._queue())
+            self._call("zlm_gemm_tc_experts", self._at(z), self._at(u16), self._at(gates), self._at(table), tiles,
+                       blocks * Tp, blocks, 2 * bs, bs, 2 * bs, STORE_F32, self._queue())
+            self._call("zlm_rglru_cluster", self._at(out), out.stride(0), self._at(z), self._at(proj), proj.stride(0),
+                       x_off, y_off, self._at(bx), self._at(by), self._at(conv_w), self._at(conv_b), self._at(c_r),
+                       self._at(c_i), self._at(lam), c_float(c_decay), self._at(state), self._at(plan.seq_slot),
+                       self._at(plan.seq_start), self._at(plan.cu_seqlens), T, plan.R, W, blocks,
+                       taps, c_float(out_scale), self.lib.zlm_rglru_cluster_size(plan.R, T, max_new, W),
+                       self._queue())
             return
         u = plan.scratch("rglru.u", (T, W), torch.float32)
         z = plan.scratch("rglru.z", (T, blocks, 2 * bs), torch.float32)
@@ -1057,32 +1073,32 @@ class CudaKernels:
         u16 = plan.scratch("rglru.u16", (T, W), dt) if by_products else None
 
         def call(phase: int) -> None:
-            self._call("zlm_rglru", self._p(out), c_int(out.stride(0)), self._p(u), self._p(u16), self._p(z), self._p(proj),
-                       c_int(proj.stride(0)), c_int(x_off), c_int(y_off), self._p(bx), self._p(by), self._p(conv_w),
-                       self._p(conv_b), self._p(a_r), self._p(a_i), self._p(c_r), self._p(c_i), self._p(lam), c_float(c_decay),
-                       self._p(state), c_int(_dt(proj)), self._p(plan.token_pos), self._p(plan.token_slot),
-                       self._p(plan.token_seq), self._p(plan.seq_start), self._p(plan.cu_seqlens), self._p(plan.seq_slot),
-                       c_int(T), c_int(plan.R), c_int(W), c_int(blocks), c_int(taps), c_float(out_scale), c_int(max_new),
-                       self._p(part), c_int(phase), self._stream())
+            self._call("zlm_rglru", self._at(out), out.stride(0), self._at(u), self._at(u16), self._at(z), self._at(proj),
+                       proj.stride(0), x_off, y_off, self._at(bx), self._at(by), self._at(conv_w),
+                       self._at(conv_b), self._at(a_r), self._at(a_i), self._at(c_r), self._at(c_i), self._at(lam), c_float(c_decay),
+                       self._at(state), _dt(proj), self._at(plan.token_pos), self._at(plan.token_slot),
+                       self._at(plan.token_seq), self._at(plan.seq_start), self._at(plan.cu_seqlens), self._at(plan.seq_slot),
+                       T, plan.R, W, blocks, taps, c_float(out_scale), max_new,
+                       self._at(part), phase, self._queue())
         if not by_products:
             call(0)
             return
         assert gates.shape == (blocks, 2 * bs, bs) and gates.is_contiguous() and gates.dtype == dt
         call(1)
         N, K, ldx, ldy = 2 * bs, bs, W, 2 * W
-        if self.bounds_check or not self.lib.zlm_gemm_tc_supported(T, N, K, ldx):
+        if self.bounds_check or not self._ask("zlm_gemm_tc_supported", T, N, K, ldx):
             for b in range(blocks):
                 self.linear(z[:, b], u16[:, b * bs:(b + 1) * bs], gates[b])
         else:
             # the same product a block, without the host's work of ``linear`` for each (operands of one tensor each,
             # a block's share found by address)
             self.flush_shares()
-            ks = int(self.lib.zlm_gemm_tc_ksplit(T, N, K))
+            ks = self._ask("zlm_gemm_tc_ksplit", T, N, K)
             scratch = self.scratch("gemm_tc.partials", ks * T * N, torch.float32, z.device) if ks > 1 else None
-            pz, pu, pg, ps, st = self._p(z).value, self._p(u16).value, self._p(gates).value, self._p(scratch), self._stream()
+            pz, pu, pg, ps, st = self._at(z), self._at(u16), self._at(gates), self._at(scratch), self._queue()
             for b in range(blocks):
-                self._call("zlm_gemm_tc", c_void_p(pz + b * N * 4), c_void_p(pu + b * K * 2), c_void_p(pg + b * N * K * 2),
-                           c_int(T), c_int(N), c_int(K), c_int(ldx), c_int(ldy), c_int(STORE_F32), ps, st)
+                self._call("zlm_gemm_tc", pz + b * N * 4, pu + b * K * 2, pg + b * N * K * 2,
+                           T, N, K, ldx, ldy, STORE_F32, ps, st)
         call(2)
 
     def mingru(self, out: torch.Tensor, proj: torch.Tensor, z_off: int, x_off: int, g_off: int, bz: Optional[torch.Tensor],
@@ -1100,10 +1116,10 @@ class CudaKernels:
         if cluster is None:
             cluster = int(getattr(plan, "max_new", 0) or 0) >= self.RECURRENT_PIECES_FROM
         b = bz if bz is not None else bx
-        self._call("zlm_mingru", self._p(out), c_int(out.stride(0)), self._p(proj), c_int(proj.stride(0)), c_int(z_off),
-                   c_int(x_off), c_int(g_off), self._p(bz), self._p(bx), c_int(_dt(b) if b is not None else F32), self._p(state),
-                   c_int(_dt(proj)), self._p(plan.seq_slot), self._p(plan.cu_seqlens), c_int(T), c_int(plan.R), c_int(W),
-                   c_int(1 if cluster else 0), self._stream())
+        self._call("zlm_mingru", self._at(out), out.stride(0), self._at(proj), proj.stride(0), z_off,
+                   x_off, g_off, self._at(bz), self._at(bx), _dt(b) if b is not None else F32, self._at(state),
+                   _dt(proj), self._at(plan.seq_slot), self._at(plan.cu_seqlens), T, plan.R, W,
+                   1 if cluster else 0, self._queue())
 
     def mlstm_step(self, out: torch.Tensor, proj: torch.Tensor, q_off: int, k_off: int, v_off: int, g_off: int, z: torch.Tensor,
                    i_off: int, f_off: int, b_i: Optional[torch.Tensor], b_f: Optional[torch.Tensor], cap: float,
@@ -1115,12 +1131,12 @@ class CudaKernels:
         assert plan.is_decode and plan.R == T and N == heads * v_dim and out.stride(1) == 1
         assert w_norm.shape == (N,) and w_norm.is_contiguous()
         b = b_i if b_i is not None else b_f
-        self._call("zlm_mlstm_step", self._p(out), c_int(out.stride(0)), c_int(_dt(out)), self._p(proj), c_int(proj.stride(0)),
-                   c_int(_dt(proj)), c_int(q_off), c_int(k_off), c_int(v_off), c_int(g_off), self._p(z), c_int(z.stride(0)),
-                   c_int(i_off), c_int(f_off), self._p(b_i), self._p(b_f), c_int(_dt(b) if b is not None else F32), c_float(cap),
-                   self._p(S), self._p(n), self._p(m), self._p(plan.seq_slot), self._p(plan.cu_seqlens), c_int(plan.R),
-                   c_int(heads), c_int(dim), c_int(v_dim), c_float(q_scale), self._p(w_norm), c_int(_dt(w_norm)), c_float(eps),
-                   self._stream())
+        self._call("zlm_mlstm_step", self._at(out), out.stride(0), _dt(out), self._at(proj), proj.stride(0),
+                   _dt(proj), q_off, k_off, v_off, g_off, self._at(z), z.stride(0),
+                   i_off, f_off, self._at(b_i), self._at(b_f), _dt(b) if b is not None else F32, c_float(cap),
+                   self._at(S), self._at(n), self._at(m), self._at(plan.seq_slot), self._at(plan.cu_seqlens), plan.R,
+                   heads, dim, v_dim, c_float(q_scale), self._at(w_norm), _dt(w_norm), c_float(eps),
+                   self._queue())
 
     def mlstm(self, o: torch.Tensor, proj: torch.Tensor, q_off: int, k_off: int, v_off: int, z: torch.Tensor, i_off: int,
               f_off: int, b_i: Optional[torch.Tensor], b_f: Optional[torch.Tensor], cap: float, state, plan, heads: int,
@@ -1134,17 +1150,16 @@ class CudaKernels:
         S, n, m = self._check_mlstm(proj, z, b_i, b_f, state, heads, dim, v_dim)
         assert o.shape == (T, heads * v_dim) and o.dtype == torch.float32 and o.is_contiguous()
         max_new = int(plan.max_new)
-        self.lib.zlm_mlstm_scratch.restype = ctypes.c_longlong
         part = plan.scratch("mlstm.pieces", (int(self.lib.zlm_mlstm_scratch(plan.R, heads, dim, v_dim, max_new)),), torch.float32)
         b = b_i if b_i is not None else b_f
         y, g, w, eps = _gate if _gate is not None else (None, None, None, 0.0)
-        self._call("zlm_mlstm", self._p(o), self._p(proj), c_int(proj.stride(0)), c_int(_dt(proj)), c_int(q_off), c_int(k_off),
-                   c_int(v_off), self._p(z), c_int(z.stride(0)), c_int(i_off), c_int(f_off), self._p(b_i), self._p(b_f),
-                   c_int(_dt(b) if b is not None else F32), c_float(cap), self._p(S), self._p(n), self._p(m),
-                   self._p(plan.seq_slot), self._p(plan.cu_seqlens), c_int(T), c_int(plan.R), c_int(heads), c_int(dim),
-                   c_int(v_dim), c_float(q_scale), c_int(max_new), self._p(part), self._p(y), c_int(y.stride(0) if y is not None else 0),
-                   self._p(g), c_int(g.stride(0) if g is not None else 0), self._p(w), c_int(_dt(w) if w is not None else F32),
-                   c_float(eps), self._stream())
+        self._call("zlm_mlstm", self._at(o), self._at(proj), proj.stride(0), _dt(proj), q_off, k_off,
+                   v_off, self._at(z), z.stride(0), i_off, f_off, self._at(b_i), self._at(b_f),
+                   _dt(b) if b is not None else F32, c_float(cap), self._at(S), self._at(n), self._at(m),
+                   self._at(plan.seq_slot), self._at(plan.cu_seqlens), T, plan.R, heads, dim,
+                   v_dim, c_float(q_scale), max_new, self._at(part), self._at(y), y.stride(0) if y is not None else 0,
+                   self._at(g), g.stride(0) if g is not None else 0, self._at(w), _dt(w) if w is not None else F32,
+                   c_float(eps), self._queue())
 
     def mlstm_gated(self, y: torch.Tensor, g: torch.Tensor, w_norm: torch.Tensor, eps: float, o: torch.Tensor, proj: torch.Tensor,
                     q_off: int, k_off: int, v_off: int, z: torch.Tensor, i_off: int, f_off: int, b_i: Optional[torch.Tensor],
@@ -1154,8 +1169,8 @@ class CudaKernels:
         args = (proj, q_off, k_off, v_off, z, i_off, f_off, b_i, b_f, cap, state, plan, heads, dim, v_dim, q_scale)
         if (y.dtype == g.dtype == torch.bfloat16 and v_dim <= 128 and y.stride(1) == g.stride(1) == 1
                 and (y.stride(0) | g.stride(0)) % 8 == 0 and (proj.data_ptr() | y.data_ptr() | g.data_ptr()) % 16 == 0
-                and self.lib.zlm_mlstm_products(c_int(_dt(proj)), c_int(proj.stride(0)), c_int(q_off), c_int(k_off), c_int(v_off),
-                                                c_int(dim), c_int(v_dim))):
+                and self._ask("zlm_mlstm_products", _dt(proj), proj.stride(0), q_off, k_off, v_off,
+                                                dim, v_dim)):
             assert y.shape == g.shape == (proj.shape[0], heads * v_dim)
             assert w_norm.is_contiguous() and w_norm.numel() == heads * v_dim
             self.mlstm(o, *args, _gate=(y, g, w_norm, eps))
@@ -1181,8 +1196,8 @@ class CudaKernels:
         C, rank = w2.shape
         assert alpha.shape == (T, C) and alpha.dtype == torch.float32 and alpha.is_contiguous() and proj.stride(1) == 1
         assert w2.is_contiguous() and w2.dtype == proj.dtype and (b is None or (b.numel() == C and b.dtype == proj.dtype and b.is_contiguous()))
-        self._call("zlm_lowrank_decay", self._p(alpha), self._p(proj), c_int(proj.stride(0)), c_int(lo_off), self._p(w2),
-                   self._p(b), c_int(_dt(proj)), c_int(T), c_int(C), c_int(rank), c_float(tau), self._stream())
+        self._call("zlm_lowrank_decay", self._at(alpha), self._at(proj), proj.stride(0), lo_off, self._at(w2),
+                   self._at(b), _dt(proj), T, C, rank, c_float(tau), self._queue())
 
     def linear_attention(self, o: torch.Tensor, proj: torch.Tensor, q_off: int, k_off: int, v_off: int,
                          alpha: Optional[torch.Tensor], head_decay: Optional[torch.Tensor], state: torch.Tensor, plan,
@@ -1208,12 +1223,12 @@ class CudaKernels:
             maxp = (max_new + self.RECURRENT_PIECE - 1) // self.RECURRENT_PIECE
             part = plan.scratch("linear_attention.pieces", (plan.R * maxp * heads * dim * (v_dim + 1),), torch.float32)
         y, g, w, eps, act = _gate if _gate is not None else (None, None, None, 0.0, "silu")
-        self._call("zlm_linear_attention", self._p(o), self._p(proj), c_int(proj.stride(0)), c_int(q_off), c_int(k_off),
-                   c_int(v_off), self._p(alpha), self._p(head_decay if alpha is None else None), self._p(state), c_int(_dt(proj)),
-                   self._p(plan.seq_slot), self._p(plan.cu_seqlens), c_int(T), c_int(plan.R), c_int(heads), c_int(dim),
-                   c_int(v_dim), c_float(q_scale), c_int(max_new), self._p(part), self._p(y),
-                   c_int(y.stride(0) if y is not None else 0), self._p(g), c_int(g.stride(0) if g is not None else 0), self._p(w),
-                   c_int(_dt(w) if w is not None else F32), c_float(eps), c_int({"sigmoid": 0, "silu": 1}[act]), self._stream())
+        self._call("zlm_linear_attention", self._at(o), self._at(proj), proj.stride(0), q_off, k_off,
+                   v_off, self._at(alpha), self._at(head_decay if alpha is None else None), self._at(state), _dt(proj),
+                   self._at(plan.seq_slot), self._at(plan.cu_seqlens), T, plan.R, heads, dim,
+                   v_dim, c_float(q_scale), max_new, self._at(part), self._at(y),
+                   y.stride(0) if y is not None else 0, self._at(g), g.stride(0) if g is not None else 0, self._at(w),
+                   _dt(w) if w is not None else F32, c_float(eps), {"sigmoid": 0, "silu": 1}[act], self._queue())
 
     def linear_attention_gated(self, y: torch.Tensor, g: torch.Tensor, w_norm: torch.Tensor, eps: float, act: str, o: torch.Tensor,
                                proj: torch.Tensor, q_off: int, k_off: int, v_off: int, alpha: Optional[torch.Tensor],
@@ -1240,28 +1255,28 @@ class CudaKernels:
         if blank is not None and blank.data_ptr() == out.data_ptr() and tuple(blank.shape) == tuple(out.shape):
             self._blank = None
             accumulate = False
-        self._call("zlm_scaled_sum", self._p(out), self._p(a), c_float(alpha), self._p(b), c_float(beta),
-                   ctypes.c_longlong(out.numel()), c_int(1 if accumulate else 0), self._stream())
+        self._call("zlm_scaled_sum", self._at(out), self._at(a), c_float(alpha), self._at(b), c_float(beta),
+                   out.numel(), 1 if accumulate else 0, self._queue())
 
     def softcap_(self, x: torch.Tensor, cap: float) -> None:
         """x = cap * tanh(x / cap) for a contiguous fp32 tensor (logits)."""
         assert x.dtype == torch.float32 and x.is_contiguous()
         if self._candidates is not None and self._candidates[0] == x.data_ptr():
             self._candidates = None
-        self._call("zlm_softcap_f32", self._p(x), ctypes.c_longlong(x.numel()), c_float(cap), self._stream())
+        self._call("zlm_softcap_f32", self._at(x), x.numel(), c_float(cap), self._queue())
 
     def silu_rows(self, x: torch.Tensor, cols: int) -> None:
         """x[:, :cols] = silu(x[:, :cols]) in place."""
         T = x.shape[0]
         assert x.stride(1) == 1 and 0 <= cols <= x.shape[1]
-        self._call("zlm_silu_rows", self._p(x), c_int(x.stride(0)), c_int(_dt(x)), c_int(T), c_int(cols), self._stream())
+        self._call("zlm_silu_rows", self._at(x), x.stride(0), _dt(x), T, cols, self._queue())
 
     def gated_limit(self, out: torch.Tensor, gu: torch.Tensor, limit: float, alpha: float) -> None:
         """out[t, i] = g sigmoid(alpha g) (u + 1) with g = min(gu[t, i], limit), u = clamp(gu[t, I + i], -limit, limit)."""
         T, I = out.shape
         assert gu.shape == (T, 2 * I) and gu.dtype == out.dtype and out.is_contiguous() and gu.is_contiguous()
-        self._call("zlm_gated_limit", self._p(out), self._p(gu), c_int(_dt(out)), c_int(T), c_int(I), c_float(limit),
-                   c_float(alpha), self._stream())
+        self._call("zlm_gated_limit", self._at(out), self._at(gu), _dt(out), T, I, c_float(limit),
+                   c_float(alpha), self._queue())
 
     # -- latent attention (see csrc/latent_attention.cu) --------------------
     def latent_prep(self, q: torch.Tensor, q_rot: torch.Tensor, dkv: Optional[torch.Tensor],
@@ -1289,14 +1304,14 @@ class CudaKernels:
             assert pool is not None and pool.dtype == q.dtype and pool.is_contiguous()
             assert tuple(pool.shape[1:]) == (PAGE_TOKENS, kv_rank + rot_dim) and block_table.dtype == torch.int32
             assert c_weight is not None and c_weight.shape == (kv_rank,) and c_weight.is_contiguous()
-        self._call("zlm_latent_prep", self._p(q), c_int(q.stride(0)), self._p(q_rot), c_int(q_rot.stride(0)),
-                   c_int(q_rot.stride(1)), self._p(dkv),
-                   c_int(dkv.stride(0) if dkv is not None else 0), c_int(_dt(q)), self._p(c_weight if dkv is not None else None),
-                   c_int(_dt(c_weight) if dkv is not None else F32), c_float(eps), self._p(inv_freq), c_int(n_rot),
-                   self._p(token_pos), self._p(token_slot), self._p(block_table if dkv is not None else None),
-                   c_int(block_table.stride(0) if dkv is not None else 0), self._p(pool if dkv is not None else None),
-                   c_int(T), c_int(heads), c_int(dim), c_int(rot_dim), c_int(kv_rank), self._p(rec_out),
-                   c_int(rec_out.stride(0) if rec_out is not None else 0), self._stream())
+        self._call("zlm_latent_prep", self._at(q), q.stride(0), self._at(q_rot), q_rot.stride(0),
+                   q_rot.stride(1), self._at(dkv),
+                   dkv.stride(0) if dkv is not None else 0, _dt(q), self._at(c_weight if dkv is not None else None),
+                   _dt(c_weight) if dkv is not None else F32, c_float(eps), self._at(inv_freq), n_rot,
+                   self._at(token_pos), self._at(token_slot), self._at(block_table if dkv is not None else None),
+                   block_table.stride(0) if dkv is not None else 0, self._at(pool if dkv is not None else None),
+                   T, heads, dim, rot_dim, kv_rank, self._at(rec_out),
+                   rec_out.stride(0) if rec_out is not None else 0, self._queue())
 
     def latent_down(self, cq: torch.Tensor, down: torch.Tensor, q_weight: torch.Tensor, eps: float,
                     dkv: Optional[torch.Tensor] = None, c_weight: Optional[torch.Tensor] = None,
@@ -1322,12 +1337,12 @@ class CudaKernels:
             inv_freq = block_table = pool = c_weight = token_pos = token_slot = None
         assert rec_out is None or (dkv is not None and rec_out.shape == (T, kv_rank + rot_dim) and rec_out.stride(1) == 1
                                    and rec_out.dtype == down.dtype)
-        self._call("zlm_latent_down", self._p(cq), c_int(cq.stride(0)), c_int(cq.shape[1]), self._p(down), c_int(down.stride(0)),
-                   c_int(_dt(down)), c_int(qr), self._p(q_weight), c_int(_dt(q_weight)), self._p(dkv), self._p(c_weight),
-                   c_int(_dt(c_weight) if c_weight is not None else F32), c_float(eps), self._p(inv_freq), c_int(n_rot),
-                   self._p(token_pos), self._p(token_slot), self._p(block_table),
-                   c_int(block_table.stride(0) if block_table is not None else 0), self._p(pool), c_int(T), c_int(rot_dim),
-                   c_int(kv_rank), self._p(rec_out), c_int(rec_out.stride(0) if rec_out is not None else 0), self._stream())
+        self._call("zlm_latent_down", self._at(cq), cq.stride(0), cq.shape[1], self._at(down), down.stride(0),
+                   _dt(down), qr, self._at(q_weight), _dt(q_weight), self._at(dkv), self._at(c_weight),
+                   _dt(c_weight) if c_weight is not None else F32, c_float(eps), self._at(inv_freq), n_rot,
+                   self._at(token_pos), self._at(token_slot), self._at(block_table),
+                   block_table.stride(0) if block_table is not None else 0, self._at(pool), T, rot_dim,
+                   kv_rank, self._at(rec_out), rec_out.stride(0) if rec_out is not None else 0, self._queue())
 
     def latent_gather(self, rec: torch.Tensor, pool: torch.Tensor, block_table: torch.Tensor, token_pos: torch.Tensor,
                       token_slot: torch.Tensor) -> None:
@@ -1335,8 +1350,8 @@ class CudaKernels:
         T, R = rec.shape
         assert rec.is_contiguous() and pool.is_contiguous() and rec.dtype == pool.dtype
         assert tuple(pool.shape[1:]) == (PAGE_TOKENS, R) and block_table.dtype == torch.int32
-        self._call("zlm_latent_gather", self._p(rec), self._p(pool), self._p(block_table), c_int(block_table.stride(0)),
-                   self._p(token_pos), self._p(token_slot), c_int(_dt(rec)), c_int(T), c_int(R), self._stream())
+        self._call("zlm_latent_gather", self._at(rec), self._at(pool), self._at(block_table), block_table.stride(0),
+                   self._at(token_pos), self._at(token_slot), _dt(rec), T, R, self._queue())
 
     def latent_unfold(self, spool: torch.Tensor, stable: torch.Tensor, kv: torch.Tensor, rec: torch.Tensor,
                       token_pos: torch.Tensor, token_seq: torch.Tensor, heads: int, dim: int, rot_dim: int, v_dim: int,
@@ -1349,10 +1364,10 @@ class CudaKernels:
         assert kv.shape == (T, heads * (dim + v_dim)) and kv.stride(1) == 1 and rec.shape[0] == T and rec.stride(1) == 1
         assert spool.is_contiguous() and tuple(spool.shape[1:]) == (2, heads, PAGE_TOKENS, hd) and spool.dtype == kv.dtype
         assert stable.dtype == torch.int32 and stable.dim() == 2
-        self._call("zlm_latent_unfold", self._p(spool), self._p(stable), c_int(stable.stride(0)), self._p(kv),
-                   c_int(kv.stride(0)), self._p(rec), c_int(rec.stride(0)), self._p(token_pos), self._p(token_seq),
-                   c_int(_dt(kv)), c_int(T), c_int(heads), c_int(dim), c_int(rot_dim), c_int(v_dim), c_int(kv_rank),
-                   self._stream())
+        self._call("zlm_latent_unfold", self._at(spool), self._at(stable), stable.stride(0), self._at(kv),
+                   kv.stride(0), self._at(rec), rec.stride(0), self._at(token_pos), self._at(token_seq),
+                   _dt(kv), T, heads, dim, rot_dim, v_dim, kv_rank,
+                   self._queue())
 
     def head_linear(self, out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, impl: Optional[str] = None) -> None:
         """out[t, h, :] = w[h] @ x[t, h, :] for per-head matrices w [heads, N, K]; x [T, heads, K] and out
@@ -1362,15 +1377,15 @@ class CudaKernels:
         assert w.shape == (H, N, K) and w.is_contiguous() and out.shape == (T, H, N)
         assert x.dtype == w.dtype == out.dtype and x.stride(2) == 1 and out.stride(2) == 1
         if (x.dtype == torch.bfloat16 and T > 16 and impl != "plain" and x.data_ptr() % 16 == 0
-                and self.lib.zlm_head_linear_mma_supported(c_int(K), c_int(x.stride(0)), c_int(x.stride(1)))):
+                and self._ask("zlm_head_linear_mma_supported", K, x.stride(0), x.stride(1))):
             # many tokens: tiles of tokens per head on the tensor cores
-            self._call("zlm_head_linear_mma", self._p(out), c_int(out.stride(0)), c_int(out.stride(1)), self._p(x),
-                       c_int(x.stride(0)), c_int(x.stride(1)), self._p(w), c_int(T), c_int(H), c_int(N), c_int(K),
-                       self._stream())
+            self._call("zlm_head_linear_mma", self._at(out), out.stride(0), out.stride(1), self._at(x),
+                       x.stride(0), x.stride(1), self._at(w), T, H, N, K,
+                       self._queue())
             return
-        self._call("zlm_head_linear", self._p(out), c_int(out.stride(0)), c_int(out.stride(1)), self._p(x),
-                   c_int(x.stride(0)), c_int(x.stride(1)), self._p(w), c_int(_dt(x)), c_int(T), c_int(H), c_int(N),
-                   c_int(K), self._stream())
+        self._call("zlm_head_linear", self._at(out), out.stride(0), out.stride(1), self._at(x),
+                   x.stride(0), x.stride(1), self._at(w), _dt(x), T, H, N,
+                   K, self._queue())
 
     def latent_attention(self, out: torch.Tensor, q: torch.Tensor, pool: torch.Tensor, block_table: torch.Tensor,
                          token_pos: torch.Tensor, token_slot: torch.Tensor, heads: int, kv_rank: int, rot_dim: int,
@@ -1392,7 +1407,7 @@ class CudaKernels:
         assert q.stride(1) == 1 and out.stride(1) == 1 and pool.is_contiguous()
         assert tuple(pool.shape[1:]) == (PAGE_TOKENS, D)
         if (q.dtype == torch.bfloat16 and plan is not None and impl != "plain"
-                and self.lib.zlm_latent_attention_mma_supported(c_int(heads), c_int(kv_rank), c_int(rot_dim))
+                and self._ask("zlm_latent_attention_mma_supported", heads, kv_rank, rot_dim)
                 and q.data_ptr() % 16 == 0 and (q.stride(0) * 2) % 16 == 0 and out.stride(0) % 2 == 0):
             # the tensor-core kernel: a decode step cuts the sequences' pages into splits (all heads of a tile
             # share one pass over the records: the head tiles stand where the other attention has kv heads);
@@ -1402,26 +1417,26 @@ class CudaKernels:
                 if len_bucket is None:
                     len_bucket = attention_len_bucket(plan.max_len)
                 wave = self.decode_blocks or self.sm_count * int(
-                    self.lib.zlm_latent_attention_mma_blocks_per_sm(c_int(kv_rank), c_int(rot_dim)))
+                    self._ask("zlm_latent_attention_mma_blocks_per_sm", kv_rank, rot_dim))
                 splits, per = latent_decode_splits(T, tiles, len_bucket, wave)
                 qt, fresh = 1, max(1, int(getattr(plan, "max_new", 1) or 1))
             else:
                 splits, per = 1, max(1, (int(plan.max_len) + PAGE_TOKENS - 1) // PAGE_TOKENS)
-                qt, fresh = int(self.lib.zlm_latent_attention_mma_tokens(c_int(kv_rank), c_int(rot_dim))), 0
+                qt, fresh = self._ask("zlm_latent_attention_mma_tokens", kv_rank, rot_dim), 0
             part_o = part_ml = None
             if splits > 1:
                 part_o = plan.scratch("lat.part_o", (T * heads * splits * kv_rank,), torch.float32)
                 part_ml = plan.scratch("lat.part_ml", (T * heads * splits * 2,), torch.float32)
-            self._call("zlm_latent_attention_mma", self._p(out), c_int(out.stride(0)), self._p(q), c_int(q.stride(0)),
-                       self._p(pool), self._p(block_table), c_int(block_table.stride(0)), self._p(token_pos),
-                       self._p(token_slot), c_int(T), c_int(heads), c_int(kv_rank), c_int(rot_dim), c_float(scale),
-                       c_int(window), c_int(qt), c_int(splits), c_int(per), self._p(part_o), self._p(part_ml),
-                       c_int(fresh), c_int(chunk), self._p(sinks), self._stream())
+            self._call("zlm_latent_attention_mma", self._at(out), out.stride(0), self._at(q), q.stride(0),
+                       self._at(pool), self._at(block_table), block_table.stride(0), self._at(token_pos),
+                       self._at(token_slot), T, heads, kv_rank, rot_dim, c_float(scale),
+                       window, qt, splits, per, self._at(part_o), self._at(part_ml),
+                       fresh, chunk, self._at(sinks), self._queue())
             return
-        self._call("zlm_latent_attention", self._p(out), c_int(out.stride(0)), self._p(q), c_int(q.stride(0)),
-                   c_int(_dt(q)), self._p(pool), self._p(block_table), c_int(block_table.stride(0)),
-                   self._p(token_pos), self._p(token_slot), c_int(T), c_int(heads), c_int(kv_rank), c_int(rot_dim),
-                   c_float(scale), c_int(window), c_int(chunk), self._p(sinks), self._stream())
+        self._call("zlm_latent_attention", self._at(out), out.stride(0), self._at(q), q.stride(0),
+                   _dt(q), self._at(pool), self._at(block_table), block_table.stride(0),
+                   self._at(token_pos), self._at(token_slot), T, heads, kv_rank, rot_dim,
+                   c_float(scale), window, chunk, self._at(sinks), self._queue())
 
     # -- the stream of designs that norm a sublayer's output (see csrc/stream_ops.cu) -------------------------
     def embed_scaled(self, out: torch.Tensor, table: torch.Tensor, ids: torch.Tensor, scale: float,
@@ -1438,11 +1453,11 @@ class CudaKernels:
             assert pair.shape == (buckets + 1, H) and pair.dtype == table.dtype and pair.is_contiguous()
             assert prev_state is not None and prev_state.dtype == torch.int32 and plan is not None
         ll = ctypes.c_longlong
-        self._call("zlm_embed_scaled", self._p(out), self._p(table), c_int(_dt(table)), c_float(scale), self._p(pair),
-                   c_int(buckets), ll(mul_prev), ll(mul_cur), self._p(ids),
-                   self._p(plan.token_pos if pair is not None else None), self._p(plan.token_seq if pair is not None else None),
-                   self._p(plan.cu_seqlens if pair is not None else None), self._p(plan.seq_slot if pair is not None else None),
-                   self._p(prev_state if pair is not None else None), c_int(T), c_int(H), c_int(table.shape[0]), self._stream())
+        self._call("zlm_embed_scaled", self._at(out), self._at(table), _dt(table), c_float(scale), self._at(pair),
+                   buckets, mul_prev, mul_cur, self._at(ids),
+                   self._at(plan.token_pos if pair is not None else None), self._at(plan.token_seq if pair is not None else None),
+                   self._at(plan.cu_seqlens if pair is not None else None), self._at(plan.seq_slot if pair is not None else None),
+                   self._at(prev_state if pair is not None else None), T, H, table.shape[0], self._queue())
 
     def norm_scale_add(self, stream: torch.Tensor, y: torch.Tensor, w: torch.Tensor, eps: float,
                        layer_scale: Optional[torch.Tensor] = None, cast_out: Optional[torch.Tensor] = None) -> None:
@@ -1453,9 +1468,9 @@ class CudaKernels:
         assert stream.is_contiguous() and y.is_contiguous() and w.is_contiguous()
         assert layer_scale is None or (layer_scale.shape == (H,) and layer_scale.is_contiguous())
         assert cast_out is None or (cast_out.dtype == torch.bfloat16 and cast_out.shape == (R, H) and cast_out.is_contiguous())
-        self._call("zlm_norm_scale_add", self._p(stream), self._p(y), c_int(_dt(y)), self._p(w), c_int(_dt(w)),
-                   self._p(layer_scale), c_int(_dt(layer_scale) if layer_scale is not None else F32), c_int(R), c_int(H),
-                   c_float(eps), self._p(cast_out), self._stream())
+        self._call("zlm_norm_scale_add", self._at(stream), self._at(y), _dt(y), self._at(w), _dt(w),
+                   self._at(layer_scale), _dt(layer_scale) if layer_scale is not None else F32, R, H,
+                   c_float(eps), self._at(cast_out), self._queue())
 
     NORM_ADD_NORM_MAX = 11264        # the widest row the fused pair of norms holds in shared memory
 
@@ -1476,10 +1491,10 @@ class CudaKernels:
             mixed, cw, state, plan = conv
             taps, slots = self._check_input_conv(mixed, out2, cw, state), plan.seq_slot
             assert plan.is_decode and plan.R == R
-        self._call("zlm_norm_add_norm", self._p(stream), self._p(y), self._p(w1), c_int(_dt(w1)), c_float(eps1),
-                   self._p(out2), c_int(_dt(out2)), self._p(w2), c_int(_dt(w2)), c_float(eps2), c_int(R), c_int(H),
-                   c_int(1 if center else 0), self._p(cw), c_int(taps), self._p(state if taps > 1 else None), self._p(slots),
-                   self._p(mixed), self._stream())
+        self._call("zlm_norm_add_norm", self._at(stream), self._at(y), self._at(w1), _dt(w1), c_float(eps1),
+                   self._at(out2), _dt(out2), self._at(w2), _dt(w2), c_float(eps2), R, H,
+                   1 if center else 0, self._at(cw), taps, self._at(state if taps > 1 else None), self._at(slots),
+                   self._at(mixed), self._queue())
 
     @staticmethod
     def _check_input_conv(out, h, w, state) -> int:
@@ -1496,9 +1511,9 @@ class CudaKernels:
         first, which is brought up to date."""
         taps = self._check_input_conv(out, h, w, state)
         T, C = h.shape
-        self._call("zlm_input_conv", self._p(out), self._p(h), self._p(w), self._p(state if taps > 1 else None), c_int(_dt(h)),
-                   self._p(plan.token_seq), self._p(plan.cu_seqlens), self._p(plan.seq_slot), c_int(T), c_int(C), c_int(taps),
-                   self._stream())
+        self._call("zlm_input_conv", self._at(out), self._at(h), self._at(w), self._at(state if taps > 1 else None), _dt(h),
+                   self._at(plan.token_seq), self._at(plan.cu_seqlens), self._at(plan.seq_slot), T, C, taps,
+                   self._queue())
 
     def poly_norm(self, out: torch.Tensor, z: torch.Tensor, coef: torch.Tensor, eps: float) -> None:
         """out[t] = a N(z[t]) + b N(z[t]^2) + c N(z[t]^3) + e, powers element by element, N(u) = u / sqrt(mean(u^2) + eps)
@@ -1506,8 +1521,8 @@ class CudaKernels:
         T, F = z.shape
         assert out.shape[0] == T and out.shape[1] >= F and out.dtype == z.dtype and out.stride(1) == 1 and z.stride(1) == 1
         assert coef.shape == (4,) and coef.is_contiguous()
-        self._call("zlm_poly_norm", self._p(out), c_int(out.stride(0)), c_int(out.shape[1]), self._p(z), c_int(z.stride(0)),
-                   c_int(_dt(z)), self._p(coef), c_int(_dt(coef)), c_int(T), c_int(F), c_float(eps), self._stream())
+        self._call("zlm_poly_norm", self._at(out), out.stride(0), out.shape[1], self._at(z), z.stride(0),
+                   _dt(z), self._at(coef), _dt(coef), T, F, c_float(eps), self._queue())
 
     # -- a layer's second look at its tokens (see csrc/token_input.cu) -------------------------------------------
     def token_gate(self, g: torch.Tensor, z: torch.Tensor, side: torch.Tensor, off: int, ids: torch.Tensor) -> None:
@@ -1515,12 +1530,12 @@ class CudaKernels:
         T, dim = z.shape
         assert g.shape[0] == T and g.shape[1] >= dim and g.dtype == z.dtype == side.dtype and ids.dtype == torch.int32
         assert g.stride(1) == 1 and z.stride(1) == 1 and side.is_contiguous() and 0 <= off and off + dim <= side.shape[1]
-        self._call("zlm_token_gate", self._p(g), c_int(g.stride(0)), c_int(g.shape[1]), self._p(z), c_int(z.stride(0)),
-                   self._p(side), c_int(side.shape[1]), c_int(off), self._p(ids), c_int(_dt(z)), c_int(T), c_int(dim),
-                   c_int(side.shape[0]), self._stream())
+        self._call("zlm_token_gate", self._at(g), g.stride(0), g.shape[1], self._at(z), z.stride(0),
+                   self._at(side), side.shape[1], off, self._at(ids), _dt(z), T, dim,
+                   side.shape[0], self._queue())
 
     def token_gate_few_supported(self, tokens: int, w: torch.Tensor) -> bool:
-        return w.dtype == torch.bfloat16 and bool(self.lib.zlm_token_gate_few_supported(c_int(tokens), c_int(w.shape[1])))
+        return w.dtype == torch.bfloat16 and bool(self._ask("zlm_token_gate_few_supported", tokens, w.shape[1]))
 
     def token_gate_few(self, g: torch.Tensor, x: torch.Tensor, w: torch.Tensor, side: torch.Tensor, off: int,
                        ids: torch.Tensor) -> None:
@@ -1530,36 +1545,36 @@ class CudaKernels:
         assert x.dtype == torch.float32 and x.is_contiguous() and w.shape == (dim, K) and w.is_contiguous()
         assert g.shape[0] == T and g.shape[1] >= dim and g.dtype == w.dtype == side.dtype == torch.bfloat16
         assert g.stride(1) == 1 and side.is_contiguous() and 0 <= off and off + dim <= side.shape[1] and ids.dtype == torch.int32
-        self._call("zlm_token_gate_few", self._p(g), c_int(g.stride(0)), c_int(g.shape[1]), self._p(x), self._p(w),
-                   self._p(side), c_int(side.shape[1]), c_int(off), self._p(ids), c_int(T), c_int(K), c_int(dim),
-                   c_int(side.shape[0]), self._stream())
+        self._call("zlm_token_gate_few", self._at(g), g.stride(0), g.shape[1], self._at(x), self._at(w),
+                   self._at(side), side.shape[1], off, self._at(ids), T, K, dim,
+                   side.shape[0], self._queue())
 
     def cast_rows(self, out: torch.Tensor, x: torch.Tensor) -> None:
         """out = x rounded to bfloat16 (x fp32, both contiguous and of one shape)."""
         assert x.dtype == torch.float32 and out.dtype == torch.bfloat16 and out.shape == x.shape
         assert x.is_contiguous() and out.is_contiguous()
-        self._call("zlm_cast_rows", self._p(out), self._p(x), ctypes.c_longlong(x.numel()), self._stream())
+        self._call("zlm_cast_rows", self._at(out), self._at(x), x.numel(), self._queue())
 
     def gated_act(self, out: torch.Tensor, gu: torch.Tensor, act: str = "silu") -> None:
         """out[t, i] = act(gu[t, i]) * gu[t, I + i]; act "silu" or "gelu_tanh"."""
         T, I = out.shape
         assert gu.shape == (T, 2 * I) and gu.dtype == out.dtype and out.is_contiguous() and gu.is_contiguous()
-        self._call("zlm_gated_act", self._p(out), self._p(gu), c_int(_dt(out)), c_int(T), c_int(I),
-                   c_int({"silu": 0, "gelu_tanh": 1}[act]), self._stream())
+        self._call("zlm_gated_act", self._at(out), self._at(gu), _dt(out), T, I,
+                   {"silu": 0, "gelu_tanh": 1}[act], self._queue())
 
     def scale_(self, x: torch.Tensor, s: float) -> None:
         """x *= s for a contiguous fp32 tensor (logits times a constant)."""
         assert x.dtype == torch.float32 and x.is_contiguous()
         if self._candidates is not None and self._candidates[0] == x.data_ptr():
             self._candidates = None         # the candidates a few-token product left hold the unscaled values
-        self._call("zlm_scale_f32", self._p(x), ctypes.c_longlong(x.numel()), c_float(s), self._stream())
+        self._call("zlm_scale_f32", self._at(x), x.numel(), c_float(s), self._queue())
 
     def head_scalar_gate(self, x: torch.Tensor, g: torch.Tensor) -> None:
         """x[t, h, :] *= sigmoid(g[t, h]) in place; x [T, heads, V] and g [T, heads] may be views (innermost contiguous)."""
         T, H, V = x.shape
         assert g.shape == (T, H) and g.dtype == x.dtype and x.stride(2) == 1 and g.stride(1) == 1
-        self._call("zlm_head_scalar_gate", self._p(x), c_int(x.stride(0)), c_int(x.stride(1)), self._p(g), c_int(g.stride(0)),
-                   c_int(_dt(x)), c_int(T), c_int(H), c_int(V), self._stream())
+        self._call("zlm_head_scalar_gate", self._at(x), x.stride(0), x.stride(1), self._at(g), g.stride(0),
+                   _dt(x), T, H, V, self._queue())
 
     def expect_blank(self, t: Optional[torch.Tensor]) -> None:
         """An arrangement's word that ``t`` (fp32) is to be taken as zeros although it holds anything: the next product
@@ -1593,11 +1608,11 @@ class CudaKernels:
             assert inv_freq.dtype == torch.float32 and inv_freq.numel() * 2 == n_rot
         else:
             n_rot = 0
-        self._call("zlm_diff_prep", self._p(q_out), c_int(q_out.stride(0)), self._p(proj), c_int(proj.stride(0)),
-                   c_int(_dt(proj)), self._p(q_w), self._p(k_w), c_int(_dt(q_w)), c_float(eps),
-                   self._p(inv_freq if n_rot else None), c_int(n_rot), self._p(token_pos), self._p(token_slot),
-                   self._p(block_table), c_int(block_table.stride(0)), self._p(pool), c_int(T), c_int(heads), c_int(kv_heads),
-                   c_int(dim), c_int(vdim), c_int(hdp), self._stream())
+        self._call("zlm_diff_prep", self._at(q_out), q_out.stride(0), self._at(proj), proj.stride(0),
+                   _dt(proj), self._at(q_w), self._at(k_w), _dt(q_w), c_float(eps),
+                   self._at(inv_freq if n_rot else None), n_rot, self._at(token_pos), self._at(token_slot),
+                   self._at(block_table), block_table.stride(0), self._at(pool), T, heads, kv_heads,
+                   dim, vdim, hdp, self._queue())
 
     def diff_combine(self, out: torch.Tensor, a: torch.Tensor, heads: int, kv_heads: int, vdim: int, hdp: int, lam: float,
                      post: float, eps: float) -> None:
@@ -1606,9 +1621,9 @@ class CudaKernels:
         T = a.shape[0]
         assert a.shape == (T, 2 * heads * hdp) and out.shape == (T, heads * vdim) and a.dtype == out.dtype
         assert a.stride(1) == 1 and out.stride(1) == 1
-        self._call("zlm_diff_combine", self._p(out), c_int(out.stride(0)), self._p(a), c_int(a.stride(0)), c_int(_dt(a)),
-                   c_int(T), c_int(heads), c_int(kv_heads), c_int(vdim), c_int(hdp), c_float(lam), c_float(post), c_float(eps),
-                   self._stream())
+        self._call("zlm_diff_combine", self._at(out), out.stride(0), self._at(a), a.stride(0), _dt(a),
+                   T, heads, kv_heads, vdim, hdp, c_float(lam), c_float(post), c_float(eps),
+                   self._queue())
 
     # -- routed experts (see csrc/moe.cu) -------------------------------------
     def moe_route(self, idx: torch.Tensor, wgt: torch.Tensor, x: torch.Tensor, w_router: torch.Tensor, top: int,
@@ -1629,16 +1644,16 @@ class CudaKernels:
         if w_gate is not None:
             assert w_gate.numel() == K and w_gate.is_contiguous() and w_gate.dtype == x.dtype
             assert gate is not None and gate.dtype == torch.float32 and gate.numel() >= T
-        self._call("zlm_moe_route", self._p(idx), self._p(wgt), self._p(gate if w_gate is not None else None), self._p(x),
-                   c_int(x.stride(0)), self._p(w_router), self._p(w_gate), c_int(_dt(x)), c_int(T), c_int(E), c_int(K),
-                   c_int(top), c_int({"sigmoid": 0, "softmax": 1}[score]), c_int(1 if renormalize else 0),
-                   *self._route_extras(correction, E, groups, keep, weight_scale, group_top), self._stream())
+        self._call("zlm_moe_route", self._at(idx), self._at(wgt), self._at(gate if w_gate is not None else None), self._at(x),
+                   x.stride(0), self._at(w_router), self._at(w_gate), _dt(x), T, E, K,
+                   top, {"sigmoid": 0, "softmax": 1}[score], 1 if renormalize else 0,
+                   *self._route_extras(correction, E, groups, keep, weight_scale, group_top), self._queue())
 
     def _route_extras(self, correction, E, groups, keep, weight_scale, group_top=1):
         if correction is not None:
             assert correction.dtype == torch.float32 and correction.shape == (E,) and correction.is_contiguous()
         assert group_top in (1, 2)
-        return self._p(correction), c_int(groups), c_int(keep), c_int(group_top), c_float(weight_scale)
+        return self._at(correction), groups, keep, group_top, c_float(weight_scale)
 
     def moe_choose(self, idx: torch.Tensor, wgt: torch.Tensor, logits: torch.Tensor, experts: int, top: int,
                    gate: Optional[torch.Tensor] = None, score: str = "sigmoid", renormalize: bool = False,
@@ -1650,10 +1665,10 @@ class CudaKernels:
         assert logits.dtype == torch.float32 and logits.stride(1) == 1 and logits.shape[1] >= experts + (1 if gate is not None else 0)
         assert idx.dtype == torch.int32 and wgt.dtype == torch.float32 and idx.shape == (T, top) and wgt.shape == (T, top)
         assert idx.is_contiguous() and wgt.is_contiguous()
-        self._call("zlm_moe_choose", self._p(idx), self._p(wgt), self._p(gate), self._p(logits), c_int(logits.stride(0)),
-                   c_int(T), c_int(experts), c_int(top), c_int(1 if gate is not None else 0),
-                   c_int({"sigmoid": 0, "softmax": 1}[score]), c_int(1 if renormalize else 0),
-                   *self._route_extras(correction, experts, groups, keep, weight_scale, group_top), self._stream())
+        self._call("zlm_moe_choose", self._at(idx), self._at(wgt), self._at(gate), self._at(logits), logits.stride(0),
+                   T, experts, top, 1 if gate is not None else 0,
+                   {"sigmoid": 0, "softmax": 1}[score], 1 if renormalize else 0,
+                   *self._route_extras(correction, experts, groups, keep, weight_scale, group_top), self._queue())
 
     _ACT_KINDS = {"relu2": 0, "swiglu": 1, "swiglu_interleaved": 2, "swish_limit": 3, "swish_limit_interleaved": 4}
 
@@ -1672,9 +1687,9 @@ class CudaKernels:
         E = w_up.shape[0]
         assert w_up.shape == (E, F * (2 if kind else 1), K) and w_up.is_contiguous() and act.shape == (T, top, F) and act.is_contiguous()
         assert x.dtype == w_up.dtype == act.dtype and x.stride(1) == 1
-        self._call("zlm_moe_up", self._p(act), self._p(x), c_int(x.stride(0)), self._p(w_up), self._p(idx), self._p(wgt),
-                   c_int(_dt(x)), c_int(T), c_int(top), c_int(F), c_int(K), c_int(1 if scale_input else 0), c_int(kind),
-                   c_int(E), c_float(limit), c_float(alpha), self._stream())
+        self._call("zlm_moe_up", self._at(act), self._at(x), x.stride(0), self._at(w_up), self._at(idx), self._at(wgt),
+                   _dt(x), T, top, F, K, 1 if scale_input else 0, kind,
+                   E, c_float(limit), c_float(alpha), self._queue())
 
     def moe_down(self, stream: torch.Tensor, act: torch.Tensor, w_down: torch.Tensor, idx: torch.Tensor,
                  identity_input: Optional[torch.Tensor] = None, wgt: Optional[torch.Tensor] = None) -> None:
@@ -1687,9 +1702,9 @@ class CudaKernels:
         x = identity_input
         if x is not None:
             assert x.shape == (T, N) and x.stride(1) == 1 and x.dtype == act.dtype and wgt is not None and wgt.is_contiguous()
-        self._call("zlm_moe_down", self._p(stream), self._p(act), self._p(w_down), self._p(idx), c_int(_dt(act)), c_int(T),
-                   c_int(top), c_int(F), c_int(N), c_int(E), self._p(x), c_int(x.stride(0) if x is not None else 0),
-                   self._p(wgt if x is not None else None), self._stream())
+        self._call("zlm_moe_down", self._at(stream), self._at(act), self._at(w_down), self._at(idx), _dt(act), T,
+                   top, F, N, E, self._at(x), x.stride(0) if x is not None else 0,
+                   self._at(wgt if x is not None else None), self._queue())
 
     def moe_grouped(self, stream: torch.Tensor, x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor,
                     idx: torch.Tensor, wgt: torch.Tensor, scale_input: bool = True, impl: Optional[str] = None,
@@ -1731,37 +1746,37 @@ class CudaKernels:
             act = self.scratch("moe.sorted_act", P * F, torch.bfloat16, x.device)
             y = self.scratch("moe.sorted_out", P * K, torch.float32, x.device)
             inv, table = ints[:P], ints[P:P + 3 * tiles]
-            self._call("zlm_moe_sort", self._p(idx), c_int(P), c_int(E), c_int(tiles), self._p(inv), self._p(table), self._stream())
-            self._call("zlm_moe_gather", self._p(xs), self._p(x), c_int(x.stride(0)), self._p(inv), self._p(wgt), c_int(T),
-                       c_int(top), c_int(K), c_int(1 if scale_input else 0), self._stream())
+            self._call("zlm_moe_sort", self._at(idx), P, E, tiles, self._at(inv), self._at(table), self._queue())
+            self._call("zlm_moe_gather", self._at(xs), self._at(x), x.stride(0), self._at(inv), self._at(wgt), T,
+                       top, K, 1 if scale_input else 0, self._queue())
             if activation == "swish_limit_interleaved":
                 assert limit > 0
-                self._call("zlm_set_gate_gemm_tcgen05", c_float(limit), c_float(alpha), self._stream())
-            self._call("zlm_gemm_tc_experts", self._p(act), self._p(xs), self._p(w_up), self._p(table), c_int(tiles), c_int(P),
-                       c_int(E), c_int(2 * F if gated else F), c_int(K), c_int(F),
-                       c_int({"relu2": 6, "swiglu_interleaved": 3, "swish_limit_interleaved": GATED_LIMIT}[activation]), self._stream())
-            self._call("zlm_gemm_tc_experts", self._p(y), self._p(act), self._p(w_down), self._p(table), c_int(tiles), c_int(P),
-                       c_int(E), c_int(K), c_int(F), c_int(K), c_int(2), self._stream())
-            self._call("zlm_moe_combine", self._p(stream), self._p(y), self._p(inv), self._p(None if scale_input else wgt),
-                       c_int(T), c_int(top), c_int(K), self._p(x if identity else None), c_int(x.stride(0)),
-                       self._p(wgt if identity else None), self._stream())
+                self._call("zlm_set_gate_gemm_tcgen05", c_float(limit), c_float(alpha), self._queue())
+            self._call("zlm_gemm_tc_experts", self._at(act), self._at(xs), self._at(w_up), self._at(table), tiles, P,
+                       E, 2 * F if gated else F, K, F,
+                       {"relu2": 6, "swiglu_interleaved": 3, "swish_limit_interleaved": GATED_LIMIT}[activation], self._queue())
+            self._call("zlm_gemm_tc_experts", self._at(y), self._at(act), self._at(w_down), self._at(table), tiles, P,
+                       E, K, F, K, 2, self._queue())
+            self._call("zlm_moe_combine", self._at(stream), self._at(y), self._at(inv), self._at(None if scale_input else wgt),
+                       T, top, K, self._at(x if identity else None), x.stride(0),
+                       self._at(wgt if identity else None), self._queue())
             return
-        bm = int(self.lib.zlm_moe_grouped_tile_rows(c_int(P), c_int(E)))
-        tiles = int(self.lib.zlm_moe_grouped_max_tiles(c_int(P), c_int(E), c_int(bm)))
+        bm = self._ask("zlm_moe_grouped_tile_rows", P, E)
+        tiles = self._ask("zlm_moe_grouped_max_tiles", P, E, bm)
         ints = self.scratch("moe.sorted", 2 * P + 3 * tiles, torch.int32, x.device)
         act = self.scratch("moe.sorted_act", P * F, torch.bfloat16, x.device)
         y = self.scratch("moe.sorted_out", P * K, torch.float32, x.device)
-        self._call("zlm_moe_grouped", self._p(stream), self._p(x), c_int(x.stride(0)), self._p(w_up), self._p(w_down),
-                   self._p(idx), self._p(wgt), c_int(T), c_int(top), c_int(E), c_int(F), c_int(K),
-                   c_int(1 if scale_input else 0), self._p(ints), self._p(act), self._p(y), self._stream())
+        self._call("zlm_moe_grouped", self._at(stream), self._at(x), x.stride(0), self._at(w_up), self._at(w_down),
+                   self._at(idx), self._at(wgt), T, top, E, F, K,
+                   1 if scale_input else 0, self._at(ints), self._at(act), self._at(y), self._queue())
 
     def relu2_scale(self, out: torch.Tensor, u: torch.Tensor, row_scale: Optional[torch.Tensor] = None) -> None:
         """out[t, i] = relu(u[t, i])^2 * row_scale[t]."""
         T, F = u.shape
         assert out.shape == (T, F) and out.dtype == u.dtype and out.is_contiguous() and u.is_contiguous()
         assert row_scale is None or (row_scale.dtype == torch.float32 and row_scale.numel() >= T)
-        self._call("zlm_relu2_scale", self._p(out), self._p(u), self._p(row_scale), c_int(_dt(u)), c_int(T), c_int(F),
-                   self._stream())
+        self._call("zlm_relu2_scale", self._at(out), self._at(u), self._at(row_scale), _dt(u), T, F,
+                   self._queue())
 
     def argmax(self, out: torch.Tensor, logits: torch.Tensor, fresh: bool = False) -> None:
         """out[r] = index of the highest logit of row r, ties to the lowest index.  ``fresh``: the
@@ -1774,18 +1789,18 @@ class CudaKernels:
         if cand is not None and cand[0] == logits.data_ptr() and cand[1] >= R and cand[2] == V and logits.is_contiguous():
             # these logits came from the few-token product just before: it left the candidates
             _, _, _, nb, cv, ci = cand
-            self._call("zlm_argmax_candidates", self._p(out), self._p(cv), self._p(ci), c_int(R), c_int(nb), self._stream())
+            self._call("zlm_argmax_candidates", self._at(out), self._at(cv), self._at(ci), R, nb, self._queue())
             return
         sv = self.scratch("argmax.values", R * 64, torch.float32, logits.device)
         si = self.scratch("argmax.indices", R * 64, torch.int32, logits.device)
-        self._call("zlm_argmax", self._p(out), self._p(logits), c_int(R), c_int(V),
-                   c_int(logits.stride(0)), self._p(sv), self._p(si), self._stream())
+        self._call("zlm_argmax", self._at(out), self._at(logits), R, V,
+                   logits.stride(0), self._at(sv), self._at(si), self._queue())
 
     def set_pdl(self, on: bool) -> None:
         """Launch the decode-path kernels with programmatic dependent launch (a kernel's
         blocks are scheduled, and its weights start streaming, while the kernel before it
         drains) or in plain stream order."""
-        self.lib.zlm_set_pdl(c_int(1 if on else 0))
+        self._ask("zlm_set_pdl", 1 if on else 0)
 
     def gemm_tc_status(self) -> int:
         """0 unless a bounded wait inside a tcgen05 kernel (product or attention) gave up
@@ -1799,8 +1814,8 @@ class CudaKernels:
         flag, nanoseconds the kernel took, its TMA copy had landed)."""
         src = torch.zeros((128, 64), dtype=torch.bfloat16, device="cuda")
         out = torch.zeros(4, dtype=torch.int32, device="cuda")
-        self._call("zlm_test_bounded_wait", self._p(src), self._p(out), ctypes.c_ulonglong(int(limit_ns)),
-                   self._stream())
+        self._call("zlm_test_bounded_wait", self._at(src), self._at(out), ctypes.c_ulonglong(int(limit_ns)),
+                   self._queue())
         torch.cuda.synchronize()
         code, released, ns, landed = out.tolist()
         return code, bool(released), ns, bool(landed)
@@ -1815,10 +1830,10 @@ class CudaKernels:
         R, V = logits.shape
         assert logits.dtype == torch.float32 and logits.stride(1) == 1 and out.dtype == torch.int32
         assert request.dtype == torch.int32 and position.dtype == torch.int32
-        self._call("zlm_sample", self._p(out), self._p(logits), c_int(R), c_int(V),
-                   c_int(logits.stride(0)), c_float(temperature), c_int(top_k), c_float(top_p),
-                   ctypes.c_ulonglong(seed & 0xFFFFFFFFFFFFFFFF), self._p(request),
-                   self._p(position), c_int({None: 0, "block": 1, "cluster": 2}[form]), self._stream())
+        self._call("zlm_sample", self._at(out), self._at(logits), R, V,
+                   logits.stride(0), c_float(temperature), top_k, c_float(top_p),
+                   ctypes.c_ulonglong(seed & 0xFFFFFFFFFFFFFFFF), self._at(request),
+                   self._at(position), {None: 0, "block": 1, "cluster": 2}[form], self._queue())
 
 
 _KERNELS: Optional[CudaKernels] = None

@@ -94,22 +94,31 @@ class Workspace:
 
     def __init__(self, device):
         self.device = device
-        self._bufs: Dict[str, torch.Tensor] = {}
+        self._bufs: Dict[Tuple[str, torch.dtype], torch.Tensor] = {}
+        self._views: Dict[Any, torch.Tensor] = {}      # (a view costs the host as much as a launch's arguments: kept by name and shape)
         self.generation = 0
 
     def get(self, name: str, shape: Sequence[int], dtype: torch.dtype) -> torch.Tensor:
+        shape = tuple(shape)
+        view = self._views.get((name, dtype, shape))
+        if view is not None:
+            return view
         n = 1
         for s in shape:
             n *= int(s)
-        key = f"{name}:{dtype}"
+        key = (name, dtype)
         buf = self._bufs.get(key)
         if buf is None or buf.numel() < n:
             if buf is not None and buf.is_cuda and not torch.cuda.is_current_stream_capturing():
                 torch.cuda.synchronize(buf.device)      # (kernels of another stream may still be at the old memory)
             buf = torch.empty(max(n, 1), dtype=dtype, device=self.device)
             self._bufs[key] = buf
+            self._views.clear()
             self.generation += 1
-        return buf[:n].view(*shape)
+        if len(self._views) >= 1024:                    # (steps of ever new sizes)
+            self._views.clear()
+        view = self._views[(name, dtype, shape)] = buf[:n].view(*shape)
+        return view
 
 
 class Runtime:
