@@ -51,7 +51,7 @@ static int launch_decode(__nv_bfloat16* out, int out_stride, const __nv_bfloat16
                          int window, int splits, int per, float* part_o, float* part_ml, int fresh, int sink, AttnOpts opt,
                          cudaStream_t st) {
     const size_t stage_bytes = (size_t)4 * ZLM_PAGE * HD * sizeof(__nv_bfloat16);
-    const size_t merge_bytes = (size_t)DEC_WARPS * 16 * (HD + 2) * sizeof(float);
+    const size_t merge_bytes = (size_t)DEC_WARPS * 16 * (HD + 8 + 2) * sizeof(float);
     const size_t smem = stage_bytes > merge_bytes ? stage_bytes : merge_bytes;
     auto kern = attention_decode_kernel<HD>;
     static bool attr_set_dev[64] = {}; bool& attr_set = attr_set_dev[zlm_device_index()];
