@@ -632,11 +632,13 @@ mlstm_out_kernel(float* __restrict__ o, const TA* __restrict__ proj, int stride,
 }
 
 // ---------------------------------------------------------------------------- the outputs as tensor-core products
-// The third pass for bfloat16 projections and heads of up to 128 coordinates, every fp32 operand cut into three bfloat16
-// pieces (split_mma.cuh), the heads' norm and gate along with it.  3,001 tokens of four sequences, 16 heads of 128 x 128: 108 us
-// on the FFMA pipe (three shared-memory reads for 48 FMAs) and 28 us norm and gate, 99 us so (56 bytes of spills); outputs 3.7e-7 off 64-bit
-// sums before, 2.1e-7 now.  (The first pass stays an FFMA chain: as products it took 37 instead of 58 us, but its states, which
-// exponential weights make the sum of a few last tokens, were 7e-8 off instead of 6e-8.)
+// The third pass for bfloat16 projections and heads of up to 128 coordinates.  Queries and keys stay bfloat16 (q_scale goes to
+// the sums, which are 32-bit either way), so a score takes one product and a number read from the state three, of the
+// state cut into three bfloat16 pieces (split_mma.cuh); the weights of the values are cut likewise.  The heads' norm and gate
+// go along with it.  3,001 tokens of four sequences, 16 heads of 128 x 128: 108 us on the FFMA pipe (three shared-memory reads
+// for 48 FMAs) and 28 us norm and gate; 99 us with queries, scaled first, and keys in pieces too (six products each).  (The
+// first pass stays an FFMA chain: as products it took 37 instead of 58 us, but its states, which exponential weights make the sum
+// of a few last tokens, were 7e-8 off instead of 6e-8.)
 // grid (R * maxp * H, ceil(V / 128)); a warp owns 16 tokens and 64 value columns
 __global__ void __launch_bounds__(ML_THREADS, 2)
 mlstm_out_products_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, int stride, int q_off, int k_off, int v_off,
@@ -644,12 +646,13 @@ mlstm_out_products_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, int
                           const float2* __restrict__ ahead, float* __restrict__ mmax, const int* __restrict__ seq_slot,
                           const int* __restrict__ cu_seqlens, int H, int D, int V, int maxp, float q_scale) {
     extern __shared__ __align__(128) __nv_bfloat16 ml_tiles[];
-    __nv_bfloat16* qt = ml_tiles;                    // [3][SM_L][128]
-    __nv_bfloat16* kt = qt + 3 * SM_L * 128;         // [3][SM_L][128], later the weights and the state's rows:
+    __nv_bfloat16* qt = ml_tiles;                    // [SM_L][128]
+    __nv_bfloat16* vt = qt + SM_L * 128;             // [SM_L][128]
+    __nv_bfloat16* kt = vt + SM_L * 128;             // [SM_L][128], later the weights and the state's rows:
     __nv_bfloat16* pt = kt;                          // [3][SM_L][SM_L]
-    __nv_bfloat16* st = pt + 3 * SM_L * SM_L;        // [3][32][128], later the gate's columns
-    __nv_bfloat16* vt = kt + 3 * SM_L * 128;         // [SM_L][128]
-    // (with the tiles this is all that two blocks an SM have room for: what comes later takes the place of what is read)
+    __nv_bfloat16* st = pt + 3 * SM_L * SM_L;        // [2][3][32][128], then one of the two the gate's columns
+    constexpr int ST = 3 * 32 * 128;
+    // (what comes later takes the place of what is read)
     __shared__ __align__(16) double se[SM_L], sm[SM_L];
     float* m_of = (float*)se;                        // [SM_L], after the weights
     float (*sums)[2] = (float (*)[2])sm;             // [SM_L][2], after the weights; once more for the heads' norms
@@ -661,7 +664,11 @@ mlstm_out_products_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, int
     if (!ZLM_CHK(ahead + pc.at, 8)) return;
     const float2 ma = ahead[pc.at];
     const __nv_bfloat16* rows = proj + (size_t)pc.row0 * stride;
+    sm_stage_values(qt, rows + q_off + (size_t)pc.h * D, stride, pc.n, 0, D, tid);
+    sm_stage_values(kt, rows + k_off + (size_t)pc.h * D, stride, pc.n, 0, D, tid);
     sm_stage_values(vt, rows + v_off + (size_t)pc.h * V, stride, pc.n, c0, V, tid);
+    const float* S = part + pc.at * D * V;
+    SmRows next = sm_fetch_state(S, 0, D, V, c0, tid);
     float m0 = 0.f, m1 = 0.f;
     if (warp == 0) {
         const MlPieceGates g = ml_piece_gates(gates, pc.row0, pc.n, pc.h);
@@ -676,10 +683,6 @@ mlstm_out_products_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, int
             if (ZLM_CHK(dst, 4)) *dst = ma.y;
         }
     }
-    sm_stage_rows(qt, rows + q_off + (size_t)pc.h * D, stride, pc.n, D, q_scale, tid);
-    sm_stage_rows(kt, rows + k_off + (size_t)pc.h * D, stride, pc.n, D, 1.f, tid);
-    const float* S = part + pc.at * D * V;
-    SmRows next = sm_fetch_state(S, 0, D, V, c0, tid);
     const float* np = part_n + pc.at * D + lane * 4;
     const float4 n_ahead = lane * 4 < D && ZLM_CHK(np, 16) ? *(const float4*)np : make_float4(0.f, 0.f, 0.f, 0.f);
     dec_wait<0>();
@@ -688,7 +691,7 @@ mlstm_out_products_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, int
     float s[4][4], keep[2], sum[2] = {0.f, 0.f};
     {
         SmSum<4> dots;
-        sm_scores(dots, qt, kt, r0, half * 32, D, lane);
+        sm_scores_plain(dots, qt, kt, r0, half * 32, D, lane);
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
             const int j = j0 + 8 * x;
@@ -699,7 +702,7 @@ mlstm_out_products_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, int
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const int l = half * 32 + i * 8 + (lane & 3) * 2 + e;
-                    s[i][2 * x + e] = (l <= j && l < pc.n) ? dots.get(i, 2 * x + e) * expf((float)(se[l] - M)) : 0.f;
+                    s[i][2 * x + e] = (l <= j && l < pc.n) ? dots.get(i, 2 * x + e) * q_scale * expf((float)(se[l] - M)) : 0.f;
                     sum[x] += s[i][2 * x + e];
                 }
             sum[x] += __shfl_xor_sync(0xffffffffu, sum[x], 1);
@@ -711,19 +714,18 @@ mlstm_out_products_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, int
         const int row = r0 + (lane >> 1);
         float nq = 0.f;
         for (int c = 0; c < D >> 3; c += 2) {
-            float f[3][8];
-#pragma unroll
-            for (int x = 0; x < 3; ++x) widen8(*(const uint4*)(qt + x * SM_L * 128 + tile_off<128>(row, c + (lane & 1))), f[x]);
+            float f[8];
+            widen8(*(const uint4*)(qt + tile_off<128>(row, c + (lane & 1))), f);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
                 const float mine = (e & 3) == 0 ? n_ahead.x : (e & 3) == 1 ? n_ahead.y : (e & 3) == 2 ? n_ahead.z : n_ahead.w;
                 const float nv = __shfl_sync(0xffffffffu, mine, 2 * (c + (lane & 1)) + (e >> 2));
-                nq = fmaf(nv, sm_odd(f[0][e]) ? f[0][e] : f[0][e] + (f[1][e] + f[2][e]), nq);
+                nq = fmaf(nv, f[e], nq);
             }
         }
         nq += __shfl_xor_sync(0xffffffffu, nq, 1);
 #pragma unroll
-        for (int x = 0; x < 2; ++x) sum[x] = fmaf(keep[x], __shfl_sync(0xffffffffu, nq, 2 * (lane >> 2) + 16 * x), sum[x]);
+        for (int x = 0; x < 2; ++x) sum[x] = fmaf(keep[x] * q_scale, __shfl_sync(0xffffffffu, nq, 2 * (lane >> 2) + 16 * x), sum[x]);
     }
     __syncthreads();                                 // (the keys, e and the maxima are read)
     sm_put_weights(pt, s, r0, half * 32, lane);
@@ -731,17 +733,19 @@ mlstm_out_products_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, int
     if ((lane & 3) == 0) { sums[j0][half] = sum[0]; sums[j0 + 8][half] = sum[1]; }
     SmSum<8> acc;
     acc.zero();
-    for (int d0 = 0; d0 < D; d0 += 32) {
+    for (int d0 = 0; d0 < D; d0 += 32, st = pt + 3 * SM_L * SM_L + (d0 & 32 ? ST : 0)) {
+        // (whoever is here has passed the barrier of the 32 rows before, and with it everybody's reading of the two before)
         sm_put_state(st, next, tid);
         if (d0 + 32 < D) next = sm_fetch_state(S, d0 + 32, D, V, c0, tid);
         __syncthreads();
-        sm_read_state(acc, qt, st, r0, half * 64, d0, D, lane);
-        __syncthreads();
+        sm_read_state_plain(acc, qt, st, r0, half * 64, d0, D, lane);
     }
     if (out.y) sm_stage_values(st, out.g + (size_t)pc.row0 * out.g_stride + (size_t)pc.h * V, out.g_stride, pc.n, 0, V, tid);      // (the state is read)
+    keep[0] *= q_scale;
+    keep[1] *= q_scale;
     acc.scale(keep[0], keep[1]);
     sm_read_values(acc, pt, vt, r0, half * 64, lane);
-    sm_mend_out(acc, SmSeen{qt, pt, vt, S + c0, rows + v_off + (size_t)pc.h * V + c0, (size_t)stride, D, V}, keep[0], keep[1], taken, pc.n,
+    sm_mend_out(acc, SmSeen{qt, pt, vt, S + c0, rows + v_off + (size_t)pc.h * V + c0, (size_t)stride, D, V, q_scale}, keep[0], keep[1], taken, pc.n,
                 V - c0, r0, half * 64, lane);
     float inv[2];
 #pragma unroll
@@ -886,7 +890,7 @@ extern "C" int zlm_mlstm(float* o, const void* proj, int stride, int dtype, int 
     ZLM_REQUIRE(!y || (products && V <= 128 && y_stride % 8 == 0 && g_stride % 8 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)g % 16 == 0),
                 "mlstm: heads of %d x %d do not take their gate along", D, V);
     if (products) {
-        const size_t t3 = (size_t)7 * SM_L * 128 * sizeof(__nv_bfloat16);
+        const size_t t3 = (size_t)(2 * SM_L * 128 + 3 * SM_L * SM_L + 2 * 3 * 32 * 128) * sizeof(__nv_bfloat16);
         static bool attr_set_dev[64] = {};
         bool& attr_set = attr_set_dev[zlm_device_index()];
         if (!attr_set) {

@@ -440,7 +440,7 @@ retention_piece_out_kernel(SmOut out, const __nv_bfloat16* __restrict__ proj, in
     const float keep0 = pw[r0 + (lane >> 2) + 1], keep8 = pw[r0 + (lane >> 2) + 9];
     acc.scale(keep0, keep8);
     sm_read_values(acc, pt, vt, r0, part * 64, lane);
-    sm_mend_out(acc, SmSeen{qt, pt, vt, S + c0, rows + v_off + (size_t)h * V + c0, (size_t)ld, D, V}, keep0, keep8, taken, n, V - c0, r0,
+    sm_mend_out(acc, SmSeen{qt, pt, vt, S + c0, rows + v_off + (size_t)h * V + c0, (size_t)ld, D, V, 0.f}, keep0, keep8, taken, n, V - c0, r0,
                 part * 64, lane);
     sm_write(acc, 1.f, 1.f, out, st, red, row0, n, h, H, V, c0, r0, part, lane);
 }

@@ -101,6 +101,22 @@ template <int NP> __device__ __forceinline__ void sm_mma3(float (*acc)[4], const
 #pragma unroll
         for (int e = 0; e < 4; ++e) acc[t][e] += d[t][e];
 }
+// the same with A in bfloat16 as it is and B in pieces
+template <int NP> __device__ __forceinline__ void sm_mma3b(float (*acc)[4], const unsigned (&a)[4], const unsigned (&b)[NP][3][4]) {
+    float d[2 * NP][4];
+#pragma unroll
+    for (int x = 2; x >= 0; --x)
+#pragma unroll
+        for (int t = 0; t < 2 * NP; ++t) {
+            const unsigned* p = b[t / 2][x] + (t & 1) * 2;
+            if (x == 2) sm_mma_zero(d[t], a, p[0], p[1]);
+            else dec_mma(d[t], a, p[0], p[1]);
+        }
+#pragma unroll
+    for (int t = 0; t < 2 * NP; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[t][e] += d[t][e];
+}
 // sums of NT tiles of 16 x 8
 template <int NT> struct SmSum {
     float v[NT][4];
@@ -187,13 +203,15 @@ static __device__ __noinline__ void sm_mend_state(float (*s)[4], const __nv_bflo
             s[i][e] = t;
         }
 }
-// what an output is made of: S the state's column of the head's value column c0 + c, v the piece's values of that column
+// what an output is made of: S the state's column of the head's value column c0 + c, v the piece's values of that column;
+// q_scale: 0 where the queries' tile holds pieces, else the factor of queries that are bfloat16 as they are
 struct SmSeen {
     const __nv_bfloat16 *qt, *pt, *vt;
     const float* S;
     const __nv_bfloat16* v;
     size_t stride;
     int D, V;
+    float q_scale;
 };
 static __device__ __noinline__ void sm_mend_outputs(float (*acc)[4], const SmSeen& s, float keep0, float keep8, bool taken, int n, int cols,
                                                     int r0, int n0, int lane) {
@@ -206,9 +224,10 @@ static __device__ __noinline__ void sm_mend_outputs(float (*acc)[4], const SmSee
                 x = 0.f;
                 for (int d = 0; d < s.D; ++d) {
                     const float* p = s.S + (size_t)d * s.V + c;
-                    if (ZLM_CHK(p, 4)) x = fmaf(sm_whole<128>(s.qt, SM_L * 128, j, d), *p, x);
+                    const float q = s.q_scale == 0.f ? sm_whole<128>(s.qt, SM_L * 128, j, d) : to_f32(s.qt[tile_off<128>(j, d >> 3) + (d & 7)]);
+                    if (ZLM_CHK(p, 4)) x = fmaf(q, *p, x);
                 }
-                x *= e < 2 ? keep0 : keep8;
+                x *= e < 2 ? keep0 : keep8;            // (the queries' factor among them)
                 for (int l = 0; l <= j; ++l)
                     x = fmaf(sm_whole<SM_L>(s.pt, SM_L * SM_L, j, l), to_f32(s.vt[tile_off<128>(l, c >> 3) + (c & 7)]), x);
             }
@@ -286,6 +305,25 @@ __device__ __forceinline__ void sm_scores(SmSum<4>& s, const __nv_bfloat16* qt, 
     sm_mend_scores(t.v, qt, kt, r0, n0, dim, lane);
     s = t;
 }
+// the same of queries and keys that are bfloat16 as they are [SM_L][128]: their products are exact, and what is not finite
+// comes out as from FFMA chains
+__device__ __forceinline__ void sm_scores_plain(SmSum<4>& s, const __nv_bfloat16* qt, const __nv_bfloat16* kt, int r0, int n0, int dim, int lane) {
+    s.zero();
+    if (n0 > r0 + 15) return;
+    for (int k0 = 0; k0 < dim; k0 += 16) {
+        unsigned a[4], b[2][4];
+        dec_ldsm4(a[0], a[1], a[2], a[3], sm_a_rows<128>(qt, r0, k0, lane));
+#pragma unroll
+        for (int y = 0; y < 2; ++y) dec_ldsm4(b[y][0], b[y][1], b[y][2], b[y][3], sm_b_rows<128>(kt, n0 + y * 16, k0, lane));
+        float d[4][4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) sm_mma_zero(d[t], a, b[t / 2][(t & 1) * 2], b[t / 2][(t & 1) * 2 + 1]);
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s.v[t][e] += d[t][e];
+    }
+}
 // 32 rows of the state, 128 columns: fetched into registers (a thread's four float4), then cut into pieces [32][128]
 struct SmRows { float4 f[4]; };
 __device__ __forceinline__ SmRows sm_fetch_state(const float* S, int d0, int dim, int V, int c0, int tid) {
@@ -324,6 +362,26 @@ __device__ __forceinline__ void sm_read_state(SmSum<8>& acc, const __nv_bfloat16
                 for (int x = 0; x < 3; ++x)
                     dec_ldsm4t(b[y][x][0], b[y][x][1], b[y][x][2], b[y][x][3], sm_b_cols<128>(st + x * 32 * 128, n0 + n * 8 + y * 16, k0, lane));
             sm_mma6<2>(acc.v + n, a, b);
+        }
+    }
+}
+// the same with queries that are bfloat16 as they are
+__device__ __forceinline__ void sm_read_state_plain(SmSum<8>& acc, const __nv_bfloat16* qt, const __nv_bfloat16* st, int r0, int n0, int d0, int dim,
+                                                    int lane) {
+#pragma unroll
+    for (int k0 = 0; k0 < 32; k0 += 16) {
+        if (d0 + k0 >= dim) return;
+        unsigned a[4];
+        dec_ldsm4(a[0], a[1], a[2], a[3], sm_a_rows<128>(qt, r0, d0 + k0, lane));
+#pragma unroll
+        for (int n = 0; n < 8; n += 4) {
+            unsigned b[2][3][4];
+#pragma unroll
+            for (int y = 0; y < 2; ++y)
+#pragma unroll
+                for (int x = 0; x < 3; ++x)
+                    dec_ldsm4t(b[y][x][0], b[y][x][1], b[y][x][2], b[y][x][3], sm_b_cols<128>(st + x * 32 * 128, n0 + n * 8 + y * 16, k0, lane));
+            sm_mma3b<2>(acc.v + n, a, b);
         }
     }
 }
