@@ -1640,6 +1640,19 @@ extern "C" int zlm_gemm_tc_tile_width(int T, int N, int K) {
     return best;
 }
 
+// The width for a mode: 240 columns, and 224 of gate and up, are no whole boxes of the copy engine's (32 bf16 outputs, 64 sums
+// of gate and up), and with them a tile's results leave row by row.  2,048 tokens, bf16 outputs, 240 / 256 columns: N = 4,096 at
+// K = 512 20.0 / 13.0 us, N = 6,144 at K = 4,096 79.2 / 72.0; 5,000 tokens x 4,096 at K = 1,024 48.9 / 33.0.
+static int tile_width(int T, int N, int K, int mode) {
+    const int width = zlm_gemm_tc_tile_width(T, N, K);
+    if (g_tc_width || g_tc_form == 1 || width == 0 || width == 128 || width == 256) return width;
+    if (ZLM_GATED(mode)) return 256;
+    if (mode != 0 || width != 240) return width;
+    const long long m_tiles = (T + TCQ_BM - 1) / TCQ_BM, slots = sm_count() / 2;
+    auto cost = [&](int bn) { return ((m_tiles * ((N + bn - 1) / bn) + slots - 1) / slots) * bn; };
+    return cost(224) * 100 < cost(256) * 95 ? 224 : 256;
+}
+
 // mode 0: Y bf16 = X W^T; mode 1: Y fp32 += X W^T; mode 2: Y fp32 = X W^T;
 // mode 3: Y bf16 [T, N/2] = silu(gate) * up, W's rows in groups of 8 gate + 8 up (N a multiple of 16);
 // mode 7: the same with gelu_tanh(gate).
@@ -1668,7 +1681,7 @@ extern "C" int zlm_gemm_tc(void* Y, const void* X, const void* W, int T, int N, 
         if (T <= 64) return launch_tc_few<64, 8>(Y, X, W, T, N, K, ldx, ldy, mode, plan, scratch, st);
         return launch_tc_few<128, 6>(Y, X, W, T, N, K, ldx, ldy, mode, plan, scratch, st);
     }
-    const int width = zlm_gemm_tc_tile_width(T, N, K);
+    const int width = tile_width(T, N, K, mode);
     if (g_tc_form != 1) {
         if (width == 128) return launch_tc_pair<128, 8>(Y, X, W, T, N, K, ldx, ldy, mode, st);
         if (width == 240) return launch_tc_pair<240, 6>(Y, X, W, T, N, K, ldx, ldy, mode, st);
