@@ -1,6 +1,6 @@
 // bf16 matrix product Y[T,N] = X[T,K] . W[N,K]^T for prefill-sized T on the
 // 5th-generation tensor cores: operands staged in shared memory by TMA
-// (cp.async.bulk.tensor, 128-byte swizzle), products issued by one thread with
+// (cp.async.bulk.tensor, 128-byte swizzle), products issued by one lane with
 // tcgen05.mma (128 x 256 x 16 per instruction), fp32 accumulators in tensor
 // memory, read back with tcgen05.ld for the epilogue.
 //
@@ -15,7 +15,7 @@
 //    where the tiles alone would not fill the SMs, and a second kernel adds the shares in a
 //    fixed order.
 // In all of them warp 0 is the TMA producer, warp 1 allocates tensor memory and issues the
-// products, warps 2..5 are the epilogue.  A ring of (first-operand tile 128x64,
+// products (TcIssue), warps 2..5 are the epilogue.  A ring of (first-operand tile 128x64,
 // second-operand tile x64) is handed back and forth with mbarriers: `full` is completed by
 // the TMA's byte count, `empty` by tcgen05.commit when the products that read a stage have
 // retired.
@@ -147,7 +147,7 @@ __device__ __forceinline__ void store_swapped16(const float* v, void* Y, int row
 // product to Y [gridDim.z][T][N]; zlm_gemm_tc adds the shares up in a second kernel.
 // The few-token form as stand-alone blocks: the first operand is W (128 outputs), the second X
 // (a tile of BN tokens); one block per tile and share of K.
-template <int BN, int STAGES, int MODE>
+template <int BN, int STAGES, int MODE, bool WHOLE>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                void* __restrict__ Y, int T, int N, int K, int ldy) {
@@ -220,7 +220,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        using I = TcIssue<WHOLE>;
+        if ((WHOLE || lane == 0)) {
             // instruction descriptor: fp32 accumulate, bf16 x bf16, both K-major, N = BN, M = 128
             const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) |
                                    ((unsigned)(TC_BM >> 4) << 24);
@@ -228,18 +229,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             for (int kb = 0; kb < KB && ok; ++kb) {
                 const int s = kb % STAGES;
                 const unsigned round = kb / STAGES;
-                ok = mbar_wait(&full[s], round & 1, abort_flag, 2);
+                ok = I::wait(&full[s], round & 1, abort_flag, 2);
                 if (!ok) break;
                 tc_fence_after();
                 // one descriptor per stage, advanced by constants (the start address field counts
                 // 16-byte units and does not carry): the issuing thread has no instruction to spare
                 const uint64_t ad = make_desc(smem_u32(sA + s * A_BYTES)), bd = make_desc(smem_u32(sB + s * B_BYTES));
-#pragma unroll
-                for (int k = 0; k < TC_BK / 16; ++k)
-                    tc_mma(tmem_base, ad + ((k * 32) >> 4), bd + ((k * 32) >> 4), idesc, (kb | k) != 0);
-                tc_commit(&empty[s]);          // the stage is free once these products have read it
+                I::mma4(tmem_base, ad, bd, idesc, kb != 0);
+                I::commit(&empty[s]);          // the stage is free once these products have read it
             }
-            tc_commit(acc_full);               // arrives when every product issued so far has retired
+            I::commit(acc_full);               // arrives when every product issued so far has retired
         }
     } else {
         // epilogue: warp w may touch tensor-memory lanes 32 (w % 4) .. + 31; a lane is a row of the tile
@@ -308,7 +307,7 @@ static int tile_group(int bm, int K) {
 }
 
 #define TCP_ACC 256          // tensor-memory columns between the two accumulators (an allocation is a power of two)
-template <int BN, int STAGES, int MODE>
+template <int BN, int STAGES, int MODE, bool WHOLE = false>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                           void* __restrict__ Y, int T, int N, int K, int ldy, int gm) {
@@ -370,7 +369,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        using I = TcIssue<WHOLE>;
+        if ((WHOLE || lane == 0)) {
             const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) |
                                    ((unsigned)(TC_BM >> 4) << 24);
             unsigned it = 0, local = 0;
@@ -378,24 +378,22 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
                 const unsigned buf = local & 1;
                 // the epilogue must have drained this accumulator (two tiles ago)
-                ok = mbar_wait(&acc_empty[buf], ((local >> 1) & 1) ^ 1, abort_flag, 4);
+                ok = I::wait(&acc_empty[buf], ((local >> 1) & 1) ^ 1, abort_flag, 4);
                 if (!ok) break;
                 tc_fence_after();
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     const int s = it % STAGES;
-                    ok = mbar_wait(&full[s], (it / STAGES) & 1, abort_flag, 2);
+                    ok = I::wait(&full[s], (it / STAGES) & 1, abort_flag, 2);
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t ad = make_desc(smem_u32(sA + s * A_BYTES)), bd = make_desc(smem_u32(sB + s * B_BYTES));
-#pragma unroll
-                    for (int k = 0; k < TC_BK / 16; ++k)
-                        tc_mma(tmem_base + buf * TCP_ACC, ad + ((k * 32) >> 4), bd + ((k * 32) >> 4), idesc, (kb | k) != 0);
-                    tc_commit(&empty[s]);
+                    I::mma4(tmem_base + buf * TCP_ACC, ad, bd, idesc, kb != 0);
+                    I::commit(&empty[s]);
                 }
-                tc_commit(&acc_full[buf]);
+                I::commit(&acc_full[buf]);
                 ++local;
             }
-            if (!ok) { tc_commit(&acc_full[0]); tc_commit(&acc_full[1]); }     // let the epilogue out
+            if (!ok) { I::commit(&acc_full[0]); I::commit(&acc_full[1]); }     // let the epilogue out
         }
     } else {
         const int lg = warp & 3;
@@ -620,7 +618,7 @@ __device__ __forceinline__ void qkv_epilogue_rows(const QkvEpilogue& ep, const Q
 // 25,000 (61,037 tokens, 16 + 2 x 8 heads of 128: 772 us); the other modes lose 3 to 5 % with eight.
 #define TCQ_THREADS(MODE) ((MODE) == 5 ? 320 : TC_THREADS)
 #define TCQ_NORM_BYTES 1024          // MODE 5: the norm weights of q and k as fp32, heads of up to 128
-template <int BN, int STAGES, int MODE>
+template <int BN, int STAGES, int MODE, bool WHOLE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCQ_THREADS(MODE), 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_y, void* __restrict__ Y, int T, int N, int K, int ldy, int gm,
@@ -715,7 +713,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        using I = TcIssuePair<WHOLE>;
+        if (rank == 0 && (WHOLE || lane == 0)) {
             // fp32 accumulate, bf16 x bf16, both K-major, N = BN, M = 256 over the two blocks
             const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) |
                                    ((unsigned)(TCQ_BM >> 4) << 24);
@@ -723,23 +722,21 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             bool ok = true;
             for (int tile = pair; tile < tiles && ok; tile += pairs, ++local) {
                 const unsigned buf = local & 1;
-                ok = mbar_wait_pair(&acc_empty[buf], ((local >> 1) & 1) ^ 1, abort_flag, 4);
+                ok = I::wait_pair(&acc_empty[buf], ((local >> 1) & 1) ^ 1, abort_flag, 4);
                 if (!ok) break;
                 tc_fence_after();
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     const int s = it % STAGES;
-                    ok = mbar_wait(&full[s], (it / STAGES) & 1, abort_flag, 2);
+                    ok = I::wait(&full[s], (it / STAGES) & 1, abort_flag, 2);
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t ad = make_desc(smem_u32(sA + s * A_BYTES)), bd = make_desc(smem_u32(sB + s * B_BYTES));
-#pragma unroll
-                    for (int k = 0; k < TC_BK / 16; ++k)
-                        tc_mma_pair(tmem_base + buf * TCP_ACC, ad + ((k * 32) >> 4), bd + ((k * 32) >> 4), idesc, (kb | k) != 0);
-                    tc_commit_pair(&empty[s]);
+                    I::mma4(tmem_base + buf * TCP_ACC, ad, bd, idesc, kb != 0);
+                    I::commit(&empty[s]);
                 }
-                tc_commit_pair(&acc_full[buf]);
+                I::commit(&acc_full[buf]);
             }
-            if (!ok) { tc_commit_pair(&acc_full[0]); tc_commit_pair(&acc_full[1]); }     // let the epilogues out
+            if (!ok) { I::commit(&acc_full[0]); I::commit(&acc_full[1]); }     // let the epilogues out
         }
     } else {
         const int lg = warp & 3;
@@ -875,7 +872,7 @@ __device__ __forceinline__ ExpertTile expert_tile(int tile, int n_tiles, int max
 // scheduler had one warp whose loads, shuffles and stores wait for one another, and the product into fp32 rows ran at the
 // epilogue's pace (84 us; 21 % of the tensor cores' time, 3 of the memory's 6.5 TB/s).
 #define TCE_THREADS 320
-template <int STAGES, int MODE>
+template <int STAGES, int MODE, bool WHOLE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TCE_THREADS, 1)
 gemm_tc_experts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ ExpertMaps map_x, void* __restrict__ Y,
                        int N, int K, int ldy, int max_tiles, const int* __restrict__ tile_expert,
@@ -945,7 +942,8 @@ gemm_tc_experts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        using I = TcIssuePair<WHOLE>;
+        if (rank == 0 && (WHOLE || lane == 0)) {
             unsigned it = 0, local = 0;
             bool ok = true;
             ExpertTile next = ZLM_TILE_AT(pair);
@@ -956,23 +954,21 @@ gemm_tc_experts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                 const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((t.rows + 31) / 32 * 4) << 17) |
                                        ((unsigned)(TCQ_BM >> 4) << 24);
                 const unsigned buf = local & 1;
-                ok = mbar_wait_pair(&acc_empty[buf], ((local >> 1) & 1) ^ 1, abort_flag, 4);
+                ok = I::wait_pair(&acc_empty[buf], ((local >> 1) & 1) ^ 1, abort_flag, 4);
                 if (!ok) break;
                 tc_fence_after();
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     const int s = it % STAGES;
-                    ok = mbar_wait(&full[s], (it / STAGES) & 1, abort_flag, 2);
+                    ok = I::wait(&full[s], (it / STAGES) & 1, abort_flag, 2);
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t ad = make_desc(smem_u32(sA + s * A_BYTES)), bd = make_desc(smem_u32(sB + s * B_BYTES));
-#pragma unroll
-                    for (int k = 0; k < TC_BK / 16; ++k)
-                        tc_mma_pair(tmem_base + buf * TCP_ACC, ad + ((k * 32) >> 4), bd + ((k * 32) >> 4), idesc, (kb | k) != 0);
-                    tc_commit_pair(&empty[s]);
+                    I::mma4(tmem_base + buf * TCP_ACC, ad, bd, idesc, kb != 0);
+                    I::commit(&empty[s]);
                 }
-                tc_commit_pair(&acc_full[buf]);
+                I::commit(&acc_full[buf]);
             }
-            if (!ok) { tc_commit_pair(&acc_full[0]); tc_commit_pair(&acc_full[1]); }     // let the epilogues out
+            if (!ok) { I::commit(&acc_full[0]); I::commit(&acc_full[1]); }     // let the epilogues out
         }
     } else {
         const int lg = warp & 3, turn = (warp - 2) >> 2;
@@ -1057,7 +1053,7 @@ gemm_tc_experts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 // item that finishes a tile last, was built and gave the same bits; under the load of the weight
 // stream its reads of the shares took several times as long as the whole second kernel does.)
 // ---------------------------------------------------------------------------
-template <int BN, int STAGES, int MODE>
+template <int BN, int STAGES, int MODE, bool WHOLE>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                    void* __restrict__ Y, int T, int N, int K, int ldy, int whole, int ks,
@@ -1147,7 +1143,8 @@ gemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        using I = TcIssue<WHOLE>;
+        if ((WHOLE || lane == 0)) {
             const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) |
                                    ((unsigned)(TC_BM >> 4) << 24);
             unsigned it = 0, local = 0;
@@ -1156,23 +1153,21 @@ gemm_tc_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 ZLM_ITEM(item)
                 (void)a0row; (void)b0row; (void)split;
                 const unsigned buf = local & 1;
-                ok = mbar_wait(&acc_empty[buf], ((local >> 1) & 1) ^ 1, abort_flag, 4);
+                ok = I::wait(&acc_empty[buf], ((local >> 1) & 1) ^ 1, abort_flag, 4);
                 if (!ok) break;
                 tc_fence_after();
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     const int s = it % STAGES;
-                    ok = mbar_wait(&full[s], (it / STAGES) & 1, abort_flag, 2);
+                    ok = I::wait(&full[s], (it / STAGES) & 1, abort_flag, 2);
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t ad = make_desc(smem_u32(sA + s * A_BYTES)), bd = make_desc(smem_u32(sB + s * B_BYTES));
-#pragma unroll
-                    for (int k = 0; k < TC_BK / 16; ++k)
-                        tc_mma(tmem_base + buf * ACC, ad + ((k * 32) >> 4), bd + ((k * 32) >> 4), idesc, (kb | k) != 0);
-                    tc_commit(&empty[s]);
+                    I::mma4(tmem_base + buf * ACC, ad, bd, idesc, kb != 0);
+                    I::commit(&empty[s]);
                 }
-                tc_commit(&acc_full[buf]);
+                I::commit(&acc_full[buf]);
             }
-            if (!ok) { tc_commit(&acc_full[0]); tc_commit(&acc_full[1]); }     // let the epilogue out
+            if (!ok) { I::commit(&acc_full[0]); I::commit(&acc_full[1]); }     // let the epilogue out
         }
     } else {
         const int lg = warp & 3;
@@ -1339,9 +1334,9 @@ static int make_map(CUtensorMap* m, const void* ptr, int rows, int K, int ld, in
     return zlm_make_map_2d(m, ptr, rows, K, ld, box_rows, TC_BK);
 }
 
-template <int BN, int STAGES>
-static int launch_tc(void* Y, const void* X, const void* W, int T, int N, int K, int ldx, int ldy, int mode,
-                     int ksplit, float* scratch, cudaStream_t st, bool add_shares = true) {
+template <int BN, int STAGES, bool WHOLE>
+static int launch_tc_as(void* Y, const void* X, const void* W, int T, int N, int K, int ldx, int ldy, int mode,
+                     int ksplit, float* scratch, cudaStream_t st, bool add_shares) {
     CUtensorMap mx, mw;
     int rc = make_map(&mx, X, T, K, ldx, BN);
     if (rc) return rc;
@@ -1354,7 +1349,7 @@ static int launch_tc(void* Y, const void* X, const void* W, int T, int N, int K,
     void* dst = ksplit > 1 ? (void*)scratch : Y;
 #define ZLM_TC_LAUNCH(M)                                                                                   \
     {                                                                                                      \
-        auto kern = gemm_tc_kernel<BN, STAGES, M>;                                                         \
+        auto kern = gemm_tc_kernel<BN, STAGES, M, WHOLE>;                                                  \
         static bool attr_set_dev[64] = {}; bool& attr_set = attr_set_dev[zlm_device_index()];                                                                      \
         if (!attr_set) {                                                                                   \
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
@@ -1377,6 +1372,13 @@ static int launch_tc(void* Y, const void* X, const void* W, int T, int N, int K,
     rc = zlm_check_launch("gemm_tc");
     if (rc || ksplit <= 1 || !add_shares) return rc;
     return launch_reduce(Y, scratch, T, N, ldy, mode, ksplit, 0, st);
+}
+template <int BN, int STAGES>
+static int launch_tc(void* Y, const void* X, const void* W, int T, int N, int K, int ldx, int ldy, int mode, int ksplit, float* scratch,
+                     cudaStream_t st, bool add_shares = true) {
+    const int stages = ((K + TC_BK - 1) / TC_BK + ksplit - 1) / ksplit;
+    return tc_issue_whole(stages, BN) ? launch_tc_as<BN, STAGES, true>(Y, X, W, T, N, K, ldx, ldy, mode, ksplit, scratch, st, add_shares)
+                                      : launch_tc_as<BN, STAGES, false>(Y, X, W, T, N, K, ldx, ldy, mode, ksplit, scratch, st, add_shares);
 }
 
 static int sm_count() {
@@ -1424,9 +1426,9 @@ static int launch_tc_persistent(void* Y, const void* X, const void* W, int T, in
     return zlm_check_launch("gemm_tc_persistent");
 }
 
-template <int BN, int STAGES>
-static int launch_tc_pair(void* Y, const void* X, const void* W, int T, int N, int K, int ldx, int ldy, int mode,
-                          cudaStream_t st, const QkvEpilogue* qkv = nullptr) {
+template <int BN, int STAGES, bool WHOLE>
+static int launch_tc_pair_as(void* Y, const void* X, const void* W, int T, int N, int K, int ldx, int ldy, int mode,
+                          cudaStream_t st, const QkvEpilogue* qkv) {
     const QkvEpilogue ep = qkv ? *qkv : QkvEpilogue{};
     CUtensorMap mx, mw;
     int rc = make_map(&mx, X, T, K, ldx, TC_BM);
@@ -1448,7 +1450,7 @@ static int launch_tc_pair(void* Y, const void* X, const void* W, int T, int N, i
     const int pairs = (int)(tiles < sm_count() / 2 ? tiles : sm_count() / 2);
 #define ZLM_TCQ_LAUNCH(M)                                                                                  \
     {                                                                                                      \
-        auto kern = gemm_tc_pair_kernel<BN, STAGES, M>;                                                    \
+        auto kern = gemm_tc_pair_kernel<BN, STAGES, M, WHOLE>;                                             \
         static bool attr_set_dev[64] = {}; bool& attr_set = attr_set_dev[zlm_device_index()];                                                                      \
         if (!attr_set) {                                                                                   \
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
@@ -1471,6 +1473,14 @@ static int launch_tc_pair(void* Y, const void* X, const void* W, int T, int N, i
     else ZLM_TCQ_LAUNCH(8)
 #undef ZLM_TCQ_LAUNCH
     return zlm_check_launch("gemm_tc_pair");
+}
+template <int BN, int STAGES>
+static int launch_tc_pair(void* Y, const void* X, const void* W, int T, int N, int K, int ldx, int ldy, int mode, cudaStream_t st,
+                          const QkvEpilogue* qkv = nullptr) {
+    // (narrow tiles gain at every K)
+    if (BN < 240 || tc_issue_whole((K + TC_BK - 1) / TC_BK, BN)) return launch_tc_pair_as<BN, STAGES, true>(Y, X, W, T, N, K, ldx, ldy, mode, st, qkv);
+    if constexpr (BN >= 240) return launch_tc_pair_as<BN, STAGES, false>(Y, X, W, T, N, K, ldx, ldy, mode, st, qkv);
+    return ZLM_OK;
 }
 
 // Which many-token form runs, and how wide its tiles are: 0 lets the dispatcher choose (pairs of
@@ -1506,8 +1516,8 @@ static FewPlan few_plan(int T, int N, int K) {
     return p;
 }
 
-template <int BN, int STAGES>
-static int launch_tc_few(void* Y, const void* X, const void* W, int T, int N, int K, int ldx, int ldy, int mode,
+template <int BN, int STAGES, bool WHOLE>
+static int launch_tc_few_as(void* Y, const void* X, const void* W, int T, int N, int K, int ldx, int ldy, int mode,
                          const FewPlan& plan, float* scratch, cudaStream_t st) {
     CUtensorMap mx, mw;
     int rc = make_map(&mx, X, T, K, ldx, BN);
@@ -1520,7 +1530,7 @@ static int launch_tc_few(void* Y, const void* X, const void* W, int T, int N, in
     const int blocks = (int)(items < sm_count() ? items : sm_count());
 #define ZLM_TCF_LAUNCH(M)                                                                                  \
     {                                                                                                      \
-        auto kern = gemm_tc_few_kernel<BN, STAGES, M>;                                                     \
+        auto kern = gemm_tc_few_kernel<BN, STAGES, M, WHOLE>;                                              \
         static bool attr_set_dev[64] = {}; bool& attr_set = attr_set_dev[zlm_device_index()];                                                                      \
         if (!attr_set) {                                                                                   \
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
@@ -1543,24 +1553,17 @@ static int launch_tc_few(void* Y, const void* X, const void* W, int T, int N, in
     if (rc || plan.ks <= 1) return rc;
     return launch_reduce(Y, scratch, T, N, ldy, mode, plan.ks, plan.whole / plan.t_tiles * TC_BM, st);
 }
+template <int BN, int STAGES>
+static int launch_tc_few(void* Y, const void* X, const void* W, int T, int N, int K, int ldx, int ldy, int mode, const FewPlan& plan,
+                         float* scratch, cudaStream_t st) {
+    // (143 tokens x 4,096 at K = 1,024: 0.1 us slower with it)
+    return K > 24 * TC_BK ? launch_tc_few_as<BN, STAGES, true>(Y, X, W, T, N, K, ldx, ldy, mode, plan, scratch, st)
+                          : launch_tc_few_as<BN, STAGES, false>(Y, X, W, T, N, K, ldx, ldy, mode, plan, scratch, st);
+}
 
-// The products of routed experts.  X [rows, K]: the (token, choice) rows sorted by expert; tile tt of the table holds
-// rows tile_row0[tt] .. + tile_rows[tt] (at most 256) of expert tile_expert[tt] (-1: the table ends), which multiply that
-// expert's matrix, rows [e * N, e * N + N) of W [experts * N, K]; Y [rows, ldy].
-// mode 2: Y fp32; mode 6: Y bf16 = relu(.)^2; mode 3: Y bf16 [.., N / 2] = silu(gate) * up, an expert's rows in sixteens
-// of 8 gate rows and the 8 matching up rows; mode 8: the same with the clamped activation, whose constants
-// zlm_set_gate_gemm_tcgen05 has set before.
-extern "C" int zlm_gemm_tc_experts(void* Y, const void* X, const void* W, const int* table, int max_tiles, int rows,
-                                   int experts, int N, int K, int ldy, int mode, cudaStream_t st) {
-    if (max_tiles == 0 || rows == 0 || N == 0) return ZLM_OK;
-    ZLM_REQUIRE(max_tiles > 0 && rows > 0 && experts > 0 && N >= 8 && K >= 8 && K % 8 == 0 && N % 2 == 0,
-                "gemm_tc_experts: tiles=%d rows=%d experts=%d N=%d K=%d", max_tiles, rows, experts, N, K);
-    ZLM_REQUIRE((long long)experts * N < (1ll << 31), "gemm_tc_experts: %d experts of %d rows", experts, N);
-    ZLM_REQUIRE(((uintptr_t)X % 16 == 0) && ((uintptr_t)W % 16 == 0) && table && (uintptr_t)Y % 4 == 0,
-                "gemm_tc_experts: operands must be 16-byte aligned");
-    ZLM_REQUIRE(mode == 2 || mode == 3 || mode == 6 || mode == 8, "gemm_tc_experts: mode %d", mode);
-    ZLM_REQUIRE(!ZLM_GATED(mode) || N % 16 == 0, "gemm_tc_experts: gated rows come in groups of 16, N=%d", N);
-    ZLM_REQUIRE(mode != 6 || ldy % 2 == 0, "gemm_tc_experts: rows of %d outputs", ldy);
+template <bool WHOLE>
+static int launch_tc_experts(void* Y, const void* X, const void* W, const int* table, int max_tiles, int rows, int experts, int N, int K,
+                             int ldy, int mode, cudaStream_t st) {
     constexpr int STAGES = 6;
     CUtensorMap mw;
     ExpertMaps mx;
@@ -1576,7 +1579,7 @@ extern "C" int zlm_gemm_tc_experts(void* Y, const void* X, const void* W, const 
     const int pairs = (int)(tiles < sm_count() / 2 ? tiles : sm_count() / 2);
 #define ZLM_TCE_LAUNCH(M)                                                                                  \
     {                                                                                                      \
-        auto kern = gemm_tc_experts_kernel<STAGES, M>;                                                     \
+        auto kern = gemm_tc_experts_kernel<STAGES, M, WHOLE>;                                              \
         static bool attr_set_dev[64] = {}; bool& attr_set = attr_set_dev[zlm_device_index()];              \
         if (!attr_set) {                                                                                   \
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
@@ -1595,6 +1598,28 @@ extern "C" int zlm_gemm_tc_experts(void* Y, const void* X, const void* W, const 
     else ZLM_TCE_LAUNCH(6)
 #undef ZLM_TCE_LAUNCH
     return zlm_check_launch("gemm_tc_experts");
+}
+
+// The products of routed experts.  X [rows, K]: the (token, choice) rows sorted by expert; tile tt of the table holds
+// rows tile_row0[tt] .. + tile_rows[tt] (at most 256) of expert tile_expert[tt] (-1: the table ends), which multiply that
+// expert's matrix, rows [e * N, e * N + N) of W [experts * N, K]; Y [rows, ldy].
+// mode 2: Y fp32; mode 6: Y bf16 = relu(.)^2; mode 3: Y bf16 [.., N / 2] = silu(gate) * up, an expert's rows in sixteens
+// of 8 gate rows and the 8 matching up rows; mode 8: the same with the clamped activation, whose constants
+// zlm_set_gate_gemm_tcgen05 has set before.
+extern "C" int zlm_gemm_tc_experts(void* Y, const void* X, const void* W, const int* table, int max_tiles, int rows,
+                                   int experts, int N, int K, int ldy, int mode, cudaStream_t st) {
+    if (max_tiles == 0 || rows == 0 || N == 0) return ZLM_OK;
+    ZLM_REQUIRE(max_tiles > 0 && rows > 0 && experts > 0 && N >= 8 && K >= 8 && K % 8 == 0 && N % 2 == 0,
+                "gemm_tc_experts: tiles=%d rows=%d experts=%d N=%d K=%d", max_tiles, rows, experts, N, K);
+    ZLM_REQUIRE((long long)experts * N < (1ll << 31), "gemm_tc_experts: %d experts of %d rows", experts, N);
+    ZLM_REQUIRE(((uintptr_t)X % 16 == 0) && ((uintptr_t)W % 16 == 0) && table && (uintptr_t)Y % 4 == 0,
+                "gemm_tc_experts: operands must be 16-byte aligned");
+    ZLM_REQUIRE(mode == 2 || mode == 3 || mode == 6 || mode == 8, "gemm_tc_experts: mode %d", mode);
+    ZLM_REQUIRE(!ZLM_GATED(mode) || N % 16 == 0, "gemm_tc_experts: gated rows come in groups of 16, N=%d", N);
+    ZLM_REQUIRE(mode != 6 || ldy % 2 == 0, "gemm_tc_experts: rows of %d outputs", ldy);
+    // (a table of 60 experts of which two bring 1,700 rows and more, K = 2,048: 100.9 us a thread, 97.3 a warp; K = 768 no difference)
+    return K >= 24 * TC_BK ? launch_tc_experts<true>(Y, X, W, table, max_tiles, rows, experts, N, K, ldy, mode, st)
+                           : launch_tc_experts<false>(Y, X, W, table, max_tiles, rows, experts, N, K, ldy, mode, st);
 }
 
 // 1 if the tensor-memory kernel takes this product (else use zlm_gemm_bf16_mma)

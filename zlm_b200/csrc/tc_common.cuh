@@ -74,15 +74,42 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tc_mma(unsigned tmem_d, uint64_t desc_a, uint64_t desc_b, unsigned idesc, unsigned accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
+// The issuing side of a product kernel, for the whole warp (one elected lane issues) or for one thread of it.  mma4: the four
+// products of a stage (64 of K, 32 bytes on in both operands each) from one block of instructions; commit: an arrival at
+// `bar` once what this issuer has issued has retired; wait: a bounded wait.  A product issued from a thread in a branch of its
+// own takes it about 108 cycles, from an elected lane of a whole warp 50 to 65: less than 256 x 128 x 16 takes the tensor cores,
+// where the thread is what bounds the kernel.  But a kernel built with it is 0.2 to 0.3 us slower to get going (measured; not
+// explained), so that it pays from some stages on (tc_issue_whole): built as kernels of their own.
+#define TC_MMA4(GROUP, LEADER)                                                                                          \
+    asm volatile("{\n\t.reg .pred q, p0, p1;\n\t.reg .b64 da, db;\n\t" LEADER                                         \
+                 "setp.ne.b32 p0, %4, 0;\n\tsetp.eq.b32 p1, 0, 0;\n\t"                                                  \
+                 "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], %1, %2, %3, p0;\n\t"                              \
+                 "add.u64 da, %1, 2;\n\tadd.u64 db, %2, 2;\n\t@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], da, db, %3, p1;\n\t" \
+                 "add.u64 da, %1, 4;\n\tadd.u64 db, %2, 4;\n\t@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], da, db, %3, p1;\n\t" \
+                 "add.u64 da, %1, 6;\n\tadd.u64 db, %2, 6;\n\t@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], da, db, %3, p1;\n\t" \
+                 "}\n" ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory")
+#define TC_COMMIT(FORM, LEADER, ...)                                                                                    \
+    asm volatile("{\n\t.reg .pred q;\n\t" LEADER "@q tcgen05.commit." FORM ";\n\t}\n" ::"r"(smem_u32(bar)), ##__VA_ARGS__ : "memory")
+#define TC_ELECT "elect.sync _|q, 0xffffffff;\n\t"
+#define TC_THIS "setp.eq.b32 q, 0, 0;\n\t"
+template <bool WHOLE> struct TcIssue {
+    static __device__ __forceinline__ void mma4(unsigned tmem_d, uint64_t desc_a, uint64_t desc_b, unsigned idesc, unsigned accumulate) {
+        if (WHOLE) TC_MMA4("1", TC_ELECT);
+        else TC_MMA4("1", TC_THIS);
+    }
+    static __device__ __forceinline__ void commit(uint64_t* bar) {
+        if (WHOLE) TC_COMMIT("cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0]", TC_ELECT);
+        else TC_COMMIT("cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0]", TC_THIS);
+    }
+    static __device__ __forceinline__ bool wait(uint64_t* bar, unsigned parity, volatile int* abort_flag, int where) {
+        return WHOLE ? mbar_wait_warp(bar, parity, abort_flag, where) : mbar_wait(bar, parity, abort_flag, where);
+    }
+};
+// Single thread / whole warp, us: 128 tokens x 1,024 x 1,024 (8 stages a block) 11.1 / 11.4; 384 x 6,144 x 4,096 (32 stages) 27.2 /
+// 22.9; pairs, 512 x 1,024 x 1,024 in tiles of 128 columns 11.4 / 10.8, 1,024 x 2,048 x 2,048 17.4 / 15.9; in tiles of 224, 2,999 x
+// 5,120 x 2,048 48.0 / 45.9; of 240 and 256, 2,048 x 2,048 x 1,024 13.4 / 13.9, 2,048 x 2,048 x 2,048 19.0 / 19.5, 2,048 x 4,096 x
+// 4,096 52.2 / 51.2.
+static inline bool tc_issue_whole(int stages, int width) { return stages >= (width < 240 ? 12 : 48); }
 // 16 columns of this thread's lane, without the wait: several loads can be in flight, then tc_wait_ld()
 __device__ __forceinline__ void tc_ld16_nowait(unsigned taddr, float* v) {
     unsigned* r = (unsigned*)v;
@@ -169,17 +196,6 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
         ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(bar_rank0) : "memory");
 }
-__device__ __forceinline__ void tc_mma_pair(unsigned tmem_d, uint64_t desc_a, uint64_t desc_b, unsigned idesc, unsigned accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
-// arrives, once the products issued so far have retired, at the mbarrier at this place in both blocks
-__device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
-                 ::"r"(smem_u32(bar)), "h"((unsigned short)3) : "memory");
-}
 __device__ __forceinline__ void mbar_arrive_at(unsigned cluster_address) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_address) : "memory");
 }
@@ -203,6 +219,28 @@ __device__ __forceinline__ bool mbar_wait_pair(uint64_t* bar, unsigned parity, v
     zlm_report_status((TC_FAMILY << 8) | where);
     return false;
 }
+
+// TcIssue for a pair; the arrival goes to the mbarrier at this place in both blocks
+template <bool WHOLE> struct TcIssuePair {
+    static __device__ __forceinline__ void mma4(unsigned tmem_d, uint64_t desc_a, uint64_t desc_b, unsigned idesc, unsigned accumulate) {
+        if (WHOLE) TC_MMA4("2", TC_ELECT);
+        else TC_MMA4("2", TC_THIS);
+    }
+    static __device__ __forceinline__ void commit(uint64_t* bar) {
+        if (WHOLE) TC_COMMIT("cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1", TC_ELECT, "h"((unsigned short)3));
+        else TC_COMMIT("cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1", TC_THIS, "h"((unsigned short)3));
+    }
+    static __device__ __forceinline__ bool wait(uint64_t* bar, unsigned parity, volatile int* abort_flag, int where) {
+        return TcIssue<WHOLE>::wait(bar, parity, abort_flag, where);
+    }
+    // on a barrier at which the other block arrives too
+    static __device__ __forceinline__ bool wait_pair(uint64_t* bar, unsigned parity, volatile int* abort_flag, int where) {
+        if (!WHOLE) return mbar_wait_pair(bar, parity, abort_flag, where);
+        int ok = 0;
+        if ((threadIdx.x & 31) == 0) ok = mbar_wait_pair(bar, parity, abort_flag, where) ? 1 : 0;
+        return __shfl_sync(0xffffffffu, ok, 0) != 0;
+    }
+};
 
 typedef CUresult (*ZlmEncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                      const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
