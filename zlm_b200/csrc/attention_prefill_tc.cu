@@ -409,6 +409,14 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             if (inner) {
 #pragma unroll
                 for (int e = 0; e < FA_BK; ++e) mx4[e & 3] = fmaxf(mx4[e & 3], sv[e]);
+            } else if (!KEEP && kb0 >= last_lo) {
+                // the last keys only: one comparison with a constant a score (three for the general mask below)
+                const int last = row_ok ? pos - kb0 : -1;
+#pragma unroll
+                for (int e = 0; e < FA_BK; ++e) {
+                    sv[e] = e <= last ? sv[e] : -INFINITY;
+                    mx4[e & 3] = fmaxf(mx4[e & 3], sv[e]);
+                }
             } else {
 #pragma unroll
                 for (int e = 0; e < FA_BK; ++e) {
@@ -471,26 +479,34 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         if (ok && NS > 0) ok = mbar_wait_warp(&pv_done[hh], (NS - 1) & 1, abort_flag, 8);
         tc_fence_after();
         if (ok && !*abort_flag) {
+            // The warp's rows go out through its own rows of P, which nothing reads any more, in P's layout: eight lanes store 128
+            // bytes of one row.  (A thread that stored its own row touched 32 rows and half a sector of each per instruction.)
             const float inv = row_ok ? 1.0f / l : 0.f;
-            __nv_bfloat16* orow = out + (size_t)(tok0 + row0 + i) * out_stride + (size_t)head * KD;
-#pragma unroll 1
+#pragma unroll 2
             for (int c = 0; c < FA_HD; c += 16) {
                 float ov[16];
                 tc_ld16(tmem_o + lane_addr + c, ov);
-                if (row_ok && ZLM_CHK(orow + c, 32)) {
-                    uint4 a, bq;
-                    a.x = fa_pack(ov[0] * inv, ov[1] * inv); a.y = fa_pack(ov[2] * inv, ov[3] * inv);
-                    a.z = fa_pack(ov[4] * inv, ov[5] * inv); a.w = fa_pack(ov[6] * inv, ov[7] * inv);
-                    bq.x = fa_pack(ov[8] * inv, ov[9] * inv); bq.y = fa_pack(ov[10] * inv, ov[11] * inv);
-                    bq.z = fa_pack(ov[12] * inv, ov[13] * inv); bq.w = fa_pack(ov[14] * inv, ov[15] * inv);
-                    *(uint4*)(orow + c) = a;
-                    *(uint4*)(orow + c + 8) = bq;
-                }
-            }
-            // (out's rows are as wide as the keys: the columns beyond the values become zeros)
-            if (KD > FA_HD && row_ok && ZLM_CHK(orow + FA_HD, (KD - FA_HD) * 2)) {
 #pragma unroll
-                for (int c = FA_HD; c < KD; c += 8) *(uint4*)(orow + c) = make_uint4(0u, 0u, 0u, 0u);
+                for (int e = 0; e < 16; ++e) ov[e] *= inv;
+                unsigned char* const row = sP_h + (c >> 6) * (P_BYTES / 2) + i * 128;
+                const int ch = (c >> 3) & 7;
+                *(uint4*)(row + ((ch ^ (i & 7)) << 4)) = make_uint4(fa_pack(ov[0], ov[1]), fa_pack(ov[2], ov[3]), fa_pack(ov[4], ov[5]), fa_pack(ov[6], ov[7]));
+                *(uint4*)(row + (((ch + 1) ^ (i & 7)) << 4)) = make_uint4(fa_pack(ov[8], ov[9]), fa_pack(ov[10], ov[11]), fa_pack(ov[12], ov[13]), fa_pack(ov[14], ov[15]));
+            }
+            __syncwarp();
+            const int piece = lane & 7;
+#pragma unroll
+            for (int it = 0; it < 8; ++it) {
+                const int r = lg * 32 + it * 4 + (lane >> 3);
+                if (r >= rows) continue;
+                __nv_bfloat16* const orow = out + (size_t)(tok0 + row0 + r) * out_stride + (size_t)head * KD + piece * 8;
+                const unsigned char* const row = sP_h + r * 128 + ((piece ^ (r & 7)) << 4);
+                if (ZLM_CHK(orow, 16)) *(uint4*)orow = *(const uint4*)row;
+                if (ZLM_CHK(orow + 64, 16)) *(uint4*)(orow + 64) = *(const uint4*)(row + P_BYTES / 2);
+                // (out's rows are as wide as the keys: the columns beyond the values become zeros)
+#pragma unroll
+                for (int c = FA_HD; c < KD; c += 64)
+                    if (ZLM_CHK(orow + c, 16)) *(uint4*)(orow + c) = make_uint4(0u, 0u, 0u, 0u);
             }
         }
     }
