@@ -41,7 +41,7 @@ def test_recurrences_over_prompts_and_32_bit_kernels_stay_inside_their_tensors()
 
 def test_sorted_experts_and_decode_attention_stay_inside_their_tensors():
     rc, out = _run(["-m", "pytest", "-x", "-q", "--zlm-bounds-check", "-m", "gpu", "-p", "no:cacheprovider",
-                    "tests/test_expert_products_gpu.py", "tests/test_decode_attention_rows_gpu.py", "tests/test_issue_forms_gpu.py"])
+                    "tests/test_expert_products_gpu.py", "tests/test_decode_attention_rows_gpu.py", "tests/test_issue_forms_gpu.py", "tests/test_gate_rows_gpu.py"])
     assert rc == 0, out
     assert " passed" in out and "failed" not in out, out
 
