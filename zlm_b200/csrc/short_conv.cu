@@ -144,12 +144,17 @@ conv_norm_write_run_kernel(TA* __restrict__ q_out, int q_out_stride, const TA* _
     const int kind = unit < nq ? 0 : (unit < nq + nkv ? 1 : 2);
     const int width = kind == 2 ? vdim : dim, e = lane * 4;
     const int c = (kind == 0 ? unit * dim : (kind == 1 ? nq * dim + (unit - nq) * dim : (nq + nkv) * dim + (unit - nq - nkv) * vdim)) + e;
+    // (four channels' taps stand next to each other: four numbers a read instead of 4 TAPS reads of one)
     float w[4][TAPS];
 #pragma unroll
-    for (int v = 0; v < 4; ++v)
+    for (int x = 0; x < TAPS; ++x) {
+        Raw r;
+        memset(&r, 0, sizeof(r));
+        const TA* p = conv_w + (size_t)c * TAPS + 4 * x;
+        if (e < width && ZLM_CHK(p, sizeof(Raw))) r = *(const Raw*)p;
 #pragma unroll
-        for (int j = 0; j < TAPS; ++j)
-            w[v][j] = (e < width && ZLM_CHK(conv_w + (size_t)(c + v) * TAPS + j, sizeof(TA))) ? to_f32(conv_w[(size_t)(c + v) * TAPS + j]) : 0.f;
+        for (int v = 0; v < 4; ++v) w[(4 * x + v) / TAPS][(4 * x + v) % TAPS] = to_f32(r.v[v]);
+    }
     // the run's tokens, one a lane (the step's integers do not wait for the kernel before): read token by token inside the loop,
     // two trips to memory stood before every store
     const int tl = t0 + (lane & (SC_RUN - 1));
@@ -269,7 +274,7 @@ static void launch_conv(void* q_out, int q_out_stride, const void* proj, int pro
     const bool vec = dim % 4 == 0 && vdim % 4 == 0 && hdp % 4 == 0 && proj_stride % 4 == 0 && q_out_stride % 4 == 0 && C0 % 4 == 0 &&
                      (uintptr_t)proj % al == 0 && (uintptr_t)q_out % al == 0 && (uintptr_t)pool % al == 0 &&
                      (state == nullptr || (uintptr_t)state % al == 0);
-    if (vec && zlm_conv_runs(T, R, units, hdp, taps)) {
+    if (vec && (uintptr_t)conv_w % al == 0 && zlm_conv_runs(T, R, units, hdp, taps)) {
         const dim3 grid((T + SC_RUN - 1) / SC_RUN, (units + SC_WARPS - 1) / SC_WARPS);
 #define ZLM_SC(N)                                                                                                               \
     case N:                                                                                                                     \
