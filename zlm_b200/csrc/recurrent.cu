@@ -475,13 +475,32 @@ rglru_conv_blocks_kernel(__nv_bfloat16* __restrict__ u16, int* __restrict__ tabl
     const int c = (blockIdx.y * 128 + threadIdx.x) * 8, t0 = blockIdx.x * RC_RUN;
     float w[8][TAPS], b[8], bias[8];
     if (c < W) {
+        // (eight channels' taps and biases stand next to each other: eight numbers a read where they start at 16 bytes)
+        if (((uintptr_t)conv_w | (uintptr_t)bx | (uintptr_t)cb) % 16 == 0) {
+            auto read8 = [](const __nv_bfloat16* p, float* f) {
+                const uint4 u = p && ZLM_CHK(p, 16) ? *(const uint4*)p : make_uint4(0, 0, 0, 0);
+                const unsigned x[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-        for (int v = 0; v < 8; ++v) {
-            b[v] = bx && ZLM_CHK(bx + c + v, 2) ? to_f32(bx[c + v]) : 0.f;
-            bias[v] = cb && ZLM_CHK(cb + c + v, 2) ? to_f32(cb[c + v]) : 0.f;
+                for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(i & 1 ? x[i / 2] & 0xffff0000u : x[i / 2] << 16);
+            };
+            read8(bx ? bx + c : nullptr, b);
+            read8(cb ? cb + c : nullptr, bias);
 #pragma unroll
-            for (int j = 0; j < TAPS; ++j)
-                w[v][j] = ZLM_CHK(conv_w + (size_t)(c + v) * TAPS + j, 2) ? to_f32(conv_w[(size_t)(c + v) * TAPS + j]) : 0.f;
+            for (int x = 0; x < TAPS; ++x) {
+                float f[8];
+                read8(conv_w + (size_t)c * TAPS + 8 * x, f);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) w[(8 * x + i) / TAPS][(8 * x + i) % TAPS] = f[i];
+            }
+        } else {
+#pragma unroll
+            for (int v = 0; v < 8; ++v) {
+                b[v] = bx && ZLM_CHK(bx + c + v, 2) ? to_f32(bx[c + v]) : 0.f;
+                bias[v] = cb && ZLM_CHK(cb + c + v, 2) ? to_f32(cb[c + v]) : 0.f;
+#pragma unroll
+                for (int j = 0; j < TAPS; ++j)
+                    w[v][j] = ZLM_CHK(conv_w + (size_t)(c + v) * TAPS + j, 2) ? to_f32(conv_w[(size_t)(c + v) * TAPS + j]) : 0.f;
+            }
         }
     }
     pdl_wait();
