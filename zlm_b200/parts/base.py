@@ -95,30 +95,33 @@ class Workspace:
     def __init__(self, device):
         self.device = device
         self._bufs: Dict[Tuple[str, torch.dtype], torch.Tensor] = {}
-        self._views: Dict[Any, torch.Tensor] = {}      # (a view costs the host as much as a launch's arguments: kept by name and shape)
+        self._views: Dict[Any, torch.Tensor] = {}      # by name, type and shape; never handed out themselves
         self.generation = 0
 
     def get(self, name: str, shape: Sequence[int], dtype: torch.dtype) -> torch.Tensor:
+        """The buffer's first numbers as a tensor of that shape.  The memory is shared with every other tensor of the name and
+        type, the tensor object is the caller's own: what it does to the object (``squeeze_``, ``requires_grad_``) nobody else
+        sees.  (Cut and shaped anew, a view costs the host 2.8 to 5 us, as much as a launch's arguments; as an alias of one that
+        is kept, 0.6.)"""
         shape = tuple(shape)
         view = self._views.get((name, dtype, shape))
-        if view is not None:
-            return view
-        n = 1
-        for s in shape:
-            n *= int(s)
-        key = (name, dtype)
-        buf = self._bufs.get(key)
-        if buf is None or buf.numel() < n:
-            if buf is not None and buf.is_cuda and not torch.cuda.is_current_stream_capturing():
-                torch.cuda.synchronize(buf.device)      # (kernels of another stream may still be at the old memory)
-            buf = torch.empty(max(n, 1), dtype=dtype, device=self.device)
-            self._bufs[key] = buf
-            self._views.clear()
-            self.generation += 1
-        if len(self._views) >= 1024:                    # (steps of ever new sizes)
-            self._views.clear()
-        view = self._views[(name, dtype, shape)] = buf[:n].view(*shape)
-        return view
+        if view is None:
+            n = 1
+            for s in shape:
+                n *= int(s)
+            key = (name, dtype)
+            buf = self._bufs.get(key)
+            if buf is None or buf.numel() < n:
+                if buf is not None and buf.is_cuda and not torch.cuda.is_current_stream_capturing():
+                    torch.cuda.synchronize(buf.device)      # (kernels of another stream may still be at the old memory)
+                buf = torch.empty(max(n, 1), dtype=dtype, device=self.device)
+                self._bufs[key] = buf
+                self._views.clear()
+                self.generation += 1
+            if len(self._views) >= 1024:                    # (steps of ever new sizes)
+                self._views.clear()
+            view = self._views[(name, dtype, shape)] = buf[:n].view(*shape)
+        return view.detach()
 
 
 class Runtime:
