@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import operator
 from ctypes import c_float, c_int, c_void_p
 from typing import Optional
 
@@ -140,6 +141,13 @@ def _dt(t: torch.Tensor) -> int:
         return _DT[t.dtype]
     except KeyError:
         raise KernelError(f"unsupported dtype {t.dtype}") from None
+
+
+def _whole(*numbers) -> None:
+    """Refuses what is no whole number.  (An entry point takes None for 0, which is right for an address and not for a column, a
+    window or a number of sequences.)"""
+    for n in numbers:
+        operator.index(n)
 
 
 def _span_bytes(t: torch.Tensor) -> int:
@@ -656,6 +664,7 @@ class CudaKernels:
 
     def qkv_rope_supported(self, x: torch.Tensor, w: torch.Tensor, nq: int, nkv: int, hd: int, n_rot: int) -> bool:
         """Whether ``linear_qkv_rope`` takes this step: bf16, many tokens, heads that divide a tile."""
+        _whole(nq, nkv, hd, n_rot)
         if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
             return False
         return bool(self._ask("zlm_gemm_tc_qkv_supported", x.shape[0], w.shape[0], w.shape[1],
@@ -743,6 +752,7 @@ class CudaKernels:
         value heads] of [PAGE_TOKENS, hd] each (with 1, the ordinary [2, nkv, PAGE_TOKENS, hd]).  ``keep``: with a
         window, the sequence's first ``keep`` keys stay visible beside it.  ``bias``: ``pad_bias`` of numbers b [nq, n] that
         are added to the scores after scale and cap, b[h, min(distance, n - 1)]."""
+        _whole(window)
         T = q.shape[0]
         bias_n = 0
         if bias is not None:
@@ -781,6 +791,7 @@ class CudaKernels:
         if (plan is not None and not plan.is_decode and q.dtype == torch.bfloat16
                 and getattr(plan, "cu_seqlens", None) is not None
                 and self._ask("zlm_attention_prefill_supported", nq, nkv, hd)):
+            _whole(plan.R, plan.max_new)
             impl = getattr(plan, "attention_impl", None)
             if (impl != "mma" and not (keep and bias is not None)
                     and self._ask("zlm_attention_prefill_tc_supported", nq, nkv, hd, q.stride(0), out.stride(0))):
@@ -848,6 +859,7 @@ class CudaKernels:
         step's first token come from ``state`` [slots, taps-1, channels], which is brought up to date afterwards), then
         q and k heads divided by their root mean square over ``dim`` (``norm``); q goes to ``q_out`` [T, nq*hdp], k and v
         to the token's place in the paged ``pool`` [pages, 2, nkv, PAGE_TOKENS, hdp], heads padded with zeros to hdp."""
+        _whole(plan.R)
         T = proj.shape[0]
         hdp = pool.shape[-1]
         C = (nq + nkv) * dim + nkv * vdim
@@ -892,6 +904,7 @@ class CudaKernels:
         steps.  Long prompts run in pieces side by side (``pieces`` forces or forbids that).  ``cos_sin``: the step's
         rotation table [2, n_rot/2, T] (``rope_table``) where a step computes it once for all layers; without it the
         kernel forms cosines and sines itself."""
+        _whole(q_off, k_off, v_off, plan.R)
         T = proj.shape[0]
         assert o.shape == (T, heads * v_dim) and o.dtype == torch.float32 and o.is_contiguous() and proj.stride(1) == 1
         assert state.dtype == torch.float32 and tuple(state.shape[1:]) == (heads, dim, v_dim) and state.is_contiguous()
@@ -953,6 +966,7 @@ class CudaKernels:
         ``rot_scale`` (``interleaved``: 2i against 2i + 1).  ``q_temp`` (coef, every): q is multiplied by
         1 + coef * ln(floor((pos + 1) / every) + 1).  ``v_first`` [T, nkv*vdim]: v becomes (1 - v_lambda) v + v_lambda
         v_first.  ``v_keep`` [T, nkv*vdim] receives v as it was before that."""
+        _whole(plan.R)
         T = proj.shape[0]
         hdp = pool.shape[-1]
         C = (nq + nkv) * dim + nkv * vdim
@@ -1026,6 +1040,7 @@ class CudaKernels:
         ``gates`` [blocks, 2*width/blocks, width/blocks] (the rows of a_r[b], then of a_i[b]): bfloat16 steps of more than 16
         tokens compute the gates' logits block by block as products of the library with fp32 sums and fp32 output.  Long
         prompts run in pieces side by side (``pieces`` forces or forbids that)."""
+        _whole(plan.R)
         T = proj.shape[0]
         W = width
         dt = proj.dtype
@@ -1107,6 +1122,7 @@ class CudaKernels:
         and sigmoid(u) elsewhere; zp, xp and g are the W columns of ``proj`` from z_off, x_off and g_off on, ``state``
         [slots, W] fp32.  Long prompts run on clusters of blocks that share a sequence's tokens
         (``cluster`` forces or forbids that)."""
+        _whole(z_off, x_off, g_off, plan.R)
         T = proj.shape[0]
         W = state.shape[1]
         assert out.shape == (T, W) and out.dtype == proj.dtype and out.stride(1) == 1 and proj.stride(1) == 1
@@ -1126,6 +1142,7 @@ class CudaKernels:
                    state, plan, heads: int, dim: int, v_dim: int, q_scale: float, w_norm: torch.Tensor, eps: float) -> None:
         """One token of a matrix memory (see ``mlstm``) for every sequence of a decode step, with what follows it:
         out [T, heads*v_dim] = o / rms(o, per head) * w_norm * sigmoid(g), g the columns of ``proj`` from g_off on."""
+        _whole(q_off, k_off, v_off, g_off, i_off, f_off, dim)
         T, N = out.shape
         S, n, m = self._check_mlstm(proj, z, b_i, b_f, state, heads, dim, v_dim)
         assert plan.is_decode and plan.R == T and N == heads * v_dim and out.stride(1) == 1
@@ -1146,6 +1163,7 @@ class CudaKernels:
         o = S_t^T q / (max(|n_t . q|, exp(-m_t)) + 1e-6).  q (times ``q_scale``), k, v are columns of ``proj`` from q_off,
         k_off, v_off on; zi and zf columns i_off + h and f_off + h of ``z`` (fp32); ``state`` (S [slots, heads, dim, v_dim],
         n [slots, heads, dim], m [slots, heads]), all fp32.  A sequence's tokens run in pieces side by side."""
+        _whole(q_off, k_off, v_off, i_off, f_off, dim, plan.R)
         T = proj.shape[0]
         S, n, m = self._check_mlstm(proj, z, b_i, b_f, state, heads, dim, v_dim)
         assert o.shape == (T, heads * v_dim) and o.dtype == torch.float32 and o.is_contiguous()
@@ -1192,6 +1210,7 @@ class CudaKernels:
     def lowrank_decay(self, alpha: torch.Tensor, proj: torch.Tensor, lo_off: int, w2: torch.Tensor, b: Optional[torch.Tensor],
                       tau: float) -> None:
         """alpha [T, C] fp32 = sigmoid(w2 lo + b)^(1/tau), lo = ``rank`` columns of proj from lo_off on, w2 [C, rank]."""
+        _whole(lo_off)
         T = proj.shape[0]
         C, rank = w2.shape
         assert alpha.shape == (T, C) and alpha.dtype == torch.float32 and alpha.is_contiguous() and proj.stride(1) == 1
@@ -1208,6 +1227,7 @@ class CudaKernels:
         key channel, or ``head_decay`` [heads] fp32 one per head; ``state`` [slots, heads, dim, v_dim] fp32.  Long prompts
         run in pieces of 32 tokens side by side: every piece from a zero state, the pieces' states chained, and a
         product that adds what the state before a piece gives its tokens (``pieces`` forces or forbids that)."""
+        _whole(q_off, k_off, v_off, plan.R)
         T = proj.shape[0]
         assert o.shape == (T, heads * v_dim) and o.dtype == torch.float32 and o.is_contiguous() and proj.stride(1) == 1
         assert state.dtype == torch.float32 and tuple(state.shape[1:]) == (heads, dim, v_dim) and state.is_contiguous()
@@ -1359,6 +1379,7 @@ class CudaKernels:
         """Per-head keys and values of the step's tokens into a pool of the attention kernels' layout
         [pages, 2, heads, PAGE_TOKENS, dim + rot_dim]: K = [kv[t, h*dim : (h+1)*dim] | rec[t, kv_rank:]],
         V = [kv[t, heads*dim + h*v_dim : ...] | 0]; ``stable`` [sequences of the step, pages] names the pages."""
+        _whole(kv_rank)
         T = kv.shape[0]
         hd = dim + rot_dim
         assert kv.shape == (T, heads * (dim + v_dim)) and kv.stride(1) == 1 and rec.shape[0] == T and rec.stride(1) == 1
@@ -1399,6 +1420,7 @@ class CudaKernels:
         Both kernels have both options.
         ``sinks`` [heads] fp32: exp(sinks[h]) joins the softmax's denominator of head h, without a value.  ``chunk``:
         a query sees only the records of its own chunk of that many positions."""
+        _whole(window, chunk)
         T = q.shape[0]
         D = kv_rank + rot_dim
         if sinks is not None:
@@ -1446,6 +1468,7 @@ class CudaKernels:
         (ids[t-1] * mul_prev + ids[t] * mul_cur) mod buckets (the row ``buckets`` for a sequence's first token).  The
         token before a step's first one comes from ``prev_state`` [slots] int32, which then receives the step's last
         token of every sequence."""
+        _whole(mul_prev, mul_cur)
         T, H = out.shape
         assert out.dtype == torch.float32 and ids.dtype == torch.int32 and table.shape[1] == H
         assert out.is_contiguous() and table.is_contiguous()
@@ -1535,6 +1558,7 @@ class CudaKernels:
                    side.shape[0], self._queue())
 
     def token_gate_few_supported(self, tokens: int, w: torch.Tensor) -> bool:
+        _whole(tokens)
         return w.dtype == torch.bfloat16 and bool(self._ask("zlm_token_gate_few_supported", tokens, w.shape[1]))
 
     def token_gate_few(self, g: torch.Tensor, x: torch.Tensor, w: torch.Tensor, side: torch.Tensor, off: int,
@@ -1618,6 +1642,7 @@ class CudaKernels:
                      post: float, eps: float) -> None:
         """out[t, h, :] = unit_rms(a1 - lam * a2) * post over vdim, where a1, a2 are the attention's outputs of head h's
         two maps in ``a`` [T, 2 heads, hdp] (the order ``diff_prep`` gives the query heads)."""
+        _whole(kv_heads)
         T = a.shape[0]
         assert a.shape == (T, 2 * heads * hdp) and out.shape == (T, heads * vdim) and a.dtype == out.dtype
         assert a.stride(1) == 1 and out.stride(1) == 1
@@ -1650,6 +1675,7 @@ class CudaKernels:
                    *self._route_extras(correction, E, groups, keep, weight_scale, group_top), self._queue())
 
     def _route_extras(self, correction, E, groups, keep, weight_scale, group_top=1):
+        _whole(groups, keep)
         if correction is not None:
             assert correction.dtype == torch.float32 and correction.shape == (E,) and correction.is_contiguous()
         assert group_top in (1, 2)
@@ -1827,6 +1853,7 @@ class CudaKernels:
         (seed, request[r], position[r]).  ``form`` forces one of the kernel's two forms
         (tests): "cluster" (8 blocks per row, the row in distributed shared memory) or
         "block" (one block per row; rows too long for the cluster form)."""
+        _whole(top_k)
         R, V = logits.shape
         assert logits.dtype == torch.float32 and logits.stride(1) == 1 and out.dtype == torch.int32
         assert request.dtype == torch.int32 and position.dtype == torch.int32
