@@ -50,3 +50,31 @@ def test_runs_give_the_bits_of_single_tokens(nq, nkv, dim, vdim, hdp, taps, dtyp
     assert not any(k.lib.zlm_conv_runs(sum(step), sum(n > 0 for n in step), units, hdp, taps) for step in cut)
     for a, b in zip(whole, run(cut)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("taps", [2, 3, 4, 5])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("off", [1, 2, 4])
+def test_taps_that_start_off_a_read_of_four(taps, dtype, off):
+    """Runs are taken wherever the taps start, and give the bits that they give of aligned taps."""
+    from zlm_b200.kernels import PAGE_TOKENS, get_kernels
+    k = get_kernels()
+    nq, nkv, dim, vdim, T = 6, 2, 128, 64, 1031
+    g = torch.Generator(device="cuda").manual_seed(taps)
+    C = (nq + nkv) * dim + nkv * vdim
+    proj = torch.randn((T, C), generator=g, device="cuda").to(dtype)
+    taps_at = torch.zeros(C * taps + 16, device="cuda", dtype=dtype)
+    values = torch.randn((C, taps), generator=g, device="cuda").to(dtype)
+    first = torch.randn((1, taps - 1, C), generator=g, device="cuda").to(dtype)
+    table = torch.arange(-(-T // PAGE_TOKENS), device="cuda", dtype=torch.int32).view(1, -1)
+    assert k.lib.zlm_conv_runs(T, 1, nq + 2 * nkv, dim, taps)
+    got = []
+    for at in (0, off):
+        w = taps_at[at:at + C * taps].view(C, taps)
+        w.copy_(values)
+        q, state = torch.empty((T, nq * dim), device="cuda", dtype=dtype), first.clone()
+        pool = torch.zeros((table.numel(), 2, nkv, PAGE_TOKENS, dim), device="cuda", dtype=dtype)
+        k.conv_norm_write(q, proj, w, state, plan_of([T], [0]), table, pool, nq, nkv, dim, vdim, taps, True, 1e-6)
+        got.append((q, state, pool))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
