@@ -43,62 +43,47 @@ __device__ __forceinline__ void attention_decode_item(
     const int p_end = min(walk.n, p_begin + per);
     if (p_begin >= p_end && splits > 1) return;      // the combine kernel skips this split too
 
-    // q and this step's keys and values come from the kernel before; all other rows of the first two pages are asked for
-    // before the wait for that kernel, its own rows after it.  `fresh` is how many of a sequence's newest positions this
-    // step may have written (0: not known, nothing is read early).  (A page used to wait whole if it held one fresh row: a
-    // sequence of less than a page, and every sequence's newest page, then came a trip to memory after the wait.)
-    const int fresh_lo = fresh > 0 ? max(0, pos + 1 - fresh) : 0;
-    auto has_fresh = [&](int w) { return walk.page(w) * ZLM_PAGE + ZLM_PAGE > fresh_lo && walk.page(w) * ZLM_PAGE <= pos; };
-    // rows r_lo .. r_hi - 1 of page w, without those in s_lo .. s_hi - 1
-    auto load_rows = [&](int w, int stage, int r_lo, int r_hi, int s_lo, int s_hi) {
+    // q and this step's keys and values come from the kernel before; pages that hold only positions
+    // from earlier steps do not, and their loads start before the wait for that kernel.  `fresh`
+    // is how many of a sequence's newest positions this step may have written (0: not known,
+    // nothing is read early).
+    // (Asking for the older rows of a page that also holds fresh ones before the wait, and for those after it, was built: sequences
+    // of two and three pages on a GPU with blocks to spare took 0.6 us longer, 4 sequences of 65 keys, 8 kv heads, 5.6 and 6.2 us,
+    // and 32 of 4,096 keys 99.0 and 104.8.)
+    const int old_pages = fresh > 0 ? max(0, pos + 1 - fresh) / ZLM_PAGE : 0;
+    const bool early0 = PDL && p_begin < p_end && walk.page(p_begin) < old_pages;
+    const bool early1 = early0 && p_begin + 1 < p_end && walk.page(p_begin + 1) < old_pages;
+    auto load_page = [&](int w, int stage) {
         const int p = walk.page(w);
         if (!ZLM_CHK(pages + p, 4)) return;
         const __nv_bfloat16* kb = pool + (size_t)pages[p] * page_stride + (size_t)kvh * TILE;
         const __nv_bfloat16* vb = kb + v_off;
         __nv_bfloat16* ks_ = Ks + stage * TILE;
         __nv_bfloat16* vs_ = Vs + stage * TILE;
-        for (int id = r_lo * CH + tid; id < r_hi * CH; id += DEC_THREADS) {
+        for (int id = tid; id < ZLM_PAGE * CH; id += DEC_THREADS) {
             const int r = id / CH, c = id % CH;
-            if (r >= s_lo && r < s_hi) continue;
             dec_cp_async16(ks_ + tile_off<HD>(r, c), kb + r * HD + c * 8);
             dec_cp_async16(vs_ + tile_off<HD>(r, c), vb + r * HD + c * 8);
         }
     };
-    auto load_page = [&](int w, int stage) { load_rows(w, stage, 0, ZLM_PAGE, 0, 0); };
-    auto fresh_from = [&](int w) { return min(ZLM_PAGE, max(0, fresh_lo - walk.page(w) * ZLM_PAGE)); };
-    auto fresh_to = [&](int w) { return max(0, min(ZLM_PAGE, pos + 1 - walk.page(w) * ZLM_PAGE)); };
 
-    const bool early = PDL && fresh > 0 && p_begin < p_end, second = p_begin + 1 < p_end;
-    bool late0 = false, late1 = false;
-    if (early) {
-        late0 = has_fresh(p_begin);
-        late1 = second && (late0 || has_fresh(p_begin + 1));
-        load_rows(p_begin, 0, 0, ZLM_PAGE, late0 ? fresh_from(p_begin) : 0, late0 ? fresh_to(p_begin) : 0);
-        if (!late0) dec_commit();
-        if (!late0 && second) {
-            load_rows(p_begin + 1, 1, 0, ZLM_PAGE, late1 ? fresh_from(p_begin + 1) : 0, late1 ? fresh_to(p_begin + 1) : 0);
-            if (!late1) dec_commit();
+    if (early0) {
+        load_page(p_begin, 0);
+        dec_commit();
+        if (early1) {
+            load_page(p_begin + 1, 1);
+            dec_commit();
         }
     }
     if (PDL) pdl_wait();
     // the other pages do not depend on q either: they land while q is fetched
-    if (!early) {
+    if (!early0) {
         if (p_begin < p_end) load_page(p_begin, 0);
         dec_commit();
-        if (second) load_page(p_begin + 1, 1);
+    }
+    if (!early1) {
+        if (p_begin + 1 < p_end) load_page(p_begin + 1, 1);
         dec_commit();
-    } else {
-        if (late0) {
-            load_rows(p_begin, 0, fresh_from(p_begin), fresh_to(p_begin), 0, 0);
-            dec_commit();
-            if (second) load_page(p_begin + 1, 1);
-            dec_commit();
-        } else if (late1) {
-            load_rows(p_begin + 1, 1, fresh_from(p_begin + 1), fresh_to(p_begin + 1), 0, 0);
-            dec_commit();
-        } else if (!second) {
-            dec_commit();
-        }
     }
     // Q fragments: row i of the 16-row tile is head kvh*G + i (zero beyond the group)
     unsigned qf[KS][4] = {};
@@ -239,8 +224,8 @@ __device__ __forceinline__ void attention_decode_item(
     l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-    // (only the group's rows, 8 floats beside each so that eight rows meet all banks: without that, a block's end took a
-    // microsecond of conflicts)
+    // (only the group's rows, 8 floats beside each so that eight rows meet all banks: 16 sequences of 51 keys, 8 kv heads, 7.6 us
+    // with the conflicts, 6.2 without)
     constexpr int OLD = HD + 8;
     float* so = (float*)smem_raw;                 // [DEC_WARPS][16][OLD]
     float* sm_ = so + DEC_WARPS * 16 * OLD;       // [DEC_WARPS][16]
