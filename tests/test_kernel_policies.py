@@ -78,6 +78,19 @@ def test_many_token_tile_width(lib, T, N, K, width):
     assert lib.zlm_gemm_tc_tile_width(T, N, K) == width
 
 
+@pytest.mark.parametrize("T,N,K,modes,width", [
+    (2048, 4096, 4096, (1, 2), 240), (2048, 4096, 4096, (0,), 256),          # bf16 rows are no whole boxes of 240 columns
+    (2048, 6144, 4096, (1, 2), 240), (2048, 6144, 4096, (0,), 256),
+    (2048, 5120, 8192, (0, 1, 2), 224),
+    (512, 12288, 2048, (3, 7, 8), 224), (2048, 8192, 1024, (3, 7, 8), 224),  # gate and up: the rule whatever the boxes
+    (385, 12288, 2048, (3, 7, 8), 224), (1500, 11008, 2048, (3, 7, 8), 240),
+    (2048, 24576, 4096, (0, 1, 2, 3, 7, 8), 256), (512, 2048, 1024, (0, 1, 2, 3, 7, 8), 128),
+])
+def test_many_token_tile_width_by_what_leaves_the_tile(lib, T, N, K, modes, width):
+    for mode in modes:
+        assert lib.zlm_gemm_tc_mode_width(T, N, K, mode) == width
+
+
 @pytest.mark.parametrize("R,max_new,nq,nkv,heads", [
     (1, 2048, 32, 8, 2),     # 256 blocks of two heads: enough for 148 SMs
     (1, 2048, 16, 8, 1),     # two heads per block would be 128 blocks, the longest twice as long

@@ -1647,8 +1647,8 @@ extern "C" int zlm_gemm_tc_ksplit(int T, int N, int K) {
 // in rounds of one per SM (or pair of SMs), and a round costs its width: N = 4096 at 2,048 tokens
 // is 128 tiles of 256 columns on 74 pairs (2 rounds, the second 73 % full) or 144 of 240 (2 rounds,
 // 97 % full).  A narrower tile re-reads the activations more often, so it has to win by more than
-// 5 % in rounds x width (measured at 2,048 tokens: N = 4096 and 6144 gain 2-3 % with 240 columns,
-// N = 24576 loses 3 % with 224 although it saves a round of 12).  128 columns (pairs only): half
+// 5 % in rounds x width (measured at 2,048 tokens with fp32 sums: N = 4096 and 6144 gain 2-3 % with
+// 240 columns, N = 24576 loses 3 % with 224 although it saves a round of 12).  128 columns (pairs only): half
 // the reuse of the activations per product, so only where the wider tiles would leave a third of
 // the pairs idle (N = 1024 at 2,048 tokens: 32 tiles on 74 pairs).
 extern "C" int zlm_gemm_tc_tile_width(int T, int N, int K) {
@@ -1665,14 +1665,16 @@ extern "C" int zlm_gemm_tc_tile_width(int T, int N, int K) {
     return best;
 }
 
-// The width for a mode: 240 columns, and 224 of gate and up, are no whole boxes of the copy engine's (32 bf16 outputs, 64 sums
-// of gate and up), and with them a tile's results leave row by row.  2,048 tokens, bf16 outputs, 240 / 256 columns: N = 4,096 at
-// K = 512 20.0 / 13.0 us, N = 6,144 at K = 4,096 79.2 / 72.0; 5,000 tokens x 4,096 at K = 1,024 48.9 / 33.0.
-static int tile_width(int T, int N, int K, int mode) {
+// The width for a mode.  240 columns are no whole boxes of the copy engine's bf16 results (32 columns), and with them a tile's
+// rows leave one by one: bf16 outputs never take them.  2,048 tokens, 240 / 256 columns: N = 4,096 at K = 512 20.0 / 13.0 us,
+// N = 6,144 at K = 4,096 79.2 / 72.0; 5,000 tokens x 4,096 at K = 1,024 48.9 / 33.0.  Gate and up, whose boxes are 64 columns, leave
+// row by row from 224 and 240 as well and keep the rule all the same: half as many results, and rows beyond the step's tokens,
+// zeros whose activation the division takes its slow path for, are left out.  Us, 256 / the rule: 512 tokens x 12,288 x 2,048 35.1
+// / 33.8, 2,048 x 8,192 x 1,024 49.2 / 46.1; 385 x 12,288 x 2,048 64.1 / 33.3, 1,500 x 11,008 x 2,048 85.8 / 57.3; only where tiles are
+// many rounds does 256 gain: 4,096 x 9,728 x 2,560 145.8 / 153.3.
+extern "C" int zlm_gemm_tc_mode_width(int T, int N, int K, int mode) {
     const int width = zlm_gemm_tc_tile_width(T, N, K);
-    if (g_tc_width || g_tc_form == 1 || width == 0 || width == 128 || width == 256) return width;
-    if (ZLM_GATED(mode)) return 256;
-    if (mode != 0 || width != 240) return width;
+    if (g_tc_width || g_tc_form == 1 || mode != 0 || width != 240) return width;
     const long long m_tiles = (T + TCQ_BM - 1) / TCQ_BM, slots = sm_count() / 2;
     auto cost = [&](int bn) { return ((m_tiles * ((N + bn - 1) / bn) + slots - 1) / slots) * bn; };
     return cost(224) * 100 < cost(256) * 95 ? 224 : 256;
@@ -1706,7 +1708,7 @@ extern "C" int zlm_gemm_tc(void* Y, const void* X, const void* W, int T, int N, 
         if (T <= 64) return launch_tc_few<64, 8>(Y, X, W, T, N, K, ldx, ldy, mode, plan, scratch, st);
         return launch_tc_few<128, 6>(Y, X, W, T, N, K, ldx, ldy, mode, plan, scratch, st);
     }
-    const int width = tile_width(T, N, K, mode);
+    const int width = zlm_gemm_tc_mode_width(T, N, K, mode);
     if (g_tc_form != 1) {
         if (width == 128) return launch_tc_pair<128, 8>(Y, X, W, T, N, K, ldx, ldy, mode, st);
         if (width == 240) return launch_tc_pair<240, 6>(Y, X, W, T, N, K, ldx, ldy, mode, st);
