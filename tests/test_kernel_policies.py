@@ -59,6 +59,19 @@ def test_few_token_shares_of_k(lib, T, N, K, shares):
     assert lib.zlm_gemm_tc_ksplit(T, N, K) == shares
 
 
+@pytest.mark.parametrize("T,K,shares", [
+    (384, 1024, 2), (385, 1024, 1), (9472, 1024, 1),            # up to 384 tokens as ever; beyond, what is saved has to pay
+    (385, 1536, 3), (1024, 1536, 3), (1500, 1536, 1),
+    (385, 2048, 4), (2048, 2048, 4), (3000, 2048, 4), (4096, 2048, 1), (8192, 2048, 1),
+    (2048, 4096, 8), (6000, 4096, 3), (8192, 4096, 1),
+    (2048, 8192, 8), (9472, 8192, 2), (9473, 8192, 1),          # 75 tiles of 128 tokens: two shares are more than a round
+])
+def test_few_outputs_over_many_tokens_are_cut_where_that_wins(lib, T, K, shares):
+    for N in (8, 64, 128):
+        assert lib.zlm_gemm_tc_ksplit(T, N, K) == shares
+    assert lib.zlm_gemm_tc_ksplit(max(T, 385), 129, K) == 1     # two tiles of outputs: never
+
+
 def test_tcgen05_product_takes_what_tma_can_address(lib):
     assert lib.zlm_gemm_tc_supported(64, 4096, 4096, 4096) == 1
     assert lib.zlm_gemm_tc_supported(64, 4096, 4100, 4100) == 0      # rows of K elements must be 16-byte multiples

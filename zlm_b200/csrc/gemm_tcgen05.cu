@@ -13,7 +13,8 @@
 //    full-height products; one block per tile and share of K where that is one round of the
 //    GPU (gemm_tc_kernel), else persistent blocks (gemm_tc_few_kernel); K is cut into shares
 //    where the tiles alone would not fill the SMs, and a second kernel adds the shares in a
-//    fixed order.
+//    fixed order.  Products of up to 128 outputs over some thousand tokens, cut so, run as its
+//    stand-alone blocks too (few_form).
 // In all of them warp 0 is the TMA producer, warp 1 allocates tensor memory and issues the
 // products (TcIssue), warps 2..5 are the epilogue.  A ring of (first-operand tile 128x64,
 // second-operand tile x64) is handed back and forth with mbarriers: `full` is completed by
@@ -1627,14 +1628,18 @@ extern "C" int zlm_gemm_tc_supported(int T, int N, int K, int ldx) {
     return (T >= 1 && N >= 8 && K >= 8 && K % 8 == 0 && ldx % 8 == 0) ? 1 : 0;
 }
 
-// Whether a product runs in a few-token form: up to 384 tokens; and with more where it has one tile of outputs and all its
-// tiles, cut along K, are one round of the GPU (a router's logits, a mixer's gates: 2,048 tokens x 64 outputs x 2,048 is 8 tiles
-// for 74 pairs of blocks, and 64 blocks of a quarter of K each here: 15.5 us and 13.3 with the shares' sum).
+// Whether a product runs in a few-token form: up to 384 tokens; and with more where it has one tile of outputs (a router's logits,
+// a mixer's gates), all its tiles, cut along K, are one round of the GPU, and the cut saves a block enough of its stages of K: a
+// stage less is 0.29 us, and the shares' store and sum cost what 12 stages do and one more for every 300 tokens.  bf16 outputs, us
+// in tiles of pairs / cut: 64 outputs at K = 2,048, 385 tokens 13.8 / 10.4, 2,048 14.7 / 12.2, 3,000 14.8 / 12.9, 8,192 15.9 / 18.2;
+// K = 1,024 9.2 / 10.4 and 10.9 / 14.6 for 385 and 8,192; 8 outputs at K = 2,048, 4,096 tokens 14.8 / 14.8; 128 at K = 4,096, 6,000 25.4 /
+// 22.3, 8,192 25.9 / 25.9; 128 at K = 8,192, 2,048 42.9 / 18.2, 9,472 45.1 / 43.1.
 static bool few_form(int T, int N, int K) {
     if (T <= 384) return true;
     if (N > TC_BM || g_tc_form) return false;
     const FewPlan plan = few_plan(T, N, K);
-    return plan.ks > 1 && plan.whole == 0;
+    const int kb = (K + TC_BK - 1) / TC_BK;
+    return plan.whole == 0 && kb - (kb + plan.ks - 1) / plan.ks > 12 + T / 300;
 }
 
 // shares of K whose fp32 partial products need scratch memory (T * N floats each)
