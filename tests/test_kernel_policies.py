@@ -72,6 +72,19 @@ def test_few_outputs_over_many_tokens_are_cut_where_that_wins(lib, T, K, shares)
     assert lib.zlm_gemm_tc_ksplit(max(T, 385), 129, K) == 1     # two tiles of outputs: never
 
 
+@pytest.mark.parametrize("T,N,K,whole", [
+    (1024, 1024, 704, 0), (1024, 1024, 768, 1), (385, 4096, 512, 0), (1024, 1024, 64, 0),         # pairs, tiles of 128 columns: from 12 stages
+    (700, 8192, 1984, 0), (700, 8192, 2048, 1),                                                 # of 224: from 32
+    (2048, 2048, 2048, 0), (2048, 24576, 3008, 0), (2048, 24576, 3072, 1),                      # of 256: from 48
+    (143, 6144, 4096, 1), (300, 4096, 1024, 1), (300, 4096, 704, 0), (143, 2048, 2048, 0),      # stand-alone, two token tiles and more
+    (17, 4096, 4096, 0), (64, 8192, 2048, 0), (100, 6144, 4096, 0), (128, 4096, 12288, 0),      # one: the weights come from memory
+    (2048, 64, 2048, 0), (4096, 128, 8192, 0),                                                  # few outputs over many tokens
+    (300, 8192, 1536, 0), (300, 8192, 2048, 1),                                                 # persistent few-token blocks
+])
+def test_who_issues_a_product(lib, T, N, K, whole):
+    assert lib.zlm_gemm_tc_issues_whole(T, N, K, 2) == whole
+
+
 def test_tcgen05_product_takes_what_tma_can_address(lib):
     assert lib.zlm_gemm_tc_supported(64, 4096, 4096, 4096) == 1
     assert lib.zlm_gemm_tc_supported(64, 4096, 4100, 4100) == 0      # rows of K elements must be 16-byte multiples

@@ -1378,8 +1378,9 @@ template <int BN, int STAGES>
 static int launch_tc(void* Y, const void* X, const void* W, int T, int N, int K, int ldx, int ldy, int mode, int ksplit, float* scratch,
                      cudaStream_t st, bool add_shares = true) {
     const int stages = ((K + TC_BK - 1) / TC_BK + ksplit - 1) / ksplit;
-    return tc_issue_whole(stages, BN) ? launch_tc_as<BN, STAGES, true>(Y, X, W, T, N, K, ldx, ldy, mode, ksplit, scratch, st, add_shares)
-                                      : launch_tc_as<BN, STAGES, false>(Y, X, W, T, N, K, ldx, ldy, mode, ksplit, scratch, st, add_shares);
+    if constexpr (BN == 128)
+        if (tc_issue_whole_alone(T, stages)) return launch_tc_as<BN, STAGES, true>(Y, X, W, T, N, K, ldx, ldy, mode, ksplit, scratch, st, add_shares);
+    return launch_tc_as<BN, STAGES, false>(Y, X, W, T, N, K, ldx, ldy, mode, ksplit, scratch, st, add_shares);
 }
 
 static int sm_count() {
@@ -1478,10 +1479,8 @@ static int launch_tc_pair_as(void* Y, const void* X, const void* W, int T, int N
 template <int BN, int STAGES>
 static int launch_tc_pair(void* Y, const void* X, const void* W, int T, int N, int K, int ldx, int ldy, int mode, cudaStream_t st,
                           const QkvEpilogue* qkv = nullptr) {
-    // (narrow tiles gain at every K)
-    if (BN < 240 || tc_issue_whole((K + TC_BK - 1) / TC_BK, BN)) return launch_tc_pair_as<BN, STAGES, true>(Y, X, W, T, N, K, ldx, ldy, mode, st, qkv);
-    if constexpr (BN >= 240) return launch_tc_pair_as<BN, STAGES, false>(Y, X, W, T, N, K, ldx, ldy, mode, st, qkv);
-    return ZLM_OK;
+    return tc_issue_whole((K + TC_BK - 1) / TC_BK, BN) ? launch_tc_pair_as<BN, STAGES, true>(Y, X, W, T, N, K, ldx, ldy, mode, st, qkv)
+                                                       : launch_tc_pair_as<BN, STAGES, false>(Y, X, W, T, N, K, ldx, ldy, mode, st, qkv);
 }
 
 // Which many-token form runs, and how wide its tiles are: 0 lets the dispatcher choose (pairs of
@@ -1557,7 +1556,8 @@ static int launch_tc_few_as(void* Y, const void* X, const void* W, int T, int N,
 template <int BN, int STAGES>
 static int launch_tc_few(void* Y, const void* X, const void* W, int T, int N, int K, int ldx, int ldy, int mode, const FewPlan& plan,
                          float* scratch, cudaStream_t st) {
-    // (143 tokens x 4,096 at K = 1,024: 0.1 us slower with it)
+    // (us, a thread / a whole warp: 143 tokens x 24,576 x 4,096 66.9 / 58.9, 384 x 32,000 x 4,096 117.4 / 103.3, 300 x 8,192 x 2,048 26.7 /
+    // 25.4; 384 x 8,192 x 1,024 20.5 / 20.7; no difference up to 128 tokens, where the weights come from memory)
     return K > 24 * TC_BK ? launch_tc_few_as<BN, STAGES, true>(Y, X, W, T, N, K, ldx, ldy, mode, plan, scratch, st)
                           : launch_tc_few_as<BN, STAGES, false>(Y, X, W, T, N, K, ldx, ldy, mode, plan, scratch, st);
 }
@@ -1723,6 +1723,16 @@ extern "C" int zlm_gemm_tc(void* Y, const void* X, const void* W, int T, int N, 
     if (width == 240) return launch_tc_persistent<240, 4>(Y, X, W, T, N, K, ldx, ldy, mode, st);
     if (width == 224) return launch_tc_persistent<224, 4>(Y, X, W, T, N, K, ldx, ldy, mode, st);
     return launch_tc_persistent<256, 4>(Y, X, W, T, N, K, ldx, ldy, mode, st);
+}
+
+// For tests: whether a whole warp issues this product (0: one thread of it)
+extern "C" int zlm_gemm_tc_issues_whole(int T, int N, int K, int mode) {
+    const int kb = (K + TC_BK - 1) / TC_BK;
+    if (!few_form(T, N, K)) return g_tc_form != 1 && tc_issue_whole(kb, zlm_gemm_tc_mode_width(T, N, K, mode));
+    const FewPlan plan = few_plan(T, N, K);
+    const long long tiles = (long long)((N + TC_BM - 1) / TC_BM) * plan.t_tiles;
+    if (plan.whole + (tiles - plan.whole) * plan.ks <= sm_count()) return tc_issue_whole_alone(T, (kb + plan.ks - 1) / plan.ks);
+    return K > 24 * TC_BK;
 }
 
 // A few-token product that runs as one round of stand-alone blocks cuts K into shares and leaves

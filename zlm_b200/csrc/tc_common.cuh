@@ -78,8 +78,8 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 // products of a stage (64 of K, 32 bytes on in both operands each) from one block of instructions; commit: an arrival at
 // `bar` once what this issuer has issued has retired; wait: a bounded wait.  A product issued from a thread in a branch of its
 // own takes it about 108 cycles, from an elected lane of a whole warp 50 to 65: less than 256 x 128 x 16 takes the tensor cores,
-// where the thread is what bounds the kernel.  But a kernel built with it is 0.2 to 0.3 us slower to get going (measured; not
-// explained), so that it pays from some stages on (tc_issue_whole): built as kernels of their own.
+// where the thread is what bounds the kernel.  But a kernel built with it is 0.2 to 0.6 us slower to get going (measured; not
+// explained), so that it pays from some stages on (tc_issue_whole, tc_issue_whole_alone): built as kernels of their own.
 #define TC_MMA4(GROUP, LEADER)                                                                                          \
     asm volatile("{\n\t.reg .pred q, p0, p1;\n\t.reg .b64 da, db;\n\t" LEADER                                         \
                  "setp.ne.b32 p0, %4, 0;\n\tsetp.eq.b32 p1, 0, 0;\n\t"                                                  \
@@ -105,11 +105,16 @@ template <bool WHOLE> struct TcIssue {
         return WHOLE ? mbar_wait_warp(bar, parity, abort_flag, where) : mbar_wait(bar, parity, abort_flag, where);
     }
 };
-// Single thread / whole warp, us: 128 tokens x 1,024 x 1,024 (8 stages a block) 11.1 / 11.4; 384 x 6,144 x 4,096 (32 stages) 27.2 /
-// 22.9; pairs, 512 x 1,024 x 1,024 in tiles of 128 columns 11.4 / 10.8, 1,024 x 2,048 x 2,048 17.4 / 15.9; in tiles of 224, 2,999 x
-// 5,120 x 2,048 48.0 / 45.9; of 240 and 256, 2,048 x 2,048 x 1,024 13.4 / 13.9, 2,048 x 2,048 x 2,048 19.0 / 19.5, 2,048 x 4,096 x
-// 4,096 52.2 / 51.2.
-static inline bool tc_issue_whole(int stages, int width) { return stages >= (width < 240 ? 12 : 48); }
+// Pairs of blocks, `stages` of K a tile.  Whole warp in per cent of a single thread's time, at K = 512 / 768 / 1,024 / 1,536 / 2,048 / 4,096:
+// tiles of 128 columns, 1,024 tokens x 1,024 outputs 102 / 99 / 97 / 94 / 92 / -; of 224, 700 x 8,192, 103 / 101 / 103 / 100 / 98 / 97;
+// of 240, 2,048 x 4,096, 103 / 103 / 105 / 101 / 99 / 98; of 256, 2,048 x 6,144, 104 / 106 / 103 / 101 / 100 / 99.
+static inline bool tc_issue_whole(int stages, int width) { return stages >= (width < 224 ? 12 : width < 240 ? 32 : 48); }
+// The few-token form's stand-alone blocks: only where two token tiles and more read the weights, so that they come from L2 and the
+// issuing thread, not memory, sets the pace; and up to 384 tokens.  Us: 143 tokens x 6,144 x 4,096 (64 stages) 25.9 / 22.0, 300 x 4,096 x
+// 1,536 (24) 13.3 / 12.4, 300 x 4,096 x 1,024 (16) 10.6 / 10.3, 143 x 4,096 x 1,536 (12) 15.5 / 15.2, 143 x 2,048 x 2,048 (8) 13.2 / 13.2, 256 x
+// 1,024 x 1,024 (8) 11.8 / 12.0; one tile: 17 x 4,096 x 4,096 (16) 12.4 / 13.0, 100 x 6,144 x 4,096 (21) 20.9 / 21.7, 100 x 4,096 x 12,288 (48)
+// 29.8 / 30.7; few outputs: 4,096 x 128 x 8,192 (32) 23.8 / 24.5.
+static inline bool tc_issue_whole_alone(int tokens, int stages) { return tokens > 128 && tokens <= 384 && stages >= 12; }
 // 16 columns of this thread's lane, without the wait: several loads can be in flight, then tc_wait_ld()
 __device__ __forceinline__ void tc_ld16_nowait(unsigned taddr, float* v) {
     unsigned* r = (unsigned*)v;
