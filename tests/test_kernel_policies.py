@@ -85,6 +85,14 @@ def test_who_issues_a_product(lib, T, N, K, whole):
     assert lib.zlm_gemm_tc_issues_whole(T, N, K, 2) == whole
 
 
+@pytest.mark.parametrize("T,N,hd,width", [
+    (2048, 128, 128, 128), (2048, 128, 32, 128), (9472, 128, 128, 128),      # one head in all: half of a wide tile would be empty
+    (2048, 512, 128, 128), (512, 4096, 128, 128), (512, 4096, 256, 256), (2048, 4096, 128, 256), (30000, 4096, 128, 256),
+])
+def test_projection_tile_width(lib, T, N, hd, width):
+    assert lib.zlm_gemm_tc_qkv_width(T, N, hd) == width
+
+
 def test_tcgen05_product_takes_what_tma_can_address(lib):
     assert lib.zlm_gemm_tc_supported(64, 4096, 4096, 4096) == 1
     assert lib.zlm_gemm_tc_supported(64, 4096, 4100, 4100) == 0      # rows of K elements must be 16-byte multiples

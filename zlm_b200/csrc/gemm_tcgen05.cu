@@ -1648,7 +1648,7 @@ extern "C" int zlm_gemm_tc_ksplit(int T, int N, int K) {
     return few_plan(T, N, K).ks;
 }
 
-// The width of the many-token forms' tiles (0 for the few-token forms).  Tiles run
+// The width of the many-token forms' tiles.  Tiles run
 // in rounds of one per SM (or pair of SMs), and a round costs its width: N = 4096 at 2,048 tokens
 // is 128 tiles of 256 columns on 74 pairs (2 rounds, the second 73 % full) or 144 of 240 (2 rounds,
 // 97 % full).  A narrower tile re-reads the activations more often, so it has to win by more than
@@ -1656,8 +1656,7 @@ extern "C" int zlm_gemm_tc_ksplit(int T, int N, int K) {
 // 240 columns, N = 24576 loses 3 % with 224 although it saves a round of 12).  128 columns (pairs only): half
 // the reuse of the activations per product, so only where the wider tiles would leave a third of
 // the pairs idle (N = 1024 at 2,048 tokens: 32 tiles on 74 pairs).
-extern "C" int zlm_gemm_tc_tile_width(int T, int N, int K) {
-    if (few_form(T, N, K)) return 0;
+static int many_width(int T, int N) {
     if (g_tc_width) return g_tc_width;
     const bool pairs = g_tc_form != 1;
     const long long m_tiles = pairs ? (T + TCQ_BM - 1) / TCQ_BM : (T + TC_BM - 1) / TC_BM;
@@ -1669,6 +1668,8 @@ extern "C" int zlm_gemm_tc_tile_width(int T, int N, int K) {
     if (pairs && cost(128) * 100 < cost(best) * 70) best = 128;
     return best;
 }
+// (0 for the few-token forms)
+extern "C" int zlm_gemm_tc_tile_width(int T, int N, int K) { return few_form(T, N, K) ? 0 : many_width(T, N); }
 
 // The width for a mode.  240 columns are no whole boxes of the copy engine's bf16 results (32 columns), and with them a tile's
 // rows leave one by one: bf16 outputs never take them.  2,048 tokens, 240 / 256 columns: N = 4,096 at K = 512 20.0 / 13.0 us,
@@ -1774,6 +1775,10 @@ extern "C" int zlm_gemm_tc_qkv_supported(int T, int N, int K, int ldx, int nq, i
     return 1;
 }
 
+// Its tiles, of whole heads: 256 columns, or 128 where 256 would leave pairs of SMs idle (however few its outputs: it always runs
+// on pairs of blocks)
+extern "C" int zlm_gemm_tc_qkv_width(int T, int N, int hd) { return many_width(T, N) == 128 && 128 % hd == 0 ? 128 : 256; }
+
 // q [T, nq*hd] bf16 (row stride ldy) = norm+rotate(X Wq^T); k (normed, rotated) and v go to the
 // tokens' places in the paged pool.  cos_sin: [2][hd/2][T] from zlm_rope_table, or null.
 extern "C" int zlm_gemm_tc_qkv(void* Y, const void* X, const void* W, int T, int N, int K, int ldx, int ldy,
@@ -1790,9 +1795,7 @@ extern "C" int zlm_gemm_tc_qkv(void* Y, const void* X, const void* W, int T, int
     ZLM_REQUIRE(nkv == 0 || (pool && block_table && token_slot), "gemm_tc_qkv: the cache is missing");
     QkvEpilogue ep{q_w, k_w, w_dtype, eps, cos_sin, token_pos, token_slot, block_table, table_stride,
                    (__nv_bfloat16*)pool, nq, nkv, hd};
-    // tiles of whole heads: 256 columns, or 128 where 256 would leave pairs of SMs idle
-    int width = g_tc_width ? g_tc_width : zlm_gemm_tc_tile_width(T, N, K);
-    if (width != 128 || 128 % hd != 0) width = 256;
+    const int width = zlm_gemm_tc_qkv_width(T, N, hd);
     if (width == 128) return launch_tc_pair<128, 8>(Y, X, W, T, N, K, ldx, ldy, 5, st, &ep);
     return launch_tc_pair<256, 6>(Y, X, W, T, N, K, ldx, ldy, 5, st, &ep);
 }
