@@ -495,17 +495,18 @@ __device__ __forceinline__ void qkv_flush(const unsigned char* stage, __nv_bfloa
     __syncwarp();
 }
 
-// the heads first, first + step, .. of one warp's 32 token rows (this thread's: lane `taddr` of tensor memory, tile columns
+// the heads first, first + step, .. of one warp's 32 token rows; part 1, 2: only the first, the second half of a head's angles (this thread's: lane `taddr` of tensor memory, tile columns
 // [n0, n0 + BN)); ws: the norm weights of q and of k, widened, in shared memory (null: read them where they are)
 template <int BN>
 __device__ __forceinline__ void qkv_epilogue_rows(const QkvEpilogue& ep, const QkvRow& at, unsigned taddr, __nv_bfloat16* Y, int row,
-                                                  int n0, int T, int N, int ldy, int first, int step, unsigned char* stage,
+                                                  int n0, int T, int N, int ldy, int first, int step, int part, unsigned char* stage,
                                                   const float* ws, int lane) {
     const int hd = ep.hd, half = hd >> 1;
     // the table is [2][hd/2][T]: the warp's 32 rows read 32 neighbouring floats of one angle
     const float* cs_row = ep.cos_sin ? ep.cos_sin + min(row, T - 1) : nullptr;
     const float* sn_row = ep.cos_sin ? ep.cos_sin + (size_t)half * T + min(row, T - 1) : nullptr;
     unsigned char* const mine = stage + lane * 128;
+    const int c_lo = part == 2 ? half >> 1 : 0, c_hi = part == 1 ? half >> 1 : half;
     for (int c0 = first * hd; c0 < BN; c0 += step * hd) { // the tile's heads; warp-uniform
         const int n = n0 + c0;
         if (n >= N) break;
@@ -526,8 +527,8 @@ __device__ __forceinline__ void qkv_epilogue_rows(const QkvEpilogue& ep, const Q
         if (turn) {                                       // (on their way while the squares are summed)
 #pragma unroll
             for (int e = 0; e < 16; ++e) {
-                cc[e] = __ldg(cs_row + (size_t)e * T);
-                sn[e] = __ldg(sn_row + (size_t)e * T);
+                cc[e] = __ldg(cs_row + (size_t)(c_lo + e) * T);
+                sn[e] = __ldg(sn_row + (size_t)(c_lo + e) * T);
             }
         }
         float inv = 1.f;
@@ -545,7 +546,7 @@ __device__ __forceinline__ void qkv_epilogue_rows(const QkvEpilogue& ep, const Q
             inv = 1.0f / sqrtf(ss / (float)hd + ep.eps);
         }
 #pragma unroll 1
-        for (int c = 0, k = 0; c < half; c += 16, k ^= 1) {
+        for (int c = c_lo, k = 0; c < c_hi; c += 16, k ^= 1) {
             float lo[16], hi[16];
             tc_ld16_nowait(taddr + (unsigned)(c0 + c), lo);
             tc_ld16_nowait(taddr + (unsigned)(c0 + half + c), hi);
@@ -568,7 +569,7 @@ __device__ __forceinline__ void qkv_epilogue_rows(const QkvEpilogue& ep, const Q
                     lo[e] = x0 * cc[e] - x1 * sn[e];
                     hi[e] = x0 * sn[e] + x1 * cc[e];
                 }
-                if (c + 16 < half)                        // the next sixteen angles, while these results go out
+                if (c + 16 < c_hi)                        // the next sixteen angles, while these results go out
 #pragma unroll
                     for (int e = 0; e < 16; ++e) {
                         cc[e] = __ldg(cs_row + (size_t)(c + 16 + e) * T);
@@ -583,7 +584,7 @@ __device__ __forceinline__ void qkv_epilogue_rows(const QkvEpilogue& ep, const Q
             *(uint4*)(mine + (((2 * k + 4) ^ sw) << 4)) = ZLM_PK8(hi);
             *(uint4*)(mine + (((2 * k + 5) ^ sw) << 4)) = ZLM_PK8((hi + 8));
 #undef ZLM_PK8
-            if (k == 1 || c + 16 >= half) qkv_flush(stage, dst, c - 16 * k, half, k + 1, lane);
+            if (k == 1 || c + 16 >= c_hi) qkv_flush(stage, dst, c - 16 * k, half, k + 1, lane);
         }
     }
 }
@@ -614,9 +615,11 @@ __device__ __forceinline__ void qkv_epilogue_rows(const QkvEpilogue& ep, const Q
 #define TCQ_BOX_BYTES (32 * 64)
 #define TCQ_BOX_ACC(MODE) (ZLM_GATED(MODE) ? 64 : (MODE) == 0 ? 32 : 16)
 #define TCQ_OUT_BYTES (4 * TCQ_RING * TCQ_BOX_BYTES)
-// MODE 5 has eight epilogue warps, two for every quarter of the accumulators' lanes: they share a tile's heads, or take the
-// tiles in turn where a tile is one head.  At K = 1,024 a tile's products take 8,200 cycles, and four warps' epilogue took
-// 25,000 (61,037 tokens, 16 + 2 x 8 heads of 128: 772 us); the other modes lose 3 to 5 % with eight.
+// MODE 5 has eight epilogue warps, two for every quarter of the accumulators' lanes.  They share a tile's heads; where a tile is
+// one head they take half of its angles each, or, if it has a norm, whose sum of squares needs all of it, the tiles in turn.
+// At K = 1,024 a tile's products take 8,200 cycles, and four warps' epilogue took 25,000 (61,037 tokens, 16 + 2 x 8 heads of 128:
+// 772 us); plain heads of a tile each in turn: 512 tokens, 16 + 2 x 8 heads of 128, K = 1,024 14.6 us, 13.2 by halves (13.7 with four warps
+// that store their rows directly).  The other modes lose 3 to 5 % with eight.
 #define TCQ_THREADS(MODE) ((MODE) == 5 ? 320 : TC_THREADS)
 #define TCQ_NORM_BYTES 1024          // MODE 5: the norm weights of q and k as fp32, heads of up to 128
 template <int BN, int STAGES, int MODE, bool WHOLE>
@@ -637,7 +640,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     unsigned* tmem_slot = (unsigned*)(acc_empty + 2);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     float* norm_w = (float*)(((uintptr_t)(tmem_slot + 2) + 15) & ~(uintptr_t)15);       // MODE 5
-    const bool share_tile = MODE == 5 && BN / ep.hd >= 2;       // both sets of epilogue warps work on every tile
+    // both sets of epilogue warps work on every tile: on its heads in turn, or on half of one head's angles each
+    const bool heads_in_turn = MODE == 5 && BN / ep.hd >= 2, share_tile = MODE == 5 && (heads_in_turn || !ep.q_w);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned rank = cluster_rank();
@@ -758,7 +762,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (!ok || *abort_flag) break;
             if constexpr (MODE == 5) {
                 qkv_epilogue_rows<BN>(ep, at, tmem_base + ((unsigned)(lg * 32) << 16) + buf * TCP_ACC, (__nv_bfloat16*)Y, arow,
-                                      b0row, T, N, ldy, share_tile ? set : 0, share_tile ? 2 : 1,
+                                      b0row, T, N, ldy, heads_in_turn ? set : 0, heads_in_turn ? 2 : 1,
+                                      share_tile && !heads_in_turn ? 1 + set : 0,
                                       sOut + (warp - 2) * (TCQ_OUT_BYTES / 8),
                                       8 * ep.hd <= TCQ_NORM_BYTES ? norm_w : nullptr, lane);
             } else if (y_tma && BN % TCQ_BOX_ACC(MODE) == 0) {
