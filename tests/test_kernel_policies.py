@@ -59,16 +59,20 @@ def test_few_token_shares_of_k(lib, T, N, K, shares):
     assert lib.zlm_gemm_tc_ksplit(T, N, K) == shares
 
 
-@pytest.mark.parametrize("T,K,shares", [
-    (384, 1024, 2), (385, 1024, 1), (9472, 1024, 1),            # up to 384 tokens as ever; beyond, what is saved has to pay
-    (385, 1536, 3), (1024, 1536, 3), (1500, 1536, 1),
-    (385, 2048, 4), (2048, 2048, 4), (3000, 2048, 4), (4096, 2048, 1), (8192, 2048, 1),
-    (2048, 4096, 8), (6000, 4096, 3), (8192, 4096, 1),
-    (2048, 8192, 8), (9472, 8192, 2), (9473, 8192, 1),          # 75 tiles of 128 tokens: two shares are more than a round
+@pytest.mark.parametrize("T,K,shares,bf16", [
+    (384, 1024, 2, 1), (385, 1024, 2, 0), (9472, 1024, 2, 0), (385, 512, 1, 0),      # up to 384 tokens as ever
+    (385, 1536, 3, 1), (1024, 1536, 3, 1), (1500, 1536, 3, 0),
+    (385, 2048, 4, 1), (2048, 2048, 4, 1), (3000, 2048, 4, 1), (4096, 2048, 4, 0), (8192, 2048, 2, 0),
+    (2048, 4096, 8, 1), (6000, 4096, 3, 1), (8192, 4096, 2, 0),
+    (2048, 8192, 8, 1), (9472, 8192, 2, 1), (9473, 8192, 1, 0),                      # 75 tiles of 128 tokens: two shares are more than a round
 ])
-def test_few_outputs_over_many_tokens_are_cut_where_that_wins(lib, T, K, shares):
-    for N in (8, 64, 128):
+def test_few_outputs_over_many_tokens_are_cut(lib, T, K, shares, bf16):
+    """fp32 results wherever they can be cut, whose sums are the more exact for it; bf16 results where that is faster."""
+    for N in (16, 64, 128):
         assert lib.zlm_gemm_tc_ksplit(T, N, K) == shares
+        assert all(lib.zlm_gemm_tc_takes_few_form(T, N, K, m) == (T <= 384 or shares > 1) for m in (1, 2))
+        assert all(lib.zlm_gemm_tc_takes_few_form(T, N, K, m) == bf16 for m in (0, 3, 7, 8))
+        assert bf16 or lib.zlm_gemm_tc_mode_width(T, N, K, 0) == 128
     assert lib.zlm_gemm_tc_ksplit(max(T, 385), 129, K) == 1     # two tiles of outputs: never
 
 

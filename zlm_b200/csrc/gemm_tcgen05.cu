@@ -1633,21 +1633,32 @@ extern "C" int zlm_gemm_tc_supported(int T, int N, int K, int ldx) {
     return (T >= 1 && N >= 8 && K >= 8 && K % 8 == 0 && ldx % 8 == 0) ? 1 : 0;
 }
 
-// Whether a product runs in a few-token form: up to 384 tokens; and with more where it has one tile of outputs (a router's logits,
-// a mixer's gates), all its tiles, cut along K, are one round of the GPU, and the cut saves a block enough of its stages of K: a
-// stage less is 0.29 us, and the shares' store and sum cost what 12 stages do and one more for every 300 tokens.  bf16 outputs, us
-// in tiles of pairs / cut: 64 outputs at K = 2,048, 385 tokens 13.8 / 10.4, 2,048 14.7 / 12.2, 3,000 14.8 / 12.9, 8,192 15.9 / 18.2;
-// K = 1,024 9.2 / 10.4 and 10.9 / 14.6 for 385 and 8,192; 8 outputs at K = 2,048, 4,096 tokens 14.8 / 14.8; 128 at K = 4,096, 6,000 25.4 /
-// 22.3, 8,192 25.9 / 25.9; 128 at K = 8,192, 2,048 42.9 / 18.2, 9,472 45.1 / 43.1.
+// Whether a product runs in a few-token form: up to 384 tokens; and with more where it has one tile of outputs and all its
+// tiles, cut along K, are one round of the GPU (a router's logits, a mixer's gates: 2,048 tokens x 64 outputs x 2,048 is 8 tiles
+// for 74 pairs of blocks, and 64 blocks of a quarter of K each here).  fp32 results are cut wherever that can be done, also where
+// it costs time: the chains of sums are shorter, and the results' error, which grows with them, 2 to 4 times smaller.  us whole /
+// cut and error of either against 64 bits, 64 outputs: K = 1,024, 385 tokens 9.7 / 10.3, 1.0e-6 / 4.7e-7, 8,192 11.5 / 14.6; K = 2,048,
+// 385 14.2 / 10.4, 2.1e-6 / 4.7e-7, 2,048 15.0 / 12.3, 8,192 16.2 / 18.2, 2.1e-6 / 9.9e-7; K = 4,096, 385 23.6 / 11.4, 8,192 25.7 / 23.7.
 static bool few_form(int T, int N, int K) {
     if (T <= 384) return true;
     if (N > TC_BM || g_tc_form) return false;
     const FewPlan plan = few_plan(T, N, K);
-    const int kb = (K + TC_BK - 1) / TC_BK;
-    return plan.whole == 0 && kb - (kb + plan.ks - 1) / plan.ks > 12 + T / 300;
+    return plan.ks > 1 && plan.whole == 0;
 }
+// The same by what leaves the product.  bf16 results, whose rounding hides those errors, are cut only where the stages of K that a
+// block is spared pay for it: a stage less is 0.29 us, and the shares' store and sum cost what 12 stages do and one more for every
+// 300 tokens.  us whole / cut: 64 outputs at K = 2,048, 385 tokens 13.8 / 10.4, 2,048 14.7 / 12.2, 3,000 14.8 / 12.9, 8,192 15.9 / 18.2;
+// K = 1,024 9.2 / 10.4 and 10.9 / 14.6 for 385 and 8,192; 8 outputs at K = 2,048, 4,096 tokens 14.8 / 14.8; 128 at K = 4,096, 6,000 25.4 /
+// 22.3, 8,192 25.9 / 25.9; 128 at K = 8,192, 2,048 42.9 / 18.2, 9,472 45.1 / 43.1.
+static bool few_form(int T, int N, int K, int mode) {
+    if (T <= 384 || mode == 1 || mode == 2) return few_form(T, N, K);
+    const int kb = (K + TC_BK - 1) / TC_BK, ks = few_plan(T, N, K).ks;
+    return few_form(T, N, K) && kb - (kb + ks - 1) / ks > 12 + T / 300;
+}
+// (for tests)
+extern "C" int zlm_gemm_tc_takes_few_form(int T, int N, int K, int mode) { return few_form(T, N, K, mode); }
 
-// shares of K whose fp32 partial products need scratch memory (T * N floats each)
+// shares of K whose fp32 partial products need scratch memory (T * N floats each), whatever the mode
 extern "C" int zlm_gemm_tc_ksplit(int T, int N, int K) {
     if (!few_form(T, N, K)) return 1;
     return few_plan(T, N, K).ks;
@@ -1684,7 +1695,7 @@ extern "C" int zlm_gemm_tc_tile_width(int T, int N, int K) { return few_form(T, 
 // / 33.8, 2,048 x 8,192 x 1,024 49.2 / 46.1; 385 x 12,288 x 2,048 64.1 / 33.3, 1,500 x 11,008 x 2,048 85.8 / 57.3; only where tiles are
 // many rounds does 256 gain: 4,096 x 9,728 x 2,560 145.8 / 153.3.
 extern "C" int zlm_gemm_tc_mode_width(int T, int N, int K, int mode) {
-    const int width = zlm_gemm_tc_tile_width(T, N, K);
+    const int width = few_form(T, N, K, mode) ? 0 : many_width(T, N);
     if (g_tc_width || g_tc_form == 1 || mode != 0 || width != 240) return width;
     const long long m_tiles = (T + TCQ_BM - 1) / TCQ_BM, slots = sm_count() / 2;
     auto cost = [&](int bn) { return ((m_tiles * ((N + bn - 1) / bn) + slots - 1) / slots) * bn; };
@@ -1705,7 +1716,7 @@ extern "C" int zlm_gemm_tc(void* Y, const void* X, const void* W, int T, int N, 
     const int ks = zlm_gemm_tc_ksplit(T, N, K);
     ZLM_REQUIRE(ks == 1 || scratch, "gemm_tc: scratch for %d shares of K is missing", ks);
     // few tokens: W is the 128-row operand so that it streams at full height
-    if (few_form(T, N, K)) {
+    if (few_form(T, N, K, mode)) {
         const FewPlan plan = few_plan(T, N, K);
         const long long tiles = (long long)((N + TC_BM - 1) / TC_BM) * plan.t_tiles;
         if (plan.whole + (tiles - plan.whole) * plan.ks <= sm_count()) {
@@ -1734,7 +1745,7 @@ extern "C" int zlm_gemm_tc(void* Y, const void* X, const void* W, int T, int N, 
 // For tests: whether a whole warp issues this product (0: one thread of it)
 extern "C" int zlm_gemm_tc_issues_whole(int T, int N, int K, int mode) {
     const int kb = (K + TC_BK - 1) / TC_BK;
-    if (!few_form(T, N, K)) return g_tc_form != 1 && tc_issue_whole(kb, zlm_gemm_tc_mode_width(T, N, K, mode));
+    if (!few_form(T, N, K, mode)) return g_tc_form != 1 && tc_issue_whole(kb, zlm_gemm_tc_mode_width(T, N, K, mode));
     const FewPlan plan = few_plan(T, N, K);
     const long long tiles = (long long)((N + TC_BM - 1) / TC_BM) * plan.t_tiles;
     if (plan.whole + (tiles - plan.whole) * plan.ks <= sm_count()) return tc_issue_whole_alone(T, (kb + plan.ks - 1) / plan.ks);
