@@ -82,7 +82,7 @@ def test_few_outputs_over_many_tokens_are_cut(lib, T, K, shares, bf16):
     (2048, 2048, 2048, 0), (2048, 24576, 3008, 0), (2048, 24576, 3072, 1),                      # of 256: from 48
     (143, 6144, 4096, 1), (300, 4096, 1024, 1), (300, 4096, 704, 0), (143, 2048, 2048, 0),      # stand-alone, two token tiles and more
     (17, 4096, 4096, 0), (64, 8192, 2048, 0), (100, 6144, 4096, 0), (128, 4096, 12288, 0),      # one: the weights come from memory
-    (2048, 64, 2048, 0), (4096, 128, 8192, 0),                                                  # few outputs over many tokens
+    (512, 128, 8192, 1), (2048, 128, 8192, 0), (4096, 128, 8192, 0),                                                  # few outputs over many tokens
     (300, 8192, 1536, 0), (300, 8192, 2048, 1),                                                 # persistent few-token blocks
 ])
 def test_who_issues_a_product(lib, T, N, K, whole):

@@ -110,11 +110,11 @@ template <bool WHOLE> struct TcIssue {
 // of 240, 2,048 x 4,096, 103 / 103 / 105 / 101 / 99 / 98; of 256, 2,048 x 6,144, 104 / 106 / 103 / 101 / 100 / 99.
 static inline bool tc_issue_whole(int stages, int width) { return stages >= (width < 224 ? 12 : width < 240 ? 32 : 48); }
 // The few-token form's stand-alone blocks: only where two token tiles and more read the weights, so that they come from L2 and the
-// issuing thread, not memory, sets the pace; and up to 384 tokens.  Us: 143 tokens x 6,144 x 4,096 (64 stages) 25.9 / 22.0, 300 x 4,096 x
+// issuing thread, not memory, sets the pace; and up to 512 tokens.  Us: 143 tokens x 6,144 x 4,096 (64 stages) 25.9 / 22.0, 300 x 4,096 x
 // 1,536 (24) 13.3 / 12.4, 300 x 4,096 x 1,024 (16) 10.6 / 10.3, 143 x 4,096 x 1,536 (12) 15.5 / 15.2, 143 x 2,048 x 2,048 (8) 13.2 / 13.2, 256 x
 // 1,024 x 1,024 (8) 11.8 / 12.0; one tile: 17 x 4,096 x 4,096 (16) 12.4 / 13.0, 100 x 6,144 x 4,096 (21) 20.9 / 21.7, 100 x 4,096 x 12,288 (48)
-// 29.8 / 30.7; few outputs: 4,096 x 128 x 8,192 (32) 23.8 / 24.5.
-static inline bool tc_issue_whole_alone(int tokens, int stages) { return tokens > 128 && tokens <= 384 && stages >= 12; }
+// 29.8 / 30.7; few outputs: 512 x 128 x 8,192 (16) 14.3 / 13.9, 2,048 (16) 17.7 / 18.2, 4,096 (32) 23.8 / 24.5.
+static inline bool tc_issue_whole_alone(int tokens, int stages) { return tokens > 128 && tokens <= 512 && stages >= 12; }
 // 16 columns of this thread's lane, without the wait: several loads can be in flight, then tc_wait_ld()
 __device__ __forceinline__ void tc_ld16_nowait(unsigned taddr, float* v) {
     unsigned* r = (unsigned*)v;
