@@ -156,7 +156,7 @@ class GQAAttention(Mixer):
 
     def _attend(self, q: torch.Tensor, residual: torch.Tensor, ctx: StepContext, cache) -> None:
         rt, k = self.rt, self.rt.k
-        out = rt.ws.get("attn.out", (q.shape[0], self.Q), rt.dtype)
+        out = rt.ws.kept("attn.out", (q.shape[0], self.Q), rt.dtype)
         key = self.step_key(ctx)
         k.attention(out, q, cache.pool, cache.block_table, ctx.token_pos, ctx.token_slot,
                     self.nq, self.nkv, self.hd, self.scale, self.window, ctx,

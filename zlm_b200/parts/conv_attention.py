@@ -209,9 +209,9 @@ class ConvAttention(Mixer):
         rt, k = self.rt, self.rt.k
         T = x.shape[0]
         cache = io.cache
-        proj = rt.ws.get("conv_attn.proj", (T, self.C + self.GW), rt.dtype)
+        proj = rt.ws.kept("conv_attn.proj", (T, self.C + self.GW), rt.dtype)
         k.linear(proj, x, self.w_in)
-        q = rt.ws.get("conv_attn.q", (T, self.H * self.hdp), rt.dtype)
+        q = rt.ws.kept("conv_attn.q", (T, self.H * self.hdp), rt.dtype)
         if self.general:
             v_first, v_keep = self._values(ctx, T)
             k.attn_prep(q, proj, self.w_conv, io.state, ctx, cache.block_table, cache.pool, self.H, self.G, self.D, self.V,
@@ -222,7 +222,7 @@ class ConvAttention(Mixer):
         else:
             k.conv_norm_write(q, proj, self.w_conv, io.state, ctx, cache.block_table, cache.pool, self.H, self.G, self.D,
                               self.V, self.taps, self.qk_norm == "unit", self.eps)
-        out = rt.ws.get("conv_attn.out", (T, self.H * self.hdp), rt.dtype)
+        out = rt.ws.kept("conv_attn.out", (T, self.H * self.hdp), rt.dtype)
         key = self.step_key(ctx)
         k.attention(out, q, cache.pool, cache.block_table, ctx.token_pos, ctx.token_slot, self.H, self.G, self.hdp,
                     self.scale, self.window, ctx, len_bucket=key[1] if key else None,
@@ -231,6 +231,6 @@ class ConvAttention(Mixer):
         if self.gate == "none":
             y = out             # (the output projection has zero columns where the heads are padded)
         else:
-            y = rt.ws.get("conv_attn.gated", (T, self.HV), rt.dtype)
+            y = rt.ws.kept("conv_attn.gated", (T, self.HV), rt.dtype)
             k.head_gate(y, out.view(T, self.H, self.hdp), proj[:, self.C:], self.H, self.V, False, self.eps, self.gate)
         k.linear(residual, y, self.w_o, accumulate=True, defer=True)       # a norm reads the stream next

@@ -113,16 +113,16 @@ class DiffAttention(Mixer):
         T = x.shape[0]
         H, G, hdp = self.H, self.G, self.hdp
         cache = io.cache
-        proj = rt.ws.get("diff_attn.proj", (T, self.w_in.shape[0]), rt.dtype)
+        proj = rt.ws.kept("diff_attn.proj", (T, self.w_in.shape[0]), rt.dtype)
         k.linear(proj, x, self.w_in)
-        q = rt.ws.get("diff_attn.q", (T, 2 * H * hdp), rt.dtype)
+        q = rt.ws.kept("diff_attn.q", (T, 2 * H * hdp), rt.dtype)
         k.diff_prep(q, proj, self.q_norm, self.k_norm, self.eps, self.position.inv_freq, self.position.n_rot,
                     ctx.token_pos, ctx.token_slot, cache.block_table, cache.pool, H, G, self.D, self.V)
-        a = rt.ws.get("diff_attn.maps", (T, 2 * H * hdp), rt.dtype)
+        a = rt.ws.kept("diff_attn.maps", (T, 2 * H * hdp), rt.dtype)
         key = self.step_key(ctx)
         k.attention(a, q, cache.pool, cache.block_table, ctx.token_pos, ctx.token_slot, 2 * H, 2 * G, hdp, self.scale,
                     self.window, ctx, len_bucket=key[1] if key else None, v_dim=self.V if self.V < hdp else None,
                     chunk=self.chunk, softcap=self.softcap, v_share=2)
-        o = rt.ws.get("diff_attn.out", (T, H * self.V), rt.dtype)
+        o = rt.ws.kept("diff_attn.out", (T, H * self.V), rt.dtype)
         k.diff_combine(o, a, H, G, self.V, hdp, self.lam, 1.0 - self.diff, self.eps)
         k.linear(residual, o, self.w_o, accumulate=True, defer=True)       # a norm reads the stream next

@@ -183,22 +183,22 @@ class LatentAttention(Mixer):
                 and not any(ctx.h_seq_start)):
             self._forward_unfolded(x, residual, ctx, cache, writes)
             return
-        qd = rt.ws.get("lat.qd", (T, self.N_in), rt.dtype)
+        qd = rt.ws.kept("lat.qd", (T, self.N_in), rt.dtype)
         k.linear(qd, x, self.w_in)
         # the folded query [q' | rotated part] of every head
-        ql = rt.ws.get("lat.ql", (T, H, R), rt.dtype)
+        ql = rt.ws.kept("lat.ql", (T, H, R), rt.dtype)
         q = self._queries_and_records(qd, lambda q3: ql[:, :, r:], ctx, cache, writes)
         q3 = q.as_strided((T, H, self.Dq), (q.stride(0), self.Dq, 1))
         if dn:
             k.head_linear(ql[:, :, :r], q3[:, :, :dn], self.w_uk_t)
         else:
             ql[:, :, :r].zero_()
-        ol = rt.ws.get("lat.ol", (T, H * r), rt.dtype)
+        ol = rt.ws.kept("lat.ol", (T, H * r), rt.dtype)
         key = self.step_key(ctx)
         k.latent_attention(ol, ql.view(T, H * R), cache.pool, cache.block_table, ctx.token_pos, ctx.token_slot,
                            H, r, dr, self.scale, self.window, ctx, len_bucket=key[1] if key else None,
                            **self._options())
-        ov = rt.ws.get("lat.ov", (T, self.w_o_even.shape[1]), rt.dtype)
+        ov = rt.ws.kept("lat.ov", (T, self.w_o_even.shape[1]), rt.dtype)
         if ov.shape[1] > H * dv:
             ov[:, H * dv:].zero_()
         heads = ov.as_strided((T, H, dv), (ov.stride(0), dv, 1))
@@ -219,10 +219,10 @@ class LatentAttention(Mixer):
         freq, n_rot = self.position.inv_freq, self.position.n_rot
         extra = {} if rec_out is None else {"rec_out": rec_out}
         if self.qr:
-            cq = rt.ws.get("lat.cq", (T, self.w_uq.shape[1]), rt.dtype)
+            cq = rt.ws.kept("lat.cq", (T, self.w_uq.shape[1]), rt.dtype)
             k.latent_down(cq, qd[:, :self.qr], self.q_norm, self.eps, dkv, self.c_norm, freq, n_rot, ctx.token_pos,
                           ctx.token_slot, cache.block_table, cache.pool, dr, r, **extra)
-            q = rt.ws.get("lat.q", (T, (self.Q + 7) // 8 * 8), rt.dtype)[:, :self.Q]
+            q = rt.ws.kept("lat.q", (T, (self.Q + 7) // 8 * 8), rt.dtype)[:, :self.Q]
             k.linear(q, cq, self.w_uq)
             dkv, extra = None, {}
             if not dr:
@@ -277,18 +277,18 @@ class LatentAttention(Mixer):
         T = x.shape[0]
         H, dn, dr, dv, r, R = self.H, self.dn, self.dr, self.dv, self.r, self.R
         hd = dn + dr
-        qd = rt.ws.get("lat.qd", (T, self.N_in), rt.dtype)
+        qd = rt.ws.kept("lat.qd", (T, self.N_in), rt.dtype)
         k.linear(qd, x, self.w_in)
         # rotated query parts in place; the records into their pages and, for this step's products, into plain rows
         # (a layer that reads another layer's records gathers them from the pages instead)
-        rec = rt.ws.get("lat.rec", (T, R), rt.dtype)
+        rec = rt.ws.kept("lat.rec", (T, R), rt.dtype)
         q = self._queries_and_records(qd, lambda q3: q3[:, :, dn:], ctx, cache, writes, rec_out=rec if writes else None)
         if not writes:
             k.latent_gather(rec, cache.pool, cache.block_table, ctx.token_pos, ctx.token_slot)
-        kv = rt.ws.get("lat.kv", (T, H * (dn + dv)), rt.dtype)
+        kv = rt.ws.kept("lat.kv", (T, H * (dn + dv)), rt.dtype)
         k.linear(kv, rec[:, :r], self.w_ukv)
         table, rows, pages = self._step_pages(ctx)
-        spool = rt.ws.get("lat.unfolded", (pages, 2, H, PAGE_TOKENS, hd), rt.dtype)
+        spool = rt.ws.kept("lat.unfolded", (pages, 2, H, PAGE_TOKENS, hd), rt.dtype)
         # places beyond a sequence's last token are never written and are multiplied by weights of zero: fresh memory
         # there must hold numbers, so a buffer that has grown is cleared once
         seen = getattr(rt, "_unfolded_cleared", (0, 0))
@@ -299,7 +299,7 @@ class LatentAttention(Mixer):
         plan = types.SimpleNamespace(is_decode=False, cu_seqlens=ctx.cu_seqlens, seq_slot=rows, seq_start=ctx.seq_start,
                                      R=ctx.R, max_new=ctx.max_new, max_len=ctx.max_len, scratch=ctx.scratch,
                                      h_seq_start=ctx.h_seq_start, h_seq_new=ctx.h_seq_new)
-        ao = rt.ws.get("lat.ao", (T, H * hd), rt.dtype)
+        ao = rt.ws.kept("lat.ao", (T, H * hd), rt.dtype)
         k.attention(ao, q, spool, table, ctx.token_pos, ctx.token_seq, H, H, hd, self.scale, self.window, plan,
                     v_dim=dv, **self._options())
         if self.gate:

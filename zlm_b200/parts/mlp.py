@@ -69,7 +69,7 @@ class SwiGLU(FeedForward):
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx: StepContext) -> None:
         rt, k = self.rt, self.rt.k
         T = x.shape[0]
-        act = rt.ws.get("ffn.act", (T, self.cols), rt.dtype)
+        act = rt.ws.kept("ffn.act", (T, self.cols), rt.dtype)
         if self.fused:
             if self.act == "silu":
                 k.linear_swiglu(act, x, self.w_gu)
@@ -78,7 +78,7 @@ class SwiGLU(FeedForward):
             else:
                 k.linear_swiglu(act, x, self.w_gu, act=self.act)
         else:
-            gu = rt.ws.get("ffn.gu", (T, 2 * self.cols), rt.dtype)
+            gu = rt.ws.kept("ffn.gu", (T, 2 * self.cols), rt.dtype)
             k.linear(gu, x, self.w_gu)
             if self.act == "silu":
                 k.swiglu(act, gu)
@@ -117,8 +117,8 @@ class PolyNormMLP(FeedForward):
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx: StepContext) -> None:
         rt, k = self.rt, self.rt.k
         T, cols = x.shape[0], self.w_down.shape[1]
-        z = rt.ws.get("ffn.z", (T, cols), rt.dtype)[:, :self.inter]
+        z = rt.ws.kept("ffn.z", (T, cols), rt.dtype)[:, :self.inter]
         k.linear(z, x, self.w_up)
-        act = rt.ws.get("ffn.act", (T, cols), rt.dtype)
+        act = rt.ws.kept("ffn.act", (T, cols), rt.dtype)
         k.poly_norm(act, z, self.coef, self.eps)
         k.linear(residual, act, self.w_down, accumulate=True, defer=True)      # a norm reads the stream next

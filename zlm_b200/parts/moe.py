@@ -175,11 +175,11 @@ class RoutedExperts(FeedForward):
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx: StepContext) -> None:
         rt, k = self.rt, self.rt.k
         T = x.shape[0]
-        idx = rt.ws.get("moe.idx", (T, self.top), torch.int32)
-        wgt = rt.ws.get("moe.wgt", (T, self.top), torch.float32)
-        gate = rt.ws.get("moe.gate", (T,), torch.float32) if self.shared_gate else None
+        idx = rt.ws.kept("moe.idx", (T, self.top), torch.int32)
+        wgt = rt.ws.kept("moe.wgt", (T, self.top), torch.float32)
+        gate = rt.ws.kept("moe.gate", (T,), torch.float32) if self.shared_gate else None
         if self.w_route is not None:
-            logits = rt.ws.get("moe.logits", (T, self.w_route.shape[0]), torch.float32)
+            logits = rt.ws.kept("moe.logits", (T, self.w_route.shape[0]), torch.float32)
             k.linear(logits, x, self.w_route)
             k.moe_choose(idx, wgt, logits, self.routes, self.top, gate, self.score, self.renormalize, self.correction,
                          self.groups, self.keep, self.route_scale, self.group_top)
@@ -198,12 +198,12 @@ class RoutedExperts(FeedForward):
                           activation=self.up_layout, identity=bool(self.identity), **clamp)
         else:
             # few tokens (and the 32-bit path): every (token, choice) streams its expert's matrices
-            act = rt.ws.get("moe.act", (T, self.top, self.cols), rt.dtype)
+            act = rt.ws.kept("moe.act", (T, self.top, self.cols), rt.dtype)
             k.moe_up(act, x, self.w_up, idx, wgt, self.scale_input, self.up_layout, **clamp)
             k.moe_down(residual, act, self.w_down, idx, x if self.identity else None, wgt)
         if self.SF:
-            u = rt.ws.get("moe.shared_u", (T, self.SF), rt.dtype)
+            u = rt.ws.kept("moe.shared_u", (T, self.SF), rt.dtype)
             k.linear(u, x, self.w_sup)
-            a = rt.ws.get("moe.shared_a", (T, self.SF), rt.dtype)
+            a = rt.ws.kept("moe.shared_a", (T, self.SF), rt.dtype)
             k.relu2_scale(a, u, gate)
             k.linear(residual, a, self.w_sdown, accumulate=True, defer=True)     # a norm reads the stream next

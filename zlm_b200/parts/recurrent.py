@@ -94,9 +94,9 @@ class RecurrentGatedUnit(Mixer):
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx: StepContext, io: LayerIO) -> None:
         rt, k, p = self.rt, self.rt.k, self.small
         T = x.shape[0]
-        proj = rt.ws.get("rglru.proj", (T, 2 * self.W), rt.dtype)
+        proj = rt.ws.kept("rglru.proj", (T, 2 * self.W), rt.dtype)
         k.linear(proj, x, self.w_in)
-        gated = rt.ws.get("rglru.gated", (T, self.W), rt.dtype)
+        gated = rt.ws.kept("rglru.gated", (T, self.W), rt.dtype)
         k.rglru(gated, proj, self.W, 0, p["x_proj.bias"], p["y_proj.bias"], p["conv.weight"], p["conv.bias"],
                 p["a_gate.weight"], p["i_gate.weight"], p["a_gate.bias"], p["i_gate.bias"], p["lam"], self.c_decay, io.state,
                 ctx, self.W, self.B, self.taps, self.out_scale, gates=self.w_gates)
@@ -155,12 +155,12 @@ class GatedLinearAttention(Mixer):
         rt, k = self.rt, self.rt.k
         T = x.shape[0]
         QK, VV = self.QK, self.VV
-        proj = rt.ws.get("gla.proj", (T, 2 * QK + 2 * VV + self.rank), rt.dtype)
+        proj = rt.ws.kept("gla.proj", (T, 2 * QK + 2 * VV + self.rank), rt.dtype)
         k.linear(proj, x, self.w_in)
-        alpha = rt.ws.get("gla.alpha", (T, QK), torch.float32)
+        alpha = rt.ws.kept("gla.alpha", (T, QK), torch.float32)
         k.lowrank_decay(alpha, proj, 2 * QK + 2 * VV, self.a_up, self.a_bias, self.tau)
-        o = rt.ws.get("gla.o", (T, VV), torch.float32)
-        y = rt.ws.get("gla.gated", (T, VV), rt.dtype)
+        o = rt.ws.kept("gla.o", (T, VV), torch.float32)
+        y = rt.ws.kept("gla.gated", (T, VV), rt.dtype)
         k.linear_attention_gated(y, proj[:, 2 * QK + VV: 2 * QK + 2 * VV], self.w_norm, self.eps, self.gate, o, proj, 0, QK, 2 * QK,
                                  alpha, None, io.state, ctx, self.H, self.D, self.V, self.D ** -0.5)
         k.linear(residual, y, self.w_o, accumulate=True, defer=True)       # a norm reads the stream next
@@ -201,9 +201,9 @@ class MinGRU(Mixer):
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx: StepContext, io: LayerIO) -> None:
         rt, k, W = self.rt, self.rt.k, self.W
         T, cols = x.shape[0], self.w_o.shape[1]
-        proj = rt.ws.get("mingru.proj", (T, 3 * W), rt.dtype)
+        proj = rt.ws.kept("mingru.proj", (T, 3 * W), rt.dtype)
         k.linear(proj, x, self.w_in)
-        gated = rt.ws.get("mingru.gated", (T, cols), rt.dtype)
+        gated = rt.ws.kept("mingru.gated", (T, cols), rt.dtype)
         if cols > W:
             gated[:, W:].zero_()
         k.mingru(gated[:, :W], proj, 0, W, 2 * W, self.b_z, self.b_x, io.state, ctx)
@@ -267,22 +267,22 @@ class MatrixLSTM(Mixer):
         step = ctx.is_decode and ctx.T == ctx.R
         if rt.dtype == torch.float32 or (step and T <= 16):
             # (few tokens: one product with fp32 outputs serves the gates too)
-            proj = rt.ws.get("mlstm.proj", (T, self.w_in.shape[0]), torch.float32)
+            proj = rt.ws.kept("mlstm.proj", (T, self.w_in.shape[0]), torch.float32)
             k.linear(proj, x, self.w_in)
             z, i_off = proj, N
         else:
-            proj = rt.ws.get("mlstm.proj", (T, N), rt.dtype)
+            proj = rt.ws.kept("mlstm.proj", (T, N), rt.dtype)
             k.linear(proj, x, self.w_in[:N])
-            z, i_off = rt.ws.get("mlstm.gates", (T, self.w_in.shape[0] - N), torch.float32), 0
+            z, i_off = rt.ws.kept("mlstm.gates", (T, self.w_in.shape[0] - N), torch.float32), 0
             k.linear(z, x, self.w_in[N:])
         cols = self.w_o.shape[1]
-        y = rt.ws.get("mlstm.gated", (T, cols), rt.dtype)
+        y = rt.ws.kept("mlstm.gated", (T, cols), rt.dtype)
         if cols > VV:
             y[:, VV:].zero_()
         gates = (z, i_off, i_off + H, self.b_i, self.b_f, self.cap, io.state, ctx, H, D, V, D ** -0.5)
         if step:
             k.mlstm_step(y[:, :VV], proj, q_off, k_off, v_off, g_off, *gates, self.w_norm, self.eps)
         else:
-            o = rt.ws.get("mlstm.o", (T, VV), torch.float32)
+            o = rt.ws.kept("mlstm.o", (T, VV), torch.float32)
             k.mlstm_gated(y[:, :VV], proj[:, g_off:g_off + VV], self.w_norm, self.eps, o, proj, q_off, k_off, v_off, *gates)
         k.linear(residual, y, self.w_o, accumulate=True, defer=True)       # a norm reads the stream next

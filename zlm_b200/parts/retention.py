@@ -84,15 +84,15 @@ class Retention(Mixer):
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx: StepContext, io: LayerIO) -> None:
         rt, k = self.rt, self.rt.k
         T = x.shape[0]
-        proj = rt.ws.get("retention.proj", (T, 2 * self.QK + 2 * self.VV), rt.dtype)
+        proj = rt.ws.kept("retention.proj", (T, 2 * self.QK + 2 * self.VV), rt.dtype)
         k.linear(proj, x, self.w_in)
         if self.qkv_act == "silu":
             k.silu_rows(proj, 2 * self.QK + self.VV)
-        o = rt.ws.get("retention.o", (T, self.VV), torch.float32)
+        o = rt.ws.kept("retention.o", (T, self.VV), torch.float32)
         # many tokens: the step's cosines and sines come from the table that the position encoding computes once a
         # step for all layers with its frequencies; few tokens: the kernel forms its own
         table = self.position.table(ctx) if (T > 16 and self.position.n_rot and hasattr(self.position, "table")) else None
-        y = rt.ws.get("retention.gated", (T, self.VV), rt.dtype)
+        y = rt.ws.kept("retention.gated", (T, self.VV), rt.dtype)
         args = (o, proj, 0, self.QK, 2 * self.QK, self.position.inv_freq, self.position.n_rot, self.decay, io.state, ctx,
                 self.H, self.D, self.V, self.k_scale)
         if self.out_norm == "row":
