@@ -122,19 +122,19 @@ class GQAAttention(Mixer):
         n_rot = getattr(self.position, "n_rot", 0) if fused_pos else -1
         if (fused_pos and hasattr(k, "qkv_rope_supported") and (n_rot == 0 or hasattr(self.position, "table"))
                 and k.qkv_rope_supported(x, w_in, self.nq, self.nkv if writes else 0, self.hd, n_rot)):
-            q = rt.ws.get("attn.q", (T, self.Q), rt.dtype)
+            q = rt.ws.kept("attn.q", (T, self.Q), rt.dtype)
             k.linear_qkv_rope(q, x, w_in, self.q_norm, self.k_norm if writes else None, self.eps,
                               self.position.table(ctx) if n_rot else None, ctx.token_pos, ctx.token_slot, tbl, pool,
                               self.nq, self.nkv if writes else 0, self.hd)
             self._attend(q, residual, ctx, cache)
             return
         if writes:
-            qkv = rt.ws.get("attn.qkv", (T, self.Q + 2 * self.KV), rt.dtype)
+            qkv = rt.ws.kept("attn.qkv", (T, self.Q + 2 * self.KV), rt.dtype)
             # (the norm / rotation / cache write kernel reads the projection next, where there is one)
             k.linear(qkv, x, self.w_qkv, defer=fused_pos or self.qk_norm)
             nkv = self.nkv
         else:
-            qkv = rt.ws.get("attn.qkv", (T, self.Q), rt.dtype)
+            qkv = rt.ws.kept("attn.qkv", (T, self.Q), rt.dtype)
             k.linear(qkv, x, self.w_q, defer=fused_pos or self.qk_norm)
             nkv = 0
         q = qkv[:, : self.Q]
