@@ -47,25 +47,30 @@ __device__ __forceinline__ void attention_decode_item(
     // from earlier steps do not, and their loads start before the wait for that kernel.  `fresh`
     // is how many of a sequence's newest positions this step may have written (0: not known,
     // nothing is read early).
-    // (Asking for the older rows of a page that also holds fresh ones before the wait, and for those after it, was built: sequences
-    // of two and three pages on a GPU with blocks to spare took 0.6 us longer, 4 sequences of 65 keys, 8 kv heads, 5.6 and 6.2 us,
-    // and 32 of 4,096 keys 99.0 and 104.8.)
+    // A sequence of one page, whose rows all came after the wait with that, has its older rows asked for before it, and only the
+    // step's own after it (16 sequences of 51 keys, 8 kv heads, 6.2 us by pages, 5.9 so).  Done for every page with fresh
+    // rows it cost what it was to save: 4 sequences of 65 keys 5.6 and 6.2 us, 32 of 4,096 99.0 and 104.8.
     const int old_pages = fresh > 0 ? max(0, pos + 1 - fresh) / ZLM_PAGE : 0;
     const bool early0 = PDL && p_begin < p_end && walk.page(p_begin) < old_pages;
     const bool early1 = early0 && p_begin + 1 < p_end && walk.page(p_begin + 1) < old_pages;
-    auto load_page = [&](int w, int stage) {
+    const bool by_rows = PDL && fresh > 0 && splits == 1 && pos < ZLM_PAGE;
+    const int own_lo = by_rows ? max(0, pos + 1 - fresh) : 0, own_hi = by_rows ? pos + 1 : ZLM_PAGE;
+    // rows lo .. hi - 1 of page w, without those from s_lo to s_hi - 1
+    auto load_rows = [&](int w, int stage, int lo, int hi, int s_lo, int s_hi) {
         const int p = walk.page(w);
         if (!ZLM_CHK(pages + p, 4)) return;
         const __nv_bfloat16* kb = pool + (size_t)pages[p] * page_stride + (size_t)kvh * TILE;
         const __nv_bfloat16* vb = kb + v_off;
         __nv_bfloat16* ks_ = Ks + stage * TILE;
         __nv_bfloat16* vs_ = Vs + stage * TILE;
-        for (int id = tid; id < ZLM_PAGE * CH; id += DEC_THREADS) {
+        for (int id = lo * CH + tid; id < hi * CH; id += DEC_THREADS) {
             const int r = id / CH, c = id % CH;
+            if (r >= s_lo && r < s_hi) continue;
             dec_cp_async16(ks_ + tile_off<HD>(r, c), kb + r * HD + c * 8);
             dec_cp_async16(vs_ + tile_off<HD>(r, c), vb + r * HD + c * 8);
         }
     };
+    auto load_page = [&](int w, int stage) { load_rows(w, stage, 0, ZLM_PAGE, 0, 0); };
 
     if (early0) {
         load_page(p_begin, 0);
@@ -74,11 +79,13 @@ __device__ __forceinline__ void attention_decode_item(
             load_page(p_begin + 1, 1);
             dec_commit();
         }
+    } else if (by_rows) {
+        load_rows(p_begin, 0, 0, ZLM_PAGE, own_lo, own_hi);
     }
     if (PDL) pdl_wait();
     // the other pages do not depend on q either: they land while q is fetched
     if (!early0) {
-        if (p_begin < p_end) load_page(p_begin, 0);
+        if (p_begin < p_end) load_rows(p_begin, 0, own_lo, own_hi, 0, 0);
         dec_commit();
     }
     if (!early1) {
