@@ -32,3 +32,26 @@ def test_rows_equal_heads(T, H, V, act, in_place):
     ref = v * torch.sigmoid(z) * (z if act == "silu" else 1.0)
     mine = (got[1:] if T > 1 else got[:, 8:]).double()
     assert ((mine - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-30).all()         # one rounding to bfloat16, and 32-bit functions
+
+
+@pytest.mark.parametrize("off,pad", [(0, 4), (4, 0), (1, 0), (8, 8), (0, 1)])
+@pytest.mark.parametrize("which", ["out", "o", "g"])
+def test_rows_off_sixteen_bytes(off, pad, which):
+    """Starts and strides that are no multiple of eight numbers go to the form of a warp a head, with the same bits."""
+    k = get_kernels()
+    T, H, V = 65, 4, 128
+    N = H * V
+    g = torch.Generator(device="cuda").manual_seed(off + pad)
+    values = {n: torch.randn((T, N), generator=g, device="cuda").bfloat16() for n in ("out", "o", "g")}
+
+    def placed(name):
+        if name != which:
+            return values[name].clone()
+        t = torch.zeros(T * (N + pad) + off, device="cuda", dtype=torch.bfloat16)[off:].as_strided((T, N), (N + pad, 1))
+        return t.copy_(values[name])
+
+    want = torch.empty((T, N), device="cuda", dtype=torch.bfloat16)
+    k.head_gate(want, values["o"].view(T, H, V), values["g"], H, V, False, 0.0, "silu")
+    out, o, gate = placed("out"), placed("o"), placed("g")
+    k.head_gate(out, o.as_strided((T, H, V), (o.stride(0), V, 1)), gate, H, V, False, 0.0, "silu")
+    assert torch.equal(out, want)

@@ -44,3 +44,32 @@ def test_what_is_no_argument_is_refused(call, wrong):
     entry = ctypes.CFUNCTYPE(c_int, c_int)(lambda a: 0)
     with pytest.raises(TypeError):
         call(ctypes.cast(entry, c_void_p).value, wrong)
+
+
+def test_the_native_caller_is_the_one_that_runs():
+    """Where it can be built: on Linux on one of the two processors, with a compiler and Python's headers."""
+    import os
+    import platform
+    import shutil
+    import sys
+    import sysconfig
+    if not (sys.platform.startswith("linux") and platform.machine() in ("x86_64", "aarch64") and (shutil.which("gcc") or shutil.which("cc"))
+            and os.path.isfile(os.path.join(sysconfig.get_paths()["include"], "Python.h"))):
+        pytest.skip("host_call.c cannot be built here")
+    assert host_call(verbose=False) is not _through_ctypes
+
+
+def test_as_many_arguments_as_there_are_places():
+    call = host_call(verbose=False)
+    if call is _through_ctypes:
+        pytest.skip("the stand-in has no limit")
+    got = []
+    entry = ctypes.CFUNCTYPE(c_int, *[c_longlong] * 64, *[c_float] * 8)(lambda *a: (got.extend(a), 3)[1])
+    at = ctypes.cast(entry, c_void_p).value
+    ints, floats = [n * n - (1 << 40) for n in range(64)], [c_float(n + 0.3) for n in range(8)]
+    assert call(at, *ints, *floats) == 3
+    assert got == ints + [f.value for f in floats]
+    for more in (ints + [0] + floats, ints + floats + [c_float(0.0)]):
+        with pytest.raises(TypeError):
+            call(at, *more)
+    assert len(got) == 72                                     # (nothing was called with too many)
