@@ -1,5 +1,6 @@
-"""Decode attention around the edges of a page: what is read before the wait for the kernel before (all rows but the step's
-own) and after it give the bits of reading everything after it, whatever the group, the head size and the split."""
+"""Decode attention around the edges of a page: what is read before the wait for the kernel before (pages without a row of the
+step's own, and the older rows of a sequence of one page) and after it give the bits of reading everything after it, whatever
+the group, the head size and the split."""
 import pytest
 import torch
 

@@ -250,7 +250,7 @@ class CudaKernels:
             self.check_bounds(name)
 
     def _p(self, t: Optional[torch.Tensor]) -> c_void_p:
-        """``_at`` as an object of ctypes, for calls of other libraries."""
+        """``_at`` as an object of ctypes."""
         return c_void_p(self._at(t))
 
     def _at(self, t: Optional[torch.Tensor]) -> int:
@@ -606,7 +606,7 @@ class CudaKernels:
         px = self._at(lazy[4]) if lazy is not None else self._at(x)
         self._call("zlm_gemv_bf16_norms", self._at(out), px, self._at(w), T, N, K,
                    ldx, ldy, mode, self._at(cv), self._at(ci),
-                   self._at(lazy[5]) if lazy is not None else (0), lazy[6] if lazy is not None else 0,
+                   self._at(lazy[5]) if lazy is not None else 0, lazy[6] if lazy is not None else 0,
                    c_float(lazy[3] if lazy is not None else 0.0), self._at(norm_weight),
                    _dt(norm_weight) if norm_weight is not None else 0, self._at(nxt), self._at(sq), self._queue())
         if cv is not None:
@@ -667,8 +667,7 @@ class CudaKernels:
         _whole(nq, nkv, hd, n_rot)
         if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
             return False
-        return bool(self._ask("zlm_gemm_tc_qkv_supported", x.shape[0], w.shape[0], w.shape[1],
-                                                       x.stride(0), nq, nkv, hd, n_rot))
+        return bool(self._ask("zlm_gemm_tc_qkv_supported", x.shape[0], w.shape[0], w.shape[1], x.stride(0), nq, nkv, hd, n_rot))
 
     def linear_qkv_rope(self, q_out: torch.Tensor, x: torch.Tensor, w: torch.Tensor, q_w: Optional[torch.Tensor],
                         k_w: Optional[torch.Tensor], eps: float, cos_sin: Optional[torch.Tensor],
@@ -836,9 +835,8 @@ class CudaKernels:
         if (q.dtype == torch.float32 and plan is not None and getattr(plan, "cu_seqlens", None) is not None
                 and int(getattr(plan, "max_len", 0) or plan.max_new) >= (32 if int(plan.max_new) > 1 else 512)
                 and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
-                and self._ask("zlm_attention_f32_tile_supported", nq, nkv, hd, q.stride(0),
-                                                              out.stride(0), c_float(softcap), v_share, keep,
-                                                              bias is not None, plan.R, int(plan.max_new))):
+                and self._ask("zlm_attention_f32_tile_supported", nq, nkv, hd, q.stride(0), out.stride(0), c_float(softcap), v_share,
+                              keep, bias is not None, plan.R, int(plan.max_new))):
             self._call("zlm_attention_f32_tile", self._at(out), out.stride(0), self._at(q), q.stride(0), self._at(pool),
                        self._at(block_table), block_table.stride(0), self._at(plan.cu_seqlens), self._at(plan.seq_slot),
                        self._at(plan.seq_start), plan.R, plan.max_new, nq, nkv, hd, c_float(scale),
@@ -946,7 +944,7 @@ class CudaKernels:
                 and y.stride(1) == g.stride(1) == 1 and (y.stride(0) | g.stride(0)) % 8 == 0
                 and (proj.data_ptr() | y.data_ptr() | g.data_ptr()) % 16 == 0
                 and self._ask("zlm_retention_products", _dt(proj), proj.stride(0), q_off, k_off, v_off,
-                                                    n_rot if inv_freq is not None else 0, dim, v_dim)):
+                              n_rot if inv_freq is not None else 0, dim, v_dim)):
             assert y.shape == g.shape == (proj.shape[0], heads * v_dim)
             self.retention(o, *args, cos_sin=cos_sin, _gate=(y, g, eps, act))
             return
@@ -1187,8 +1185,7 @@ class CudaKernels:
         args = (proj, q_off, k_off, v_off, z, i_off, f_off, b_i, b_f, cap, state, plan, heads, dim, v_dim, q_scale)
         if (y.dtype == g.dtype == torch.bfloat16 and v_dim <= 128 and y.stride(1) == g.stride(1) == 1
                 and (y.stride(0) | g.stride(0)) % 8 == 0 and (proj.data_ptr() | y.data_ptr() | g.data_ptr()) % 16 == 0
-                and self._ask("zlm_mlstm_products", _dt(proj), proj.stride(0), q_off, k_off, v_off,
-                                                dim, v_dim)):
+                and self._ask("zlm_mlstm_products", _dt(proj), proj.stride(0), q_off, k_off, v_off, dim, v_dim)):
             assert y.shape == g.shape == (proj.shape[0], heads * v_dim)
             assert w_norm.is_contiguous() and w_norm.numel() == heads * v_dim
             self.mlstm(o, *args, _gate=(y, g, w_norm, eps))
@@ -1438,8 +1435,7 @@ class CudaKernels:
             if plan.is_decode:
                 if len_bucket is None:
                     len_bucket = attention_len_bucket(plan.max_len)
-                wave = self.decode_blocks or self.sm_count * int(
-                    self._ask("zlm_latent_attention_mma_blocks_per_sm", kv_rank, rot_dim))
+                wave = self.decode_blocks or self.sm_count * self._ask("zlm_latent_attention_mma_blocks_per_sm", kv_rank, rot_dim)
                 splits, per = latent_decode_splits(T, tiles, len_bucket, wave)
                 qt, fresh = 1, max(1, int(getattr(plan, "max_new", 1) or 1))
             else:
@@ -1475,7 +1471,6 @@ class CudaKernels:
         if pair is not None:
             assert pair.shape == (buckets + 1, H) and pair.dtype == table.dtype and pair.is_contiguous()
             assert prev_state is not None and prev_state.dtype == torch.int32 and plan is not None
-        ll = ctypes.c_longlong
         self._call("zlm_embed_scaled", self._at(out), self._at(table), _dt(table), c_float(scale), self._at(pair),
                    buckets, mul_prev, mul_cur, self._at(ids),
                    self._at(plan.token_pos if pair is not None else None), self._at(plan.token_seq if pair is not None else None),
