@@ -150,6 +150,11 @@ def _whole(*numbers) -> None:
         operator.index(n)
 
 
+def _kept(plan, name: str, shape, dtype: torch.dtype) -> torch.Tensor:
+    """Scratch of the step that a kernel alone is given: the workspace's own object where the plan offers it."""
+    return getattr(plan, "kept", plan.scratch)(name, shape, dtype)
+
+
 def _span_bytes(t: torch.Tensor) -> int:
     """Bytes from the tensor's first element to the end of its last one."""
     if t.numel() == 0:
@@ -775,8 +780,8 @@ class CudaKernels:
             splits, per = decode_splits(T, nkv, len_bucket, self.decode_blocks or self.sm_count * DECODE_BLOCKS_PER_SM)
             part_o = part_ml = None
             if splits > 1:
-                part_o = plan.scratch("attn.part_o", (T * nq * splits * hd,), torch.float32)
-                part_ml = plan.scratch("attn.part_ml", (T * nq * splits * 2,), torch.float32)
+                part_o = _kept(plan, "attn.part_o", (T * nq * splits * hd,), torch.float32)
+                part_ml = _kept(plan, "attn.part_ml", (T * nq * splits * 2,), torch.float32)
             # (a decode step writes one position per sequence: every page below that one is from earlier
             # steps, and its load need not wait for the kernel that wrote this step's keys and values)
             self._call("zlm_attention_decode_fresh", self._at(out), out.stride(0),
@@ -924,7 +929,7 @@ class CudaKernels:
             # about the step's sequences has to be carried to the device beyond what the step has there already
             L = self.RETENTION_PIECE
             maxp = (int(plan.max_new) + L - 1) // L
-            part = plan.scratch("retention.part_state", (plan.R * maxp * heads * dim * v_dim,), torch.float32)
+            part = _kept(plan, "retention.part_state", (plan.R * maxp * heads * dim * v_dim,), torch.float32)
             # (the gate rides in the last kernel where the pieces run as products)
             y, g, eps, act = (_gate[0], _gate[1], _gate[2], _gate[3]) if _gate is not None else (None, None, 0.0, "silu")
             self._call("zlm_retention_parts", *head, maxp, L, self._at(part), *tail[:-1], self._at(y),
@@ -1059,10 +1064,10 @@ class CudaKernels:
             # three launches: the convolution, all blocks' gate logits as one grouped product, the recurrence on clusters
             assert gates.shape == (blocks, 2 * bs, bs) and gates.is_contiguous() and gates.dtype == dt
             Tp = -(-T // 128) * 128
-            u16 = plan.scratch("rglru.u16", (blocks, Tp, bs), dt)
-            z = plan.scratch("rglru.z", (blocks * Tp, 2 * bs), torch.float32)
+            u16 = _kept(plan, "rglru.u16", (blocks, Tp, bs), dt)
+            z = _kept(plan, "rglru.z", (blocks * Tp, 2 * bs), torch.float32)
             tiles = blocks * (-(-T // 256))
-            table = plan.scratch("rglru.tiles", (3 * tiles,), torch.int32)
+            table = _kept(plan, "rglru.tiles", (3 * tiles,), torch.int32)
             self._call("zlm_rglru_conv_blocks", self._at(u16), self._at(table), self._at(proj), proj.stride(0), x_off,
                        self._at(bx), self._at(conv_w), self._at(conv_b), self._at(state), self._at(plan.token_pos),
                        self._at(plan.token_slot), self._at(plan.token_seq), self._at(plan.seq_start), T, W,
@@ -1076,14 +1081,14 @@ class CudaKernels:
                        taps, c_float(out_scale), self.lib.zlm_rglru_cluster_size(plan.R, T, max_new, W),
                        self._queue())
             return
-        u = plan.scratch("rglru.u", (T, W), torch.float32)
-        z = plan.scratch("rglru.z", (T, blocks, 2 * bs), torch.float32)
+        u = _kept(plan, "rglru.u", (T, W), torch.float32)
+        z = _kept(plan, "rglru.z", (T, blocks, 2 * bs), torch.float32)
         part = None
         if pieces:
             maxp = (max_new + self.RECURRENT_PIECE - 1) // self.RECURRENT_PIECE
-            part = plan.scratch("rglru.pieces", (2 * plan.R * maxp * W,), torch.float32)
+            part = _kept(plan, "rglru.pieces", (2 * plan.R * maxp * W,), torch.float32)
         by_products = (gates is not None and dt == torch.bfloat16 and T > 16 and bs % 8 == 0 and W % 8 == 0)
-        u16 = plan.scratch("rglru.u16", (T, W), dt) if by_products else None
+        u16 = _kept(plan, "rglru.u16", (T, W), dt) if by_products else None
 
         def call(phase: int) -> None:
             self._call("zlm_rglru", self._at(out), out.stride(0), self._at(u), self._at(u16), self._at(z), self._at(proj),
@@ -1166,7 +1171,7 @@ class CudaKernels:
         S, n, m = self._check_mlstm(proj, z, b_i, b_f, state, heads, dim, v_dim)
         assert o.shape == (T, heads * v_dim) and o.dtype == torch.float32 and o.is_contiguous()
         max_new = int(plan.max_new)
-        part = plan.scratch("mlstm.pieces", (int(self.lib.zlm_mlstm_scratch(plan.R, heads, dim, v_dim, max_new)),), torch.float32)
+        part = _kept(plan, "mlstm.pieces", (int(self.lib.zlm_mlstm_scratch(plan.R, heads, dim, v_dim, max_new)),), torch.float32)
         b = b_i if b_i is not None else b_f
         y, g, w, eps = _gate if _gate is not None else (None, None, None, 0.0)
         self._call("zlm_mlstm", self._at(o), self._at(proj), proj.stride(0), _dt(proj), q_off, k_off,
@@ -1238,7 +1243,7 @@ class CudaKernels:
         part = None
         if pieces:
             maxp = (max_new + self.RECURRENT_PIECE - 1) // self.RECURRENT_PIECE
-            part = plan.scratch("linear_attention.pieces", (plan.R * maxp * heads * dim * (v_dim + 1),), torch.float32)
+            part = _kept(plan, "linear_attention.pieces", (plan.R * maxp * heads * dim * (v_dim + 1),), torch.float32)
         y, g, w, eps, act = _gate if _gate is not None else (None, None, None, 0.0, "silu")
         self._call("zlm_linear_attention", self._at(o), self._at(proj), proj.stride(0), q_off, k_off,
                    v_off, self._at(alpha), self._at(head_decay if alpha is None else None), self._at(state), _dt(proj),
@@ -1443,8 +1448,8 @@ class CudaKernels:
                 qt, fresh = self._ask("zlm_latent_attention_mma_tokens", kv_rank, rot_dim), 0
             part_o = part_ml = None
             if splits > 1:
-                part_o = plan.scratch("lat.part_o", (T * heads * splits * kv_rank,), torch.float32)
-                part_ml = plan.scratch("lat.part_ml", (T * heads * splits * 2,), torch.float32)
+                part_o = _kept(plan, "lat.part_o", (T * heads * splits * kv_rank,), torch.float32)
+                part_ml = _kept(plan, "lat.part_ml", (T * heads * splits * 2,), torch.float32)
             self._call("zlm_latent_attention_mma", self._at(out), out.stride(0), self._at(q), q.stride(0),
                        self._at(pool), self._at(block_table), block_table.stride(0), self._at(token_pos),
                        self._at(token_slot), T, heads, kv_rank, rot_dim, c_float(scale),

@@ -186,6 +186,10 @@ class StepContext:
         """A scratch buffer that lives until the next kernel asks for the same name."""
         return self.workspace.get(name, shape, dtype)
 
+    def kept(self, name: str, shape, dtype) -> torch.Tensor:
+        """The same for a buffer that only kernels are given (``Workspace.kept``)."""
+        return self.workspace.kept(name, shape, dtype)
+
 
 class Part:
     """Base of every part.  ``rt`` is set by ``attach`` before ``bind``."""
